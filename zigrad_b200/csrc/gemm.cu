@@ -1,7 +1,7 @@
 // GEMM entry points: zg_bmm (include/zg_b200.h), gemm / gemv / ger
 // (include/blas_conflux.h).  Large, TMA-addressable problems go to the
-// tcgen05 kernel (gemm_tc.cuh); everything else (tiny shapes, rows whose byte
-// stride is not a multiple of 16, fp64) runs on a register-tiled FFMA kernel.
+// tcgen05 kernel (gemm_tc.cuh); everything else (small shapes, rows whose byte
+// stride is not a multiple of 16, fp64) runs on the FFMA kernel of gemm_block.cuh.
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -11,132 +11,13 @@
 #include "gemm_tc.cuh"
 #include "gemm_tc_persistent.cuh"
 #include "gemm_skinny.cuh"
+#include "gemm_block.cuh"
 #include "mlp_tail.cuh"
 #include "../../include/blas_conflux.h"
 
 namespace zg {
 
 static int g_math_mode = ZG_MATH_FP32X3;
-
-// =====================================================================
-// FFMA kernel: 64x64 tile, 16-deep k-slabs, 256 threads x (4x4) outputs.
-// Generic in element type (double / float / bf16 inputs with float math),
-// operand transposes and leading dimensions.  gridDim.z = batches * splits.
-// =====================================================================
-template <typename T> struct Acc { using type = float; };
-template <> struct Acc<double> { using type = double; };
-
-template <typename T> __device__ __forceinline__ typename Acc<T>::type to_acc(T v) { return (typename Acc<T>::type)v; }
-template <> __device__ __forceinline__ float to_acc<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
-template <typename TC, typename A> __device__ __forceinline__ TC from_acc(A v) { return (TC)v; }
-template <> __device__ __forceinline__ __nv_bfloat16 from_acc<__nv_bfloat16, float>(float v) { return __float2bfloat16_rn(v); }
-
-struct SimtParams {
-  size_t nA, nB, m, n, k, lda, ldb, ldc, a_stride, b_stride, c_stride;
-  bool ta, tb;
-  double alpha, beta;
-  int epilogue;
-  const float* bias;
-  const void* mask;
-  float* colsum;
-  unsigned splits;
-  size_t k_per_split;
-};
-
-template <typename TI, typename TC>
-__global__ void __launch_bounds__(256) gemm_simt_kernel(const TI* __restrict__ A, const TI* __restrict__ B, TC* C, const SimtParams p) {
-  using AT = typename Acc<TI>::type;
-  constexpr int TM = 64, TN = 64, TK = 16;
-  pdl_sync();
-  __shared__ AT As[TK][TM + 1];
-  __shared__ AT Bs[TK][TN + 1];
-  const unsigned batch = blockIdx.z / p.splits, split = blockIdx.z % p.splits;
-  const TI* a = A + (batch % p.nA) * p.a_stride;
-  const TI* b = B + (batch % p.nB) * p.b_stride;
-  TC* c = C + (size_t)batch * p.c_stride;
-  const size_t m0 = (size_t)blockIdx.y * TM, n0 = (size_t)blockIdx.x * TN;
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  AT acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = AT(0);
-  const size_t kb = split * p.k_per_split;
-  size_t ke = kb + p.k_per_split;
-  if (ke > p.k) ke = p.k;
-  // Cooperative loads: 1024 elements per operand slab, 4 per thread; the
-  // fastest-varying thread index follows the contiguous dimension in memory.
-  // The next slab is fetched into registers while the current one is being
-  // multiplied, so a trip costs the arithmetic, not a round trip to memory.
-  AT ar[4], br[4];
-  auto fetch = [&](size_t k0) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = threadIdx.x + q * 256;
-      int mm, kk;
-      if (p.ta) { mm = e % TM; kk = e / TM; } else { kk = e % TK; mm = e / TK; }
-      const size_t gm = m0 + mm, gk = k0 + kk;
-      ar[q] = (gm < p.m && gk < ke) ? to_acc<TI>(p.ta ? a[gk * p.lda + gm] : a[gm * p.lda + gk]) : AT(0);
-      int nn;
-      if (p.tb) { kk = e % TK; nn = e / TK; } else { nn = e % TN; kk = e / TN; }
-      const size_t gn = n0 + nn, gk2 = k0 + kk;
-      br[q] = (gn < p.n && gk2 < ke) ? to_acc<TI>(p.tb ? b[gn * p.ldb + gk2] : b[gk2 * p.ldb + gn]) : AT(0);
-    }
-  };
-  if (kb < ke) fetch(kb);
-  for (size_t k0 = kb; k0 < ke; k0 += TK) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = threadIdx.x + q * 256;
-      int mm, kk, nn;
-      if (p.ta) { mm = e % TM; kk = e / TM; } else { kk = e % TK; mm = e / TK; }
-      As[kk][mm] = ar[q];
-      if (p.tb) { kk = e % TK; nn = e / TK; } else { nn = e % TN; kk = e / TN; }
-      Bs[kk][nn] = br[q];
-    }
-    __syncthreads();
-    if (k0 + TK < ke) fetch(k0 + TK);
-#pragma unroll
-    for (int kk = 0; kk < TK; ++kk) {
-      AT av[4], bv[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) av[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bv[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] += av[i] * bv[j];
-    }
-    __syncthreads();
-  }
-  const AT alpha = (AT)p.alpha, beta = (AT)p.beta;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const size_t gm = m0 + ty * 4 + i;
-    if (gm >= p.m) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const size_t gn = n0 + tx + 16 * j;
-      if (gn >= p.n) continue;
-      const size_t o = gm * p.ldc + gn;
-      AT v = alpha * acc[i][j];
-      if (p.splits > 1) {
-        if constexpr (sizeof(TC) == 4 || sizeof(TC) == 8) atomicAdd(reinterpret_cast<AT*>(c) + o, v);
-        continue;
-      }
-      if (beta != AT(0)) v += beta * to_acc<TC>(c[o]);
-      if (p.epilogue == ZG_EPI_BIAS) v += (AT)p.bias[gn];
-      else if (p.epilogue == ZG_EPI_BIAS_RELU) { v += (AT)p.bias[gn]; v = v > AT(0) ? v : AT(0); }
-      else if (p.epilogue == ZG_EPI_RELU_MASK) {
-        const TC* mk = static_cast<const TC*>(p.mask) + (size_t)batch * p.c_stride;
-        if (to_acc<TC>(mk[o]) <= AT(0)) v = AT(0);
-      }
-      c[o] = from_acc<TC, AT>(v);
-      if (p.colsum) atomicAdd(p.colsum + gn, (float)v);
-    }
-  }
-}
 
 // C[b][i][j] *= beta over an [m, n] window with leading dimension ldc
 template <typename T>
@@ -156,33 +37,47 @@ static void prescale_c(cudaStream_t s, T* C, size_t batches, size_t m, size_t n,
   launch_pdl(scale_c_kernel<T>, dim3(grid_for(batches * m * n, 1024)), dim3(256), 0, s, C, batches, m, n, ldc, c_stride, (T)beta);
 }
 
+// Cluster size of a small problem: enough CTAs to occupy the SMs, no k range under 32.
+static unsigned block_splits(size_t tiles, len_t k) {
+  unsigned s = 1;
+  while (s < 8 && tiles * s * 2 <= (size_t)sm_count() * 2 && k >= (len_t)s * 2 * 32) s *= 2;
+  return s;
+}
+
+template <typename TI, typename TC, int TM, int TN, int MI>
+static void launch_block_inst(cudaStream_t s, const void* A, const void* B, void* C, block::Params& p, len_t nC, unsigned splits) {
+  using L = block::Layout<TI, TM, TN, MI>;
+  auto kern = block::gemm_block_kernel<TI, TC, TM, TN, MI>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    if (!ZG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kSmem))) return;
+    attr_set = true;
+  }
+  p.tiles_m = (uint32_t)((p.m + TM - 1) / TM);
+  p.tiles_n = (uint32_t)((p.n + TN - 1) / TN);
+  p.splits = splits;
+  p.k_per_split = splits > 1 ? ((p.k + splits - 1) / splits + 7) / 8 * 8 : p.k;
+  const size_t ctas = (size_t)p.tiles_m * p.tiles_n * nC * splits;
+  if (ctas > 0x7fffffffu) { set_error(kBadArgument, "gemm: grid too large (m=%lu, batches=%lu)", (len_t)p.m, nC); return; }
+  launch_pdl_cluster(kern, dim3((unsigned)ctas), dim3(block::kThreads), L::kSmem, s, splits, static_cast<const TI*>(A),
+                     static_cast<const TI*>(B), static_cast<TC*>(C), p);
+}
+
 template <typename TI, typename TC>
-static void launch_simt(cudaStream_t s, const void* A, const void* B, void* C, len_t nA, len_t nB, len_t nC, len_t m, len_t n, len_t k,
-                        bool ta, bool tb, len_t lda, len_t ldb, len_t ldc, double alpha, double beta, int epilogue, const void* bias,
-                        const void* mask, void* colsum) {
-  SimtParams p;
-  p.colsum = static_cast<float*>(colsum);
+static void launch_block(cudaStream_t s, const void* A, const void* B, void* C, len_t nA, len_t nB, len_t nC, len_t m, len_t n, len_t k,
+                         bool ta, bool tb, len_t lda, len_t ldb, len_t ldc, double alpha, double beta, int epilogue, const void* bias,
+                         const void* mask, void* colsum) {
+  block::Params p;
+  memset(&p, 0, sizeof(p));
   p.nA = nA; p.nB = nB; p.m = m; p.n = n; p.k = k; p.lda = lda; p.ldb = ldb; p.ldc = ldc;
   p.a_stride = (ta ? k : m) * lda; p.b_stride = (tb ? n : k) * ldb; p.c_stride = m * ldc;
   p.ta = ta; p.tb = tb; p.alpha = alpha; p.beta = beta; p.epilogue = epilogue;
-  p.bias = static_cast<const float*>(bias); p.mask = mask;
-  const size_t tiles = ((m + 63) / 64) * ((n + 63) / 64) * nC;
-  unsigned splits = 1;
-  // deep-k, few-tile problems (weight gradients): split K over more CTAs
-  if (epilogue == ZG_EPI_NONE && !colsum && sizeof(TC) >= 4 && k >= 128 && tiles * 2 <= (size_t)sm_count()) {
-    size_t want = (size_t)sm_count() * 2 / tiles;
-    size_t maxs = k / 32;  // at least two 16-deep slabs per split
-    splits = (unsigned)(want < maxs ? want : maxs);
-    if (splits < 1) splits = 1;
-  }
-  p.splits = splits;
-  p.k_per_split = splits > 1 ? ((k + splits - 1) / splits + 15) / 16 * 16 : k;
-  if (splits > 1) {
-    if constexpr (sizeof(TC) >= 4) prescale_c<TC>(s, static_cast<TC*>(C), nC, m, n, ldc, p.c_stride, beta);
-  }
-  dim3 grid((unsigned)((n + 63) / 64), (unsigned)((m + 63) / 64), (unsigned)(nC * splits));
-  if (grid.y > 65535 || grid.z > 65535) { set_error(kBadArgument, "gemm: grid too large (m=%lu, batches=%lu)", m, nC); return; }
-  launch_pdl(gemm_simt_kernel<TI, TC>, grid, dim3(256), 0, s, static_cast<const TI*>(A), static_cast<const TI*>(B), static_cast<TC*>(C), p);
+  p.bias = static_cast<const float*>(bias); p.mask = mask; p.colsum = static_cast<float*>(colsum);
+  const size_t t64 = ((m + 63) / 64) * ((n + 63) / 64) * nC, t32 = ((m + 31) / 32) * ((n + 31) / 32) * nC;
+  // 64 x 64 tiles (half the copies per multiply-add) once there is one for every SM; below that, parallelism counts
+  // for more: 1000x301x501 takes 21 us with 32 x 32, 30 with 64 x 64; 4096x1023x1023 379 and 280
+  if (t64 > (size_t)sm_count()) launch_block_inst<TI, TC, 64, 64, 8>(s, A, B, C, p, nC, 1);
+  else launch_block_inst<TI, TC, 32, 32, 4>(s, A, B, C, p, nC, block_splits(t32, k));
 }
 
 // =====================================================================
@@ -366,9 +261,16 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   if (!host_aligned16(A) || !host_aligned16(B) || (lda * es) % 16 || (ldb * es) % 16) return false;
   if (m == 0 || n == 0 || nC == 0) return false;
   if (m > 0x7fffffffu || n > 0x7fffffffu || k > 0x7fffffffu || ldc > 0xffffffffu) return false;
-  // tiny problems are launch-bound either way; keep them on the FFMA kernel
-  const char* force = getenv("ZG_GEMM_FORCE_TC");
-  if (!(force && force[0] == '1') && (double)m * (double)n * (double)k < 64.0 * 64.0 * 64.0) return false;
+  // Small problems are a latency chain on the tensor cores (descriptor fetch, TMA round trip, operand split, MMA,
+  // TMEM read-back, and for split K a pre-scaled C and a second pass); the FFMA kernel with its clusters needs 3 us
+  // + 1 us per 9.5 M multiply-adds.  Measured crossovers: fp32 in three passes 36 M (512x256x256: 6.7 us against 6.9;
+  // 64x128x784: 4.1 against 13.8), 100 M where a fused epilogue keeps a deep k in few CTAs (1024x128x784: 13.8
+  // against 18.3; 2048 rows: 21.0 against 19.7); single pass 4 M (bf16 64x128x784 = 6.4 M: 6.0 against 5.6).
+  const bool fused = epilogue != ZG_EPI_NONE || colsum;
+  const double small = (bf16 || g_math_mode == ZG_MATH_TF32) ? 4e6 : (fused && k >= 512 ? 1e8 : 3.6e7);
+  static const bool force = [] { const char* e = getenv("ZG_GEMM_FORCE_TC"); return e && e[0] == '1'; }();
+  const double macs = (double)((m + 31) / 32 * 32) * (double)((n + 31) / 32 * 32) * (double)k * (double)nC;  // its tiles are 32 x 32
+  if (!force && macs < small) return false;
 
   const int mode = bf16 ? tc::kBF16 : (g_math_mode == ZG_MATH_TF32 ? tc::kTF32 : tc::kFP32X3);
   const int atom = bf16 ? 64 : 32;        // M/N elements per 128-byte column block
@@ -377,10 +279,10 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   const bool b_kmajor = tb;               // B stored [n,k] -> K contiguous
   // Large single-pass problems: persistent kernel over 128 x 256 tiles
   // (at least one tile per SM, k deep enough to amortise the tile hand-over).
-  const char* no_persist = getenv("ZG_GEMM_NO_PERSISTENT");
+  static const bool no_persist = [] { const char* e = getenv("ZG_GEMM_NO_PERSISTENT"); return e && e[0] == '1'; }();
   const size_t ptiles = ((m + 127) / 128) * ((n + 255) / 256) * nC;
   const bool persistent = mode != tc::kFP32X3 && n > 128 && k >= 8 * (size_t)bk && ptiles * 2 >= (size_t)sm_count() &&
-                          ptiles <= 0x3fffffffu && !(no_persist && no_persist[0] == '1');
+                          ptiles <= 0x3fffffffu && !no_persist;
   int bn = persistent ? 256 : (n <= 32 ? 32 : (n <= 64 ? 64 : 128));
   if (bn < atom) bn = atom;               // MN-major B needs whole column blocks; bf16 has no BN=32 instance
   size_t tiles = ((m + 127) / 128) * ((n + bn - 1) / bn) * nC;
@@ -496,10 +398,10 @@ void bmm_dispatch(dtype id, dtype c_id, cudaStream_t s, const void* A, const voi
   if (colsum && id == DOUBLE) { set_error(kUnsupported, "bmm: column sums are fp32 only"); return; }
   if (try_skinny(id, c_id, s, A, B, C, nA, nB, nC, m, n, k, ta, tb, lda, ldb, ldc, alpha, beta, epilogue, bias, mask, colsum)) return;
   if (try_tensor_core(id, c_id, s, A, B, C, nA, nB, nC, m, n, k, ta, tb, lda, ldb, ldc, alpha, beta, epilogue, bias, mask, colsum)) return;
-  if (id == SINGLE && c_id == SINGLE) launch_simt<float, float>(s, A, B, C, nA, nB, nC, m, n, k, ta, tb, lda, ldb, ldc, alpha, beta, epilogue, bias, mask, colsum);
-  else if (id == DOUBLE && c_id == DOUBLE) launch_simt<double, double>(s, A, B, C, nA, nB, nC, m, n, k, ta, tb, lda, ldb, ldc, alpha, beta, epilogue, bias, mask, colsum);
-  else if (id == BF16 && c_id == SINGLE) launch_simt<__nv_bfloat16, float>(s, A, B, C, nA, nB, nC, m, n, k, ta, tb, lda, ldb, ldc, alpha, beta, epilogue, bias, mask, colsum);
-  else if (id == BF16 && c_id == BF16) launch_simt<__nv_bfloat16, __nv_bfloat16>(s, A, B, C, nA, nB, nC, m, n, k, ta, tb, lda, ldb, ldc, alpha, beta, epilogue, bias, mask, colsum);
+  if (id == SINGLE && c_id == SINGLE) launch_block<float, float>(s, A, B, C, nA, nB, nC, m, n, k, ta, tb, lda, ldb, ldc, alpha, beta, epilogue, bias, mask, colsum);
+  else if (id == DOUBLE && c_id == DOUBLE) launch_block<double, double>(s, A, B, C, nA, nB, nC, m, n, k, ta, tb, lda, ldb, ldc, alpha, beta, epilogue, bias, mask, colsum);
+  else if (id == BF16 && c_id == SINGLE) launch_block<__nv_bfloat16, float>(s, A, B, C, nA, nB, nC, m, n, k, ta, tb, lda, ldb, ldc, alpha, beta, epilogue, bias, mask, colsum);
+  else if (id == BF16 && c_id == BF16) launch_block<__nv_bfloat16, __nv_bfloat16>(s, A, B, C, nA, nB, nC, m, n, k, ta, tb, lda, ldb, ldc, alpha, beta, epilogue, bias, mask, colsum);
   else set_error(kUnsupported, "bmm: unsupported dtype combination %d -> %d", (int)id, (int)c_id);
 }
 
