@@ -2,6 +2,7 @@
 // (include/blas_conflux.h).  Large, TMA-addressable problems go to the
 // tcgen05 kernel (gemm_tc.cuh); everything else (small shapes, rows whose byte
 // stride is not a multiple of 16, fp64) runs on the FFMA kernel of gemm_block.cuh.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -116,22 +117,16 @@ static bool make_tmap(CUtensorMap* map, bool bf16, const void* base, uint64_t in
   return ZG_CU(r);
 }
 
-template <int BN, bool AK, bool BK_, int MODE, bool ATM = false>
+template <int BN, bool AK, bool BK_, int MODE, bool DIRECT = false>
 static bool launch_tc_inst(cudaStream_t s, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tcm, const tc::Params& p, dim3 grid) {
-  using SL = tc::SmemLayout<BN, MODE, ATM>;
-  auto kern = tc::gemm_tc_kernel<BN, AK, BK_, MODE, ATM>;
+  using SL = tc::SmemLayout<BN, MODE>;
+  auto kern = tc::gemm_tc_kernel<BN, AK, BK_, MODE, DIRECT>;
   static bool attr_set = false;
   if (!attr_set) {
     if (!ZG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SL::kTotal))) return false;
     attr_set = true;
   }
-  return launch_pdl(kern, grid, dim3(tc::tc_threads(MODE)), (size_t)SL::kTotal, s, ta, tb, tcm, p);
-}
-
-// FP32X3: the hi/lo parts of A live in tensor memory (ZG_X3_TMEM_A=0 keeps them in shared memory)
-static bool x3_tmem_a() {
-  static const bool on = [] { const char* e = getenv("ZG_X3_TMEM_A"); return !(e && e[0] == '0'); }();
-  return on;
+  return launch_pdl_cluster(kern, grid, dim3(SL::kThreads + (DIRECT ? 128 : 0)), (size_t)SL::kTotal, s, p.cluster ? p.splits : 1, ta, tb, tcm, p);
 }
 
 template <int MODE>
@@ -139,14 +134,6 @@ static bool launch_tc_mode(cudaStream_t s, int bn, bool a_kmajor, bool b_kmajor,
                            const CUtensorMap& tcm, const tc::Params& p, dim3 grid) {
 #define ZG_TC_CASE(BNV)                                                                       \
   if (bn == BNV) {                                                                            \
-    if constexpr (MODE == tc::kFP32X3) {                                                      \
-      if (x3_tmem_a()) {                                                                      \
-        if (a_kmajor && b_kmajor) return launch_tc_inst<BNV, true, true, MODE, true>(s, ta, tb, tcm, p, grid);   \
-        if (a_kmajor) return launch_tc_inst<BNV, true, false, MODE, true>(s, ta, tb, tcm, p, grid);              \
-        if (b_kmajor) return launch_tc_inst<BNV, false, true, MODE, true>(s, ta, tb, tcm, p, grid);              \
-        return launch_tc_inst<BNV, false, false, MODE, true>(s, ta, tb, tcm, p, grid);                           \
-      }                                                                                       \
-    }                                                                                         \
     if (a_kmajor && b_kmajor) return launch_tc_inst<BNV, true, true, MODE>(s, ta, tb, tcm, p, grid);   \
     if (a_kmajor && !b_kmajor) return launch_tc_inst<BNV, true, false, MODE>(s, ta, tb, tcm, p, grid); \
     if (!a_kmajor && b_kmajor) return launch_tc_inst<BNV, false, true, MODE>(s, ta, tb, tcm, p, grid); \
@@ -158,6 +145,45 @@ static bool launch_tc_mode(cudaStream_t s, int bn, bool a_kmajor, bool b_kmajor,
 #undef ZG_TC_CASE
   set_error(kBadArgument, "gemm: no tensor-core instance for BN=%d", bn);
   return false;
+}
+
+static void launch_tc_direct(cudaStream_t s, int bn, bool a_kmajor, bool b_kmajor, const CUtensorMap& ta, const CUtensorMap& tb,
+                             const CUtensorMap& tcm, const tc::Params& p, dim3 grid) {
+#define ZG_DIRECT_CASE(BNV)                                                                                        \
+  if (a_kmajor && b_kmajor) launch_tc_inst<BNV, true, true, tc::kFP32X3, true>(s, ta, tb, tcm, p, grid);     \
+  else if (a_kmajor) launch_tc_inst<BNV, true, false, tc::kFP32X3, true>(s, ta, tb, tcm, p, grid);           \
+  else if (b_kmajor) launch_tc_inst<BNV, false, true, tc::kFP32X3, true>(s, ta, tb, tcm, p, grid);           \
+  else launch_tc_inst<BNV, false, false, tc::kFP32X3, true>(s, ta, tb, tcm, p, grid);
+  if (bn == 64) { ZG_DIRECT_CASE(64) } else { ZG_DIRECT_CASE(128) }
+#undef ZG_DIRECT_CASE
+}
+
+// Clusters of `size` CTAs that can run at once when a CTA takes a whole SM (GPCs hold different numbers of SMs, so not
+// every SM finds a place: of 148, 148 CTAs in pairs, 132 in fours and sixes, 120 in eights).
+static size_t max_clusters(unsigned size) {
+  static int cached[9] = {0};
+  if (!cached[size]) {
+    using SL = tc::SmemLayout<64, tc::kFP32X3>;
+    auto kern = tc::gemm_tc_kernel<64, true, true, tc::kFP32X3>;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(size);
+    cfg.blockDim = dim3(SL::kThreads);
+    cfg.dynamicSmemBytes = SL::kTotal;
+    cudaLaunchAttribute attr;
+    memset(&attr, 0, sizeof(attr));
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = size;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (!ZG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SL::kTotal)) ||
+        !ZG_CUDA(cudaOccupancyMaxActiveClusters(&n, kern, &cfg)))
+      return 0;
+    cached[size] = n + 1;  // 0: not asked yet
+  }
+  return (size_t)(cached[size] - 1);
 }
 
 template <bool AK, bool BK_, int MODE>
@@ -215,7 +241,8 @@ static bool try_skinny(dtype id, dtype c_id, cudaStream_t s, const void* A, cons
     return launch_pdl(skinny::skinny_m_kernel<16>, dim3(grid), dim3(skinny::kThreads), smem, s, p, rows_per_cta);
   }
   if (m < 256) return false;
-  if (n <= 16 && k >= 16 && k <= 512 && k % 4 == 0 && lda % 4 == 0 && host_aligned16(A) && epilogue != ZG_EPI_RELU_MASK && !colsum) {
+  // (deeper rows: the quad per row walks them serially, 37 us for 20000x16x500 against 10 on the tensor cores)
+  if (n <= 16 && k >= 16 && k <= 128 && k % 4 == 0 && lda % 4 == 0 && host_aligned16(A) && epilogue != ZG_EPI_RELU_MASK && !colsum) {
     const unsigned grid = (unsigned)((m + skinny::kThreads / 4 - 1) / (skinny::kThreads / 4));
     const size_t smem = (size_t)n * k * sizeof(float);
     if (n <= 4) return launch_pdl(skinny::skinny_n_kernel<4>, dim3(grid), dim3(skinny::kThreads), smem, s, p);
@@ -258,45 +285,56 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   if (id == SINGLE && (g_math_mode == ZG_MATH_FFMA || c_id != SINGLE)) return false;
   if (bf16 && !(c_id == SINGLE || c_id == BF16)) return false;
   const size_t es = bf16 ? 2 : 4;
-  if (!host_aligned16(A) || !host_aligned16(B) || (lda * es) % 16 || (ldb * es) % 16) return false;
+  // operands whose rows a TMA box cannot address: fp32 ones are copied element by element (direct_slab)
+  bool a_direct = !host_aligned16(A) || (lda * es) % 16 != 0, b_direct = !host_aligned16(B) || (ldb * es) % 16 != 0;
+  const bool direct = a_direct || b_direct;
+  if (direct && bf16) return false;
   if (m == 0 || n == 0 || nC == 0) return false;
   if (m > 0x7fffffffu || n > 0x7fffffffu || k > 0x7fffffffu || ldc > 0xffffffffu) return false;
   // Small problems are a latency chain on the tensor cores (descriptor fetch, TMA round trip, operand split, MMA,
-  // TMEM read-back, and for split K a pre-scaled C and a second pass); the FFMA kernel with its clusters needs 3 us
-  // + 1 us per 9.5 M multiply-adds.  Measured crossovers: fp32 in three passes 36 M (512x256x256: 6.7 us against 6.9;
-  // 64x128x784: 4.1 against 13.8), 100 M where a fused epilogue keeps a deep k in few CTAs (1024x128x784: 13.8
-  // against 18.3; 2048 rows: 21.0 against 19.7); single pass 4 M (bf16 64x128x784 = 6.4 M: 6.0 against 5.6).
-  const bool fused = epilogue != ZG_EPI_NONE || colsum;
-  const double small = (bf16 || g_math_mode == ZG_MATH_TF32) ? 4e6 : (fused && k >= 512 ? 1e8 : 3.6e7);
+  // TMEM read-back: 7 to 9 us in three passes, 4 in one); the FFMA kernel with its clusters needs 3 us + 1 us per 9.5 M
+  // multiply-adds.  Measured crossovers: 50 M in three passes (512x128x784: 8.5 us either way; 64x128x784 4.1
+  // against 13.8), 4 M in one (bf16 64x128x784 = 6.4 M: 6.0 against 5.6).
+  const int mode = bf16 ? tc::kBF16 : (g_math_mode == ZG_MATH_TF32 && !direct ? tc::kTF32 : tc::kFP32X3);
+  const double small = mode == tc::kFP32X3 ? 5e7 : 4e6;
   static const bool force = [] { const char* e = getenv("ZG_GEMM_FORCE_TC"); return e && e[0] == '1'; }();
   const double macs = (double)((m + 31) / 32 * 32) * (double)((n + 31) / 32 * 32) * (double)k * (double)nC;  // its tiles are 32 x 32
   if (!force && macs < small) return false;
 
-  const int mode = bf16 ? tc::kBF16 : (g_math_mode == ZG_MATH_TF32 ? tc::kTF32 : tc::kFP32X3);
   const int atom = bf16 ? 64 : 32;        // M/N elements per 128-byte column block
   const int bk = bf16 ? 64 : 32;
-  const bool a_kmajor = !ta;              // A stored [m,k] -> K contiguous
-  const bool b_kmajor = tb;               // B stored [n,k] -> K contiguous
+  // A C of few rows is computed as its transpose, so that the long dimension fills the 128 rows of the tile.
+  // (Only where the column tiles alone occupy the chip in clusters of eight.)
+  const bool swap = m <= 64 && n >= 1536;
+  const len_t M = swap ? n : m, N = swap ? m : n;
+  const bool a_kmajor = swap ? tb : !ta;  // the dimension that is contiguous in memory: K, or M / N
+  const bool b_kmajor = swap ? !ta : tb;
   // Large single-pass problems: persistent kernel over 128 x 256 tiles
   // (at least one tile per SM, k deep enough to amortise the tile hand-over).
   static const bool no_persist = [] { const char* e = getenv("ZG_GEMM_NO_PERSISTENT"); return e && e[0] == '1'; }();
   const size_t ptiles = ((m + 127) / 128) * ((n + 255) / 256) * nC;
-  const bool persistent = mode != tc::kFP32X3 && n > 128 && k >= 8 * (size_t)bk && ptiles * 2 >= (size_t)sm_count() &&
+  const bool persistent = mode != tc::kFP32X3 && !swap && n > 128 && k >= 8 * (size_t)bk && ptiles * 2 >= (size_t)sm_count() &&
                           ptiles <= 0x3fffffffu && !no_persist;
-  int bn = persistent ? 256 : (n <= 32 ? 32 : (n <= 64 ? 64 : 128));
+  int bn = persistent ? 256 : (N <= 32 && !direct ? 32 : (N <= 64 ? 64 : 128));
   if (bn < atom) bn = atom;               // MN-major B needs whole column blocks; bf16 has no BN=32 instance
-  size_t tiles = ((m + 127) / 128) * ((n + bn - 1) / bn) * nC;
-  // Deep-k problems with a plain epilogue (weight gradients) get their
-  // parallelism from K splits, so they keep the wide tile (fewer operand bytes
-  // per flop through shared memory); everything else halves BN when there are
-  // too few tiles to occupy the SMs.
-  // (with a fused epilogue or column sums the last CTA of a tile applies them to the finished sums)
-  // and that costs a second pass over the tile, so it is kept for problems with very few tiles)
-  const bool deferred = epilogue != ZG_EPI_NONE || colsum;
-  const bool can_split = !persistent && c_id == SINGLE && k >= 512 && (!deferred || tiles * 4 <= sm_share());
-  if (!can_split && bn == 128 && tiles * 2 <= sm_share() && n > 64) {
+  size_t tiles = ((M + 127) / 128) * ((N + bn - 1) / bn) * nC;
+  // Problems with few tiles get their parallelism from K splits.  Up to eight splits form a cluster, which sums its
+  // partial tiles through distributed shared memory and applies any epilogue.  A plain product of 128-wide tiles
+  // adds them into C with TMA reductions instead (128x784x1024: 7.2 us against 8.8), which also allows more
+  // than eight.  What cannot split, or only in two, halves BN when there are too few tiles to occupy the SMs
+  // (8192x128x784: 12.6 us in 64-wide tiles, 14.4 as two splits of 128-wide ones).
+  const size_t min_slabs = mode == tc::kFP32X3 ? 4 : 12;  // per split: a three-pass slab costs 450 to 750 cycles, a single-pass one 130
+  const bool can_split = !persistent && k >= 2 * min_slabs * (size_t)bk && tiles * (bn == 128 ? 3 : 2) <= sm_share();
+  if (!persistent && !can_split && bn == 128 && tiles * 2 <= sm_share() && N > 64) {
     bn = 64;
-    tiles = ((m + 127) / 128) * ((n + bn - 1) / bn) * nC;
+    tiles = ((M + 127) / 128) * ((N + bn - 1) / bn) * nC;
+  }
+  bool c_aligned;
+  {
+    const size_t ce = (c_id == SINGLE) ? 4 : 2;
+    c_aligned = host_aligned16(C) && (ldc * ce) % 16 == 0 && ((uint64_t)m * ldc * ce) % 16 == 0;
+    if (mask) c_aligned = c_aligned && host_aligned16(mask);
+    if (bias) c_aligned = c_aligned && host_aligned16(bias);
   }
 
   unsigned splits = 1;
@@ -311,23 +349,36 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
       if (eff > best + 0.03) { best = eff; splits = sp; }
     }
   }
-  if (can_split && tiles * 2 <= sm_share()) {
-    size_t want = sm_share() / tiles;
-    size_t maxs = k / (4 * (size_t)bk);  // at least four k-slabs per split
-    splits = (unsigned)(want < maxs ? want : maxs);
-    if (splits < 1) splits = 1;
+  bool cluster = false;
+  if (can_split) {
+    const bool reduces = epilogue == ZG_EPI_NONE && !colsum && c_id == SINGLE && c_aligned && !swap && bn == 128;
+    splits = (unsigned)std::max<size_t>(1, std::min(sm_share() / tiles, k / (min_slabs * bk)));
+    if (!reduces) {
+      splits = std::min(splits, 8u);
+      while (splits > 1 && tiles > max_clusters(splits)) --splits;
+      cluster = splits > 1;
+    }
   }
   const size_t k_per_split = splits > 1 ? ((k + splits - 1) / splits + bk - 1) / bk * bk : ((k + bk - 1) / bk * bk);
   if (splits > 1) splits = (unsigned)((k + k_per_split - 1) / k_per_split);
+  cluster = cluster && splits > 1;
 
+  // the tile's A and B: C's own operands, or exchanged
+  const void *pa = swap ? B : A, *pb = swap ? A : B;
+  const len_t la = swap ? ldb : lda, lb = swap ? lda : ldb, na = swap ? nB : nA, nb = swap ? nA : nB;
+  if (swap) std::swap(a_direct, b_direct);
   CUtensorMap tmA, tmB;
-  bool ok;
+  memset(&tmA, 0, sizeof(tmA));
+  memset(&tmB, 0, sizeof(tmB));
+  bool ok = true;
   // MN-major fp32 operands travel in the 128-byte swizzle with 32-byte atoms
-  if (a_kmajor) ok = make_tmap(&tmA, bf16, A, k, m, nA, lda, bk, 128, false);
-  else ok = make_tmap(&tmA, bf16, A, m, k, nA, lda, atom, bk, !bf16);
+  if (a_direct) {}
+  else if (a_kmajor) ok = make_tmap(&tmA, bf16, pa, k, M, na, la, bk, 128, false);
+  else ok = make_tmap(&tmA, bf16, pa, M, k, na, la, atom, bk, !bf16);
   if (!ok) return true;  // error recorded
-  if (b_kmajor) ok = make_tmap(&tmB, bf16, B, k, n, nB, ldb, bk, bn, false);
-  else ok = make_tmap(&tmB, bf16, B, n, k, nB, ldb, atom, bk, !bf16);
+  if (b_direct) {}
+  else if (b_kmajor) ok = make_tmap(&tmB, bf16, pb, k, N, nb, lb, bk, bn, false);
+  else ok = make_tmap(&tmB, bf16, pb, N, k, nb, lb, atom, bk, !bf16);
   if (!ok) return true;
 
   tc::Params p;
@@ -338,16 +389,18 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   p.colsum = static_cast<float*>(colsum);
   p.c_batch_stride = (uint64_t)m * ldc;
   p.m = (uint32_t)m; p.n = (uint32_t)n; p.k = (uint32_t)k; p.ldc = (uint32_t)ldc;
-  p.nA = (uint32_t)nA; p.nB = (uint32_t)nB;
+  p.nA = (uint32_t)na; p.nB = (uint32_t)nb;
+  p.swap = swap ? 1 : 0;
+  p.a_direct = a_direct; p.b_direct = b_direct;
+  if (direct) {
+    p.a_src = static_cast<const float*>(pa); p.b_src = static_cast<const float*>(pb);
+    p.a_ld = la; p.b_ld = lb;
+    p.a_batch = (a_kmajor ? M : k) * la; p.b_batch = (b_kmajor ? N : k) * lb;
+  }
+  p.tiles_n = (uint32_t)((N + bn - 1) / bn);
   p.splits = splits; p.k_per_split = (uint32_t)k_per_split;
   p.alpha = (float)alpha; p.beta = (float)beta; p.epilogue = epilogue;
-  {
-    const size_t ce = (c_id == SINGLE) ? 4 : 2;
-    bool ok = host_aligned16(C) && (ldc * ce) % 16 == 0 && ((uint64_t)m * ldc * ce) % 16 == 0;
-    if (mask) ok = ok && host_aligned16(mask);
-    if (bias) ok = ok && host_aligned16(bias);
-    p.vec_ok = ok ? 1 : 0;
-  }
+  p.vec_ok = c_aligned ? 1 : 0;
   p.error_flag = tc_error_flag();
   if (persistent) {
     const uint32_t tiles_m = (uint32_t)((m + 127) / 128), tiles_n = (uint32_t)((n + 255) / 256);
@@ -357,29 +410,22 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
     else launch_persistent<tc::kTF32>(s, a_kmajor, b_kmajor, tmA, tmB, p, tiles_m, tiles_n, items);
     return true;
   }
-  if (splits > 1) prescale_c<float>(s, static_cast<float*>(C), nC, m, n, ldc, m * ldc, beta);
-  if (splits > 1 && deferred) {
-    unsigned* unused = nullptr;
-    p.tile_tickets = static_cast<unsigned*>(workspace(s, sizeof(unsigned) * tiles, &unused, 2));
-    if (!p.tile_tickets) return true;
-    p.deferred_epilogue = epilogue;
-    p.deferred_colsum = p.colsum;
-    p.epilogue = ZG_EPI_NONE;
-    p.colsum = nullptr;
-  }
-  dim3 grid((unsigned)((n + bn - 1) / bn), (unsigned)((m + 127) / 128), (unsigned)(nC * splits));
+  p.cluster = cluster ? 1 : 0;
+  if (splits > 1 && !cluster) prescale_c<float>(s, static_cast<float*>(C), nC, m, n, ldc, m * ldc, beta);
+  dim3 grid((unsigned)((N + bn - 1) / bn * splits), (unsigned)((M + 127) / 128), (unsigned)nC);
   if (grid.y > 65535 || grid.z > 65535) return false;
   // Output through the C tensor map where the epilogue needs nothing from global memory but the bias
   // (ZG_GEMM_TMA_EPILOGUE=0 keeps the register path)
   CUtensorMap tmC;
   memset(&tmC, 0, sizeof(tmC));
   static const bool tma_epi_on = [] { const char* e = getenv("ZG_GEMM_TMA_EPILOGUE"); return !(e && e[0] == '0'); }();
-  if (tma_epi_on && c_id == SINGLE && p.vec_ok && !p.tile_tickets && !p.colsum && nC <= 0x7fffffffu &&
+  if (tma_epi_on && c_id == SINGLE && p.vec_ok && !cluster && !swap && !p.colsum && nC <= 0x7fffffffu &&
       (splits > 1 ? epilogue == ZG_EPI_NONE : (beta == 0.0 && epilogue != ZG_EPI_RELU_MASK))) {
     if (!make_tmap(&tmC, false, C, n, m, nC, ldc, 32, 32, false)) return true;
     p.tma_epilogue = splits > 1 ? 2 : 1;
   }
-  if (mode == tc::kBF16) launch_tc_mode<tc::kBF16>(s, bn, a_kmajor, b_kmajor, tmA, tmB, tmC, p, grid);
+  if (direct) launch_tc_direct(s, bn, a_kmajor, b_kmajor, tmA, tmB, tmC, p, grid);
+  else if (mode == tc::kBF16) launch_tc_mode<tc::kBF16>(s, bn, a_kmajor, b_kmajor, tmA, tmB, tmC, p, grid);
   else if (mode == tc::kTF32) launch_tc_mode<tc::kTF32>(s, bn, a_kmajor, b_kmajor, tmA, tmB, tmC, p, grid);
   else launch_tc_mode<tc::kFP32X3>(s, bn, a_kmajor, b_kmajor, tmA, tmB, tmC, p, grid);
   return true;

@@ -299,8 +299,12 @@ __global__ void __launch_bounds__(kThreads) gemm_block_kernel(const TI* __restri
     const int share = TM * TN / (int)p.splits;  // this CTA finishes one share of the tile (whole rows: splits <= 8)
     for (int e = threadIdx.x; e < share; e += kThreads) {
       const int at = (int)split * share + e;
-      AT v = AT(0);
-      for (uint32_t r = 0; r < p.splits; ++r) v += cluster.map_shared_rank(red, r)[at];
+      // all ranks' values are requested before the first is added: one round trip over the cluster network, not eight
+      AT part[8], v = AT(0);
+#pragma unroll
+      for (uint32_t r = 0; r < 8; ++r) part[r] = r < p.splits ? cluster.map_shared_rank(red, r)[at] : AT(0);
+#pragma unroll
+      for (uint32_t r = 0; r < 8; ++r) v += part[r];
       finish(at, v);
     }
     cluster.sync();  // nobody leaves while its partial tile may still be read

@@ -11,19 +11,30 @@
 //               lane measured 55 cycles per tcgen05.mma issued against 20 this
 //               way), one elected lane issues tcgen05.mma with the accumulator
 //               in tensor memory; also owns the TMEM allocation
-//   warps 2-7   FP32X3 mode only: for every fp32 operand slab write the
-//               remainder lo = x - tf32(x) to a second buffer.  The MMA reads
+//   warps 2-11  FP32X3 mode only (the other modes have 8 warps): for every fp32
+//               operand slab form the remainder lo = x - tf32(x).  The MMA reads
 //               only the top 19 bits of an fp32 word (measured: results do not
 //               change when the low 13 bits are cleared first), so the fetched
-//               slab itself serves as "hi" and Ahi*Bhi + Alo*Bhi + Ahi*Blo
-//               recovers fp32-level accuracy.  With a K-major A (hi and lo of A
-//               go to tensor memory) and tiles of up to 64 columns, warps 4-7
-//               split A, warps 2-3 most of B, each fetching its part of the
-//               next slab before it hands the current one over; one mbarrier
-//               arrival per warp
-//   warps 4-7   epilogue: tcgen05.ld of the accumulator (warp q reads TMEM
-//               lanes 32q..32q+31, one row per thread), alpha/beta/bias/ReLU/
-//               mask in registers, 128-bit row-contiguous global accesses
+//               word itself serves as "hi" and Ahi*Bhi + Alo*Bhi + Ahi*Blo
+//               recovers fp32-level accuracy.  Hi and lo of A go to tensor memory
+//               (thread = row), lo of B to a second buffer of the stage.  Warps
+//               4-7 and 8-11 take the A slabs in turn, warps 2-3 split (most of)
+//               B, each fetching its part of its next slab before it hands the
+//               current one over; one mbarrier arrival per warp.  With one set of
+//               A warps the serial chain of a slab (wait, split, tcgen05.st, wait)
+//               bounded the loop: 4096^3 650 -> 635 us, 128x784x8192 12.7 -> 12.3
+//   warps 12-15 DIRECT instances only: element-wise copies of operands whose rows no
+//               TMA box can address (1000x501x1000 with 501-float rows: 16 us
+//               against 66 on the FFMA path, 4096x1023x1023 80 against 385)
+//   warps 4-7   read the accumulator (tcgen05.ld: warp q reads TMEM lanes
+//               32q..32q+31, one row per thread); then either staged boxes go to
+//               the TMA unit, or the whole tile is staged in shared memory and
+//               all warps apply alpha / beta / bias / ReLU / mask with lanes along
+//               the rows of C, so that unaligned rows are coalesced as well.
+//               Split K forms clusters of up to 8 CTAs that sum their staged tiles
+//               through distributed shared memory in rank order: 2000x256x1000 +
+//               bias + ReLU 30 -> 14 us (before: partial sums added into a
+//               pre-scaled C by atomics, the last CTA of a tile re-reading it)
 //
 // Operand layouts.  A row-major matrix whose contiguous dimension is K is a
 // "K-major" UMMA operand; one whose contiguous dimension is M (or N) is
@@ -55,7 +66,6 @@ namespace tc {
 constexpr int kBM = 128;
 constexpr int kThreadsTc = 256;
 constexpr int kSplitThreads = kThreadsTc - 64;  // warps 2-7
-__host__ __device__ constexpr int tc_threads(int /*mode*/) { return kThreadsTc; }
 constexpr int kSlabBytes = 128;          // bytes of the contiguous dimension per smem row
 constexpr uint32_t kSpinLimit = 1u << 24;  // polls per wait before giving up
 
@@ -72,7 +82,8 @@ struct Params {
   uint32_t m, n, k;
   uint32_t ldc;
   uint32_t nA, nB;      // operand batch counts (index wraps)
-  uint32_t splits;      // K splits (gridDim.z = batches * splits)
+  uint32_t tiles_n;     // column tiles
+  uint32_t splits;      // K splits (gridDim.x = column tiles * splits)
   uint32_t k_per_split; // multiple of BK
   float alpha, beta;
   int epilogue;
@@ -85,14 +96,16 @@ struct Params {
   // lines leave the SM instead of 16-byte pieces of 32 different lines per instruction, and boxes that
   // hang over the edge of C are clipped by the unit.  0: register path below.
   int tma_epilogue;
-  // Split-K with a fused epilogue: the partial products are added into C (which
-  // the launcher scaled by beta first) with the epilogue switched off; every CTA
-  // then takes a ticket of its tile, and the one that draws the last applies
-  // bias / ReLU / mask / column sums to the finished sums.  One counter per
-  // output tile, zero before and after the launch.
-  unsigned* tile_tickets;
-  int deferred_epilogue;  // what to apply at the end (epilogue is NONE and colsum NULL during accumulation)
-  float* deferred_colsum;
+  // Split K over the CTAs of a cluster: every CTA stages its partial tile in shared memory, rank r sums rows r,
+  // r + splits, ... of all of them through distributed shared memory in rank order and applies the epilogue.
+  int cluster;
+  int swap;  // the tile is C transposed: its rows are C's columns (short C: the long dimension fills the 128 rows)
+  // Operands whose rows no TMA box can address (base or row stride not a multiple of 16 bytes) come through
+  // element-wise cp.async of four loader warps into the same swizzled slabs (DIRECT instances only).
+  int a_direct, b_direct;
+  const float* a_src;
+  const float* b_src;
+  uint64_t a_ld, b_ld, a_batch, b_batch;  // elements
 };
 
 // ------------------------------------------------------------------ PTX
@@ -292,7 +305,6 @@ struct ModeTraits {
   static constexpr int kBK = kSlabBytes / kElem;       // elements of K per stage: 32 (fp32) / 64 (bf16)
   static constexpr int kUmmaK = 32 / kElem;            // K per MMA: 8 (tf32) / 16 (bf16)
   static constexpr int kAtomMN = kSlabBytes / kElem;   // M/N elements per 128-byte column block
-  static constexpr int kBufs = (MODE == kFP32X3) ? 2 : 1;  // hi (+ lo) copies of each operand slab
 };
 
 // Epilogue of one 32-column chunk of one accumulator row (registers r, raw
@@ -453,45 +465,268 @@ __device__ __forceinline__ void load_a_row(const uint8_t* a_stage, int row, floa
   }
 }
 
-// ATM: FP32X3 keeps the hi and lo parts of the A operand in TENSOR
+// One slab (ROWS rows x 32 k) of an fp32 operand into its swizzled place by 128 threads, 4 bytes per copy, lanes along
+// the contiguous dimension of the source; zeros outside [0, rows) x [0, k).
+template <int ROWS, bool KMAJOR>
+__device__ __forceinline__ void direct_slab(uint8_t* dst, const float* src, uint64_t ld, uint32_t row0, uint32_t rows, uint32_t k0, uint32_t k, const float* safe) {
+  const int w = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
+  const uint32_t base = smem_u32(dst);
+  auto copy = [&](uint32_t to, const float* from, bool ok) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(ok ? from : safe), "r"(ok ? 4 : 0) : "memory");
+  };
+  if constexpr (KMAJOR) {
+    const bool k_ok = k0 + lane < k;
+    const float* s = src + (uint64_t)(row0 + w) * ld + k0 + lane;
+    const uint32_t d0 = base + w * kSlabBytes + (((lane >> 2) ^ w) << 4) + ((lane & 3) << 2);
+    const uint32_t d1 = base + (w + 4) * kSlabBytes + (((lane >> 2) ^ (w + 4)) << 4) + ((lane & 3) << 2);
+    const uint64_t step = 4 * ld;
+#pragma unroll
+    for (int i = 0; i < ROWS / 4; ++i) {
+      copy(((i & 1) ? d1 : d0) + (i >> 1) * (8 * kSlabBytes), s, k_ok && row0 + w + 4 * i < rows);
+      s += step;
+    }
+  } else {
+    const uint32_t d = base + w * kSlabBytes + (((lane >> 3) ^ w) << 5) + ((lane & 7) << 2);
+    const float* s = src + (uint64_t)(k0 + w) * ld + row0 + lane;
+    const uint64_t step = 4 * ld;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const bool k_ok = k0 + w + 4 * i < k;
+#pragma unroll
+      for (int b = 0; b < ROWS / 32; ++b)
+        copy(d + b * (32 * kSlabBytes) + i * (4 * kSlabBytes), s + 32 * b, k_ok && row0 + 32 * b + lane < rows);
+      s += step;
+    }
+  }
+}
+
+// FP32X3 keeps the hi and lo parts of the A operand in TENSOR
 // MEMORY (written by the split warps with tcgen05.st, read by the MMA from
 // there): shared memory then holds A once per stage (the fetched slab) and no
 // MMA reads it, which takes 64 of the 144 KB per 128x64x32 slab off the
 // shared-memory data pipe -- the unit that bounds this mode.
-template <int BN, int MODE, bool ATM = false>
+template <int BN, int MODE>
 struct SmemLayout {
+  static constexpr bool X3 = MODE == kFP32X3;
   using MT = ModeTraits<MODE>;
   static constexpr int kABytes = kBM * kSlabBytes;   // 16 KB
   static constexpr int kBBytes = BN * kSlabBytes;
-  static constexpr int kStageBytes = ATM ? (kABytes + 2 * kBBytes) : (kABytes + kBBytes) * MT::kBufs;
+  static constexpr int kStageBytes = kABytes + (X3 ? 2 : 1) * kBBytes;
   static constexpr int kEpiBytes = 0;
   static constexpr int kBudget = 220 * 1024;
   static constexpr int kAccCols = BN < 32 ? 32 : BN;
   static constexpr int kATmemCols = 64;              // per stage: 32 columns hi + 32 columns lo
   static constexpr int kStagesSmem = (kBudget - kEpiBytes - 1024) / kStageBytes;
-  static constexpr int kStagesTmem = ATM ? (512 - kAccCols) / kATmemCols : 8;
+  static constexpr int kStagesTmem = X3 ? (512 - kAccCols) / kATmemCols : 8;
   static constexpr int kStagesRaw = kStagesSmem < kStagesTmem ? kStagesSmem : kStagesTmem;
-  static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;
-  static constexpr int kTmemNeed = ATM ? kAccCols + kATmemCols * kStages : kAccCols;
+  // Even: the two sets of A warps take the slabs in turn, and a set may wait for a slab only if it has waited for the
+  // one that filled the same stage before (a parity tells two phases apart, not three).
+  static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw / 2 * 2;
+  static constexpr int kTmemNeed = X3 ? kAccCols + kATmemCols * kStages : kAccCols;
   static constexpr int kTmemCols = kTmemNeed <= 32 ? 32 : (kTmemNeed <= 64 ? 64 : (kTmemNeed <= 128 ? 128 : (kTmemNeed <= 256 ? 256 : 512)));
   static constexpr int kTotal = kStages * kStageBytes + kEpiBytes + 1024 /*alignment slack*/ + 256 /*barriers*/;
-  // ATM: 16-byte words of a B slab per thread of the two B warps / of the four A warps
+  // FP32X3: 16-byte words of a B slab per thread of the two B warps / of the four A warps
   // (BN 128: 8 + 4, BN 64: 6 + 1, BN 32: 4 + 0; 64 * kBWordsB + 128 * kBWordsA = BN * 8)
   static constexpr int kBWordsA = BN >= 128 ? 4 : (BN >= 64 ? 1 : 0);
   static constexpr int kBWordsB = (BN * 8 - 128 * kBWordsA) / 64;
+  // FP32X3: two sets of four A warps take the slabs in turn
+  static constexpr int kThreads = X3 ? 384 : kThreadsTc;  // + 128 with direct operands
+  static constexpr int kOutPitch = BN + 4;  // floats per row of the staged output tile
+  static_assert(kBM * kOutPitch * 4 <= kStages * kStageBytes, "the output tile is staged in the ring");
 };
 
-template <int BN, bool A_KMAJOR, bool B_KMAJOR, int MODE, bool ATM = false>
-__global__ void __launch_bounds__(tc_threads(MODE), 1)
+// One lane's four columns of a row of the staged tile: alpha / beta / bias / ReLU / mask and the store.  VEC: four
+// consecutive columns with 16-byte (fp32) or 8-byte (bf16) accesses; else columns `stride` apart, so that the lanes of a
+// warp run along C's row either way.
+template <bool VEC>
+__device__ __forceinline__ void store_row4(const Params& p, float (&v)[4], uint64_t row_off, uint32_t col, uint32_t stride, const float (&bias)[4]) {
+  const bool relu = p.epilogue == ZG_EPI_BIAS_RELU, masked = p.epilogue == ZG_EPI_RELU_MASK;
+  float c[4] = {0.f, 0.f, 0.f, 0.f}, mk[4] = {1.f, 1.f, 1.f, 1.f};
+  if constexpr (VEC) {
+    const uint64_t o = row_off + col;
+    if (p.splits > 1 && !p.cluster) {
+      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p.C + o), "f"(p.alpha * v[0]), "f"(p.alpha * v[1]), "f"(p.alpha * v[2]), "f"(p.alpha * v[3]) : "memory");
+      return;
+    }
+    auto get4 = [&](const float* f, const __nv_bfloat16* h, float (&d)[4]) {
+      if (f) {
+        const float4 x = *reinterpret_cast<const float4*>(f + o);
+        d[0] = x.x; d[1] = x.y; d[2] = x.z; d[3] = x.w;
+      } else {
+        const uint2 u = *reinterpret_cast<const uint2*>(h + o);
+        const float2 x = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&u)[0]), y = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&u)[1]);
+        d[0] = x.x; d[1] = x.y; d[2] = y.x; d[3] = y.y;
+      }
+    };
+    if (p.beta != 0.f) get4(p.C, p.Cb, c);
+    if (masked) get4(p.mask, p.maskb, mk);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t x = col + j * stride;
+      if (x >= p.n) continue;
+      if (p.splits > 1 && !p.cluster) { atomicAdd(p.C + row_off + x, p.alpha * v[j]); continue; }
+      if (p.beta != 0.f) c[j] = p.C ? p.C[row_off + x] : __bfloat162float(p.Cb[row_off + x]);
+      if (masked) mk[j] = p.mask ? p.mask[row_off + x] : __bfloat162float(p.maskb[row_off + x]);
+    }
+    if (p.splits > 1 && !p.cluster) return;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    v[j] = p.alpha * v[j];
+    if (p.beta != 0.f) v[j] += p.beta * c[j];
+    v[j] += bias[j];
+    if (relu) v[j] = v[j] > 0.f ? v[j] : 0.f;
+    if (masked && mk[j] <= 0.f) v[j] = 0.f;
+  }
+  if constexpr (VEC) {
+    const uint64_t o = row_off + col;
+    if (p.C) {
+      *reinterpret_cast<float4*>(p.C + o) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+      uint2 u;
+      reinterpret_cast<__nv_bfloat162*>(&u)[0] = __floats2bfloat162_rn(v[0], v[1]);
+      reinterpret_cast<__nv_bfloat162*>(&u)[1] = __floats2bfloat162_rn(v[2], v[3]);
+      *reinterpret_cast<uint2*>(p.Cb + o) = u;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t x = col + j * stride;
+      if (x >= p.n) { v[j] = 0.f; continue; }
+      if (p.C) p.C[row_off + x] = v[j];
+      else p.Cb[row_off + x] = __float2bfloat16_rn(v[j]);
+    }
+  }
+}
+
+// The same for one element (r, c) of a tile that is C transposed
+__device__ __forceinline__ float store_swapped(const Params& p, float v, uint64_t o, uint32_t col, float bias) {
+  v *= p.alpha;
+  if (p.beta != 0.f) v += p.beta * (p.C ? p.C[o] : __bfloat162float(p.Cb[o]));
+  v += bias;
+  if (p.epilogue == ZG_EPI_BIAS_RELU) v = v > 0.f ? v : 0.f;
+  if (p.epilogue == ZG_EPI_RELU_MASK && (p.mask ? p.mask[o] : __bfloat162float(p.maskb[o])) <= 0.f) v = 0.f;
+  if (p.C) p.C[o] = v;
+  else p.Cb[o] = __float2bfloat16_rn(v);
+  return v;
+}
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_rank(uint32_t smem_addr, uint32_t rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ float4 ld_cluster4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float ld_cluster(uint32_t a) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+
+// A staged tile that is C transposed: rows of the tile are columns of C, lanes run along them; a rank takes every
+// ranks-th row of C.
+template <int BN, int NT>
+__device__ __forceinline__ void staged_out_swapped(const Params& p, const float* tile, uint32_t split, uint32_t c0, uint32_t r0, uint64_t batch_off) {
+  constexpr int PITCH = BN + 4;
+  const uint32_t ranks = p.cluster ? p.splits : 1, rank = p.cluster ? split : 0, r = threadIdx.x % kBM, col = c0 + r;
+  if (col >= p.n) return;
+  const float bias = (p.epilogue == ZG_EPI_BIAS || p.epilogue == ZG_EPI_BIAS_RELU) ? __ldg(p.bias + col) : 0.f;
+  const uint32_t base = smem_u32(tile);
+  float cs = 0.f;
+#pragma unroll 2
+  for (uint32_t c = rank + threadIdx.x / kBM * ranks; c < (uint32_t)BN && r0 + c < p.m; c += NT / kBM * ranks) {
+    float v = 0.f;
+    const uint32_t at = r * PITCH + c;
+    if (ranks == 1) {
+      v = tile[at];
+    } else {
+      float x[8];
+#pragma unroll
+      for (uint32_t k = 0; k < 8; ++k) x[k] = k < ranks ? ld_cluster(map_rank(base, k) + at * 4) : 0.f;
+#pragma unroll
+      for (uint32_t k = 0; k < 8; ++k) v += x[k];
+    }
+    cs += store_swapped(p, v, batch_off + (uint64_t)(r0 + c) * p.ldc + col, col, bias);
+  }
+  if (p.colsum) atomicAdd(p.colsum + col, cs);
+}
+
+// The staged tile (128 x BN floats, pitch BN + 4, all CTAs of a cluster hold partial sums) to C: NT threads, lanes along
+// the rows of C.  col_part: BN zeroed floats.
+template <int BN, int NT, bool VEC>
+__device__ __forceinline__ void staged_out(const Params& p, const float* tile, float* col_part, uint32_t split, uint32_t m0, uint32_t n0, uint64_t batch_off) {
+  constexpr int CG = BN / 4, PITCH = BN + 4;
+  const uint32_t cg = threadIdx.x % CG, ranks = p.cluster ? p.splits : 1, rank = p.cluster ? split : 0;
+  const uint32_t local = VEC ? 4 * cg : cg, stride = VEC ? 1 : CG, col = n0 + local;
+  if (col < p.n) {
+    float bias[4] = {0.f, 0.f, 0.f, 0.f}, cs[4] = {0.f, 0.f, 0.f, 0.f};
+    if (p.epilogue == ZG_EPI_BIAS || p.epilogue == ZG_EPI_BIAS_RELU) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (col + j * stride < p.n) bias[j] = __ldg(p.bias + col + j * stride);
+    }
+    const uint32_t base = smem_u32(tile);
+    for (uint32_t r = rank + threadIdx.x / CG * ranks; r < (uint32_t)kBM && m0 + r < p.m; r += NT / CG * ranks) {
+      float v[4];
+      const uint32_t at = (r * PITCH + local) * 4;
+      if (ranks == 1) {
+        if constexpr (VEC) {
+          const float4 x = *reinterpret_cast<const float4*>(tile + r * PITCH + local);
+          v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[j] = tile[r * PITCH + local + j * stride];
+        }
+      } else {
+        // every rank's values are requested before the first is added: one round trip over the cluster network
+        float4 x[8];
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+          x[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (k < ranks) {
+            const uint32_t a = map_rank(base, k) + at;
+            if constexpr (VEC) x[k] = ld_cluster4(a);
+            else { x[k].x = ld_cluster(a); x[k].y = ld_cluster(a + 4 * stride); x[k].z = ld_cluster(a + 8 * stride); x[k].w = ld_cluster(a + 12 * stride); }
+          }
+        }
+        v[0] = v[1] = v[2] = v[3] = 0.f;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) { v[0] += x[k].x; v[1] += x[k].y; v[2] += x[k].z; v[3] += x[k].w; }
+      }
+      store_row4<VEC>(p, v, batch_off + (uint64_t)(m0 + r) * p.ldc, col, stride, bias);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) cs[j] += v[j];
+    }
+    if (p.colsum) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) atomicAdd(col_part + local + j * stride, cs[j]);
+    }
+  }
+  if (p.colsum) {
+    __syncthreads();
+    if (threadIdx.x < BN && n0 + threadIdx.x < p.n) atomicAdd(p.colsum + n0 + threadIdx.x, col_part[threadIdx.x]);
+  }
+}
+
+template <int BN, bool A_KMAJOR, bool B_KMAJOR, int MODE, bool DIRECT = false>
+__global__ void __launch_bounds__((SmemLayout<BN, MODE>::kThreads + (DIRECT ? 128 : 0)), 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
                const Params p) {
-  static_assert(!ATM || MODE == kFP32X3, "A through tensor memory: FP32X3 only");
+  static_assert(!DIRECT || MODE == kFP32X3, "direct operands: FP32X3 only");
   using MT = ModeTraits<MODE>;
-  using SL = SmemLayout<BN, MODE, ATM>;
+  using SL = SmemLayout<BN, MODE>;
   constexpr int S = SL::kStages;
   constexpr bool X3 = (MODE == kFP32X3);
   // an A operand in tensor memory is K-major by construction (row m in lane m, one k element per column)
-  constexpr uint32_t kIdesc = make_idesc(MT::kBf16, ATM ? false : !A_KMAJOR, !B_KMAJOR, BN);
+  constexpr uint32_t kIdesc = make_idesc(MT::kBf16, X3 ? false : !A_KMAJOR, !B_KMAJOR, BN);
   constexpr uint32_t kTmemCols = SL::kTmemCols;
 
   extern __shared__ uint8_t smem_raw[];
@@ -505,20 +740,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   uint64_t* accum = bars + 3 * S;   // accumulator complete
   __shared__ uint32_t tmem_base_slot;
   __shared__ volatile int failed;
+  __shared__ float col_part[BN];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t tile_n = blockIdx.x, tile_m = blockIdx.y;
-  const uint32_t batch = blockIdx.z / p.splits, split = blockIdx.z % p.splits;
+  // the splits of a tile are neighbours where they form a cluster; else the tiles are, which share their slabs of A in L2
+  const uint32_t tile_n = p.cluster ? blockIdx.x / p.splits : blockIdx.x % p.tiles_n;
+  const uint32_t split = p.cluster ? blockIdx.x % p.splits : blockIdx.x / p.tiles_n, tile_m = blockIdx.y, batch = blockIdx.z;
   const uint32_t k_begin = split * p.k_per_split;
   uint32_t k_end = k_begin + p.k_per_split;
   if (k_end > p.k) k_end = p.k;
   const int KT = (k_end > k_begin) ? (int)((k_end - k_begin + MT::kBK - 1) / MT::kBK) : 0;
 
+  if (threadIdx.x < BN) col_part[threadIdx.x] = 0.f;
   if (threadIdx.x == 0) {
     failed = 0;
     for (int s = 0; s < S; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&ready[s], kSplitThreads / 32);  // one arrival per split warp
+      mbar_init(&full[s], DIRECT ? 1 + 128 : 1);  // the TMA thread, and every loader thread's copies
+      mbar_init(&ready[s], kSplitThreads / 32);  // one arrival per split warp (of the slab's set)
       mbar_init(&empty[s], 1);
     }
     mbar_init(accum, 1);
@@ -546,24 +784,51 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (kt >= S && !mbar_wait(&empty[s], ((kt / S) & 1) ^ 1, &failed)) break;
         uint8_t* st = stage_base + s * SL::kStageBytes;
         uint8_t* a_dst = st;
-        uint8_t* b_dst = st + (ATM ? SL::kABytes : SL::kABytes * MT::kBufs);
-        mbar_expect_tx(&full[s], SL::kABytes + SL::kBBytes);
+        uint8_t* b_dst = st + SL::kABytes;
+        const bool a_tma = !DIRECT || !p.a_direct, b_tma = !DIRECT || !p.b_direct;
+        mbar_expect_tx(&full[s], (a_tma ? SL::kABytes : 0) + (b_tma ? SL::kBBytes : 0));
         const int k0 = (int)k_begin + kt * MT::kBK;
-        if (A_KMAJOR) {
-          tma_load_3d(a_dst, &tmA, &full[s], k0, (int)(tile_m * kBM), za);
-        } else {
+        if (a_tma) {
+          if (A_KMAJOR) {
+            tma_load_3d(a_dst, &tmA, &full[s], k0, (int)(tile_m * kBM), za);
+          } else {
 #pragma unroll
-          for (int j = 0; j < kBM / MT::kAtomMN; ++j)
-            tma_load_3d(a_dst + j * MT::kBK * kSlabBytes, &tmA, &full[s], (int)(tile_m * kBM) + j * MT::kAtomMN, k0, za);
+            for (int j = 0; j < kBM / MT::kAtomMN; ++j)
+              tma_load_3d(a_dst + j * MT::kBK * kSlabBytes, &tmA, &full[s], (int)(tile_m * kBM) + j * MT::kAtomMN, k0, za);
+          }
         }
-        if (B_KMAJOR) {
-          tma_load_3d(b_dst, &tmB, &full[s], k0, (int)(tile_n * BN), zb);
-        } else {
+        if (b_tma) {
+          if (B_KMAJOR) {
+            tma_load_3d(b_dst, &tmB, &full[s], k0, (int)(tile_n * BN), zb);
+          } else {
 #pragma unroll
-          for (int j = 0; j < BN / MT::kAtomMN; ++j)
-            tma_load_3d(b_dst + j * MT::kBK * kSlabBytes, &tmB, &full[s], (int)(tile_n * BN) + j * MT::kAtomMN, k0, zb);
+            for (int j = 0; j < BN / MT::kAtomMN; ++j)
+              tma_load_3d(b_dst + j * MT::kBK * kSlabBytes, &tmB, &full[s], (int)(tile_n * BN) + j * MT::kAtomMN, k0, zb);
+          }
         }
       }
+    }
+  } else if (DIRECT && warp >= SL::kThreads / 32) {
+    // ------------------------------------------------- loaders of direct operands
+    // A thread's arrival on `full` is triggered by the completion of its own copies; the split warps, which read
+    // every word of B and A, order them before the tensor core's reads (fence.proxy.async before `ready`).
+    if constexpr (DIRECT) {
+      const float* a = p.a_src + (uint64_t)(batch % p.nA) * p.a_batch;
+      const float* b = p.b_src + (uint64_t)(batch % p.nB) * p.b_batch;
+      const uint32_t rows_a = p.swap ? p.n : p.m, rows_b = p.swap ? p.m : p.n;
+      for (int kt = 0; kt < KT; ++kt) {
+        const int s = kt % S;
+        if (kt >= S) {
+          const bool got = mbar_wait(&empty[s], ((kt / S) & 1) ^ 1, &failed);
+          if (!__all_sync(0xffffffffu, got)) break;
+        }
+        uint8_t* st = stage_base + s * SL::kStageBytes;
+        const uint32_t k0 = k_begin + kt * MT::kBK;
+        if (p.a_direct) direct_slab<kBM, A_KMAJOR>(st, a, p.a_ld, tile_m * kBM, rows_a, k0, p.k, p.a_src);
+        if (p.b_direct) direct_slab<BN, B_KMAJOR>(st + SL::kABytes, b, p.b_ld, tile_n * BN, rows_b, k0, p.k, p.b_src);
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[s])) : "memory");
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer
@@ -586,9 +851,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
         tc_fence_after();
         uint8_t* st = stage_base + s * SL::kStageBytes;
-        const uint32_t a_hi = smem_u32(st), a_lo = a_hi + SL::kABytes;
-        const uint32_t b_hi = a_hi + (ATM ? SL::kABytes : SL::kABytes * MT::kBufs), b_lo = b_hi + SL::kBBytes;
-        const uint32_t a_tm = tmem_d + SL::kAccCols + (uint32_t)s * SL::kATmemCols;  // ATM: hi at +0, lo at +32
+        const uint32_t a_hi = smem_u32(st);
+        const uint32_t b_hi = a_hi + SL::kABytes, b_lo = b_hi + SL::kBBytes;
+        const uint32_t a_tm = tmem_d + SL::kAccCols + (uint32_t)s * SL::kATmemCols;  // FP32X3: hi at +0, lo at +32
         // K-major: the next MMA starts 32 bytes further inside the 128-byte rows;
         // MN-major: kUmmaK k-rows (128 bytes each) further.  MN-major 32-bit
         // operands use the 32-byte-atom swizzle with 4-row groups.
@@ -598,26 +863,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         constexpr uint32_t b_lbo = B_KMAJOR ? 16u : (uint32_t)(MT::kBK * kSlabBytes);
         constexpr uint32_t a_lay = (!A_KMAJOR && !MT::kBf16) ? 1u : 2u, b_lay = (!B_KMAJOR && !MT::kBf16) ? 1u : 2u;
         constexpr uint32_t a_h32 = desc_hi32(a_lay == 1u ? 512u : 1024u, a_lay), b_h32 = desc_hi32(b_lay == 1u ? 512u : 1024u, b_lay);
-        const uint32_t da0 = desc_lo32(a_hi, a_lbo), dal0 = desc_lo32(a_lo, a_lbo);
+        const uint32_t da0 = desc_lo32(a_hi, a_lbo);
         const uint32_t db0 = desc_lo32(b_hi, b_lbo), dbl0 = desc_lo32(b_lo, b_lbo);
         if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < MT::kBK / MT::kUmmaK; ++kk) {
           const uint64_t db = desc_pack(db0 + kk * b_step, b_h32);
           const uint32_t acc = (kt > 0 || kk > 0) ? 1u : 0u;
-          if constexpr (ATM) {
+          if constexpr (X3) {
             const uint64_t dbl = desc_pack(dbl0 + kk * b_step, b_h32);
             const uint32_t ta_hi = a_tm + kk * MT::kUmmaK, ta_lo = ta_hi + 32;
             umma_tmem_a(tmem_d, ta_lo, db, kIdesc, acc);   // Alo * Bhi
             umma_tmem_a(tmem_d, ta_hi, dbl, kIdesc, 1u);   // Ahi * Blo
             umma_tmem_a(tmem_d, ta_hi, db, kIdesc, 1u);    // Ahi * Bhi
-          } else if constexpr (X3) {
-            const uint64_t da = desc_pack(da0 + kk * a_step, a_h32);
-            const uint64_t dal = desc_pack(dal0 + kk * a_step, a_h32);
-            const uint64_t dbl = desc_pack(dbl0 + kk * b_step, b_h32);
-            umma<false>(tmem_d, dal, db, kIdesc, acc);   // Alo * Bhi
-            umma<false>(tmem_d, da, dbl, kIdesc, 1u);    // Ahi * Blo
-            umma<false>(tmem_d, da, db, kIdesc, 1u);     // Ahi * Bhi
           } else {
             const uint64_t da = desc_pack(da0 + kk * a_step, a_h32);
             umma<MT::kBf16>(tmem_d, da, db, kIdesc, acc);
@@ -629,15 +887,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       }
       if (elect_one()) umma_commit(accum);
     }
-  } else if (X3) {
+  } else if constexpr (X3) {
     // ------------------------------------------- hi/lo split (warps 2..7)
     const int t = threadIdx.x - 64;
-    const bool a_warp = warp >= 4;  // ATM: the four warps that cover the TMEM lane quadrants (warp % 4)
-    constexpr int NT = kSplitThreads;
-    // Narrow tiles run the pipelined role loops below; with BN = 128 the MMAs' operand reads load the
-    // shared-memory pipe so heavily that the plain lock-step split measured faster.
-    constexpr bool PIPE = ATM && BN <= 64;
-    if (PIPE && a_warp) {
+    const bool a_warp = warp >= 4;  // the two times four warps that cover the TMEM lane quadrants (warp % 4)
+    if (a_warp) {
       // Four warps (TMEM lane quadrant = warp % 4), thread = row of the A slab.  The row's eight
       // 16-byte chunks sit at chunk position c ^ (row % 8) (128-byte swizzle); hi = the fetched
       // word itself, lo = x - tf32(x); both go to tensor memory.  The row of the NEXT slab is
@@ -648,7 +902,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       float4 v[8];
       bool have = false;
       auto load_row = [&](int stage) { load_a_row<A_KMAJOR>(stage_base + stage * SL::kStageBytes, row, v); };
-      for (int kt = 0; kt < KT; ++kt) {
+      for (int kt = warp >= 8 ? 1 : 0; kt < KT; kt += 2) {
         const int s = kt % S;
         if (!have) {
           const bool got = mbar_wait(&full[s], (kt / S) & 1, &failed);
@@ -675,7 +929,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           float4* bl = bh + SL::kBBytes / 16;
 #pragma unroll
           for (int j = 0; j < SL::kBWordsA; ++j) {
-            const int i = 64 * SL::kBWordsB + (threadIdx.x - 128) + 128 * j;
+            const int i = 64 * SL::kBWordsB + (threadIdx.x & 127) + 128 * j;
             const float4 b = bh[i];
             float4 l;
             l.x = b.x - __uint_as_float(__float_as_uint(b.x) & 0xFFFFE000u);
@@ -686,10 +940,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           }
         }
         have = false;
-        if (kt + 1 < KT) {
-          const int s1 = (kt + 1) % S;
-          have = __all_sync(0xffffffffu, mbar_test(&full[s1], ((kt + 1) / S) & 1));
-          if (have) load_row(s1);
+        if (kt + 2 < KT) {
+          const int s2 = (kt + 2) % S;
+          have = __all_sync(0xffffffffu, mbar_test(&full[s2], ((kt + 2) / S) & 1));
+          if (have) load_row(s2);
         }
         if constexpr (SL::kBWordsA > 0) fence_async_smem();
         tmem_st_wait();
@@ -697,7 +951,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         __syncwarp();
         if (lane == 0) mbar_arrive(&ready[s]);
       }
-    } else if (PIPE) {
+    } else {
       // The two other warps split B: lo = x - tf32(x) into the second B buffer of the stage.
       // Like the A warps they fetch the next slab's part before they hand this one over.
       constexpr int NB = SL::kBWordsB;  // 16-byte words per thread and slab
@@ -736,62 +990,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         __syncwarp();
         if (lane == 0) mbar_arrive(&ready[s]);
       }
-    } else
-    for (int kt = 0; kt < KT; ++kt) {
-      const int s = kt % S;
-      if (!mbar_wait(&full[s], (kt / S) & 1, &failed)) break;
-      uint8_t* st = stage_base + s * SL::kStageBytes;
-      float4* a_hi = reinterpret_cast<float4*>(st);
-      float4* a_lo = reinterpret_cast<float4*>(st + SL::kABytes);
-      float4* b_hi = reinterpret_cast<float4*>(st + (ATM ? SL::kABytes : SL::kABytes * 2));
-      float4* b_lo = b_hi + SL::kBBytes / 16;
-      if constexpr (ATM) {
-        if (a_warp) {  // thread = row of the A slab, as in the pipelined loop above
-          const int row = (warp & 3) * 32 + lane;
-          float4 va[8];
-          load_a_row<A_KMAJOR>(st, row, va);
-          uint32_t hi[32], lo[32];
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const float x[4] = {va[c].x, va[c].y, va[c].z, va[c].w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const uint32_t h = __float_as_uint(x[e]) & 0xFFFFE000u;
-              hi[4 * c + e] = __float_as_uint(x[e]);
-              lo[4 * c + e] = __float_as_uint(x[e] - __uint_as_float(h));
-            }
-          }
-          const uint32_t ta = tmem_d + SL::kAccCols + (uint32_t)s * SL::kATmemCols + ((uint32_t)((warp & 3) * 32) << 16);
-          tmem_st32(ta, hi);
-          tmem_st32(ta + 32, lo);
-          tmem_st_wait();
-          tc_fence_before();
-        }
-      }
-      // the split is position independent, so the swizzle does not matter here
-#pragma unroll 4
-      for (int i = t; i < (ATM ? 0 : SL::kABytes / 16); i += NT) {
-        const float4 v = a_hi[i];
-        float4 h, l;
-        h.x = __uint_as_float(__float_as_uint(v.x) & 0xFFFFE000u); l.x = v.x - h.x;
-        h.y = __uint_as_float(__float_as_uint(v.y) & 0xFFFFE000u); l.y = v.y - h.y;
-        h.z = __uint_as_float(__float_as_uint(v.z) & 0xFFFFE000u); l.z = v.z - h.z;
-        h.w = __uint_as_float(__float_as_uint(v.w) & 0xFFFFE000u); l.w = v.w - h.w;
-        a_lo[i] = l;
-      }
-#pragma unroll 4
-      for (int i = t; i < SL::kBBytes / 16; i += NT) {
-        const float4 v = b_hi[i];
-        float4 h, l;
-        h.x = __uint_as_float(__float_as_uint(v.x) & 0xFFFFE000u); l.x = v.x - h.x;
-        h.y = __uint_as_float(__float_as_uint(v.y) & 0xFFFFE000u); l.y = v.y - h.y;
-        h.z = __uint_as_float(__float_as_uint(v.z) & 0xFFFFE000u); l.z = v.z - h.z;
-        h.w = __uint_as_float(__float_as_uint(v.w) & 0xFFFFE000u); l.w = v.w - h.w;
-        b_lo[i] = l;
-      }
-      fence_async_smem();  // generic-proxy writes -> visible to the tensor core's async proxy
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&ready[s]);
     }
   }
 
@@ -803,9 +1001,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int q = warp - 4;  // TMEM lane quadrant
     const bool have_acc = (KT > 0) && mbar_wait(accum, 0, &failed);
     tc_fence_after();
-    const uint32_t row = tile_m * kBM + q * 32 + lane;
-    const uint64_t c_off = (uint64_t)batch * p.c_batch_stride + (uint64_t)row * p.ldc;
-    const bool row_ok = row < p.m;
     if (p.tma_epilogue && (KT == 0 || have_acc)) {
       // The stage ring is idle by now (every fetched slab was consumed by MMAs that have completed):
       // its first bytes stage the output, 4 KB per warp and chunk, 1024-byte aligned for the swizzle.
@@ -863,10 +1058,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       }
       __syncwarp();
     } else if (KT == 0 || have_acc) {
+      // Row q * 32 + lane of the tile into the idle ring: 16-byte words whose 4-bank row offset keeps the eight rows
+      // of a quarter-warp apart.
+      float* rowp = reinterpret_cast<float*>(stage_base) + (q * 32 + lane) * SL::kOutPitch;
 #pragma unroll 1
       for (int c = 0; c < BN / 32; ++c) {
-        const uint32_t col0 = tile_n * BN + c * 32;
-        if (col0 >= p.n) break;  // uniform across the warp
         uint32_t r[32];
         if (KT > 0) {
           tmem_ld32(tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 32), r);  // warp-collective
@@ -875,46 +1071,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
           for (int j = 0; j < 32; ++j) r[j] = 0u;
         }
-        epilogue_chunk(p, r, row_ok, c_off + col0, col0, lane);
-      }
-      if (p.tile_tickets) {
-        // ---- deferred epilogue of a split-K tile (warps 4-7 only: named barrier 1)
-        __shared__ int is_last;
-        __threadfence();  // this thread's reductions into C are visible device-wide
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (threadIdx.x == 128) {
-          unsigned* ticket = p.tile_tickets + ((size_t)batch * gridDim.y + tile_m) * gridDim.x + tile_n;
-          const unsigned t = atomicAdd(ticket, 1u);
-          is_last = (t == p.splits - 1) ? 1 : 0;
-          if (is_last) *ticket = 0;
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (is_last) {
-          __threadfence();
-          Params q = p;
-          q.alpha = 1.f; q.beta = 0.f; q.splits = 1; q.epilogue = p.deferred_epilogue; q.colsum = p.deferred_colsum;
-#pragma unroll 1
-          for (int c = 0; c < BN / 32; ++c) {
-            const uint32_t col0 = tile_n * BN + c * 32;
-            if (col0 >= p.n) break;
-            uint32_t r[32];
-            const uint64_t o = c_off + col0;
-            if (row_ok && p.vec_ok && col0 + 32 <= p.n) {
 #pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                const float4 v = __ldcg(reinterpret_cast<const float4*>(p.C + o) + j);
-                r[4 * j] = __float_as_uint(v.x); r[4 * j + 1] = __float_as_uint(v.y);
-                r[4 * j + 2] = __float_as_uint(v.z); r[4 * j + 3] = __float_as_uint(v.w);
-              }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) r[j] = (row_ok && col0 + j < p.n) ? __float_as_uint(__ldcg(p.C + o + j)) : 0u;
-            }
-            epilogue_chunk(q, r, row_ok, o, col0, lane);
-          }
-        }
+        for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(rowp + c * 32 + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
       }
     }
+  }
+  __syncwarp();
+  if (!p.tma_epilogue) {
+    const float* tile = reinterpret_cast<const float*>(stage_base);
+    if (p.cluster) cluster_sync(); else __syncthreads();
+    constexpr int NT = SL::kThreads + (DIRECT ? 128 : 0);
+    const uint64_t batch_off = (uint64_t)batch * p.c_batch_stride;
+    if (p.swap) staged_out_swapped<BN, NT>(p, tile, split, tile_m * kBM, tile_n * BN, batch_off);
+    else if (p.vec_ok && (p.n & 3u) == 0) staged_out<BN, NT, true>(p, tile, col_part, split, tile_m * kBM, tile_n * BN, batch_off);
+    else staged_out<BN, NT, false>(p, tile, col_part, split, tile_m * kBM, tile_n * BN, batch_off);
+    if (p.cluster) cluster_sync();  // nobody leaves while its partial tile may still be read
   }
 
   // ---------------------------------------------------------------- teardown
