@@ -71,55 +71,140 @@ __global__ void __launch_bounds__(kIThreads) gcn_scatter_bwd_kernel(const float*
   }
 }
 
-// GCN propagation over a CSR adjacency, no atomics.  A warp owns a row: its
-// lanes fetch up to 32 neighbours at once (index, degree scale and feature
-// row: the loads of a hub node's many neighbours are in flight together) and
-// park the products in shared memory, then lane j adds column j up IN EDGE
-// ORDER.  mode 0 = forward of scatter_gcn_deg_scaled with the edges grouped by
-// TARGET (row = target t, col = source s):
+// GCN propagation over a CSR adjacency, no atomics.  A warp owns a row and FW (8, 16 or 32) features at a time.  Its lanes
+// fetch index and degree scale of up to 32 neighbours at once, then 32 / FW lane groups fetch the feature rows of
+// consecutive neighbours, lanes along the features: coalesced loads, all in flight together.  The products pass
+// through shuffles so that every lane adds its feature up IN EDGE ORDER.
+// Rows of more than kHubRow neighbours (a power-law graph of 20011 nodes has one of 1170) would be a warp's serial
+// chain of round trips while everybody else is done; they are put aside and the CTA takes them together: seven warps
+// fetch products into shared memory, the eighth adds the batch before in edge order, four cycles per neighbour.
+// That graph, 16 features: 66 us a lane per neighbour, 32 with the loads of a warp together, 12 with hubs by CTA.
+//   mode 0 = forward of scatter_gcn_deg_scaled with the edges grouped by TARGET (row = target t, col = source s):
 //     out[t, j] = sum_e (deg[s] * deg[t]) * x[s, j]            (+ bias[j], ReLU)
-// mode 1 = its gradient w.r.t. h with the edges grouped by SOURCE (row = s,
-// col = t):  out[s, j] = sum_e (x[t, j] * deg[s]) * deg[t]
+//   mode 1 = its gradient w.r.t. h with the edges grouped by SOURCE (row = s, col = t):
+//     out[s, j] = sum_e (x[t, j] * deg[s]) * deg[t]
 // -- the products in the order of host_device.zig:1356-1403, the sums in edge
 // order when the CSR was built by a stable sort of the edge list, which makes
 // the result bit-identical to the host loops.
-constexpr int kCsrWarps = kIThreads / 32;
+// Feature rows of up to NE neighbours (lane e holds node c of neighbour e).  No condition between the loads: all of them
+// are in flight before the first is used (lanes past the last neighbour hold node 0, whose row is read and not added).
+template <int FW, int NE>
+__device__ __forceinline__ void csr_load(float (&v)[NE * FW / 32], const float* __restrict__ xj, size_t ld_x, uint32_t c, int g) {
+#pragma unroll
+  for (int s = 0; s < NE * FW / 32; ++s) v[s] = __ldg(xj + (size_t)__shfl_sync(0xffffffffu, c, s * (32 / FW) + g) * ld_x);
+}
+template <int FW, int NE>
+__device__ __forceinline__ float csr_add(float acc, float (&v)[NE * FW / 32], float dc, float dr, int nk, int mode, int g, int jl) {
+  constexpr int G = 32 / FW, N = NE / G;  // neighbours per step, steps
+  float p[N][G];
+#pragma unroll
+  for (int s = 0; s < N; ++s) {
+    const float de = __shfl_sync(0xffffffffu, dc, s * G + g);
+    v[s] = mode == 0 ? (de * dr) * v[s] : (v[s] * dr) * de;
+  }
+#pragma unroll
+  for (int s = 0; s < N; ++s)
+#pragma unroll
+    for (int e = 0; e < G; ++e) p[s][e] = __shfl_sync(0xffffffffu, v[s], e * FW + jl);
+#pragma unroll
+  for (int s = 0; s < N; ++s)
+#pragma unroll
+    for (int e = 0; e < G; ++e)
+      if (s * G + e < nk) acc += p[s][e];
+  return acc;
+}
 
+constexpr int kHubRow = 64, kHubQueue = 64, kGatherWarps = kIThreads / 32 - 1;
+
+template <int FW>
 __global__ void __launch_bounds__(kIThreads) csr_gcn_propagate_kernel(float* out, const float* __restrict__ x, const float* __restrict__ deg,
                                                                       const len_t* __restrict__ row_ptr, const len_t* __restrict__ col,
                                                                       size_t n_rows, size_t F, size_t ld_x, size_t ld_out, int mode,
                                                                       int epilogue, const float* __restrict__ bias) {
-  __shared__ float prod[kCsrWarps][32][33];  // [neighbour of the chunk][feature of the tile], padded: both access patterns conflict-free
+  constexpr int EW = FW == 32 ? 16 : 32, kBatch = kGatherWarps * EW;  // neighbours per gathering warp, per batch
+  __shared__ float batch[2][kBatch][FW];
+  __shared__ uint32_t queue[kHubQueue];
+  __shared__ unsigned queued;
+  if (threadIdx.x == 0) queued = 0;
+  __syncthreads();
   pdl_sync();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane / FW, jl = lane % FW;
   const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
+  auto store = [&](size_t r, size_t j, float acc) {
+    if (epilogue == ZG_EPI_BIAS || epilogue == ZG_EPI_BIAS_RELU) acc += bias[j];
+    if (epilogue == ZG_EPI_BIAS_RELU) acc = acc > 0.f ? acc : 0.f;
+    out[r * ld_out + j] = acc;
+  };
   for (size_t r = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n_rows; r += warps) {
-    const len_t k0 = row_ptr[r], k1 = row_ptr[r + 1];
-    const float dr = deg[r];
-    for (size_t j0 = 0; j0 < F; j0 += 32) {
-      const int fw = (int)((F - j0) < 32 ? (F - j0) : 32);
-      float acc = 0.f;  // lane j < fw: feature j0 + j
+    const len_t k0 = __ldg(row_ptr + r), k1 = __ldg(row_ptr + r + 1);
+    if (k1 - k0 > kHubRow) {
+      unsigned at = 0;
+      if (lane == 0) at = atomicAdd(&queued, 1u);
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (at < kHubQueue) {
+        if (lane == 0) queue[at] = (uint32_t)r;
+        continue;
+      }
+    }
+    const float dr = __ldg(deg + r);
+    for (size_t j0 = 0; j0 < F; j0 += FW) {
+      const bool jok = j0 + jl < F;
+      const float* xj = x + j0 + (jok ? jl : 0);
+      float acc = 0.f;
       for (len_t kc = k0; kc < k1; kc += 32) {
         const int nk = (int)((k1 - kc) < 32 ? (k1 - kc) : 32);
-        if (lane < nk) {
-          const size_t c = col[kc + lane];
-          const float dc = deg[c];
-          const float* xr = x + c * ld_x + j0;
-          for (int j = 0; j < fw; ++j) {
-            const float v = xr[j];
-            prod[warp][lane][j] = mode == 0 ? (dc * dr) * v : (v * dr) * dc;
+        const uint32_t c = lane < nk ? (uint32_t)__ldg(col + kc + lane) : 0u;
+        const float dc = __ldg(deg + c);
+        if (nk > 16) { float v[FW]; csr_load<FW, 32>(v, xj, ld_x, c, g); acc = csr_add<FW, 32>(acc, v, dc, dr, nk, mode, g, jl); }
+        else if (nk > 4) { float v[FW / 2]; csr_load<FW, 16>(v, xj, ld_x, c, g); acc = csr_add<FW, 16>(acc, v, dc, dr, nk, mode, g, jl); }
+        else { float v[FW / 8]; csr_load<FW, 4>(v, xj, ld_x, c, g); acc = csr_add<FW, 4>(acc, v, dc, dr, nk, mode, g, jl); }
+      }
+      if (jok && g == 0) store(r, j0 + jl, acc);
+    }
+  }
+  __syncthreads();
+  const unsigned hubs = queued < kHubQueue ? queued : kHubQueue;
+  for (unsigned h = 0; h < hubs; ++h) {
+    const size_t r = queue[h];
+    const len_t k0 = __ldg(row_ptr + r), k1 = __ldg(row_ptr + r + 1);
+    const float dr = __ldg(deg + r);
+    for (size_t j0 = 0; j0 < F; j0 += FW) {
+      const bool jok = j0 + jl < F;
+      const float* xj = x + j0 + (jok ? jl : 0);
+      float acc = 0.f;
+      const len_t rounds = (k1 - k0 + kBatch - 1) / kBatch;
+      for (len_t i = 0; i <= rounds; ++i) {
+        if (warp > 0) {
+          const len_t kc = k0 + i * kBatch + (warp - 1) * EW;
+          if (i < rounds && kc < k1) {
+            const uint32_t c = (lane < EW && kc + lane < k1) ? (uint32_t)__ldg(col + kc + lane) : 0u;
+            const float dc = __ldg(deg + c);
+            constexpr int N = EW * FW / 32, G = 32 / FW;
+            float v[N];
+            csr_load<FW, EW>(v, xj, ld_x, c, g);
+#pragma unroll
+            for (int s = 0; s < N; ++s) {
+              const float de = __shfl_sync(0xffffffffu, dc, s * G + g);
+              batch[i & 1][(warp - 1) * EW + s * G + g][jl] = mode == 0 ? (de * dr) * v[s] : (v[s] * dr) * de;
+            }
           }
+        } else if (i > 0) {
+          const len_t left = k1 - k0 - (i - 1) * kBatch;
+          const int n = left < (len_t)kBatch ? (int)left : kBatch;
+          const float* b = &batch[(i - 1) & 1][0][jl];
+          int e = 0;
+          for (; e + 16 <= n; e += 16) {
+            float p[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) p[u] = b[(e + u) * FW];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) acc += p[u];
+          }
+          for (; e < n; ++e) acc += b[e * FW];
         }
-        __syncwarp();
-        if (lane < fw)
-          for (int l = 0; l < nk; ++l) acc += prod[warp][l][lane];
-        __syncwarp();
+        __syncthreads();
       }
-      if (lane < fw) {
-        if (epilogue == ZG_EPI_BIAS || epilogue == ZG_EPI_BIAS_RELU) acc += bias[j0 + lane];
-        if (epilogue == ZG_EPI_BIAS_RELU) acc = acc > 0.f ? acc : 0.f;
-        out[r * ld_out + j0 + lane] = acc;
-      }
+      if (warp == 0 && jok && g == 0) store(r, j0 + jl, acc);
     }
   }
 }
@@ -251,7 +336,10 @@ extern "C" void zg_csr_gcn_propagate(dtype id, StreamWrapper w, void* out, const
   if (n_rows == 0 || n_feat == 0) return;
   if (epilogue != ZG_EPI_NONE && epilogue != ZG_EPI_BIAS && epilogue != ZG_EPI_BIAS_RELU) { set_error(kBadArgument, "zg_csr_gcn_propagate: epilogue %d", epilogue); return; }
   if (epilogue != ZG_EPI_NONE && !bias) { set_error(kBadArgument, "zg_csr_gcn_propagate: bias epilogue without bias"); return; }
-  launch_pdl(csr_gcn_propagate_kernel, dim3(grid_for(n_rows, kCsrWarps)), dim3(kIThreads), 0, as_stream(w), (float*)out, (const float*)x,
+  if (n_rows > 0xffffffffu) { set_error(kBadArgument, "zg_csr_gcn_propagate: %lu rows", n_rows); return; }
+  // lane groups as wide as the feature row: 8 features take 4 neighbours per step, 32 one
+  auto kern = n_feat <= 8 ? csr_gcn_propagate_kernel<8> : (n_feat <= 16 ? csr_gcn_propagate_kernel<16> : csr_gcn_propagate_kernel<32>);
+  launch_pdl(kern, dim3(grid_for(n_rows, kIThreads / 32)), dim3(kIThreads), 0, as_stream(w), (float*)out, (const float*)x,
              (const float*)deg, row_ptr, col_idx, (size_t)n_rows, (size_t)n_feat, (size_t)ld_x, (size_t)ld_out, transpose_form ? 1 : 0, epilogue,
              (const float*)bias);
 }
