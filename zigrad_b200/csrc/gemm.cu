@@ -75,10 +75,20 @@ static void launch_block(cudaStream_t s, const void* A, const void* B, void* C, 
   p.ta = ta; p.tb = tb; p.alpha = alpha; p.beta = beta; p.epilogue = epilogue;
   p.bias = static_cast<const float*>(bias); p.mask = mask; p.colsum = static_cast<float*>(colsum);
   const size_t t64 = ((m + 63) / 64) * ((n + 63) / 64) * nC, t32 = ((m + 31) / 32) * ((n + 31) / 32) * nC;
-  // 64 x 64 tiles (half the copies per multiply-add) once there is one for every SM; below that, parallelism counts
-  // for more: 1000x301x501 takes 21 us with 32 x 32, 30 with 64 x 64; 4096x1023x1023 379 and 280
-  if (t64 > (size_t)sm_count()) launch_block_inst<TI, TC, 64, 64, 8>(s, A, B, C, p, nC, 1);
-  else launch_block_inst<TI, TC, 32, 32, 4>(s, A, B, C, p, nC, block_splits(t32, k));
+  if constexpr (sizeof(TI) == 8) {
+    // The tile whose busiest SM has the least to do (an SM holds two CTAs of any of them; a 64 x 64 tile costs about 5 %
+    // less per multiply-add than a 64 x 32 one), split over clusters while SMs are left over.
+    const size_t t6432 = ((m + 63) / 64) * ((n + 31) / 32) * nC, sms = (size_t)sm_count();
+    const double w64 = (double)((t64 + sms - 1) / sms) * 4.0, w6432 = (double)((t6432 + sms - 1) / sms) * 2.1;
+    if (t64 * 2 <= sms) launch_block_inst<TI, TC, 32, 32, 0>(s, A, B, C, p, nC, block_splits(t32, k));
+    else if (w64 <= w6432) launch_block_inst<TI, TC, 64, 64, 0>(s, A, B, C, p, nC, 1);
+    else launch_block_inst<TI, TC, 64, 32, 0>(s, A, B, C, p, nC, 1);
+  } else {
+    // 64 x 64 tiles (half the copies per multiply-add) once there is one for every SM; below that, parallelism counts
+    // for more: 1000x301x501 takes 21 us with 32 x 32, 30 with 64 x 64; 4096x1023x1023 379 and 280
+    if (t64 > (size_t)sm_count()) launch_block_inst<TI, TC, 64, 64, 8>(s, A, B, C, p, nC, 1);
+    else launch_block_inst<TI, TC, 32, 32, 4>(s, A, B, C, p, nC, block_splits(t32, k));
+  }
 }
 
 // =====================================================================

@@ -48,15 +48,17 @@ struct Params {
   int epilogue;
 };
 
-// Tile TM x TN of C per cluster, MI x MI outputs per thread: TM * TN / MI^2 threads make one k group.
+// Tile TM x TN of C per cluster.  MI x MI outputs per thread: TM * TN / MI^2 threads make one k group.  MI == 0: fp64 on
+// the tensor cores, 32 x 32 outputs per warp.
 template <typename TI, int TM, int TN, int MI>
 struct Layout {
   using AT = typename Acc<TI>::type;
-  static constexpr int kGroupThreads = TM * TN / (MI * MI);
+  static constexpr int kGroupThreads = MI ? TM * TN / (MI * MI + (MI == 0)) : TM * TN / 32;
   static constexpr int KG = kThreads / kGroupThreads;
   static constexpr int TK = sizeof(AT) == 8 ? 32 : 64;  // k depth of a stage
   static constexpr int kPerGroup = TK / KG;
-  static constexpr int kPadA = TM + 4, kPadB = TN + 4;  // 16-byte aligned rows; 8 k x 4 rows of a copy hit 32 banks
+  // 16-byte aligned rows; 8 k x 4 rows of a copy hit 32 banks, and so do the 4 k x 8 rows of an fp64 fragment
+  static constexpr int kPadA = TM + 4, kPadB = TN + 4;
   static constexpr int kStageElems = TK * (kPadA + kPadB);
   static constexpr int kStages = sizeof(TI) < 4 ? 2 : 3;
   static constexpr size_t kRedBytes = (size_t)KG * TM * TN * sizeof(AT);
@@ -127,8 +129,15 @@ __device__ __forceinline__ void load4(const T* p, T (&v)[4]) {
   }
 }
 
+// D (8 x 8) += A (8 x 4) * B (4 x 8) in fp64: lane l holds A[l / 4][l % 4], B[l % 4][l / 4] and D[l / 4][2 (l % 4)], [.. + 1].
+// Against DFMA it halves the shared-memory reads per multiply-add, which is what bounded the fp64 tiles:
+// 4 x 500x389x640 89 -> 54 us (105 on the kernel before).
+__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
+}
+
 template <typename TI, typename TC, int TM, int TN, int MI>
-__global__ void __launch_bounds__(kThreads) gemm_block_kernel(const TI* __restrict__ A, const TI* __restrict__ B, TC* C, const Params p) {
+__global__ void __launch_bounds__(kThreads, MI == 0 ? 2 : 1) gemm_block_kernel(const TI* __restrict__ A, const TI* __restrict__ B, TC* C, const Params p) {
   using L = Layout<TI, TM, TN, MI>;
   using AT = typename L::AT;
   constexpr int KG = L::KG, TK = L::TK, S = L::kStages;
@@ -202,12 +211,22 @@ __global__ void __launch_bounds__(kThreads) gemm_block_kernel(const TI* __restri
 
   const int group = threadIdx.x / L::kGroupThreads, gt = threadIdx.x % L::kGroupThreads;
   // rows ty * 4 + (i / 4) * TM / 2 + i % 4, columns likewise: 16-byte reads, consecutive threads on consecutive words
-  const int tx = gt % (TN / MI), ty = gt / (TN / MI);
-  AT acc[MI][MI];
+  constexpr int MIN = MI ? MI : 4;  // (fp64: 4 x 4 blocks of 8 x 8 per warp)
+  const int tx = MI ? gt % (TN / MIN) : gt / 32 % (TN / 32), ty = MI ? gt / (TN / MIN) : gt / 32 / (TN / 32);
+  const int lane = threadIdx.x & 31;
+  AT acc[MI ? MIN : 1][MI ? MIN : 1];
+  double dacc[MI ? 1 : 4][MI ? 1 : 4][2];
+  if constexpr (MI == 0) {
 #pragma unroll
-  for (int i = 0; i < MI; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < MI; ++j) acc[i][j] = AT(0);
+      for (int j = 0; j < 4; ++j) dacc[i][j][0] = dacc[i][j][1] = 0.0;
+  } else {
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+      for (int j = 0; j < MI; ++j) acc[i][j] = AT(0);
+  }
 
   pdl_sync();
   if constexpr (kAsync) {
@@ -222,26 +241,44 @@ __global__ void __launch_bounds__(kThreads) gemm_block_kernel(const TI* __restri
     if constexpr (kAsync) copy_wait<S - 2>();
     __syncthreads();  // slab c has landed; everyone is done with slab c - 1, whose stage the next copy reuses
     if constexpr (kAsync) issue(c + S - 1);
-    const AT* as = ring + (c % S) * L::kStageElems + group * L::kPerGroup * L::kPadA + ty * 4;
-    const AT* bs = ring + (c % S) * L::kStageElems + TK * L::kPadA + group * L::kPerGroup * L::kPadB + tx * 4;
+    const AT* as = ring + (c % S) * L::kStageElems + group * L::kPerGroup * L::kPadA + ty * (MI ? 4 : 32);
+    const AT* bs = ring + (c % S) * L::kStageElems + TK * L::kPadA + group * L::kPerGroup * L::kPadB + tx * (MI ? 4 : 32);
     const int left = depth - c * TK - group * L::kPerGroup;
-    auto mac = [&](int kk) {
-      AT av[MI], bv[MI];
+    if constexpr (MI == 0) {
+      if (left > 0) {  // the slab is padded with zeros
 #pragma unroll
-      for (int h = 0; h < MI / 4; ++h) {
-        load4(as + kk * L::kPadA + h * (TM / 2), *reinterpret_cast<AT(*)[4]>(av + 4 * h));
-        load4(bs + kk * L::kPadB + h * (TN / 2), *reinterpret_cast<AT(*)[4]>(bv + 4 * h));
+        for (int kk = 0; kk < L::kPerGroup; kk += 4) {
+          double av[4], bv[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            av[i] = as[(kk + lane % 4) * L::kPadA + 8 * i + lane / 4];
+            bv[i] = bs[(kk + lane % 4) * L::kPadB + 8 * i + lane / 4];
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) mma_f64(dacc[i][j], av[i], bv[j]);
+        }
       }
-#pragma unroll
-      for (int i = 0; i < MI; ++i)
-#pragma unroll
-        for (int j = 0; j < MI; ++j) acc[i][j] += av[i] * bv[j];
-    };
-    if (left >= L::kPerGroup) {
-#pragma unroll
-      for (int kk = 0; kk < L::kPerGroup; ++kk) mac(kk);
     } else {
-      for (int kk = 0; kk < left; ++kk) mac(kk);
+      auto mac = [&](int kk) {
+        AT av[MIN], bv[MIN];
+#pragma unroll
+        for (int h = 0; h < MI / 4; ++h) {
+          load4(as + kk * L::kPadA + h * (TM / 2), *reinterpret_cast<AT(*)[4]>(av + 4 * h));
+          load4(bs + kk * L::kPadB + h * (TN / 2), *reinterpret_cast<AT(*)[4]>(bv + 4 * h));
+        }
+#pragma unroll
+        for (int i = 0; i < MI; ++i)
+#pragma unroll
+          for (int j = 0; j < MI; ++j) acc[i][j] += av[i] * bv[j];
+      };
+      if (left >= L::kPerGroup) {
+#pragma unroll
+        for (int kk = 0; kk < L::kPerGroup; ++kk) mac(kk);
+      } else {
+        for (int kk = 0; kk < left; ++kk) mac(kk);
+      }
     }
     if constexpr (!kAsync) {
       if (c + 1 < chunks) park(c + 1);  // the other stage: its readers passed the barrier above
@@ -254,11 +291,19 @@ __global__ void __launch_bounds__(kThreads) gemm_block_kernel(const TI* __restri
   if constexpr (kAsync) copy_wait<0>();
   __syncthreads();
   AT* red = ring;
+  if constexpr (MI == 0) {
 #pragma unroll
-  for (int i = 0; i < MI; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < MI; ++j)
-      red[(group * TM + ty * 4 + (i / 4) * (TM / 2) + i % 4) * TN + tx * 4 + (j / 4) * (TN / 2) + j % 4] = acc[i][j];
+      for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<double2*>(&red[(group * TM + ty * 32 + 8 * i + lane / 4) * TN + tx * 32 + 8 * j + lane % 4 * 2]) = make_double2(dacc[i][j][0], dacc[i][j][1]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+      for (int j = 0; j < MI; ++j)
+        red[(group * TM + ty * 4 + (i / 4) * (TM / 2) + i % 4) * TN + tx * 4 + (j / 4) * (TN / 2) + j % 4] = acc[i][j];
+  }
   if (threadIdx.x < TN) col_part[threadIdx.x] = 0.f;
   __syncthreads();
   AT sum[kOut];
