@@ -57,6 +57,8 @@ EXTERN_C void zg_host_free_pinned(void* hptr);
 /* Number of kernel nodes in a saved capture (cuda_utils.h: open_capture /
  * save_capture): what one run_capture launches. */
 EXTERN_C len_t zg_capture_kernel_count(GraphWrapper graph);
+/* 1 while `stream` is being captured (by this library or by anyone else). */
+EXTERN_C int zg_stream_capturing(StreamWrapper stream);
 
 /* --------------------------------------------------------------- math mode
  * How SINGLE-precision GEMMs use the tensor cores:

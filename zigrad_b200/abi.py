@@ -175,6 +175,7 @@ SIGNATURES = {
     "zg_device_available": (i32, []),
     "zg_set_device": (None, [C.c_uint]),
     "zg_capture_kernel_count": (len_t, [GraphWrapper]),
+    "zg_stream_capturing": (i32, [S]),
     "zg_set_math_mode": (None, [i32]),
     "zg_get_math_mode": (i32, []),
     "zg_bmm_sm_budget": (None, [i32]),

@@ -536,6 +536,11 @@ extern "C" void run_capture(GraphWrapper graph, StreamWrapper stream) {
   ZG_CUDA(cudaGraphLaunch(b->exec, as_stream(stream)));
 }
 
+extern "C" int zg_stream_capturing(StreamWrapper stream) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(as_stream(stream), &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
+}
+
 extern "C" len_t zg_capture_kernel_count(GraphWrapper graph) {
   GraphBackend* b = static_cast<GraphBackend*>(graph.ptr);
   if (!b || !b->graph) return 0;

@@ -135,6 +135,8 @@ class CudaDevice:
         self._side = None  # second stream for branches of independent work, created on first use
         self._sides = {}   # further side streams by index (branch(k), k >= 1)
         self._forked = []  # side streams used since the last join()
+        self.main_stream = self.stream  # what `stream` is outside a branch() block
+        self.replaying = False  # a GraphCache (replay.py) is issuing a step
         abi.check()
 
     # ------------------------------------------------------------ lifecycle

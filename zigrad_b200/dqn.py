@@ -22,6 +22,7 @@ from . import opspec
 from .abi import SINGLE
 from .device import USIZE, CudaDevice, DeviceSlice
 from .mlp import MlpTrainer
+from .replay import GraphCache
 
 
 class DqnTrainer:
@@ -42,9 +43,24 @@ class DqnTrainer:
         self.gamma_s = d.from_numpy(np.array([gamma], np.float32))
         self.one_s = d.from_numpy(np.array([1.0], np.float32))
         self.loss = d.mem_cache_alloc(SINGLE, 1)
+        self._graphs = GraphCache(d)  # repeated steps (replay.py)
 
     def step(self, states: DeviceSlice, actions: DeviceSlice, next_states: DeviceSlice, rewards: DeviceSlice,
              dones: DeviceSlice):
+        p = self.policy
+        key = (states.ptr, actions.ptr, next_states.ptr, rewards.ptr, dones.ptr, self.gamma, self.tau, self.q_clip, p.lr, p.opt, p.beta1,
+               p.beta2, p.eps, p.clip, p.max_norm, p.delta, self.target._grads_clear, p._grads_clear)
+        self._graphs.run(key, lambda: self._step(states, actions, next_states, rewards, dones), self._host_state, self._set_host_state)
+
+    def _host_state(self):
+        return self.policy._host_state() + self.target._host_state()
+
+    def _set_host_state(self, state):
+        half = len(state) // 2
+        self.policy._set_host_state(state[:half])
+        self.target._set_host_state(state[half:])
+
+    def _step(self, states: DeviceSlice, actions: DeviceSlice, next_states: DeviceSlice, rewards: DeviceSlice, dones: DeviceSlice):
         d, B, C, qc = self.dev, self.B, self.C, self.q_clip
         pol, tgt = self.policy, self.target
         # ---- targets (gradients disabled in the reference): a chain of small kernels that does not depend
@@ -81,6 +97,7 @@ class DqnTrainer:
     def free(self):
         d = self.dev
         d.sync()
+        self._graphs.clear()
         for s in (self.maxq, self.tmp, self.targets, self.q, self.dq, self.offsets, self.gamma_s, self.one_s, self.loss):
             d.mem_cache_free(s)
         self.policy.free()

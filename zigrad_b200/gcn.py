@@ -24,6 +24,7 @@ import numpy as np
 from . import opspec
 from .abi import SINGLE
 from .device import USIZE, CudaDevice, DeviceSlice
+from .replay import GraphCache
 
 
 def _pad4(n: int) -> int:
@@ -90,6 +91,7 @@ class GcnTrainer:
         offs = (np.asarray(mask_idx, np.uint64)[:, None] * np.uint64(Cp) + np.arange(Cp, dtype=np.uint64)[None, :]).ravel()
         self.offsets = d.from_numpy(np.ascontiguousarray(offs, np.uint64))
         self.loss = alloc(1)
+        self._graphs = GraphCache(d)  # repeated steps (replay.py)
         d.sync()
 
     def _mm(self, A, B, Cbuf, m, n, k, ta, tb, lda, ldb, ldc, beta=0.0, epilogue="none", bias=None, mask=None, colsum=None):
@@ -107,6 +109,13 @@ class GcnTrainer:
 
     def step(self, T_masked: DeviceSlice):
         """T_masked: one-hot targets of the masked rows, fp32 [M, C] contiguous."""
+        key = (T_masked.ptr, T_masked.dtype, self.opt, self.lr, self.beta1, self.beta2, self.eps, self.clip, self.max_norm, self.delta)
+        self._graphs.run(key, lambda: self._step(T_masked), lambda: (self.t,), self._set_t)
+
+    def _set_t(self, state):
+        (self.t,) = state
+
+    def _step(self, T_masked: DeviceSlice):
         d, N, F, H, C, Fp, Cp, M = self.dev, self.N, self.F, self.H, self.C, self.Fp, self.Cp, self.M
         # zero_grad (model.zig:49-54) and the zero gradient the MaskLayer backward scatters into: nothing in
         # the forward pass needs them, so the two fills run on a side stream beside it
@@ -154,6 +163,7 @@ class GcnTrainer:
     def free(self):
         d = self.dev
         d.sync()
+        self._graphs.clear()
         extra = list(self.csr) + [self.deg] if self.sparse else [self.A]
         for s in extra + [self.X, self.params, self.grads, self.m, self.v, self.norms, self.h1, self.a1, self.h2, self.logits,
                   self.dlog, self.dh2, self.da1, self.dh1, self.mlog, self.dm, self.offsets, self.loss, self.t_dev]:

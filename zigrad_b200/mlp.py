@@ -39,6 +39,7 @@ import numpy as np
 from . import opspec
 from .abi import BF16, SINGLE
 from .device import CudaDevice, DeviceSlice
+from .replay import GraphCache
 
 
 def kaiming_uniform(dims: Sequence[int], seed: int):
@@ -107,12 +108,14 @@ class MlpTrainer:
         self.n_params = off
         d = dev
         self.params = d.mem_cache_alloc(SINGLE, off)
-        self.grads = d.mem_cache_alloc(SINGLE, off)
+        self._grads = d.mem_cache_alloc(SINGLE, off)
         self.norms = d.mem_cache_alloc(SINGLE, len(self.segments))
         flat = np.concatenate([np.concatenate([np.asarray(w, np.float32).ravel(), np.asarray(b, np.float32).ravel()])
                                for w, b in zip(weights, biases)])
         d.mem_transfer_htod(flat, self.params)
-        d.mem_fill(self.grads, 0.0)
+        d.mem_fill(self._grads, 0.0)
+        self._zero_due = False  # zero_grad was asked for by a forward pass and has not been issued yet
+        self._graphs = GraphCache(d)  # repeated steps (replay.py)
         if opt == "adam":
             self.m, self.v = d.mem_cache_alloc(SINGLE, off), d.mem_cache_alloc(SINGLE, off)
             d.mem_fill(self.m, 0.0)
@@ -121,8 +124,8 @@ class MlpTrainer:
             self.t_dev = d.from_numpy(np.zeros(1, np.uint64))
         self.W = [self.params.view(self.segments[2 * l][0], self.segments[2 * l][1]) for l in range(self.L)]
         self.b = [self.params.view(self.segments[2 * l + 1][0], self.segments[2 * l + 1][1]) for l in range(self.L)]
-        self.dW = [self.grads.view(self.segments[2 * l][0], self.segments[2 * l][1]) for l in range(self.L)]
-        self.db = [self.grads.view(self.segments[2 * l + 1][0], self.segments[2 * l + 1][1]) for l in range(self.L)]
+        self._dW = [self._grads.view(self.segments[2 * l][0], self.segments[2 * l][1]) for l in range(self.L)]
+        self._db = [self._grads.view(self.segments[2 * l + 1][0], self.segments[2 * l + 1][1]) for l in range(self.L)]
         # activations and their gradients.  bf16 mode: hidden activations and all
         # backward operands are bf16, logits / loss / parameter gradients fp32.
         act_t = BF16 if bf16 else SINGLE
@@ -146,18 +149,50 @@ class MlpTrainer:
             self.dlogits_bf16 = d.mem_cache_alloc(BF16, self.B * self.ld_out)
         d.sync()
 
+    # -------------------------------------------------------------- gradients
+    def _settle(self):
+        """Issue the zero_grad that is due (model.zig:57-62) as ONE fill of the flat gradient buffer."""
+        if self._zero_due:
+            self._zero_due = False
+            self.dev.mem_fill(self._grads, 0.0)
+
+    @property
+    def grads(self) -> DeviceSlice:
+        self._settle()
+        return self._grads
+
+    @property
+    def dW(self) -> List[DeviceSlice]:
+        self._settle()
+        return self._dW
+
+    @property
+    def db(self) -> List[DeviceSlice]:
+        self._settle()
+        return self._db
+
     # ------------------------------------------------------------------ pieces
     def forward(self, X: DeviceSlice):
+        if not self.fused:
+            return self._forward(X)
+        self._graphs.run(("forward", X.ptr, X.dtype), lambda: self._forward(X), self._host_state, self._set_host_state)
+        return self.act[-1]
+
+    def _host_state(self):
+        return self.t, self._grads_clear, self._zero_due
+
+    def _set_host_state(self, state):
+        self.t, self._grads_clear, self._zero_due = state
+
+    def _forward(self, X: DeviceSlice):
         d, B = self.dev, self.B
         inp = X
         if self.fused:
-            # zero_grad (model.zig:57-62) as ONE fill of the flat gradient buffer; the
-            # weight-gradient GEMMs then accumulate with beta = 1 as the reference does
-            # (kept on the main stream: as a side branch joined after the forward pass it
-            # cost more in extra graph dependencies than the 2.5 us it hides).  With
-            # zero_grads_in_update the previous step's SGD kernel has cleared them already.
-            if not self._grads_clear:
-                d.mem_fill(self.grads, 0.0)
+            # zero_grad is due from here on (the weight-gradient GEMMs accumulate with beta = 1 as the reference
+            # does) and issued when the first gradient is about to be written or somebody looks: a forward pass
+            # alone does not pay for it.  With zero_grads_in_update the previous step's SGD kernel has
+            # cleared the gradients already.
+            self._zero_due = self._zero_due or not self._grads_clear
             self._grads_clear = False
         for l in range(self.L):
             K, N = self.dims[l], self.dims[l + 1]
@@ -176,11 +211,12 @@ class MlpTrainer:
 
     def loss_and_grad(self, T: DeviceSlice):
         d, B, C = self.dev, self.B, self.dims[-1]
+        self._settle()
         if not self.fused:
             d.mem_fill(self.dact[-1], 0.0)  # ensure_grad(0), then `+=`
         if self.fused:  # the bias gradient of the last layer comes out of the same pass
             d.dispatch(opspec.softmax_ce(self.act[-1], T, B, C, self.loss, self.dact[-1], self.loss_div, accumulate=False,
-                                         ld=self.ld_out, bias_grad=self.db[-1]))
+                                         ld=self.ld_out, bias_grad=self._db[-1]))
         else:
             d.dispatch(opspec.softmax_ce(self.act[-1], T, B, C, self.loss, self.dact[-1], self.loss_div, accumulate=True))
 
@@ -203,10 +239,11 @@ class MlpTrainer:
         wide MLP the update then competes with the persistent GEMMs for memory bandwidth
         and the step got slower (2.39 ms against 2.27 ms with one update after the join)."""
         d, B = self.dev, self.B
+        self._settle()
         if self.fused and not last_bias_done:
             if self.ld_out != self.dims[-1]:
                 raise ValueError("an external output gradient needs unpadded logits (pad_logits=False)")
-            d.dispatch(opspec.unbroadcast(self.dact[-1], [B, self.dims[-1]], self.db[-1], [self.dims[-1]], None, 1.0, 0.0))
+            d.dispatch(opspec.unbroadcast(self.dact[-1], [B, self.dims[-1]], self._db[-1], [self.dims[-1]], None, 1.0, 0.0))
         for l in range(self.L - 1, -1, -1):
             K, N = self.dims[l], self.dims[l + 1]
             a_in = X if l == 0 else self.act[l - 1]
@@ -224,26 +261,26 @@ class MlpTrainer:
                 # stream (a parallel branch of a captured step), forked here where dY
                 # is ready, and runs next to this layer's dX GEMM.
                 with d.branch():
-                    d.dispatch(opspec.linear(dy, a_in, self.dW[l], N, K, B, True, False, ldy, K, K, 1.0, 1.0))
+                    d.dispatch(opspec.linear(dy, a_in, self._dW[l], N, K, B, True, False, ldy, K, K, 1.0, 1.0))
                     if on_layer_grads is not None:
                         on_layer_grads(l)
                 if l > 0:  # dX = dY . W, zeroed where the previous activation is <= 0
                     W = self.Wb[l] if self.bf16 else self.W[l]
                     d.dispatch(opspec.linear(dy, W, self.dact[l - 1], B, K, N, False, False, ldy, K, K, 1.0, 0.0,
-                                             "relu_mask", None, self.act[l - 1], colsum=self.db[l - 1]))
+                                             "relu_mask", None, self.act[l - 1], colsum=self._db[l - 1]))
                 if update_by_layer:
                     with d.branch(1, after=(0,)):
                         self._adam_layer(l, last=(l == 0))
             else:
                 if l + 1 < self.L:
                     d.dispatch(opspec.relu_inplace_bwd(self.act[l], dy))
-                d.mem_fill(self.db[l], 0.0)
-                d.dispatch(opspec.unbroadcast(dy, [B, N], self.db[l], [N], None, 1.0, 1.0))
+                d.mem_fill(self._db[l], 0.0)
+                d.dispatch(opspec.unbroadcast(dy, [B, N], self._db[l], [N], None, 1.0, 1.0))
                 if l > 0:
                     d.mem_fill(self.dact[l - 1], 0.0)
                     d.dispatch(opspec.bmm_acc(dy, self.W[l], self.dact[l - 1], (1, B, N), (1, N, K), (1, B, K), False, False, N, K, K, 1.0, 1.0))
-                d.mem_fill(self.dW[l], 0.0)
-                d.dispatch(opspec.bmm_acc(dy, a_in, self.dW[l], (1, N, B), (1, B, K), (1, N, K), True, False, N, K, K, 1.0, 1.0))
+                d.mem_fill(self._dW[l], 0.0)
+                d.dispatch(opspec.bmm_acc(dy, a_in, self._dW[l], (1, N, B), (1, B, K), (1, N, K), True, False, N, K, K, 1.0, 1.0))
         if self.fused:
             d.join()  # the weight gradients are complete before anything that follows on the main stream
 
@@ -252,7 +289,7 @@ class MlpTrainer:
         empty) so that the per-tensor step counts are those of one update over the whole model;
         the device counter is advanced by the last call of the step."""
         segs = [(off, n if j in (2 * l, 2 * l + 1) else 0) for j, (off, n) in enumerate(self.segments)]
-        self.dev.dispatch(opspec.adam(self.params, self.grads, self.m, self.v, segs, self.t + 1, self.lr, self.beta1,
+        self.dev.dispatch(opspec.adam(self.params, self._grads, self.m, self.v, segs, self.t + 1, self.lr, self.beta1,
                                       self.beta2, self.eps, self.clip, self.max_norm, self.delta, self.norms,
                                       self.params_bf16 if self.bf16 else None, self.t_dev, advance_counter=last))
         if last:
@@ -260,12 +297,13 @@ class MlpTrainer:
 
     def update(self):
         d = self.dev
+        self._settle()
         if self.opt == "sgd":
-            d.dispatch(opspec.sgd(self.params, self.grads, self.segments, self.lr, self.clip, self.max_norm, self.delta, self.norms,
+            d.dispatch(opspec.sgd(self.params, self._grads, self.segments, self.lr, self.clip, self.max_norm, self.delta, self.norms,
                                   self.zero_grads_in_update))
             self._grads_clear = self.zero_grads_in_update
         elif self.opt == "adam":
-            d.dispatch(opspec.adam(self.params, self.grads, self.m, self.v, self.segments, self.t + 1, self.lr, self.beta1,
+            d.dispatch(opspec.adam(self.params, self._grads, self.m, self.v, self.segments, self.t + 1, self.lr, self.beta1,
                                    self.beta2, self.eps, self.clip, self.max_norm, self.delta, self.norms,
                                    self.params_bf16 if self.bf16 else None, self.t_dev))
             self.t += len(self.segments)  # host mirror (eager steps only; read_t() is the truth)
@@ -276,7 +314,7 @@ class MlpTrainer:
     def layer_grads(self, l: int) -> DeviceSlice:
         """The contiguous slice [dW_l ; db_l] of the flat gradient buffer."""
         off = self.segments[2 * l][0]
-        return self.grads.view(off, self.segments[2 * l][1] + self.segments[2 * l + 1][1])
+        return self._grads.view(off, self.segments[2 * l][1] + self.segments[2 * l + 1][1])
 
     def _forward_backward_tail(self, X: DeviceSlice, T: DeviceSlice, fuse_update: bool = False):
         """forward, loss and backward with the last two layers, the loss and the
@@ -294,21 +332,21 @@ class MlpTrainer:
         layer's product; no update waits for the join of all streams.  The weights of the
         layers in between are still read by the dX products and are updated after the join."""
         d, B, L = self.dev, self.B, self.L
-        if not self._grads_clear:
-            d.mem_fill(self.grads, 0.0)
-        self._grads_clear = False
+        if self._zero_due or not self._grads_clear:
+            d.mem_fill(self._grads, 0.0)
+        self._grads_clear = self._zero_due = False
 
         in_gemm = fuse_update and self.zero_grads_in_update
         nlr = -float(np.float32(self.lr))  # lr cast f64 -> f32, then negated (optim.zig:103)
 
         def target(l):  # (C, alpha) of layer l's weight-gradient product
-            return (self.W[l], nlr) if in_gemm and l in (0, L - 2, L - 1) else (self.dW[l], 1.0)
+            return (self.W[l], nlr) if in_gemm and l in (0, L - 2, L - 1) else (self._dW[l], 1.0)
 
         def update(segs):
             if in_gemm:
                 segs = [sg for sg in segs if sg not in [self.segments[2 * l] for l in (0, L - 2, L - 1)]]
             if fuse_update and segs:
-                d.dispatch(opspec.sgd(self.params, self.grads, segs, self.lr, False, self.max_norm, self.delta, self.norms,
+                d.dispatch(opspec.sgd(self.params, self._grads, segs, self.lr, False, self.max_norm, self.delta, self.norms,
                                       self.zero_grads_in_update))
 
         weight, bias = (lambda l: self.segments[2 * l]), (lambda l: self.segments[2 * l + 1])
@@ -320,7 +358,7 @@ class MlpTrainer:
         h1, h2, C = self.dims[L - 2], self.dims[L - 1], self.dims[L]
         d.dispatch(opspec.mlp_tail(self.act[L - 3], self.W[L - 2], self.b[L - 2], self.W[L - 1], self.b[L - 1], T, B, h1, h2, C,
                                    self.ld_out, self.loss_div, self.act[L - 2], self.act[L - 1], self.loss, self.dact[L - 1],
-                                   self.dact[L - 2], self.dact[L - 3], self.db[L - 1], self.db[L - 2], self.db[L - 3],
+                                   self.dact[L - 2], self.dact[L - 3], self._db[L - 1], self._db[L - 2], self._db[L - 3],
                                    weights_ready=L - 2 >= 1))
         # the weight gradients of the two tail layers are independent of each other and of everything that follows:
         # one side stream each.
@@ -346,9 +384,9 @@ class MlpTrainer:
                 update([weight(0)])
             else:
                 with d.branch(0):
-                    d.dispatch(opspec.linear(self.dact[l], a_in, self.dW[l], N, K, B, True, False, N, K, K, 1.0, 1.0))
+                    d.dispatch(opspec.linear(self.dact[l], a_in, self._dW[l], N, K, B, True, False, N, K, K, 1.0, 1.0))
                 d.dispatch(opspec.linear(self.dact[l], self.W[l], self.dact[l - 1], B, K, N, False, False, N, K, K, 1.0, 0.0,
-                                         "relu_mask", None, self.act[l - 1], colsum=self.db[l - 1]))
+                                         "relu_mask", None, self.act[l - 1], colsum=self._db[l - 1]))
         d.join()
         if fuse_update:
             # what did not ride on the backward pass: the weights the dX products read and the biases in front of them
@@ -367,6 +405,14 @@ class MlpTrainer:
     def step(self, X: DeviceSlice, T: DeviceSlice, allreduce: Optional[Callable[[DeviceSlice], None]] = None):
         """forward + loss + backward [+ gradient all-reduce] + update, all
         asynchronous on the device stream.  The loss stays in ``self.loss``."""
+        if allreduce is not None:
+            return self._step(X, T, allreduce)
+        key = (X.ptr, X.dtype, T.ptr, T.dtype, self.lr, self.opt, self.beta1, self.beta2, self.eps, self.clip, self.max_norm, self.delta,
+               self.loss_div, self.fused, self.tail, self.fuse_update, self.update_by_layer, self.zero_grads_in_update, self._grads_clear,
+               self._zero_due)
+        self._graphs.run(key, lambda: self._step(X, T, None), self._host_state, self._set_host_state)
+
+    def _step(self, X: DeviceSlice, T: DeviceSlice, allreduce):
         if self.tail:
             fuse = self.fuse_update and allreduce is None and self.opt == "sgd" and not self.clip
             self._forward_backward_tail(X, T, fuse_update=fuse)
@@ -374,7 +420,7 @@ class MlpTrainer:
                 return
         else:
             by_layer = self.update_by_layer and self.fused and self.opt == "adam" and allreduce is None
-            self.forward(X)
+            self._forward(X)
             self.loss_and_grad(T)
             self.backward(X, update_by_layer=by_layer)
             if by_layer:
@@ -383,12 +429,12 @@ class MlpTrainer:
             fused = getattr(allreduce, "reduce_and_sgd", None)
             if fused is not None and self.opt == "sgd" and not self.clip:
                 if self.zero_grads_in_update:
-                    fused(self.grads, self.params, self.lr, True)  # reduction, update and zero_grad in one kernel
+                    fused(self._grads, self.params, self.lr, True)  # reduction, update and zero_grad in one kernel
                     self._grads_clear = True
                 else:
-                    fused(self.grads, self.params, self.lr)  # reduction and update in one kernel
+                    fused(self._grads, self.params, self.lr)  # reduction and update in one kernel
                 return
-            allreduce(self.grads)
+            allreduce(self._grads)
         self.update()
 
     def read_loss(self) -> float:
@@ -427,7 +473,8 @@ class MlpTrainer:
     def free(self):
         d = self.dev
         d.sync()
-        for s in [self.params, self.grads, self.norms, self.loss] + self.act + self.dact:
+        self._graphs.clear()
+        for s in [self.params, self._grads, self.norms, self.loss] + self.act + self.dact:
             d.mem_cache_free(s)
         if self.opt == "adam":
             d.mem_cache_free(self.m)
