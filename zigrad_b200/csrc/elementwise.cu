@@ -47,6 +47,7 @@ __device__ __forceinline__ void stv(T* p, const Pack<T, VecOf<T>::N>& v) {
 // out[i] = f(a[i], b[i], c[i]) for NIN in {1,2,3} same-length inputs.
 template <typename T, int NIN, bool VEC, typename F>
 __global__ void __launch_bounds__(kThreads) map_kernel(T* out, const T* a, const T* b, const T* c, size_t n, F f) {
+  pdl_sync();
   constexpr int N = VecOf<T>::N;
   const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t nthreads = (size_t)gridDim.x * blockDim.x;
@@ -93,8 +94,8 @@ void launch_map(cudaStream_t s, T* out, const T* a, const T* b, const T* c, size
   if (n == 0) return;
   bool vec = host_aligned16(out) && host_aligned16(a) && (NIN < 2 || host_aligned16(b)) && (NIN < 3 || host_aligned16(c));
   const unsigned g = grid_for(n, (size_t)kThreads * VecOf<T>::N * kUnroll);
-  if (vec) map_kernel<T, NIN, true, F><<<g, kThreads, 0, s>>>(out, a, b, c, n, f);
-  else map_kernel<T, NIN, false, F><<<g, kThreads, 0, s>>>(out, a, b, c, n, f);
+  if (vec) launch_pdl(map_kernel<T, NIN, true, F>, dim3(g), dim3(kThreads), 0, s, out, a, b, c, n, f);
+  else launch_pdl(map_kernel<T, NIN, false, F>, dim3(g), dim3(kThreads), 0, s, out, a, b, c, n, f);
   ZG_LAUNCH_CHECK();
 }
 
@@ -104,6 +105,7 @@ void launch_map(cudaStream_t s, T* out, const T* a, const T* b, const T* c, size
 // stride modulo L, subtract L on overflow) so no division runs per element.
 template <typename T, bool SHORT_IS_X, bool VEC, typename F>
 __global__ void __launch_bounds__(kThreads) bcast_kernel(T* out, const T* lng, const T* sht, size_t n, size_t L, F f) {
+  pdl_sync();
   constexpr int N = VecOf<T>::N;
   const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t nthreads = (size_t)gridDim.x * blockDim.x;
@@ -179,11 +181,11 @@ void binary_dispatch(cudaStream_t s, const T* x, const T* y, T* z, size_t xl, si
   const bool vec = host_aligned16(z) && host_aligned16(lng);
   const unsigned g = grid_for(zl, (size_t)kThreads * VecOf<T>::N * 2);
   if (short_is_x) {
-    if (vec) bcast_kernel<T, true, true, F><<<g, kThreads, 0, s>>>(z, lng, sht, zl, L, f);
-    else bcast_kernel<T, true, false, F><<<g, kThreads, 0, s>>>(z, lng, sht, zl, L, f);
+    if (vec) launch_pdl(bcast_kernel<T, true, true, F>, dim3(g), dim3(kThreads), 0, s, z, lng, sht, zl, L, f);
+    else launch_pdl(bcast_kernel<T, true, false, F>, dim3(g), dim3(kThreads), 0, s, z, lng, sht, zl, L, f);
   } else {
-    if (vec) bcast_kernel<T, false, true, F><<<g, kThreads, 0, s>>>(z, lng, sht, zl, L, f);
-    else bcast_kernel<T, false, false, F><<<g, kThreads, 0, s>>>(z, lng, sht, zl, L, f);
+    if (vec) launch_pdl(bcast_kernel<T, false, true, F>, dim3(g), dim3(kThreads), 0, s, z, lng, sht, zl, L, f);
+    else launch_pdl(bcast_kernel<T, false, false, F>, dim3(g), dim3(kThreads), 0, s, z, lng, sht, zl, L, f);
   }
   ZG_LAUNCH_CHECK();
 }
@@ -308,6 +310,7 @@ struct SigmInplaceBwdF { template <typename T> __device__ T operator()(T x, T xg
 //   MODE 3 clamp_mask_bwd (:630-650): bit set -> x_g += y_g
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kThreads) byte_mask_kernel(T* a, const T* b, unsigned char* mask, size_t n, T lo, T hi) {
+  pdl_sync();
   const size_t nbytes = (n + 7) / 8, nth = (size_t)gridDim.x * blockDim.x;
   const bool vec = aligned16(a) && (b == nullptr || aligned16(b));
   ClampF<T> cl{lo, hi};
@@ -370,12 +373,13 @@ __global__ void __launch_bounds__(kThreads) byte_mask_kernel(T* a, const T* b, u
 template <typename T, int MODE>
 void launch_byte_mask(cudaStream_t s, T* a, const T* b, unsigned char* mask, size_t n, T lo, T hi) {
   if (n == 0) return;
-  byte_mask_kernel<T, MODE><<<grid_for((n + 7) / 8, kThreads * 2), kThreads, 0, s>>>(a, b, mask, n, lo, hi);
+  launch_pdl(byte_mask_kernel<T, MODE>, dim3(grid_for((n + 7) / 8, kThreads * 2)), dim3(kThreads), 0, s, a, b, mask, n, lo, hi);
   ZG_LAUNCH_CHECK();
 }
 
 // fp32 <-> bf16 casts
 __global__ void __launch_bounds__(kThreads) f32_to_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, size_t n) {
+  pdl_sync();
   const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (size_t)gridDim.x * blockDim.x;
   const bool vec = aligned16(src) && ((reinterpret_cast<uintptr_t>(dst) & 7u) == 0);
   if (vec) {
@@ -394,6 +398,7 @@ __global__ void __launch_bounds__(kThreads) f32_to_bf16_kernel(const float* __re
   }
 }
 __global__ void __launch_bounds__(kThreads) bf16_to_f32_kernel(const __nv_bfloat16* __restrict__ src, float* __restrict__ dst, size_t n) {
+  pdl_sync();
   const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (size_t)gridDim.x * blockDim.x;
   if (((reinterpret_cast<uintptr_t>(src) & 7u) == 0) && aligned16(dst)) {
     // 4 elements per thread and trip: one 64-bit load, ONE 128-bit store, so that a warp's store covers
@@ -426,6 +431,7 @@ __global__ void __launch_bounds__(kThreads) bf16_to_f32_kernel(const __nv_bfloat
 // along A's rows, 128-bit stores along B's rows (needs m % 4 == n % 4 == 0
 // and 16-byte aligned bases; fp32 only).
 __global__ void __launch_bounds__(256) transpose64_kernel(const float* __restrict__ A, float* __restrict__ B, size_t m, size_t n, float alpha) {
+  pdl_sync();
   __shared__ float tile[64][65];
   const size_t bx = (size_t)blockIdx.x * 64, by = (size_t)blockIdx.y * 64;
   const int q = threadIdx.x & 15, r0 = threadIdx.x >> 4;
@@ -458,6 +464,7 @@ __global__ void __launch_bounds__(256) transpose64_kernel(const float* __restric
 
 template <typename T>
 __global__ void transpose_kernel(const T* __restrict__ A, T* __restrict__ B, size_t m, size_t n, T alpha) {
+  pdl_sync();
   __shared__ T tile[32][33];
   const size_t bx = (size_t)blockIdx.x * 32, by = (size_t)blockIdx.y * 32;
   for (int r = threadIdx.y; r < 32; r += blockDim.y) {
@@ -585,9 +592,9 @@ extern "C" void zg_cast(dtype src_id, dtype dst_id, StreamWrapper w, const void*
   if (n == 0) return;
   cudaStream_t s = as_stream(w);
   if (src_id == SINGLE && dst_id == BF16)
-    f32_to_bf16_kernel<<<grid_for(n, kThreads * 8), kThreads, 0, s>>>((const float*)src, (__nv_bfloat16*)dst, n);
+    launch_pdl(f32_to_bf16_kernel, dim3(grid_for(n, kThreads * 8)), dim3(kThreads), 0, s, (const float*)src, (__nv_bfloat16*)dst, n);
   else if (src_id == BF16 && dst_id == SINGLE)
-    bf16_to_f32_kernel<<<grid_for(n, kThreads * 8), kThreads, 0, s>>>((const __nv_bfloat16*)src, (float*)dst, n);
+    launch_pdl(bf16_to_f32_kernel, dim3(grid_for(n, kThreads * 8)), dim3(kThreads), 0, s, (const __nv_bfloat16*)src, (float*)dst, n);
   else { set_error(kUnsupported, "zg_cast: %d -> %d not supported", (int)src_id, (int)dst_id); return; }
   ZG_LAUNCH_CHECK();
 }
@@ -596,11 +603,11 @@ extern "C" void zg_transpose(dtype id, StreamWrapper w, const void* A, void* B, 
   if (m == 0 || n == 0) return;
   if (id == SINGLE && m % 4 == 0 && n % 4 == 0 && host_aligned16(A) && host_aligned16(B) && (m + 63) / 64 <= 65535) {
     dim3 grid64((unsigned)((n + 63) / 64), (unsigned)((m + 63) / 64));
-    transpose64_kernel<<<grid64, 256, 0, as_stream(w)>>>((const float*)A, (float*)B, m, n, (float)alpha);
+    launch_pdl(transpose64_kernel, dim3(grid64), dim3(256), 0, as_stream(w), (const float*)A, (float*)B, m, n, (float)alpha);
     ZG_LAUNCH_CHECK();
     return;
   }
   dim3 grid((unsigned)((n + 31) / 32), (unsigned)((m + 31) / 32)), block(32, 8);
-  ZG_FLOAT_SWITCH("zg_transpose", id, (transpose_kernel<T><<<grid, block, 0, as_stream(w)>>>((const T*)A, (T*)B, m, n, (T)alpha)));
+  ZG_FLOAT_SWITCH("zg_transpose", id, (launch_pdl(transpose_kernel<T>, dim3(grid), dim3(block), 0, as_stream(w), (const T*)A, (T*)B, m, n, (T)alpha)));
   ZG_LAUNCH_CHECK();
 }

@@ -13,6 +13,7 @@ constexpr int kIThreads = 256;
 
 template <typename T>
 __global__ void __launch_bounds__(kIThreads) scatter_add_kernel(const T* __restrict__ src, const len_t* __restrict__ offs, size_t n, T* dst) {
+  pdl_sync();
   const size_t nth = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += nth) atomicAdd(dst + offs[i], src[i]);
 }
@@ -20,6 +21,7 @@ __global__ void __launch_bounds__(kIThreads) scatter_add_kernel(const T* __restr
 template <typename T>
 __global__ void __launch_bounds__(kIThreads) gather_rows_kernel(const T* __restrict__ src, const len_t* __restrict__ idx, size_t rows, size_t cols,
                                                                 T* __restrict__ dst, len_t* __restrict__ offsets_out, int* bad) {
+  pdl_sync();
   const size_t nth = (size_t)gridDim.x * blockDim.x;
   for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += nth) {
     const size_t c = idx[r];
@@ -39,6 +41,7 @@ __global__ void __launch_bounds__(kIThreads) gather_rows_kernel(const T* __restr
 __global__ void __launch_bounds__(kIThreads) gcn_scatter_kernel(float* dst, const float* __restrict__ h, const float* __restrict__ deg,
                                                                 const len_t* __restrict__ src_idx, const len_t* __restrict__ tgt_idx,
                                                                 size_t stride, size_t n_edge) {
+  pdl_sync();
   const size_t total = n_edge * stride, nth = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nth) {
     const size_t e = i / stride, j = i % stride;
@@ -54,6 +57,7 @@ __global__ void __launch_bounds__(kIThreads) gcn_scatter_bwd_kernel(const float*
                                                                     const float* __restrict__ deg, const len_t* __restrict__ src_idx,
                                                                     const len_t* __restrict__ tgt_idx, float* grad_h, float* grad_deg,
                                                                     size_t stride, size_t n_edge) {
+  pdl_sync();
   const size_t nth = (size_t)gridDim.x * blockDim.x;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n_edge; e += nth) {
     const size_t s = src_idx[e], t = tgt_idx[e];
@@ -215,6 +219,7 @@ __global__ void __launch_bounds__(kIThreads) csr_gcn_propagate_kernel(float* out
 template <typename T>
 __global__ void __launch_bounds__(kIThreads) scatter_add_2d_kernel(const T* __restrict__ src, const len_t* __restrict__ indices, size_t n_blocks,
                                                                    size_t stride, T* dst) {
+  pdl_sync();
   const size_t total = n_blocks * stride, nth = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nth) {
     const size_t blk = i / stride, j = i - blk * stride;
@@ -226,6 +231,7 @@ __global__ void __launch_bounds__(kIThreads) scatter_add_2d_kernel(const T* __re
 // A warp walks a segment; segments do not overlap, so no atomics and the result is exact.
 template <typename T>
 __global__ void __launch_bounds__(kIThreads) scatter_add_csr_kernel(const T* __restrict__ src, const len_t* __restrict__ row_ptr, size_t n_seg, T* dst) {
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
   for (size_t r = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n_seg; r += warps) {
@@ -240,6 +246,7 @@ __global__ void __launch_bounds__(kIThreads) scatter_add_csr_kernel(const T* __r
 // folded by a shuffle tree (fixed order, so repeatable; not the host's left-to-right order).
 template <typename T>
 __global__ void __launch_bounds__(kIThreads) segment_sum_csr_kernel(const T* __restrict__ src, const len_t* __restrict__ row_ptr, size_t n_seg, T* __restrict__ dst) {
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
   for (size_t r = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n_seg; r += warps) {
@@ -267,8 +274,8 @@ extern "C" void zg_scatter_add_2d(dtype id, StreamWrapper w, const void* src, co
   if (n_blocks == 0 || stride == 0) return;
   cudaStream_t s = as_stream(w);
   const unsigned g = grid_for((size_t)n_blocks * stride, kIThreads * 2);
-  if (id == SINGLE) scatter_add_2d_kernel<float><<<g, kIThreads, 0, s>>>((const float*)src, indices, n_blocks, stride, (float*)dst);
-  else if (id == DOUBLE) scatter_add_2d_kernel<double><<<g, kIThreads, 0, s>>>((const double*)src, indices, n_blocks, stride, (double*)dst);
+  if (id == SINGLE) launch_pdl(scatter_add_2d_kernel<float>, dim3(g), dim3(kIThreads), 0, s, (const float*)src, indices, n_blocks, stride, (float*)dst);
+  else if (id == DOUBLE) launch_pdl(scatter_add_2d_kernel<double>, dim3(g), dim3(kIThreads), 0, s, (const double*)src, indices, n_blocks, stride, (double*)dst);
   else { set_error(kUnsupported, "zg_scatter_add_2d: unsupported dtype %d", (int)id); return; }
   ZG_LAUNCH_CHECK();
 }
@@ -277,8 +284,8 @@ extern "C" void zg_scatter_add_csr(dtype id, StreamWrapper w, const void* src, c
   if (n_segments == 0) return;
   cudaStream_t s = as_stream(w);
   const unsigned g = grid_for(n_segments, kIThreads / 32);
-  if (id == SINGLE) scatter_add_csr_kernel<float><<<g, kIThreads, 0, s>>>((const float*)src, row_ptr, n_segments, (float*)dst);
-  else if (id == DOUBLE) scatter_add_csr_kernel<double><<<g, kIThreads, 0, s>>>((const double*)src, row_ptr, n_segments, (double*)dst);
+  if (id == SINGLE) launch_pdl(scatter_add_csr_kernel<float>, dim3(g), dim3(kIThreads), 0, s, (const float*)src, row_ptr, n_segments, (float*)dst);
+  else if (id == DOUBLE) launch_pdl(scatter_add_csr_kernel<double>, dim3(g), dim3(kIThreads), 0, s, (const double*)src, row_ptr, n_segments, (double*)dst);
   else { set_error(kUnsupported, "zg_scatter_add_csr: unsupported dtype %d", (int)id); return; }
   ZG_LAUNCH_CHECK();
 }
@@ -287,8 +294,8 @@ extern "C" void zg_segment_sum_csr(dtype id, StreamWrapper w, const void* src, c
   if (n_segments == 0) return;
   cudaStream_t s = as_stream(w);
   const unsigned g = grid_for(n_segments, kIThreads / 32);
-  if (id == SINGLE) segment_sum_csr_kernel<float><<<g, kIThreads, 0, s>>>((const float*)src, row_offsets, n_segments, (float*)dst);
-  else if (id == DOUBLE) segment_sum_csr_kernel<double><<<g, kIThreads, 0, s>>>((const double*)src, row_offsets, n_segments, (double*)dst);
+  if (id == SINGLE) launch_pdl(segment_sum_csr_kernel<float>, dim3(g), dim3(kIThreads), 0, s, (const float*)src, row_offsets, n_segments, (float*)dst);
+  else if (id == DOUBLE) launch_pdl(segment_sum_csr_kernel<double>, dim3(g), dim3(kIThreads), 0, s, (const double*)src, row_offsets, n_segments, (double*)dst);
   else { set_error(kUnsupported, "zg_segment_sum_csr: unsupported dtype %d", (int)id); return; }
   ZG_LAUNCH_CHECK();
 }
@@ -296,8 +303,8 @@ extern "C" void zg_segment_sum_csr(dtype id, StreamWrapper w, const void* src, c
 extern "C" void zg_scatter_add(dtype id, StreamWrapper w, const void* src, const len_t* offsets, len_t n, void* dst) {
   if (n == 0) return;
   cudaStream_t s = as_stream(w);
-  if (id == SINGLE) scatter_add_kernel<float><<<grid_for(n, kIThreads * 2), kIThreads, 0, s>>>((const float*)src, offsets, n, (float*)dst);
-  else if (id == DOUBLE) scatter_add_kernel<double><<<grid_for(n, kIThreads * 2), kIThreads, 0, s>>>((const double*)src, offsets, n, (double*)dst);
+  if (id == SINGLE) launch_pdl(scatter_add_kernel<float>, dim3(grid_for(n, kIThreads * 2)), dim3(kIThreads), 0, s, (const float*)src, offsets, n, (float*)dst);
+  else if (id == DOUBLE) launch_pdl(scatter_add_kernel<double>, dim3(grid_for(n, kIThreads * 2)), dim3(kIThreads), 0, s, (const double*)src, offsets, n, (double*)dst);
   else { set_error(kUnsupported, "zg_scatter_add: unsupported dtype %d", (int)id); return; }
   ZG_LAUNCH_CHECK();
 }
@@ -306,8 +313,8 @@ extern "C" void zg_gather_rows(dtype id, StreamWrapper w, const void* src, const
                                len_t* offsets_out) {
   if (rows == 0) return;
   cudaStream_t s = as_stream(w);
-  if (id == SINGLE) gather_rows_kernel<float><<<grid_for(rows, kIThreads), kIThreads, 0, s>>>((const float*)src, idx, rows, cols, (float*)dst, offsets_out, nullptr);
-  else if (id == DOUBLE) gather_rows_kernel<double><<<grid_for(rows, kIThreads), kIThreads, 0, s>>>((const double*)src, idx, rows, cols, (double*)dst, offsets_out, nullptr);
+  if (id == SINGLE) launch_pdl(gather_rows_kernel<float>, dim3(grid_for(rows, kIThreads)), dim3(kIThreads), 0, s, (const float*)src, idx, rows, cols, (float*)dst, offsets_out, nullptr);
+  else if (id == DOUBLE) launch_pdl(gather_rows_kernel<double>, dim3(grid_for(rows, kIThreads)), dim3(kIThreads), 0, s, (const double*)src, idx, rows, cols, (double*)dst, offsets_out, nullptr);
   else { set_error(kUnsupported, "zg_gather_rows: unsupported dtype %d", (int)id); return; }
   ZG_LAUNCH_CHECK();
 }
@@ -316,7 +323,7 @@ extern "C" void zg_scatter_gcn_deg_scaled(dtype id, StreamWrapper w, void* dst, 
                                           const len_t* tgt_idx, len_t stride, len_t n_edge) {
   if (id != SINGLE) { set_error(kUnsupported, "zg_scatter_gcn_deg_scaled: only SINGLE is implemented"); return; }
   if (n_edge == 0 || stride == 0) return;
-  gcn_scatter_kernel<<<grid_for(n_edge * stride, kIThreads * 2), kIThreads, 0, as_stream(w)>>>((float*)dst, (const float*)h, (const float*)deg, src_idx, tgt_idx, stride, n_edge);
+  launch_pdl(gcn_scatter_kernel, dim3(grid_for(n_edge * stride, kIThreads * 2)), dim3(kIThreads), 0, as_stream(w), (float*)dst, (const float*)h, (const float*)deg, src_idx, tgt_idx, stride, n_edge);
   ZG_LAUNCH_CHECK();
 }
 
@@ -325,7 +332,7 @@ extern "C" void zg_scatter_gcn_deg_scaled_bwd(dtype id, StreamWrapper w, const v
                                               len_t n_edge) {
   if (id != SINGLE) { set_error(kUnsupported, "zg_scatter_gcn_deg_scaled_bwd: only SINGLE is implemented"); return; }
   if (n_edge == 0 || stride == 0) return;
-  gcn_scatter_bwd_kernel<<<grid_for(n_edge, kIThreads), kIThreads, 0, as_stream(w)>>>((const float*)grad_out, (const float*)h, (const float*)deg, src_idx, tgt_idx, (float*)grad_h, (float*)grad_deg, stride, n_edge);
+  launch_pdl(gcn_scatter_bwd_kernel, dim3(grid_for(n_edge, kIThreads)), dim3(kIThreads), 0, as_stream(w), (const float*)grad_out, (const float*)h, (const float*)deg, src_idx, tgt_idx, (float*)grad_h, (float*)grad_deg, stride, n_edge);
   ZG_LAUNCH_CHECK();
 }
 

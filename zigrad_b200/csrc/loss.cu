@@ -866,6 +866,7 @@ __global__ void __launch_bounds__(kRowThreads) softmax_ce_rows_staged_kernel(con
 // Rows wider than 1024: three passes over the row (values come back from L1/L2).
 template <bool INDEX_LABELS>
 __global__ void __launch_bounds__(kLThreads) softmax_ce_wide_kernel(const SmceArgs a) {
+  pdl_sync();
   __shared__ float sm32[32];
   const int lane = threadIdx.x & 31;
   const int C = a.C;
@@ -901,6 +902,7 @@ __global__ void __launch_bounds__(kLThreads) softmax_ce_wide_kernel(const SmceAr
 
 __global__ void __launch_bounds__(kLThreads) smooth_l1_kernel(const float* __restrict__ pred, const float* __restrict__ target, size_t n,
                                                               float beta, float* loss_out, float* grad, float* partial, unsigned* counter) {
+  pdl_sync();
   __shared__ float sm32[32];
   const size_t nth = (size_t)gridDim.x * blockDim.x;
   const float fn = (float)n;
@@ -921,6 +923,7 @@ __global__ void __launch_bounds__(kLThreads) smooth_l1_kernel(const float* __res
 
 // Plain row softmax / log-softmax (one warp per row, any width).
 __global__ void __launch_bounds__(kLThreads) softmax_rows_kernel(const float* x, float* y, size_t rows, int C, int log_mode) {
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
   for (size_t r = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
@@ -942,6 +945,7 @@ __global__ void __launch_bounds__(kLThreads) softmax_rows_kernel(const float* x,
 
 // x_grd += y * (y_grd - sum_j y_j * y_grd_j) per row
 __global__ void __launch_bounds__(kLThreads) softmax_rows_bwd_kernel(const float* __restrict__ y, const float* __restrict__ yg, float* xg, size_t rows, int C) {
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
   for (size_t r = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
@@ -954,9 +958,11 @@ __global__ void __launch_bounds__(kLThreads) softmax_rows_bwd_kernel(const float
 }
 
 __global__ void nll_index_fwd_kernel(const float* src, len_t trg, float* dst, len_t n, int mean) {
+  pdl_sync();
   if (threadIdx.x == 0 && blockIdx.x == 0) *dst = mean ? -src[trg] / (float)n : -src[trg];
 }
 __global__ void nll_encode_fwd_kernel(const float* src, const float* trg, float* dst, len_t n, int mean) {
+  pdl_sync();
   __shared__ float sm32[32];
   float acc = 0.f;
   for (len_t i = threadIdx.x; i < n; i += blockDim.x) acc -= trg[i] * src[i];
@@ -964,6 +970,7 @@ __global__ void nll_encode_fwd_kernel(const float* src, const float* trg, float*
   if (threadIdx.x == 0) *dst = mean ? acc / (float)n : acc;
 }
 __global__ void __launch_bounds__(kLThreads) nll_bwd_kernel(const float* __restrict__ x, const float* __restrict__ onehot, len_t trg, float* xg, len_t n, float denom) {
+  pdl_sync();
   const size_t nth = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += nth) {
     const float t = onehot ? onehot[i] : (i == trg ? 1.f : 0.f);
@@ -1139,7 +1146,7 @@ static void launch_softmax_ce(cudaStream_t s, SmceArgs a) {
   if (!partial) return;
   a.partial = partial;
   a.counter = counters;
-  softmax_ce_wide_kernel<IDX><<<g, kLThreads, 0, s>>>(a);
+  launch_pdl(softmax_ce_wide_kernel<IDX>, dim3(g), dim3(kLThreads), 0, s, a);
   ZG_LAUNCH_CHECK();
 }
 
@@ -1175,20 +1182,20 @@ extern "C" void zg_smooth_l1_fwd_bwd(dtype id, StreamWrapper w, const void* pred
   unsigned* counters = nullptr;
   float* partial = static_cast<float*>(workspace(s, sizeof(float) * g, &counters));
   if (!partial) return;
-  smooth_l1_kernel<<<g, kLThreads, 0, s>>>((const float*)pred, (const float*)target, n, (float)beta, (float*)loss_out, (float*)grad, partial, counters);
+  launch_pdl(smooth_l1_kernel, dim3(g), dim3(kLThreads), 0, s, (const float*)pred, (const float*)target, n, (float)beta, (float*)loss_out, (float*)grad, partial, counters);
   ZG_LAUNCH_CHECK();
 }
 
 static void softmax_rows(const char* name, dtype id, cudaStream_t s, const void* x, void* y, len_t m, len_t n, int log_mode) {
   if (id != SINGLE) { set_error(kUnsupported, "%s: only SINGLE is implemented", name); return; }
   if (m == 0 || n == 0) return;
-  softmax_rows_kernel<<<grid_for(m, kLThreads / 32), kLThreads, 0, s>>>((const float*)x, (float*)y, m, (int)n, log_mode);
+  launch_pdl(softmax_rows_kernel, dim3(grid_for(m, kLThreads / 32)), dim3(kLThreads), 0, s, (const float*)x, (float*)y, m, (int)n, log_mode);
   ZG_LAUNCH_CHECK();
 }
 static void softmax_rows_bwd(const char* name, dtype id, cudaStream_t s, const void* y, const void* yg, void* xg, len_t m, len_t n) {
   if (id != SINGLE) { set_error(kUnsupported, "%s: only SINGLE is implemented", name); return; }
   if (m == 0 || n == 0) return;
-  softmax_rows_bwd_kernel<<<grid_for(m, kLThreads / 32), kLThreads, 0, s>>>((const float*)y, (const float*)yg, (float*)xg, m, (int)n);
+  launch_pdl(softmax_rows_bwd_kernel, dim3(grid_for(m, kLThreads / 32)), dim3(kLThreads), 0, s, (const float*)y, (const float*)yg, (float*)xg, m, (int)n);
   ZG_LAUNCH_CHECK();
 }
 
@@ -1209,25 +1216,25 @@ extern "C" void nll_loss_1D_index_fwd(dtype id, CudnnWrapper w, void* src, len_t
   if (id != SINGLE) { set_error(kUnsupported, "nll_loss_1D_index_fwd: only SINGLE is implemented"); return; }
   if (n == 0 || trg >= n) { set_error(kBadArgument, "nll_loss_1D_index_fwd: target %lu out of range %lu", trg, n); return; }
   if (inplace_smax) smax_vec_fwd(id, w, src, src, n, SMAX_LOG);
-  nll_index_fwd_kernel<<<1, 32, 0, as_stream(w)>>>((const float*)src, trg, (float*)dst, n, reduxop != RDX_SUM);
+  launch_pdl(nll_index_fwd_kernel, dim3(1), dim3(32), 0, as_stream(w), (const float*)src, trg, (float*)dst, n, reduxop != RDX_SUM);
   ZG_LAUNCH_CHECK();
 }
 extern "C" void nll_loss_1D_index_bwd(dtype id, CudnnWrapper w, const void* x_val, void* x_grd, len_t trg, len_t n, reduxtype reduxop) {
   if (id != SINGLE) { set_error(kUnsupported, "nll_loss_1D_index_bwd: only SINGLE is implemented"); return; }
   if (n == 0) return;
-  nll_bwd_kernel<<<grid_for(n, kLThreads), kLThreads, 0, as_stream(w)>>>((const float*)x_val, nullptr, trg, (float*)x_grd, n, reduxop == RDX_SUM ? 1.f : (float)n);
+  launch_pdl(nll_bwd_kernel, dim3(grid_for(n, kLThreads)), dim3(kLThreads), 0, as_stream(w), (const float*)x_val, nullptr, trg, (float*)x_grd, n, reduxop == RDX_SUM ? 1.f : (float)n);
   ZG_LAUNCH_CHECK();
 }
 extern "C" void nll_loss_1D_encode_fwd(dtype id, CudnnWrapper w, void* src, const void* trg, void* dst, len_t n, bool inplace_smax, reduxtype reduxop) {
   if (id != SINGLE) { set_error(kUnsupported, "nll_loss_1D_encode_fwd: only SINGLE is implemented"); return; }
   if (n == 0) return;
   if (inplace_smax) smax_vec_fwd(id, w, src, src, n, SMAX_LOG);
-  nll_encode_fwd_kernel<<<1, kLThreads, 0, as_stream(w)>>>((const float*)src, (const float*)trg, (float*)dst, n, reduxop != RDX_SUM);
+  launch_pdl(nll_encode_fwd_kernel, dim3(1), dim3(kLThreads), 0, as_stream(w), (const float*)src, (const float*)trg, (float*)dst, n, reduxop != RDX_SUM);
   ZG_LAUNCH_CHECK();
 }
 extern "C" void nll_loss_1D_encode_bwd(dtype id, CudnnWrapper w, const void* x_val, const void* y_val, void* x_grd, len_t n, reduxtype reduxop) {
   if (id != SINGLE) { set_error(kUnsupported, "nll_loss_1D_encode_bwd: only SINGLE is implemented"); return; }
   if (n == 0) return;
-  nll_bwd_kernel<<<grid_for(n, kLThreads), kLThreads, 0, as_stream(w)>>>((const float*)x_val, (const float*)y_val, 0, (float*)x_grd, n, reduxop == RDX_SUM ? 1.f : (float)n);
+  launch_pdl(nll_bwd_kernel, dim3(grid_for(n, kLThreads)), dim3(kLThreads), 0, as_stream(w), (const float*)x_val, (const float*)y_val, 0, (float*)x_grd, n, reduxop == RDX_SUM ? 1.f : (float)n);
   ZG_LAUNCH_CHECK();
 }

@@ -21,109 +21,107 @@ constexpr int kRThreads = 256;
 
 // ------------------------------------------------------------ fold_rows
 // x: [batch][row][col] -> y: [batch][col];  y = alpha * sum_rows + beta * y.
-// Grid: (row_chunks, col_tiles, batch).  A CTA is 8 warps; with VEC a warp
-// spans 128 columns (one float4 per lane) and the 8 warps take 8 rows per
-// trip, 8 trips unrolled, so a CTA has 64 x 512-byte row segments in flight.
+// Grid: (row_chunks, col_tiles, batch).  A CTA is 8 warps; a lane owns CW columns (16 bytes where rows allow it, else
+// one) and the warps take 8 rows per trip, 8 trips unrolled: with rows of odd length one element per lane and
+// trip in flight left the launch waiting (4099x1003: 27 us, HBM's share of it 3).  The last CTA of a column tile folds
+// that tile's partial sums, so the tiles finish beside each other (per_tile: a zeroed ticket for each; without it the
+// last CTA of the grid folds all of them).
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(kRThreads) fold_rows_kernel(const T* __restrict__ x, T* y, T* __restrict__ partial,
-                                                              unsigned* counters, size_t row, size_t col, T alpha, T beta) {
-  constexpr int CW = VEC ? 4 : 1;            // columns per lane
-  constexpr int TILE = 32 * CW;              // columns per CTA
+                                                              unsigned* tickets, size_t row, size_t col, T alpha, T beta, int per_tile) {
+  pdl_sync();
+  constexpr int CW = VEC ? 16 / sizeof(T) : 1;  // columns per lane
+  constexpr int TILE = 32 * CW;                 // columns per CTA
+  constexpr int U = 8;
+  struct alignas(CW * sizeof(T)) Word { T v[CW]; };
+  __shared__ T sm[8][TILE];
+  __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const size_t b = blockIdx.z;
-  const size_t c0 = (size_t)blockIdx.y * TILE + lane * CW;
-  const size_t chunks = gridDim.x;
+  const size_t b = blockIdx.z, chunks = gridDim.x, c0 = (size_t)blockIdx.y * TILE + lane * CW;
   const T* xb = x + b * row * col;
   T acc[CW];
 #pragma unroll
   for (int j = 0; j < CW; ++j) acc[j] = T(0);
-  const bool active = c0 < col;
-  if (active) {
+  if (c0 < col) {
     size_t r = (size_t)blockIdx.x * 8 + warp;
     const size_t rstep = chunks * 8;
-    if constexpr (VEC) {
-      for (; r + 7 * rstep < row; r += 8 * rstep) {
-        float4 v[8];
+    for (; r + (U - 1) * rstep < row; r += U * rstep) {
+      Word v[U];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = *reinterpret_cast<const float4*>(xb + (r + u * rstep) * col + c0);
+      for (int u = 0; u < U; ++u) v[u] = *reinterpret_cast<const Word*>(xb + (r + u * rstep) * col + c0);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) { acc[0] += v[u].x; acc[1] += v[u].y; acc[2] += v[u].z; acc[3] += v[u].w; }
-      }
-      for (; r + 3 * rstep < row; r += 4 * rstep) {
-        float4 v[4];
+      for (int u = 0; u < U; ++u)
 #pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = *reinterpret_cast<const float4*>(xb + (r + u * rstep) * col + c0);
+        for (int j = 0; j < CW; ++j) acc[j] += v[u].v[j];
+    }
+    // the rest: every load is issued (a row past the end reads the first again and is not added) before one is used
+    if (r < row) {
+      Word v[U];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) { acc[0] += v[u].x; acc[1] += v[u].y; acc[2] += v[u].z; acc[3] += v[u].w; }
-      }
-      for (; r < row; r += rstep) {
-        const float4 v = *reinterpret_cast<const float4*>(xb + r * col + c0);
-        acc[0] += v.x; acc[1] += v.y; acc[2] += v.z; acc[3] += v.w;
-      }
-    } else {
-      for (; r < row; r += rstep) acc[0] += xb[r * col + c0];
+      for (int u = 0; u < U; ++u) v[u] = *reinterpret_cast<const Word*>(xb + (r + u * rstep < row ? r + u * rstep : 0) * col + c0);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (r + u * rstep < row)
+#pragma unroll
+          for (int j = 0; j < CW; ++j) acc[j] += v[u].v[j];
     }
   }
-  __shared__ T sm[8][TILE];
+  auto fold_warps = [&](T (&s)[CW]) {  // the 8 warps' sums of this lane's columns, in warp 0
 #pragma unroll
-  for (int j = 0; j < CW; ++j) sm[warp][lane * CW + j] = acc[j];
-  __syncthreads();
-  // warp 0 folds the 8 row-lanes and publishes the CTA partial
-  const size_t ptile = ((b * gridDim.y + blockIdx.y) * chunks + blockIdx.x) * TILE;
-  if (warp == 0) {
+    for (int j = 0; j < CW; ++j) sm[warp][lane * CW + j] = s[j];
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+      for (int j = 0; j < CW; ++j) {
+        s[j] = T(0);
+#pragma unroll
+        for (int w = 0; w < 8; ++w) s[j] += sm[w][lane * CW + j];
+      }
+    }
+  };
+  auto put = [&](size_t bb, size_t c, const T (&s)[CW]) {
 #pragma unroll
     for (int j = 0; j < CW; ++j) {
-      T s = T(0);
-#pragma unroll
-      for (int w = 0; w < 8; ++w) s += sm[w][lane * CW + j];
-      partial[ptile + lane * CW + j] = s;
+      if (c + j >= col) continue;
+      T* yo = y + bb * col + c + j;
+      *yo = (beta == T(0)) ? alpha * s[j] : alpha * s[j] + beta * (*yo);
     }
+  };
+  fold_warps(acc);
+  if (chunks == 1) {
+    if (warp == 0 && c0 < col) put(b, c0, acc);
+    return;
   }
-  __threadfence();
+  const size_t tile = b * gridDim.y + blockIdx.y;
+  if (warp == 0) {
+#pragma unroll
+    for (int j = 0; j < CW; ++j) partial[(tile * chunks + blockIdx.x) * TILE + lane * CW + j] = acc[j];
+    __threadfence();
+  }
   __syncthreads();
-  __shared__ bool last;
-  unsigned* ticket = counters + 0;
   if (threadIdx.x == 0) {
-    const unsigned total = gridDim.x * gridDim.y * gridDim.z;
-    const unsigned t = atomicAdd(ticket, 1u);
-    last = (t == total - 1);
-    if (last) *ticket = 0;  // leave the counter at zero for the next launch
+    unsigned* ticket = tickets + (per_tile ? tile : 0);
+    const unsigned total = per_tile ? gridDim.x : gridDim.x * gridDim.y * gridDim.z;
+    last = atomicAdd(ticket, 1u) == total - 1;
+    if (last) *ticket = 0;  // leave the ticket at zero for the next launch
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
-  // final fold by the last CTA: `parts` threads share one output column (each
-  // takes every parts-th chunk, four loads in flight), then a shuffle tree
-  // combines them -- a fixed order, so the result is reproducible
-  const size_t ntile = gridDim.y, nb = gridDim.z;
-  const size_t outputs = nb * ntile * TILE;
-  const unsigned parts = outputs >= 256 ? 1u : (outputs * 8 <= 256 ? 8u : (outputs * 4 <= 256 ? 4u : (outputs * 2 <= 256 ? 2u : 1u)));
-  const unsigned part = threadIdx.x % parts;
-  const size_t per_trip = blockDim.x / parts;
-  for (size_t base = 0; base < outputs; base += per_trip) {
-    const size_t idx = base + threadIdx.x / parts;
-    const size_t bb = idx / (ntile * TILE), rem = idx % (ntile * TILE);
-    const size_t tile = rem / TILE, cc = rem % TILE;
-    const size_t c = tile * TILE + cc;
-    const bool ok = idx < outputs && c < col;
-    T s0 = T(0), s1 = T(0), s2 = T(0), s3 = T(0);
-    if (ok) {
-      const T* p = partial + ((bb * ntile + tile) * chunks) * TILE + cc;
-      size_t k = part;
-      for (; k + 3 * parts < chunks; k += 4 * parts) {
-        s0 += __ldcg(p + k * TILE);
-        s1 += __ldcg(p + (k + parts) * TILE);
-        s2 += __ldcg(p + (k + 2 * parts) * TILE);
-        s3 += __ldcg(p + (k + 3 * parts) * TILE);
-      }
-      for (; k < chunks; k += parts) s0 += __ldcg(p + k * TILE);
-    }
-    T s = (s0 + s1) + (s2 + s3);
-    for (unsigned o = parts >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (ok && part == 0) {
-      T* yo = y + bb * col + c;
-      *yo = (beta == T(0)) ? alpha * s : alpha * s + beta * (*yo);
-    }
+  const size_t t0 = per_tile ? tile : 0, t1 = per_tile ? tile + 1 : (size_t)gridDim.y * gridDim.z;
+  for (size_t t = t0; t < t1; ++t) {
+    const T* p = partial + t * chunks * TILE + lane * CW;
+    T s[CW];
+#pragma unroll
+    for (int j = 0; j < CW; ++j) s[j] = T(0);
+#pragma unroll 4
+    for (size_t k = warp; k < chunks; k += 8)
+#pragma unroll
+      for (int j = 0; j < CW; ++j) s[j] += __ldcg(p + k * TILE + j);
+    __syncthreads();  // sm is free again
+    fold_warps(s);
+    const size_t c = t % gridDim.y * TILE + lane * CW;
+    if (warp == 0 && c < col) put(t / gridDim.y, c, s);
   }
 }
 
@@ -131,10 +129,10 @@ template <typename T>
 void fold_rows_launch(cudaStream_t s, const T* x, T* y, size_t batch, size_t row, size_t col, T alpha, T beta) {
   if (batch == 0 || col == 0) return;
   if (row == 0) return;
-  const bool vec = sizeof(T) == 4 && (col % 4 == 0) && host_aligned16(x);
-  const size_t tile = vec ? 128 : 32;
+  const bool vec = (col * sizeof(T)) % 16 == 0 && host_aligned16(x);
+  const size_t tile = vec ? 512 / sizeof(T) : 32;
   const size_t col_tiles = (col + tile - 1) / tile;
-  // row chunks: enough CTAs for ~4 per SM (64 KB of loads in flight on each), at least 64 rows per CTA,
+  // row chunks: enough CTAs for ~4 per SM (32 to 64 KB of loads in flight on each), at least 64 rows per CTA (one trip),
   // and a final fold that stays short (<= 64 chunks)
   size_t want = (size_t)4 * sm_count() / (col_tiles * batch);
   if (want < 1) want = 1;
@@ -143,16 +141,15 @@ void fold_rows_launch(cudaStream_t s, const T* x, T* y, size_t batch, size_t row
   if (chunks > 64) chunks = 64;
   if (chunks < 1) chunks = 1;
   if (col_tiles > 65535 || batch > 65535) { set_error(kBadArgument, "fold_rows: shape too large (%zu col tiles, batch %zu)", col_tiles, batch); return; }
-  unsigned* counters = nullptr;
-  T* partial = static_cast<T*>(workspace(s, sizeof(T) * batch * col_tiles * chunks * tile, &counters));
-  if (!partial) return;
-  dim3 grid((unsigned)chunks, (unsigned)col_tiles, (unsigned)batch);
-  if (vec) {
-    if constexpr (sizeof(T) == 4) fold_rows_kernel<T, true><<<grid, kRThreads, 0, s>>>(x, y, partial, counters, row, col, alpha, beta);
-  } else {
-    fold_rows_kernel<T, false><<<grid, kRThreads, 0, s>>>(x, y, partial, counters, row, col, alpha, beta);
+  T* partial = nullptr;
+  unsigned* tickets = nullptr;
+  if (chunks > 1) {
+    partial = static_cast<T*>(workspace(s, sizeof(T) * batch * col_tiles * chunks * tile, nullptr));
+    tickets = static_cast<unsigned*>(workspace(s, sizeof(unsigned) * batch * col_tiles, nullptr, 2));
+    if (!partial || !tickets) return;
   }
-  ZG_LAUNCH_CHECK();
+  auto kern = vec ? fold_rows_kernel<T, true> : fold_rows_kernel<T, false>;
+  launch_pdl(kern, dim3((unsigned)chunks, (unsigned)col_tiles, (unsigned)batch), dim3(kRThreads), 0, s, x, y, partial, tickets, row, col, alpha, beta, 1);
 }
 
 void fold_rows_f32(cudaStream_t s, const float* x, float* y, size_t row, size_t col) { fold_rows_launch<float>(s, x, y, 1, row, col, 1.f, 0.f); }
@@ -161,18 +158,30 @@ void fold_rows_f32(cudaStream_t s, const float* x, float* y, size_t row, size_t 
 // [row, col] -> [row]: a warp per row (wide rows) or a thread per row.
 template <typename T>
 __global__ void __launch_bounds__(kRThreads) fold_cols_warp_kernel(const T* __restrict__ x, T* y, size_t row, size_t col, T alpha, T beta) {
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
   for (size_t r = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < row; r += warps) {
     const T* xr = x + r * col;
-    T s = T(0);
-    for (size_t j = lane; j < col; j += 32) s += xr[j];
+    // eight loads of a lane in flight; rows of any length and alignment are read as coalesced single elements
+    T part[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) part[u] = T(0);
+    size_t j = lane;
+    for (; j + 224 < col; j += 256)
+#pragma unroll
+      for (int u = 0; u < 8; ++u) part[u] += xr[j + 32 * u];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (j + 32 * u < col) part[u] += xr[j + 32 * u];
+    T s = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
     s = warp_sum(s);
     if (lane == 0) y[r] = (beta == T(0)) ? alpha * s : alpha * s + beta * y[r];
   }
 }
 template <typename T>
 __global__ void __launch_bounds__(kRThreads) fold_cols_thread_kernel(const T* __restrict__ x, T* y, size_t row, size_t col, T alpha, T beta) {
+  pdl_sync();
   const size_t nth = (size_t)gridDim.x * blockDim.x;
   for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < row; r += nth) {
     const T* xr = x + r * col;
@@ -184,8 +193,8 @@ __global__ void __launch_bounds__(kRThreads) fold_cols_thread_kernel(const T* __
 template <typename T>
 void fold_cols_launch(cudaStream_t s, const T* x, T* y, size_t row, size_t col, T alpha, T beta) {
   if (row == 0 || col == 0) return;
-  if (col <= 16) fold_cols_thread_kernel<T><<<grid_for(row, kRThreads), kRThreads, 0, s>>>(x, y, row, col, alpha, beta);
-  else fold_cols_warp_kernel<T><<<grid_for(row, kRThreads / 32), kRThreads, 0, s>>>(x, y, row, col, alpha, beta);
+  if (col <= 16) launch_pdl(fold_cols_thread_kernel<T>, dim3(grid_for(row, kRThreads)), dim3(kRThreads), 0, s, x, y, row, col, alpha, beta);
+  else launch_pdl(fold_cols_warp_kernel<T>, dim3(grid_for(row, kRThreads / 32)), dim3(kRThreads), 0, s, x, y, row, col, alpha, beta);
   ZG_LAUNCH_CHECK();
 }
 
@@ -194,6 +203,7 @@ void fold_cols_launch(cudaStream_t s, const T* x, T* y, size_t row, size_t col, 
 // from -inf, strict '>' comparison (NaNs never win), as the host loop does.
 template <typename T>
 __global__ void __launch_bounds__(kRThreads) max_along_kernel(const T* __restrict__ x, T* __restrict__ y, size_t ylen, size_t d, size_t inner) {
+  pdl_sync();
   const size_t nth = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < ylen; i += nth) {
     const size_t base = (i / inner) * (inner * d) + (i % inner);
@@ -210,6 +220,7 @@ __global__ void __launch_bounds__(kRThreads) max_along_kernel(const T* __restric
 // output, lanes stride the row with 128-bit loads where the row allows.
 template <typename T>
 __global__ void __launch_bounds__(kRThreads) max_along_rows_kernel(const T* __restrict__ x, T* __restrict__ y, size_t rows, size_t d) {
+  pdl_sync();
   constexpr int V = 16 / sizeof(T);
   const int lane = threadIdx.x & 31;
   const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
@@ -239,7 +250,16 @@ __global__ void __launch_bounds__(kRThreads) max_along_rows_kernel(const T* __re
           if (e[k] > mx) mx = e[k];
       }
     } else {
-      for (size_t j = lane; j < d; j += 32) {
+      size_t j = lane;
+      for (; j + 224 < d; j += 256) {
+        T e[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) e[u] = xr[j + 32 * u];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (e[u] > mx) mx = e[u];
+      }
+      for (; j < d; j += 32) {
         const T v = xr[j];
         if (v > mx) mx = v;
       }
@@ -262,6 +282,7 @@ template <typename T, int OP>
 __global__ void __launch_bounds__(kRThreads) scalar_reduce_kernel(const T* __restrict__ a, const T* __restrict__ b, size_t n,
                                                                   double* __restrict__ partial, unsigned* counters, T* out,
                                                                   T alpha, T beta) {
+  pdl_sync();
   __shared__ double sm[32];
   const size_t nth = (size_t)gridDim.x * blockDim.x, tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   auto term = [](T v, T w) -> T {
@@ -328,7 +349,7 @@ void scalar_reduce_launch(cudaStream_t s, const T* a, const T* b, size_t n, T* o
   unsigned* counters = nullptr;
   double* partial = static_cast<double*>(workspace(s, sizeof(double) * g, &counters));
   if (!partial) return;
-  scalar_reduce_kernel<T, OP><<<g, kRThreads, 0, s>>>(a, b, n, partial, counters, out, alpha, beta);
+  launch_pdl(scalar_reduce_kernel<T, OP>, dim3(g), dim3(kRThreads), 0, s, a, b, n, partial, counters, out, alpha, beta);
   ZG_LAUNCH_CHECK();
 }
 
@@ -337,6 +358,7 @@ void scalar_reduce_launch(cudaStream_t s, const T* a, const T* b, size_t n, T* o
 template <typename T>
 __global__ void __launch_bounds__(kRThreads) amax_kernel(const T* __restrict__ x, size_t n, T* __restrict__ pval,
                                                          unsigned long long* __restrict__ pidx, unsigned* counters, T* out) {
+  pdl_sync();
   __shared__ T sv[kRThreads];
   __shared__ unsigned long long si[kRThreads];
   const size_t nth = (size_t)gridDim.x * blockDim.x, tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -417,6 +439,7 @@ __global__ void __launch_bounds__(kRThreads) amax_kernel(const T* __restrict__ x
 
 template <typename T>
 __global__ void __launch_bounds__(kRThreads) max_bwd_kernel(const T* __restrict__ x, const T* __restrict__ y, const T* __restrict__ yg, T* xg, size_t n) {
+  pdl_sync();
   const size_t nth = (size_t)gridDim.x * blockDim.x;
   const T val = y[0], g = yg[0];
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += nth)
@@ -426,6 +449,7 @@ __global__ void __launch_bounds__(kRThreads) max_bwd_kernel(const T* __restrict_
 // x *= max/(norm+delta) when norm > max; norm is read from device memory
 template <typename T>
 __global__ void __launch_bounds__(kRThreads) clip_scale_kernel(T* x, size_t n, const T* __restrict__ norm, T max_norm, T delta) {
+  pdl_sync();
   const T nv = *norm;
   if (!(nv > max_norm)) return;
   const T f = max_norm / (nv + delta);
@@ -436,6 +460,7 @@ __global__ void __launch_bounds__(kRThreads) clip_scale_kernel(T* x, size_t n, c
 // y[i] = alpha*x[i % xl] + beta*y[i]
 template <typename T>
 __global__ void __launch_bounds__(kRThreads) broadcast_kernel(const T* __restrict__ x, size_t xl, T* y, size_t yl, T alpha, T beta) {
+  pdl_sync();
   const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (size_t)gridDim.x * blockDim.x;
   size_t col = tid % xl;
   const size_t step = nth % xl;
@@ -471,13 +496,14 @@ void max_along_impl(cudaStream_t s, const T* x, const len_t* xs, size_t nd, size
   if (total == 0) return;
   const size_t ylen = total / xs[dim];
   const size_t inner = prod(xs, dim + 1, nd);
-  if (inner == 1 && xs[dim] > 8) max_along_rows_kernel<T><<<grid_for(ylen, kRThreads / 32), kRThreads, 0, s>>>(x, y, ylen, xs[dim]);
-  else max_along_kernel<T><<<grid_for(ylen, kRThreads), kRThreads, 0, s>>>(x, y, ylen, xs[dim], inner);
+  if (inner == 1 && xs[dim] > 8) launch_pdl(max_along_rows_kernel<T>, dim3(grid_for(ylen, kRThreads / 32)), dim3(kRThreads), 0, s, x, y, ylen, xs[dim]);
+  else launch_pdl(max_along_kernel<T>, dim3(grid_for(ylen, kRThreads)), dim3(kRThreads), 0, s, x, y, ylen, xs[dim], inner);
   ZG_LAUNCH_CHECK();
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kRThreads) scaled_copy_kernel(const T* __restrict__ x, T* y, size_t n, T alpha, T beta) {
+  pdl_sync();
   const size_t nth = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += nth)
     y[i] = (beta == T(0)) ? alpha * x[i] : alpha * x[i] + beta * y[i];
@@ -497,7 +523,7 @@ void unbroadcast_impl(cudaStream_t s, const T* x, const len_t* x_shape, size_t x
   const size_t xlen = prod(x_shape, 0, xnd), ylen = prod(y_shape, 0, ynd);
   if (xlen == 0) return;
   if (xlen == ylen) {
-    scaled_copy_kernel<T><<<grid_for(xlen, kRThreads * 4), kRThreads, 0, s>>>(x, y, xlen, alpha, beta);
+    launch_pdl(scaled_copy_kernel<T>, dim3(grid_for(xlen, kRThreads * 4)), dim3(kRThreads), 0, s, x, y, xlen, alpha, beta);
     ZG_LAUNCH_CHECK();
     return;
   }
@@ -586,7 +612,7 @@ extern "C" void zg_unbroadcast(dtype id, StreamWrapper w, const void* x, const l
 extern "C" void zg_broadcast(dtype id, StreamWrapper w, const void* x, len_t x_len, void* y, len_t y_len, double alpha, double beta) {
   if (y_len == 0 || x_len == 0) return;
   ZG_FLOAT_SWITCH("zg_broadcast", id,
-                  (broadcast_kernel<T><<<grid_for(y_len, kRThreads * 4), kRThreads, 0, as_stream(w)>>>((const T*)x, x_len, (T*)y, y_len, (T)alpha, (T)beta)));
+                  (launch_pdl(broadcast_kernel<T>, dim3(grid_for(y_len, kRThreads * 4)), dim3(kRThreads), 0, as_stream(w), (const T*)x, x_len, (T*)y, y_len, (T)alpha, (T)beta)));
   ZG_LAUNCH_CHECK();
 }
 
@@ -604,7 +630,7 @@ extern "C" void clip_nrm2(dtype id, CublasWrapper w, void* x, void* cur_nrm2, le
   if (n == 0) return;
   nrm2(id, w, x, cur_nrm2, n);
   ZG_FLOAT_SWITCH("clip_nrm2", id,
-                  (clip_scale_kernel<T><<<grid_for(n, kRThreads * 4), kRThreads, 0, as_stream(w)>>>((T*)x, n, (const T*)cur_nrm2, (T)max_nrm2, (T)delta)));
+                  (launch_pdl(clip_scale_kernel<T>, dim3(grid_for(n, kRThreads * 4)), dim3(kRThreads), 0, as_stream(w), (T*)x, n, (const T*)cur_nrm2, (T)max_nrm2, (T)delta)));
   ZG_LAUNCH_CHECK();
 }
 
@@ -617,7 +643,7 @@ static void max_fwd_impl(cudaStream_t s, const T* x, T* y, size_t n) {
   if (!ws) return;
   unsigned long long* pidx = reinterpret_cast<unsigned long long*>(ws);
   T* pval = reinterpret_cast<T*>(ws + 8 * (size_t)g);
-  amax_kernel<T><<<g, kRThreads, 0, s>>>(x, n, pval, pidx, counters, y);
+  launch_pdl(amax_kernel<T>, dim3(g), dim3(kRThreads), 0, s, x, n, pval, pidx, counters, y);
   ZG_LAUNCH_CHECK();
 }
 extern "C" void max_fwd(dtype id, StreamWrapper w, const void* x, void* y, len_t n) {
@@ -626,7 +652,7 @@ extern "C" void max_fwd(dtype id, StreamWrapper w, const void* x, void* y, len_t
 extern "C" void max_bwd(dtype id, StreamWrapper w, const void* x_val, void const* y_val, const void* y_grd, void* x_grd, len_t n) {
   if (n == 0) return;
   ZG_FLOAT_SWITCH("max_bwd", id,
-                  (max_bwd_kernel<T><<<grid_for(n, kRThreads * 4), kRThreads, 0, as_stream(w)>>>((const T*)x_val, (const T*)y_val, (const T*)y_grd, (T*)x_grd, n)));
+                  (launch_pdl(max_bwd_kernel<T>, dim3(grid_for(n, kRThreads * 4)), dim3(kRThreads), 0, as_stream(w), (const T*)x_val, (const T*)y_val, (const T*)y_grd, (T*)x_grd, n)));
   ZG_LAUNCH_CHECK();
 }
 
@@ -723,6 +749,7 @@ extern "C" CutensorPlanWrapper get_permutate_plan(CutensorWrapper w, dtype id, c
 namespace zg {
 template <typename T>
 __global__ void permute2d_kernel(const T* __restrict__ A, T* __restrict__ B, size_t m, size_t n, T alpha) {
+  pdl_sync();
   __shared__ T tile[32][33];
   const size_t bx = (size_t)blockIdx.x * 32, by = (size_t)blockIdx.y * 32;
   for (int r = threadIdx.y; r < 32; r += blockDim.y) {
@@ -745,10 +772,10 @@ extern "C" void permutate(CutensorWrapper w, void* plan, const void* x_vals, voi
   dim3 grid((unsigned)((p->n + 31) / 32), (unsigned)((p->m + 31) / 32)), block(32, 8);
   if (p->id == SINGLE) {
     float a; memcpy(&a, alpha, 4);
-    permute2d_kernel<float><<<grid, block, 0, as_stream(w)>>>((const float*)x_vals, (float*)y_vals, p->m, p->n, a);
+    launch_pdl(permute2d_kernel<float>, dim3(grid), dim3(block), 0, as_stream(w), (const float*)x_vals, (float*)y_vals, p->m, p->n, a);
   } else if (p->id == DOUBLE) {
     double a; memcpy(&a, alpha, 8);
-    permute2d_kernel<double><<<grid, block, 0, as_stream(w)>>>((const double*)x_vals, (double*)y_vals, p->m, p->n, a);
+    launch_pdl(permute2d_kernel<double>, dim3(grid), dim3(block), 0, as_stream(w), (const double*)x_vals, (double*)y_vals, p->m, p->n, a);
   } else { set_error(kUnsupported, "permutate: unsupported dtype"); return; }
   ZG_LAUNCH_CHECK();
 }
@@ -869,9 +896,9 @@ static void fold_rows_noalloc_launch(cudaStream_t s, const T* x, T* y, size_t ro
   if (!ZG_CUDA(cudaMemsetAsync(counters, 0, kNoAllocCounterBytes, s))) return;
   dim3 grid((unsigned)chunks, (unsigned)col_tiles, 1);
   if (vec) {
-    if constexpr (sizeof(T) == 4) fold_rows_kernel<T, true><<<grid, kRThreads, 0, s>>>(x, y, partial, counters, row, col, alpha, beta);
+    if constexpr (sizeof(T) == 4) fold_rows_kernel<T, true><<<grid, kRThreads, 0, s>>>(x, y, partial, counters, row, col, alpha, beta, 0);
   } else {
-    fold_rows_kernel<T, false><<<grid, kRThreads, 0, s>>>(x, y, partial, counters, row, col, alpha, beta);
+    fold_rows_kernel<T, false><<<grid, kRThreads, 0, s>>>(x, y, partial, counters, row, col, alpha, beta, 0);
   }
   ZG_LAUNCH_CHECK();
 }

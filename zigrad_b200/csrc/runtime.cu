@@ -98,12 +98,14 @@ __global__ void fill_kernel(T* __restrict__ p, size_t n, T v) {
 
 template <typename T>
 __global__ void sequence_kernel(T* __restrict__ p, size_t n, T init, T step) {
+  pdl_sync();
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) p[i] = init + step * (T)i;
 }
 
 template <typename T, typename I>
 __global__ void take_kernel(const T* __restrict__ src, const I* __restrict__ idx, size_t n, T* __restrict__ dst) {
+  pdl_sync();
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) dst[i] = src[idx[i]];
 }
@@ -132,6 +134,7 @@ __device__ __forceinline__ void philox4x32(uint64_t ctr, uint32_t seed, uint32_t
 
 template <typename T>
 __global__ void random_kernel(T* __restrict__ p, size_t n, int normal, uint32_t seed) {
+  pdl_sync();
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   const size_t ngroups = (n + 3) / 4;
   for (size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x; g < ngroups; g += stride) {
@@ -408,6 +411,7 @@ extern "C" void memcpy_DtoH(void* hptr, void const* dptr, len_t nbytes, StreamWr
 // 128-bit copy, four loads in flight per thread (large same-device copies: a
 // kernel reaches the HBM copy rate, the driver's device-to-device copy does not)
 __global__ void __launch_bounds__(256) copy16_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, size_t nv) {
+  pdl_sync();
   const size_t nth = (size_t)gridDim.x * blockDim.x;
   size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   for (; v + 3 * nth < nv; v += 4 * nth) {
@@ -431,7 +435,7 @@ extern "C" void memcpy_DtoD(void* dst, void const* src, len_t nbytes, StreamWrap
   if (nbytes >= ((len_t)1 << 20) && nbytes % 16 == 0 && host_aligned16(dst) && host_aligned16(src) && on_current_device(dst) &&
       on_current_device(src)) {
     const size_t nv = nbytes / 16;
-    copy16_kernel<<<grid_for(nv, 256 * 4), 256, 0, s>>>(static_cast<const uint4*>(src), static_cast<uint4*>(dst), nv);
+    launch_pdl(copy16_kernel, dim3(grid_for(nv, 256 * 4)), dim3(256), 0, s, static_cast<const uint4*>(src), static_cast<uint4*>(dst), nv);
     ZG_LAUNCH_CHECK();
     return;
   }
@@ -469,12 +473,12 @@ extern "C" void mem_sequence(dtype id, void* data, len_t n, const void* init, co
     float a, b;
     memcpy(&a, init, 4);
     memcpy(&b, step, 4);
-    sequence_kernel<float><<<grid_for(n, 256 * 8), 256, 0, s>>>(static_cast<float*>(data), n, a, b);
+    launch_pdl(sequence_kernel<float>, dim3(grid_for(n, 256 * 8)), dim3(256), 0, s, static_cast<float*>(data), n, a, b);
   } else if (id == DOUBLE) {
     double a, b;
     memcpy(&a, init, 8);
     memcpy(&b, step, 8);
-    sequence_kernel<double><<<grid_for(n, 256 * 8), 256, 0, s>>>(static_cast<double*>(data), n, a, b);
+    launch_pdl(sequence_kernel<double>, dim3(grid_for(n, 256 * 8)), dim3(256), 0, s, static_cast<double*>(data), n, a, b);
   } else {
     set_error(kUnsupported, "mem_sequence: unsupported dtype %d", (int)id);
     return;
@@ -486,8 +490,8 @@ extern "C" void mem_random(dtype id, void* x, len_t n, randtype op, unsigned see
   if (n == 0) return;
   cudaStream_t s = as_stream(stream);
   const unsigned g = grid_for((n + 3) / 4, 256 * 4);
-  if (id == SINGLE) random_kernel<float><<<g, 256, 0, s>>>(static_cast<float*>(x), n, op == NORMAL, seed);
-  else if (id == DOUBLE) random_kernel<double><<<g, 256, 0, s>>>(static_cast<double*>(x), n, op == NORMAL, seed);
+  if (id == SINGLE) launch_pdl(random_kernel<float>, dim3(g), dim3(256), 0, s, static_cast<float*>(x), n, op == NORMAL, seed);
+  else if (id == DOUBLE) launch_pdl(random_kernel<double>, dim3(g), dim3(256), 0, s, static_cast<double*>(x), n, op == NORMAL, seed);
   else { set_error(kUnsupported, "mem_random: unsupported dtype %d", (int)id); return; }
   ZG_LAUNCH_CHECK();
 }
@@ -498,9 +502,9 @@ extern "C" void mem_take(dtype id, const void* src, len_t /*src_len*/, const len
   cudaStream_t s = as_stream(stream);
   const unsigned g = grid_for(idxs_len, 256 * 4);
   if (id == SINGLE)
-    take_kernel<float, len_t><<<g, 256, 0, s>>>(static_cast<const float*>(src), idxs, idxs_len, static_cast<float*>(dst));
+    launch_pdl(take_kernel<float, len_t>, dim3(g), dim3(256), 0, s, static_cast<const float*>(src), idxs, idxs_len, static_cast<float*>(dst));
   else if (id == DOUBLE)
-    take_kernel<double, len_t><<<g, 256, 0, s>>>(static_cast<const double*>(src), idxs, idxs_len, static_cast<double*>(dst));
+    launch_pdl(take_kernel<double, len_t>, dim3(g), dim3(256), 0, s, static_cast<const double*>(src), idxs, idxs_len, static_cast<double*>(dst));
   else { set_error(kUnsupported, "mem_take: unsupported dtype %d", (int)id); return; }
   ZG_LAUNCH_CHECK();
 }
