@@ -14,6 +14,7 @@
 #include "gemm_skinny.cuh"
 #include "gemm_block.cuh"
 #include "mlp_tail.cuh"
+#include "mlp_tail_rows.cuh"
 #include "../../include/blas_conflux.h"
 
 namespace zg {
@@ -474,6 +475,18 @@ static bool launch_tail_inst(cudaStream_t s, const CUtensorMap& ta, const CUtens
   return launch_pdl(kern, dim3(grid), dim3(tail::kThreads), (size_t)tail::kSmemBytes, s, ta, tk, tn, t1, td1, td0, p);
 }
 
+template <int CP, int R, int T>
+static bool launch_tail_rows(cudaStream_t s, const tail_rows::Params& p) {
+  using L = tail_rows::Layout<CP, R, T>;
+  auto kern = tail_rows::mlp_tail_rows_kernel<CP, R, T>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    if (!ZG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kSmem))) return false;
+    attr_set = true;
+  }
+  return launch_pdl(kern, dim3((p.rows + R - 1) / R), dim3(T), L::kSmem, s, p);
+}
+
 void mlp_tail_launch(cudaStream_t s, len_t rows, len_t h1, len_t h2, len_t C, const void* act0, const void* W1, const void* b1, const void* W2,
                      const void* b2, const void* labels, int label_kind, len_t ld_out, double loss_div, void* act1, void* logits, void* loss_out,
                      void* dlogits, void* dact1, void* dact0, void* db2, void* db1, void* db0, int weights_ready) {
@@ -492,6 +505,34 @@ void mlp_tail_launch(cudaStream_t s, len_t rows, len_t h1, len_t h2, len_t C, co
     return;
   }
   if (ld_out > (len_t)tail::kCMax) { set_error(kBadArgument, "zg_mlp_tail_fwd_bwd: ld_out %lu above %d", ld_out, tail::kCMax); return; }
+  const unsigned sms = (unsigned)sm_count();
+  if (rows <= (len_t)sms * 2 * 28) {  // one wave of the row kernel; 16 rows per CTA while 28 would leave SMs idle
+    unsigned* counters = nullptr;
+    float* partial = static_cast<float*>(workspace(s, sizeof(float) * ((rows + 15) / 16), &counters));
+    if (!partial) return;
+    tail_rows::Params p;
+    memset(&p, 0, sizeof(p));
+    p.act0 = static_cast<const float*>(act0); p.W1 = static_cast<const float*>(W1); p.W2 = static_cast<const float*>(W2);
+    p.b1 = static_cast<const float*>(b1); p.b2 = static_cast<const float*>(b2);
+    p.labels = labels; p.label_index = label_kind == ZG_LABEL_INDEX ? 1 : 0;
+    p.act1 = static_cast<float*>(act1); p.dact1 = static_cast<float*>(dact1); p.dact0 = static_cast<float*>(dact0);
+    p.logits = static_cast<float*>(logits); p.dlogits = static_cast<float*>(dlogits);
+    p.db2 = static_cast<float*>(db2); p.db1 = static_cast<float*>(db1); p.db0 = static_cast<float*>(db0);
+    p.loss_out = static_cast<float*>(loss_out); p.loss_partial = partial; p.counter = counters;
+    p.rows = (uint32_t)rows; p.C = (uint32_t)C; p.ld_out = (uint32_t)ld_out;
+    p.divisor = (float)loss_div; p.inv_divisor = 1.f / p.divisor;
+    int e = 0;
+    p.exact_inv = (std::frexp(p.divisor, &e) == 0.5f && std::isnormal(p.inv_divisor)) ? 1 : 0;
+    p.early_weights = weights_ready ? 1 : 0;
+    const bool few = rows <= (len_t)sms * 16;
+#define ZG_TAIL_ROWS(CPV) few ? launch_tail_rows<CPV, 16, 256>(s, p) : launch_tail_rows<CPV, 28, 224>(s, p)
+    if (C <= 4) ZG_TAIL_ROWS(4);
+    else if (C <= 8) ZG_TAIL_ROWS(8);
+    else if (C <= 12) ZG_TAIL_ROWS(12);
+    else ZG_TAIL_ROWS(16);
+#undef ZG_TAIL_ROWS
+    return;
+  }
   CUtensorMap tmA, tmK, tmN, tm1, tmD1, tmD0;
   // outputs leave through TMA stores of [128 rows x 32 floats] slabs (rows past the end are clipped)
   if (!make_tmap(&tm1, false, act1, tail::kH2, rows, 1, tail::kH2, 32, tail::kRows, false)) return;

@@ -46,6 +46,7 @@
 // is bounded and reports through the time-out flag; after a failed wait a thread
 // skips its work but still takes part in every CTA barrier, so the CTA always
 // reaches its TMEM release.
+// For batches that fit on the chip a few rows at a time mlp_tail_rows.cuh is faster.
 #pragma once
 
 #include "gemm_tc.cuh"
