@@ -466,36 +466,57 @@ __device__ __forceinline__ void load_a_row(const uint8_t* a_stage, int row, floa
 }
 
 // One slab (ROWS rows x 32 k) of an fp32 operand into its swizzled place by 128 threads, 4 bytes per copy, lanes along
-// the contiguous dimension of the source; zeros outside [0, rows) x [0, k).
+// the contiguous dimension of the source.  The four warps' issue rate bounds it (a predicate and a pointer select per
+// copy made a 128x128 slab pair 2300 cycles, twice what its MMAs take), so a whole slab of whole k is an add and a copy
+// each.  Rows past the end of a K-major source repeat the last one (what they give lies outside C), elsewhere they are
+// zeroed: lanes that copy from one address are served one by one (2708x7x2708: 28 us against 13).  Past k the slab is zero.
 template <int ROWS, bool KMAJOR>
-__device__ __forceinline__ void direct_slab(uint8_t* dst, const float* src, uint64_t ld, uint32_t row0, uint32_t rows, uint32_t k0, uint32_t k, const float* safe) {
+__device__ __forceinline__ void direct_slab(uint8_t* dst, const float* src, uint64_t ld, uint32_t row0, uint32_t rows, uint32_t k0, uint32_t k) {
   const int w = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
   const uint32_t base = smem_u32(dst);
-  auto copy = [&](uint32_t to, const float* from, bool ok) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(ok ? from : safe), "r"(ok ? 4 : 0) : "memory");
+  auto copy = [&](uint32_t to, const float* from) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to), "l"(from) : "memory"); };
+  auto copy_if = [&](uint32_t to, const float* from, bool ok) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(ok ? from : src), "r"(ok ? 4 : 0) : "memory");
   };
+  const bool whole_k = k0 + 32 <= k;
   if constexpr (KMAJOR) {
-    const bool k_ok = k0 + lane < k;
-    const float* s = src + (uint64_t)(row0 + w) * ld + k0 + lane;
     const uint32_t d0 = base + w * kSlabBytes + (((lane >> 2) ^ w) << 4) + ((lane & 3) << 2);
     const uint32_t d1 = base + (w + 4) * kSlabBytes + (((lane >> 2) ^ (w + 4)) << 4) + ((lane & 3) << 2);
+    const uint32_t first = row0 + w < rows ? row0 + w : rows - 1;
+    const float* s = src + (uint64_t)first * ld + k0 + lane;
     const uint64_t step = 4 * ld;
+    auto to = [&](int i) { return ((i & 1) ? d1 : d0) + (i >> 1) * (8 * kSlabBytes); };
+    if (whole_k && row0 + ROWS <= rows) {
 #pragma unroll
-    for (int i = 0; i < ROWS / 4; ++i) {
-      copy(((i & 1) ? d1 : d0) + (i >> 1) * (8 * kSlabBytes), s, k_ok && row0 + w + 4 * i < rows);
-      s += step;
+      for (int i = 0; i < ROWS / 4; ++i) { copy(to(i), s); s += step; }
+    } else {
+      const bool k_ok = k0 + lane < k;
+#pragma unroll 8
+      for (int i = 0; i < ROWS / 4; ++i) {
+        copy_if(to(i), s, k_ok);
+        if (row0 + w + 4 * (i + 1) < rows) s += step;
+      }
     }
   } else {
     const uint32_t d = base + w * kSlabBytes + (((lane >> 3) ^ w) << 5) + ((lane & 7) << 2);
     const float* s = src + (uint64_t)(k0 + w) * ld + row0 + lane;
     const uint64_t step = 4 * ld;
+    if (whole_k && row0 + ROWS <= rows) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const bool k_ok = k0 + w + 4 * i < k;
+      for (int i = 0; i < 8; ++i) {
 #pragma unroll
-      for (int b = 0; b < ROWS / 32; ++b)
-        copy(d + b * (32 * kSlabBytes) + i * (4 * kSlabBytes), s + 32 * b, k_ok && row0 + 32 * b + lane < rows);
-      s += step;
+        for (int b = 0; b < ROWS / 32; ++b) copy(d + b * (32 * kSlabBytes) + i * (4 * kSlabBytes), s + 32 * b);
+        s += step;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const bool k_ok = k0 + w + 4 * i < k;
+#pragma unroll
+        for (int b = 0; b < ROWS / 32; ++b)
+          copy_if(d + b * (32 * kSlabBytes) + i * (4 * kSlabBytes), s + 32 * b, k_ok && row0 + 32 * b + lane < rows);
+        s += step;
+      }
     }
   }
 }
@@ -535,19 +556,16 @@ struct SmemLayout {
   static_assert(kBM * kOutPitch * 4 <= kStages * kStageBytes, "the output tile is staged in the ring");
 };
 
-// One lane's four columns of a row of the staged tile: alpha / beta / bias / ReLU / mask and the store.  VEC: four
-// consecutive columns with 16-byte (fp32) or 8-byte (bf16) accesses; else columns `stride` apart, so that the lanes of a
-// warp run along C's row either way.
+// One lane's four columns of a row of the staged tile.  VEC: four consecutive columns with 16-byte (fp32) or 8-byte (bf16)
+// accesses; else columns `stride` apart, so that the lanes of a warp run along C's row either way.
+// What the epilogue needs of C and the mask is requested before the sums are fetched ...
 template <bool VEC>
-__device__ __forceinline__ void store_row4(const Params& p, float (&v)[4], uint64_t row_off, uint32_t col, uint32_t stride, const float (&bias)[4]) {
-  const bool relu = p.epilogue == ZG_EPI_BIAS_RELU, masked = p.epilogue == ZG_EPI_RELU_MASK;
-  float c[4] = {0.f, 0.f, 0.f, 0.f}, mk[4] = {1.f, 1.f, 1.f, 1.f};
+__device__ __forceinline__ void fetch_row4(const Params& p, uint64_t row_off, uint32_t col, uint32_t stride, float (&c)[4], float (&mk)[4]) {
+  const bool masked = p.epilogue == ZG_EPI_RELU_MASK;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) { c[j] = 0.f; mk[j] = 1.f; }
   if constexpr (VEC) {
     const uint64_t o = row_off + col;
-    if (p.splits > 1 && !p.cluster) {
-      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p.C + o), "f"(p.alpha * v[0]), "f"(p.alpha * v[1]), "f"(p.alpha * v[2]), "f"(p.alpha * v[3]) : "memory");
-      return;
-    }
     auto get4 = [&](const float* f, const __nv_bfloat16* h, float (&d)[4]) {
       if (f) {
         const float4 x = *reinterpret_cast<const float4*>(f + o);
@@ -565,19 +583,33 @@ __device__ __forceinline__ void store_row4(const Params& p, float (&v)[4], uint6
     for (int j = 0; j < 4; ++j) {
       const uint32_t x = col + j * stride;
       if (x >= p.n) continue;
-      if (p.splits > 1 && !p.cluster) { atomicAdd(p.C + row_off + x, p.alpha * v[j]); continue; }
       if (p.beta != 0.f) c[j] = p.C ? p.C[row_off + x] : __bfloat162float(p.Cb[row_off + x]);
       if (masked) mk[j] = p.mask ? p.mask[row_off + x] : __bfloat162float(p.maskb[row_off + x]);
     }
-    if (p.splits > 1 && !p.cluster) return;
   }
+}
+// ... then alpha / beta / bias / ReLU / mask and the store (or the reduction into C)
+template <bool VEC>
+__device__ __forceinline__ void store_row4(const Params& p, float (&v)[4], uint64_t row_off, uint32_t col, uint32_t stride, const float (&bias)[4],
+                                           const float (&c)[4], const float (&mk)[4]) {
+  if (p.splits > 1 && !p.cluster) {
+    if constexpr (VEC) {
+      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p.C + row_off + col), "f"(p.alpha * v[0]), "f"(p.alpha * v[1]), "f"(p.alpha * v[2]), "f"(p.alpha * v[3]) : "memory");
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (col + j * stride < p.n) atomicAdd(p.C + row_off + col + j * stride, p.alpha * v[j]);
+    }
+    return;
+  }
+  const bool relu = p.epilogue == ZG_EPI_BIAS_RELU;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     v[j] = p.alpha * v[j];
     if (p.beta != 0.f) v[j] += p.beta * c[j];
     v[j] += bias[j];
     if (relu) v[j] = v[j] > 0.f ? v[j] : 0.f;
-    if (masked && mk[j] <= 0.f) v[j] = 0.f;
+    if (mk[j] <= 0.f) v[j] = 0.f;  // (1 where there is no mask)
   }
   if constexpr (VEC) {
     const uint64_t o = row_off + col;
@@ -641,7 +673,7 @@ __device__ __forceinline__ void staged_out_swapped(const Params& p, const float*
   const float bias = (p.epilogue == ZG_EPI_BIAS || p.epilogue == ZG_EPI_BIAS_RELU) ? __ldg(p.bias + col) : 0.f;
   const uint32_t base = smem_u32(tile);
   float cs = 0.f;
-#pragma unroll 2
+#pragma unroll 4
   for (uint32_t c = rank + threadIdx.x / kBM * ranks; c < (uint32_t)BN && r0 + c < p.m; c += NT / kBM * ranks) {
     float v = 0.f;
     const uint32_t at = r * PITCH + c;
@@ -673,37 +705,62 @@ __device__ __forceinline__ void staged_out(const Params& p, const float* tile, f
       for (int j = 0; j < 4; ++j)
         if (col + j * stride < p.n) bias[j] = __ldg(p.bias + col + j * stride);
     }
-    const uint32_t base = smem_u32(tile);
-    for (uint32_t r = rank + threadIdx.x / CG * ranks; r < (uint32_t)kBM && m0 + r < p.m; r += NT / CG * ranks) {
-      float v[4];
-      const uint32_t at = (r * PITCH + local) * 4;
-      if (ranks == 1) {
-        if constexpr (VEC) {
-          const float4 x = *reinterpret_cast<const float4*>(tile + r * PITCH + local);
-          v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-        } else {
+    const uint32_t base = smem_u32(tile), step = NT / CG * ranks;
+    constexpr int U = 2;  // rows in flight: a row is a round trip to memory (C, mask) beside one to the other ranks
+    for (uint32_t r0 = rank + threadIdx.x / CG * ranks; r0 < (uint32_t)kBM && m0 + r0 < p.m; r0 += U * step) {
+      float v[U][4], c[U][4], mk[U][4];
+      bool ok[U];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) v[j] = tile[r * PITCH + local + j * stride];
+      for (int u = 0; u < U; ++u) {
+        const uint32_t r = r0 + u * step;
+        ok[u] = r < (uint32_t)kBM && m0 + r < p.m;
+        if (ok[u]) fetch_row4<VEC>(p, batch_off + (uint64_t)(m0 + r) * p.ldc, col, stride, c[u], mk[u]);
+      }
+      if (ranks == 1) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (!ok[u]) continue;
+          const float* at = tile + (r0 + u * step) * PITCH + local;
+          if constexpr (VEC) {
+            const float4 x = *reinterpret_cast<const float4*>(at);
+            v[u][0] = x.x; v[u][1] = x.y; v[u][2] = x.z; v[u][3] = x.w;
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[u][j] = at[j * stride];
+          }
         }
       } else {
         // every rank's values are requested before the first is added: one round trip over the cluster network
-        float4 x[8];
+        float4 x[U][8];
 #pragma unroll
-        for (uint32_t k = 0; k < 8; ++k) {
-          x[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (k < ranks) {
-            const uint32_t a = map_rank(base, k) + at;
-            if constexpr (VEC) x[k] = ld_cluster4(a);
-            else { x[k].x = ld_cluster(a); x[k].y = ld_cluster(a + 4 * stride); x[k].z = ld_cluster(a + 8 * stride); x[k].w = ld_cluster(a + 12 * stride); }
+        for (int u = 0; u < U; ++u) {
+          if (!ok[u]) continue;
+          const uint32_t at = ((r0 + u * step) * PITCH + local) * 4;
+#pragma unroll
+          for (uint32_t k = 0; k < 8; ++k) {
+            x[u][k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (k < ranks) {
+              const uint32_t a = map_rank(base, k) + at;
+              if constexpr (VEC) x[u][k] = ld_cluster4(a);
+              else { x[u][k].x = ld_cluster(a); x[u][k].y = ld_cluster(a + 4 * stride); x[u][k].z = ld_cluster(a + 8 * stride); x[u][k].w = ld_cluster(a + 12 * stride); }
+            }
           }
         }
-        v[0] = v[1] = v[2] = v[3] = 0.f;
 #pragma unroll
-        for (uint32_t k = 0; k < 8; ++k) { v[0] += x[k].x; v[1] += x[k].y; v[2] += x[k].z; v[3] += x[k].w; }
+        for (int u = 0; u < U; ++u) {
+          if (!ok[u]) continue;
+          v[u][0] = v[u][1] = v[u][2] = v[u][3] = 0.f;
+#pragma unroll
+          for (uint32_t k = 0; k < 8; ++k) { v[u][0] += x[u][k].x; v[u][1] += x[u][k].y; v[u][2] += x[u][k].z; v[u][3] += x[u][k].w; }
+        }
       }
-      store_row4<VEC>(p, v, batch_off + (uint64_t)(m0 + r) * p.ldc, col, stride, bias);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) cs[j] += v[j];
+      for (int u = 0; u < U; ++u) {
+        if (!ok[u]) continue;
+        store_row4<VEC>(p, v[u], batch_off + (uint64_t)(m0 + r0 + u * step) * p.ldc, col, stride, bias, c[u], mk[u]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) cs[j] += v[u][j];
+      }
     }
     if (p.colsum) {
 #pragma unroll
@@ -824,8 +881,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
         uint8_t* st = stage_base + s * SL::kStageBytes;
         const uint32_t k0 = k_begin + kt * MT::kBK;
-        if (p.a_direct) direct_slab<kBM, A_KMAJOR>(st, a, p.a_ld, tile_m * kBM, rows_a, k0, p.k, p.a_src);
-        if (p.b_direct) direct_slab<BN, B_KMAJOR>(st + SL::kABytes, b, p.b_ld, tile_n * BN, rows_b, k0, p.k, p.b_src);
+        if (p.a_direct) direct_slab<kBM, A_KMAJOR>(st, a, p.a_ld, tile_m * kBM, rows_a, k0, p.k);
+        if (p.b_direct) direct_slab<BN, B_KMAJOR>(st + SL::kABytes, b, p.b_ld, tile_n * BN, rows_b, k0, p.k);
         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[s])) : "memory");
       }
       asm volatile("cp.async.wait_all;" ::: "memory");
