@@ -137,7 +137,7 @@ static bool launch_tc_inst(cudaStream_t s, const CUtensorMap& ta, const CUtensor
     if (!ZG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SL::kTotal))) return false;
     attr_set = true;
   }
-  return launch_pdl_cluster(kern, grid, dim3(SL::kThreads + (DIRECT ? 128 : 0)), (size_t)SL::kTotal, s, p.cluster ? p.splits : 1, ta, tb, tcm, p);
+  return launch_pdl_cluster(kern, grid, dim3(SL::kThreads + (DIRECT ? tc::kLoadWarps * 32 : 0)), (size_t)SL::kTotal, s, p.cluster ? p.splits : 1, ta, tb, tcm, p);
 }
 
 template <int MODE>

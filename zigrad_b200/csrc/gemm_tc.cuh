@@ -23,7 +23,7 @@
 //               current one over; one mbarrier arrival per warp.  With one set of
 //               A warps the serial chain of a slab (wait, split, tcgen05.st, wait)
 //               bounded the loop: 4096^3 650 -> 635 us, 128x784x8192 12.7 -> 12.3
-//   warps 12-15 DIRECT instances only: element-wise copies of operands whose rows no
+//   warps 12-19 DIRECT instances only: element-wise copies of operands whose rows no
 //               TMA box can address (1000x501x1000 with 501-float rows: 16 us
 //               against 66 on the FFMA path, 4096x1023x1023 80 against 385)
 //   warps 4-7   read the accumulator (tcgen05.ld: warp q reads TMEM lanes
@@ -101,7 +101,7 @@ struct Params {
   int cluster;
   int swap;  // the tile is C transposed: its rows are C's columns (short C: the long dimension fills the 128 rows)
   // Operands whose rows no TMA box can address (base or row stride not a multiple of 16 bytes) come through
-  // element-wise cp.async of four loader warps into the same swizzled slabs (DIRECT instances only).
+  // element-wise cp.async of loader warps into the same swizzled slabs (DIRECT instances only).
   int a_direct, b_direct;
   const float* a_src;
   const float* b_src;
@@ -465,14 +465,15 @@ __device__ __forceinline__ void load_a_row(const uint8_t* a_stage, int row, floa
   }
 }
 
-// One slab (ROWS rows x 32 k) of an fp32 operand into its swizzled place by 128 threads, 4 bytes per copy, lanes along
+constexpr int kLoadWarps = 8;
+// One slab (ROWS rows x 32 k) of an fp32 operand into its swizzled place by 256 threads, 4 bytes per copy, lanes along
 // the contiguous dimension of the source.  The four warps' issue rate bounds it (a predicate and a pointer select per
 // copy made a 128x128 slab pair 2300 cycles, twice what its MMAs take), so a whole slab of whole k is an add and a copy
 // each.  Rows past the end of a K-major source repeat the last one (what they give lies outside C), elsewhere they are
 // zeroed: lanes that copy from one address are served one by one (2708x7x2708: 28 us against 13).  Past k the slab is zero.
 template <int ROWS, bool KMAJOR>
 __device__ __forceinline__ void direct_slab(uint8_t* dst, const float* src, uint64_t ld, uint32_t row0, uint32_t rows, uint32_t k0, uint32_t k) {
-  const int w = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
+  const int w = (threadIdx.x >> 5) & 7, lane = threadIdx.x & 31;
   const uint32_t base = smem_u32(dst);
   auto copy = [&](uint32_t to, const float* from) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to), "l"(from) : "memory"); };
   auto copy_if = [&](uint32_t to, const float* from, bool ok) {
@@ -480,41 +481,40 @@ __device__ __forceinline__ void direct_slab(uint8_t* dst, const float* src, uint
   };
   const bool whole_k = k0 + 32 <= k;
   if constexpr (KMAJOR) {
-    const uint32_t d0 = base + w * kSlabBytes + (((lane >> 2) ^ w) << 4) + ((lane & 3) << 2);
-    const uint32_t d1 = base + (w + 4) * kSlabBytes + (((lane >> 2) ^ (w + 4)) << 4) + ((lane & 3) << 2);
+    const uint32_t d = base + w * kSlabBytes + (((lane >> 2) ^ w) << 4) + ((lane & 3) << 2);
     const uint32_t first = row0 + w < rows ? row0 + w : rows - 1;
     const float* s = src + (uint64_t)first * ld + k0 + lane;
-    const uint64_t step = 4 * ld;
-    auto to = [&](int i) { return ((i & 1) ? d1 : d0) + (i >> 1) * (8 * kSlabBytes); };
+    const uint64_t step = 8 * ld;
+    auto to = [&](int i) { return d + i * (8 * kSlabBytes); };
     if (whole_k && row0 + ROWS <= rows) {
 #pragma unroll
-      for (int i = 0; i < ROWS / 4; ++i) { copy(to(i), s); s += step; }
+      for (int i = 0; i < ROWS / 8; ++i) { copy(to(i), s); s += step; }
     } else {
       const bool k_ok = k0 + lane < k;
 #pragma unroll 8
-      for (int i = 0; i < ROWS / 4; ++i) {
+      for (int i = 0; i < ROWS / 8; ++i) {
         copy_if(to(i), s, k_ok);
-        if (row0 + w + 4 * (i + 1) < rows) s += step;
+        if (row0 + w + 8 * (i + 1) < rows) s += step;
       }
     }
   } else {
-    const uint32_t d = base + w * kSlabBytes + (((lane >> 3) ^ w) << 5) + ((lane & 7) << 2);
+    const uint32_t d = base + w * kSlabBytes + (((lane >> 3) ^ (w & 3)) << 5) + ((lane & 7) << 2);
     const float* s = src + (uint64_t)(k0 + w) * ld + row0 + lane;
-    const uint64_t step = 4 * ld;
+    const uint64_t step = 8 * ld;
     if (whole_k && row0 + ROWS <= rows) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
+      for (int i = 0; i < 4; ++i) {
 #pragma unroll
-        for (int b = 0; b < ROWS / 32; ++b) copy(d + b * (32 * kSlabBytes) + i * (4 * kSlabBytes), s + 32 * b);
+        for (int b = 0; b < ROWS / 32; ++b) copy(d + b * (32 * kSlabBytes) + i * (8 * kSlabBytes), s + 32 * b);
         s += step;
       }
     } else {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const bool k_ok = k0 + w + 4 * i < k;
+      for (int i = 0; i < 4; ++i) {
+        const bool k_ok = k0 + w + 8 * i < k;
 #pragma unroll
         for (int b = 0; b < ROWS / 32; ++b)
-          copy_if(d + b * (32 * kSlabBytes) + i * (4 * kSlabBytes), s + 32 * b, k_ok && row0 + 32 * b + lane < rows);
+          copy_if(d + b * (32 * kSlabBytes) + i * (8 * kSlabBytes), s + 32 * b, k_ok && row0 + 32 * b + lane < rows);
         s += step;
       }
     }
@@ -551,7 +551,7 @@ struct SmemLayout {
   static constexpr int kBWordsA = BN >= 128 ? 4 : (BN >= 64 ? 1 : 0);
   static constexpr int kBWordsB = (BN * 8 - 128 * kBWordsA) / 64;
   // FP32X3: two sets of four A warps take the slabs in turn
-  static constexpr int kThreads = X3 ? 384 : kThreadsTc;  // + 128 with direct operands
+  static constexpr int kThreads = X3 ? 384 : kThreadsTc;  // + kLoadWarps * 32 with direct operands
   static constexpr int kOutPitch = BN + 4;  // floats per row of the staged output tile
   static_assert(kBM * kOutPitch * 4 <= kStages * kStageBytes, "the output tile is staged in the ring");
 };
@@ -692,8 +692,9 @@ __device__ __forceinline__ void staged_out_swapped(const Params& p, const float*
 }
 
 // The staged tile (128 x BN floats, pitch BN + 4, all CTAs of a cluster hold partial sums) to C: NT threads, lanes along
-// the rows of C.  col_part: BN zeroed floats.
-template <int BN, int NT, bool VEC>
+// the rows of C, U rows in flight (a row of a lone CTA is a round trip to memory for C and the mask; one of a cluster
+// already has a load to every rank in flight, two measured slower).  col_part: BN zeroed floats.
+template <int BN, int NT, bool VEC, int U>
 __device__ __forceinline__ void staged_out(const Params& p, const float* tile, float* col_part, uint32_t split, uint32_t m0, uint32_t n0, uint64_t batch_off) {
   constexpr int CG = BN / 4, PITCH = BN + 4;
   const uint32_t cg = threadIdx.x % CG, ranks = p.cluster ? p.splits : 1, rank = p.cluster ? split : 0;
@@ -706,7 +707,6 @@ __device__ __forceinline__ void staged_out(const Params& p, const float* tile, f
         if (col + j * stride < p.n) bias[j] = __ldg(p.bias + col + j * stride);
     }
     const uint32_t base = smem_u32(tile), step = NT / CG * ranks;
-    constexpr int U = 2;  // rows in flight: a row is a round trip to memory (C, mask) beside one to the other ranks
     for (uint32_t r0 = rank + threadIdx.x / CG * ranks; r0 < (uint32_t)kBM && m0 + r0 < p.m; r0 += U * step) {
       float v[U][4], c[U][4], mk[U][4];
       bool ok[U];
@@ -774,7 +774,7 @@ __device__ __forceinline__ void staged_out(const Params& p, const float* tile, f
 }
 
 template <int BN, bool A_KMAJOR, bool B_KMAJOR, int MODE, bool DIRECT = false>
-__global__ void __launch_bounds__((SmemLayout<BN, MODE>::kThreads + (DIRECT ? 128 : 0)), 1)
+__global__ void __launch_bounds__((SmemLayout<BN, MODE>::kThreads + (DIRECT ? kLoadWarps * 32 : 0)), 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
                const Params p) {
   static_assert(!DIRECT || MODE == kFP32X3, "direct operands: FP32X3 only");
@@ -812,7 +812,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   if (threadIdx.x == 0) {
     failed = 0;
     for (int s = 0; s < S; ++s) {
-      mbar_init(&full[s], DIRECT ? 1 + 128 : 1);  // the TMA thread, and every loader thread's copies
+      mbar_init(&full[s], DIRECT ? 1 + kLoadWarps * 32 : 1);  // the TMA thread, and every loader thread's copies
       mbar_init(&ready[s], kSplitThreads / 32);  // one arrival per split warp (of the slab's set)
       mbar_init(&empty[s], 1);
     }
@@ -1137,11 +1137,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   if (!p.tma_epilogue) {
     const float* tile = reinterpret_cast<const float*>(stage_base);
     if (p.cluster) cluster_sync(); else __syncthreads();
-    constexpr int NT = SL::kThreads + (DIRECT ? 128 : 0);
+    constexpr int NT = SL::kThreads + (DIRECT ? kLoadWarps * 32 : 0);
     const uint64_t batch_off = (uint64_t)batch * p.c_batch_stride;
     if (p.swap) staged_out_swapped<BN, NT>(p, tile, split, tile_m * kBM, tile_n * BN, batch_off);
-    else if (p.vec_ok && (p.n & 3u) == 0) staged_out<BN, NT, true>(p, tile, col_part, split, tile_m * kBM, tile_n * BN, batch_off);
-    else staged_out<BN, NT, false>(p, tile, col_part, split, tile_m * kBM, tile_n * BN, batch_off);
+    else if (p.vec_ok && (p.n & 3u) == 0) {
+      if (p.cluster) staged_out<BN, NT, true, 1>(p, tile, col_part, split, tile_m * kBM, tile_n * BN, batch_off);
+      else staged_out<BN, NT, true, 2>(p, tile, col_part, split, tile_m * kBM, tile_n * BN, batch_off);
+    } else {
+      if (p.cluster) staged_out<BN, NT, false, 1>(p, tile, col_part, split, tile_m * kBM, tile_n * BN, batch_off);
+      else staged_out<BN, NT, false, 2>(p, tile, col_part, split, tile_m * kBM, tile_n * BN, batch_off);
+    }
     if (p.cluster) cluster_sync();  // nobody leaves while its partial tile may still be read
   }
 
