@@ -302,10 +302,22 @@ EXTERN_C void zg_adam_step_part(dtype id, StreamWrapper stream, void* params, vo
                                 double lr, double beta1, double beta2, double eps,
                                 int clip, double max_norm, double delta, void* norms, void* bf16_copy, void* step_counter,
                                 int advance_counter);
+/* zg_adam_step followed by the soft update of a target network's parameters (laid out like `params`):
+ * target = tau * params + (1 - tau) * target, in the same launch for small models. */
+EXTERN_C void zg_adam_soft_step(dtype id, StreamWrapper stream, void* params, void* grads, void* m, void* v, const zg_segment* seg, len_t n_seg,
+                                len_t t_first, double lr, double beta1, double beta2, double eps, int clip, double max_norm, double delta,
+                                void* norms, void* step_counter, void* target, double tau);
 /* out[j] = sum of squares of segment j (fp64 accumulation, deterministic two-stage): the
  * shard-local part of the per-tensor gradient norm of host_device.zig:339-346 */
 EXTERN_C void zg_segment_sumsq(dtype id, StreamWrapper stream, const void* x, const zg_segment* seg, len_t n_seg, void* out);
 /* target[i] = tau*src[i] + (1-tau)*target[i] (examples/dqn/src/dqn_agent.zig:111-123) */
+/* The ops between the forward passes of a Q-learning update and its backward pass as one launch (a dozen ops of the device
+ * interface; examples/dqn/src/dqn_agent.zig:111-228).  qn = the target network's values of the next states, q = the
+ * policy's of the states, both [batch, actions] and clamped in place; dq, dbias, loss, .. are overwritten. */
+EXTERN_C int zg_q_head_supported(dtype id, len_t batch, len_t actions);
+EXTERN_C void zg_q_head(dtype id, StreamWrapper stream, len_t batch, len_t actions, void* qn, void* q, const len_t* action, const void* rewards,
+                        const void* dones, double gamma, double q_clip, double beta, void* maxq, void* targets, void* chosen, len_t* offsets,
+                        void* loss, void* dchosen, void* dq, void* dbias);
 EXTERN_C void zg_soft_update(dtype id, StreamWrapper stream, const void* src, void* target, len_t n, double tau);
 /* fp32 -> bf16 (round to nearest even) and back */
 EXTERN_C void zg_cast(dtype src_id, dtype dst_id, StreamWrapper stream, const void* src, void* dst, len_t n);

@@ -1172,6 +1172,128 @@ extern "C" void zg_softmax_ce_fwd_bwd(dtype id, StreamWrapper w, const void* log
   else set_error(kBadArgument, "zg_softmax_ce_fwd_bwd: unknown label kind %d", label_kind);
 }
 
+// ---------------------------------------------------------------- Q learning
+// Everything between the two forward passes of a Q-learning update and its backward pass, as one launch
+// (examples/dqn/src/dqn_agent.zig:111-228): as the device interface spells it these are a dozen ops over a few kilobytes,
+// a chain of launches that takes longer than both networks' forward passes.
+//   qn, q    <- clamp +-q_clip in place;   maxq = max over the actions of qn
+//   targets   = clamp(reward + (gamma * maxq) * (1 - done))
+//   chosen    = q[action];  loss = smooth L1(chosen, targets, beta);  dchosen = its gradient
+//   dq        = dchosen scattered into zeros;  dbias = its column sums
+// Operation for operation the separate ops (clamp, max_along, mul, sub, mul, add, clamp, gather, smooth_l1, scatter_add,
+// unbroadcast).  A thread per row; loss and column sums per CTA, folded by the CTA that draws the last ticket.
+struct QHead {
+  float *qn, *q;                       // [B, A]
+  const len_t* actions;
+  const float *rewards, *dones;
+  float gamma, q_clip, beta;
+  float *maxq, *targets, *chosen, *dchosen, *dq, *dbias, *loss;
+  len_t* offsets;
+  float* partial;                      // [grid][A + 1]
+  unsigned* ticket;
+  unsigned B, A;
+};
+
+__device__ __forceinline__ float clamp_to(float x, float lo, float hi) {
+  float t = (x > lo || lo != lo) ? x : lo;  // a NaN operand is dropped, as in the clamp op
+  if (x != x) t = lo;
+  return (t < hi) ? t : hi;
+}
+
+__global__ void __launch_bounds__(kLThreads) q_head_kernel(const QHead a) {
+  extern __shared__ float cols[];  // [warps][A]
+  __shared__ float sm32[32];
+  __shared__ bool last;
+  pdl_sync();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, A = (int)a.A;
+  const float fn = (float)a.B;
+  for (int c = threadIdx.x; c < A * (kLThreads / 32); c += kLThreads) cols[c] = 0.f;
+  __syncthreads();
+  float loss = 0.f;
+  for (size_t r0 = (size_t)blockIdx.x * kLThreads; r0 < a.B; r0 += (size_t)gridDim.x * kLThreads) {
+    const size_t r = r0 + threadIdx.x;
+    const bool ok = r < a.B;
+    float g = 0.f;
+    int act = -1;
+    if (ok) {
+      float mx = -INFINITY;
+      for (int c = 0; c < A; ++c) {
+        const float x = clamp_to(a.qn[r * A + c], -a.q_clip, a.q_clip);
+        a.qn[r * A + c] = x;
+        if (x > mx) mx = x;
+        a.q[r * A + c] = clamp_to(a.q[r * A + c], -a.q_clip, a.q_clip);
+      }
+      a.maxq[r] = mx;
+      const float left = 1.f - a.dones[r];
+      float t = a.gamma * mx;
+      t = t * left;
+      t = clamp_to(a.rewards[r] + t, -a.q_clip, a.q_clip);
+      a.targets[r] = t;
+      const len_t want = a.actions[r];
+      const bool in = want < (len_t)A;  // the reference returns error.IndexOutOfBounds; never read out of range
+      act = in ? (int)want : 0;
+      const float pred = in ? a.q[r * A + act] : 0.f;
+      a.chosen[r] = pred;
+      a.offsets[r] = r * A + act;
+      const float d = pred - t, ad = fabsf(d);
+      if (ad < a.beta) {
+        loss += 0.5f * (d * d) / a.beta;
+        g = d / (a.beta * fn);
+      } else {
+        loss += ad - (0.5f * a.beta);
+        g = (float)((d > 0.f) - (d < 0.f)) / fn;
+      }
+      a.dchosen[r] = g;
+      for (int c = 0; c < A; ++c) a.dq[r * A + c] = c == act ? g : 0.f;
+    }
+    for (int c = 0; c < A; ++c) {
+      const float s = warp_sum(c == act ? g : 0.f);
+      if (lane == 0) cols[warp * A + c] += s;
+    }
+  }
+  const float bs = block_sum<float>(loss, sm32);
+  float* mine = a.partial + (size_t)blockIdx.x * (A + 1);
+  if (threadIdx.x == 0) mine[A] = bs;
+  __syncthreads();
+  for (int c = threadIdx.x; c < A; c += kLThreads) {
+    float s = 0.f;
+    for (int w = 0; w < kLThreads / 32; ++w) s += cols[w * A + c];
+    mine[c] = s;
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+    if (last) *a.ticket = 0;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int c = threadIdx.x; c <= A; c += kLThreads) {
+    float s = 0.f;
+    for (unsigned k = 0; k < gridDim.x; ++k) s += __ldcg(a.partial + (size_t)k * (A + 1) + c);
+    if (c < A) a.dbias[c] = s;
+    else *a.loss = s / fn;
+  }
+}
+
+extern "C" int zg_q_head_supported(dtype id, len_t batch, len_t actions) {
+  return id == SINGLE && batch > 0 && batch <= 0xffffffffu && actions > 0 && actions <= 64 ? 1 : 0;
+}
+extern "C" void zg_q_head(dtype id, StreamWrapper w, len_t batch, len_t actions, void* qn, void* q, const len_t* action, const void* rewards,
+                          const void* dones, double gamma, double q_clip, double beta, void* maxq, void* targets, void* chosen, len_t* offsets,
+                          void* loss, void* dchosen, void* dq, void* dbias) {
+  if (!zg_q_head_supported(id, batch, actions)) { set_error(kUnsupported, "zg_q_head: %lu x %lu", batch, actions); return; }
+  cudaStream_t s = as_stream(w);
+  const unsigned g = grid_for(batch, kLThreads);
+  unsigned* counters = nullptr;
+  float* partial = static_cast<float*>(workspace(s, sizeof(float) * g * (actions + 1), &counters));
+  if (!partial) return;
+  QHead a{(float*)qn, (float*)q, action, (const float*)rewards, (const float*)dones, (float)gamma, (float)q_clip, (float)beta, (float*)maxq, (float*)targets,
+          (float*)chosen, (float*)dchosen, (float*)dq, (float*)dbias, (float*)loss, offsets, partial, counters, (unsigned)batch, (unsigned)actions};
+  launch_pdl(q_head_kernel, dim3(g), dim3(kLThreads), sizeof(float) * actions * (kLThreads / 32), s, a);
+}
+
 extern "C" void zg_smooth_l1_fwd_bwd(dtype id, StreamWrapper w, const void* pred, const void* target, len_t n, double beta,
                                      void* loss_out, void* grad) {
   if (id != SINGLE) { set_error(kUnsupported, "zg_smooth_l1_fwd_bwd: only SINGLE is implemented"); return; }

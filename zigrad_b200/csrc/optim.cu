@@ -4,6 +4,8 @@
 #include <cmath>
 #include <cstring>
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace zg {
@@ -135,12 +137,112 @@ __global__ void __launch_bounds__(kOThreads) sgd_kernel(float* params, float* gr
   }
 }
 
-// Adam in fp32, operation for operation as the reference loop:
+// Adam in fp32, operation for operation as the reference loop (no contraction: the file is built with --fmad=false):
 //   m = b1*m + (1-b1)*g ; v = b2*v + (1-b2)*g*g ; p -= lr_t * m / (sqrt(v) + eps)
+struct AdamScalars {
+  float b1, b2, omb1, omb2, eps;
+  __device__ __forceinline__ void apply(float g, float& m, float& v, float& p, float lr_t) const {
+    m = b1 * m + omb1 * g;
+    v = b2 * v + omb2 * g * g;
+    p = p - lr_t * m / (sqrtf(v) + eps);
+  }
+  // bias-corrected step size of the tensor whose update is the t-th
+  __device__ __forceinline__ float step_size(float lr, float t) const { return lr * sqrtf(1.f - powf(b2, t)) / (1.f - powf(b1, t)); }
+};
+
+// A whole optimizer step of a small model in one launch: gradient norms, clipping, Adam, step counter and (optionally) the
+// soft update of a target network.  As separate launches these are four passes of a few microseconds over tens of
+// kilobytes; one cluster of eight CTAs holds the grid-wide barrier that the norms need.  17 K parameters (DQN): @@ us
+// against @@; the eight SMs' bandwidth makes larger models slower than separate passes over the whole chip.
+constexpr int kSmallThreads = 1024, kSmallCtas = 8;
+constexpr size_t kSmallParams = 128 * 1024;
+
+struct AdamSmall {
+  float *p, *g, *m, *v, *norms;
+  const float* given;                 // clip == 2: norms that are known already
+  float* target;                      // or nullptr: target = tau * p + (1 - tau) * target
+  __nv_bfloat16* copy;                // or nullptr
+  unsigned long long* t_dev;          // or nullptr: the sizes come from the table
+  float lr, max_norm, delta, tau;
+  int clip, advance;
+  AdamScalars a;
+};
+
+__global__ void __launch_bounds__(kSmallThreads) adam_small_kernel(const AdamSmall q, const __grid_constant__ SegTable tab) {
+  __shared__ double warp_sums[kSmallThreads / 32], sums[kMaxSeg];
+  __shared__ float norm[kMaxSeg], lr_t[kMaxSeg];
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  pdl_sync();
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const size_t tid = (size_t)blockIdx.x * kSmallThreads + t, nth = (size_t)kSmallThreads * kSmallCtas;
+  if (t < tab.n) lr_t[t] = q.t_dev ? q.a.step_size(q.lr, (float)(*q.t_dev + (unsigned long long)(t + 1))) : tab.lr_t[t];
+  if (q.clip == 1) {
+    for (int s = 0; s < tab.n; ++s) {
+      const float* g = q.g + tab.offset[s];
+      const size_t n = tab.len[s];
+      float acc = 0.f;
+#pragma unroll 4
+      for (size_t i = tid; i < n; i += nth) acc += g[i] * g[i];
+      const double w = warp_sum((double)acc);
+      if (lane == 0) warp_sums[warp] = w;
+      __syncthreads();
+      if (warp == 0) {
+        const double c = warp_sum(warp_sums[lane]);
+        if (lane == 0) sums[s] = c;
+      }
+      __syncthreads();
+    }
+  }
+  cluster.sync();  // every CTA's sums are there, and every CTA has read the counter
+  if (t < tab.n && q.clip) {
+    if (q.clip == 1) {
+      double c = 0.0;
+      for (int r = 0; r < kSmallCtas; ++r) c += cluster.map_shared_rank(sums, r)[t];
+      norm[t] = (float)sqrt(c);
+      if (blockIdx.x == 0) q.norms[t] = norm[t];
+    } else {
+      norm[t] = q.given[t];
+    }
+  }
+  if (blockIdx.x == 0 && t == 0 && q.t_dev && q.advance) *q.t_dev += (unsigned long long)tab.n;
+  __syncthreads();
+  constexpr int U = 4;
+  for (int s = 0; s < tab.n; ++s) {
+    const size_t off = tab.offset[s], n = tab.len[s];
+    const float step = lr_t[s];
+    const bool on = q.clip && norm[s] > q.max_norm;
+    const float f = on ? q.max_norm / (norm[s] + q.delta) : 1.f;
+    for (size_t i0 = tid; i0 < n; i0 += U * nth) {
+      float g[U], m[U], v[U], p[U], target[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const size_t i = off + i0 + u * nth;
+        if (i0 + u * nth < n) {
+          g[u] = q.g[i]; m[u] = q.m[i]; v[u] = q.v[i]; p[u] = q.p[i];
+          if (q.target) target[u] = q.target[i];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const size_t i = off + i0 + u * nth;
+        if (i0 + u * nth >= n) continue;
+        if (on) { g[u] *= f; q.g[i] = g[u]; }
+        q.a.apply(g[u], m[u], v[u], p[u], step);
+        q.m[i] = m[u]; q.v[i] = v[u]; q.p[i] = p[u];
+        if (q.copy) q.copy[i] = __float2bfloat16_rn(p[u]);
+        if (q.target) q.target[i] = q.tau * p[u] + (1.f - q.tau) * target[u];
+      }
+    }
+  }
+  if (q.clip == 1) cluster.sync();  // nobody leaves while its sums may still be read
+}
+
 template <bool CLIP, bool BF16COPY>
 __global__ void __launch_bounds__(kOThreads) adam_kernel(float* params, float* grads, float* ms, float* vs, const __grid_constant__ SegTable tab,
-                                                         float b1, float b2, float eps, const float* __restrict__ norms, float max_norm,
-                                                         float delta, __nv_bfloat16* copy, const unsigned long long* t_dev, float lr) {
+                                                         const AdamScalars a, const float* __restrict__ norms, float max_norm,
+                                                         float delta, __nv_bfloat16* copy, unsigned long long* t_dev, float lr,
+                                                         unsigned* ticket, unsigned long long advance) {
   pdl_sync();
   const int seg = blockIdx.y;
   const size_t off = tab.offset[seg];
@@ -151,20 +253,22 @@ __global__ void __launch_bounds__(kOThreads) adam_kernel(float* params, float* g
   const size_t n = tab.len[seg];
   float lr_t = tab.lr_t[seg];
   if (t_dev) {  // step counter kept on the device (graph replay): t = counter + position of this tensor
-    const float t_f = (float)(*t_dev + (unsigned long long)(tab.first + seg + 1));
-    lr_t = lr * sqrtf(1.f - powf(b2, t_f)) / (1.f - powf(b1, t_f));
+    lr_t = a.step_size(lr, (float)(*t_dev + (unsigned long long)(tab.first + seg + 1)));
+    if (advance) {  // the CTA that draws the last ticket moves the counter on: by then every CTA has read it
+      __syncthreads();
+      if (threadIdx.x == 0 && atomicAdd(ticket, 1u) == gridDim.x * gridDim.y - 1) {
+        *ticket = 0;
+        *t_dev += advance;
+      }
+    }
   }
-  const float omb1 = 1.f - b1, omb2 = 1.f - b2;
   bool on = false;
   float f = 1.f;
   if (CLIP) f = clip_factor(norms, tab.first + seg, max_norm, delta, &on);
   const size_t nth = (size_t)gridDim.x * blockDim.x, tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  // one element, operation for operation as the host loop (no contraction: the file is built with --fmad=false)
   auto one = [&](float& gi, float& mi, float& vi, float& pi) {
     if (CLIP && on) gi *= f;
-    mi = b1 * mi + omb1 * gi;
-    vi = b2 * vi + omb2 * gi * gi;
-    pi = pi - lr_t * mi / (sqrtf(vi) + eps);
+    a.apply(gi, mi, vi, pi, lr_t);
   };
   auto scalar = [&](size_t i) {
     float gi = g[i], mi = m[i], vi = v[i], pi = p[i];
@@ -204,11 +308,6 @@ __global__ void __launch_bounds__(kOThreads) adam_kernel(float* params, float* g
     }
   }
   for (size_t i = head + nv * 4 + tid; i < n; i += nth) scalar(i);
-}
-
-__global__ void counter_add_kernel(unsigned long long* c, unsigned long long inc) {
-  pdl_sync();
-  *c += inc;
 }
 
 static unsigned chunks_for(const zg_segment* seg, size_t n_seg) {
@@ -263,17 +362,14 @@ extern "C" void zg_sgd_step(dtype id, StreamWrapper w, void* params, void* grads
   }
 }
 
-extern "C" void zg_adam_step_part(dtype id, StreamWrapper w, void* params, void* grads, void* m, void* v, const zg_segment* seg, len_t n_seg,
-                                  len_t t_first, double lr_, double beta1_, double beta2_, double eps_, int clip, double max_norm, double delta,
-                                  void* norms, void* bf16_copy, void* step_counter, int advance_counter) {
-  if (id != SINGLE) { set_error(kUnsupported, "zg_adam_step: only SINGLE is implemented"); return; }
-  const unsigned long long* TD = static_cast<const unsigned long long*>(step_counter);
+static void adam_step(cudaStream_t s, float* P, float* G, float* M, float* V, const zg_segment* seg, len_t n_seg, len_t t_first, double lr_,
+                      double beta1_, double beta2_, double eps_, int clip, double max_norm, double delta, float* norms, __nv_bfloat16* cp,
+                      unsigned long long* t_dev, int advance, float* target, double tau) {
   if (n_seg == 0) return;
-  cudaStream_t s = as_stream(w);
-  const float lr = (float)lr_, beta1 = (float)beta1_, beta2 = (float)beta2_, eps = (float)eps_;
-  if (clip == 1 && !compute_norms(s, (const float*)grads, seg, n_seg, (float*)norms)) return;
-  if (clip == 2 && !norms) { set_error(kBadArgument, "optimizer: clip with given norms but norms is NULL"); return; }
-  for (size_t first = 0; first < n_seg; first += kMaxSeg) {
+  const float lr = (float)lr_, beta1 = (float)beta1_, beta2 = (float)beta2_;
+  const AdamScalars a{beta1, beta2, 1.f - beta1, 1.f - beta2, (float)eps_};
+  if (clip && !norms) { set_error(kBadArgument, "optimizer: clip %s but norms is NULL", clip == 2 ? "with given norms" : "requested"); return; }
+  auto table = [&](size_t first) {
     SegTable tab;
     memset(&tab, 0, sizeof(tab));
     tab.n = (int)((n_seg - first) < (size_t)kMaxSeg ? (n_seg - first) : kMaxSeg);
@@ -284,20 +380,48 @@ extern "C" void zg_adam_step_part(dtype id, StreamWrapper w, void* params, void*
       const float t_f = (float)(t_first + first + j);  // counter advances once per tensor (optim.zig:189)
       tab.lr_t[j] = lr * std::sqrt(1.f - std::pow(beta2, t_f)) / (1.f - std::pow(beta1, t_f));
     }
-    const dim3 grid(chunks_for(seg + first, tab.n), tab.n);
-    float* P = (float*)params; float* G = (float*)grads; float* M = (float*)m; float* V = (float*)v;
-    __nv_bfloat16* cp = (__nv_bfloat16*)bf16_copy;
-    const float* NR = (const float*)norms;
-    __nv_bfloat16* no_copy = nullptr;
-    const dim3 blk(kOThreads);
-    if (clip && cp) launch_pdl(adam_kernel<true, true>, grid, blk, 0, s, P, G, M, V, tab, beta1, beta2, eps, NR, (float)max_norm, (float)delta, cp, TD, lr);
-    else if (clip) launch_pdl(adam_kernel<true, false>, grid, blk, 0, s, P, G, M, V, tab, beta1, beta2, eps, NR, (float)max_norm, (float)delta, no_copy, TD, lr);
-    else if (cp) launch_pdl(adam_kernel<false, true>, grid, blk, 0, s, P, G, M, V, tab, beta1, beta2, eps, (const float*)nullptr, 0.f, 0.f, cp, TD, lr);
-    else launch_pdl(adam_kernel<false, false>, grid, blk, 0, s, P, G, M, V, tab, beta1, beta2, eps, (const float*)nullptr, 0.f, 0.f, no_copy, TD, lr);
+    return tab;
+  };
+  size_t total = 0;
+  for (len_t j = 0; j < n_seg; ++j) total += seg[j].len;
+  if (n_seg <= (len_t)kMaxSeg && total <= kSmallParams) {
+    AdamSmall q;
+    memset(&q, 0, sizeof(q));
+    q.p = P; q.g = G; q.m = M; q.v = V; q.norms = norms; q.given = norms; q.target = target; q.copy = cp; q.t_dev = t_dev;
+    q.lr = lr; q.max_norm = (float)max_norm; q.delta = (float)delta; q.tau = (float)tau; q.clip = clip; q.advance = advance; q.a = a;
+    launch_pdl_cluster(adam_small_kernel, dim3(kSmallCtas), dim3(kSmallThreads), 0, s, kSmallCtas, q, table(0));
+    return;
   }
-  if (step_counter && advance_counter) {  // advance the device counter once per tensor, after every update kernel has read it
-    launch_pdl(counter_add_kernel, dim3(1), dim3(1), 0, s, static_cast<unsigned long long*>(step_counter), (unsigned long long)n_seg);
+  if (clip == 1 && !compute_norms(s, G, seg, n_seg, norms)) return;
+  for (size_t first = 0; first < n_seg; first += kMaxSeg) {
+    const SegTable tab = table(first);
+    unsigned* ticket = nullptr;
+    if (!workspace(s, 256, &ticket, 2)) return;
+    const dim3 grid(chunks_for(seg + first, tab.n), tab.n), blk(kOThreads);
+    const unsigned long long inc = (t_dev && advance && first + kMaxSeg >= n_seg) ? (unsigned long long)n_seg : 0ull;
+    auto kern = clip ? (cp ? adam_kernel<true, true> : adam_kernel<true, false>) : (cp ? adam_kernel<false, true> : adam_kernel<false, false>);
+    if (!launch_pdl(kern, grid, blk, 0, s, P, G, M, V, tab, a, (const float*)norms, (float)max_norm, (float)delta, cp, t_dev, lr, ticket, inc)) return;
   }
+  if (target)
+    for (len_t j = 0; j < n_seg; ++j)
+      zg_soft_update(SINGLE, StreamWrapper{s}, P + seg[j].offset, target + seg[j].offset, seg[j].len, tau);
+}
+
+extern "C" void zg_adam_step_part(dtype id, StreamWrapper w, void* params, void* grads, void* m, void* v, const zg_segment* seg, len_t n_seg,
+                                  len_t t_first, double lr, double beta1, double beta2, double eps, int clip, double max_norm, double delta,
+                                  void* norms, void* bf16_copy, void* step_counter, int advance_counter) {
+  if (id != SINGLE) { set_error(kUnsupported, "zg_adam_step: only SINGLE is implemented"); return; }
+  adam_step(as_stream(w), (float*)params, (float*)grads, (float*)m, (float*)v, seg, n_seg, t_first, lr, beta1, beta2, eps, clip, max_norm, delta,
+            (float*)norms, (__nv_bfloat16*)bf16_copy, (unsigned long long*)step_counter, advance_counter, nullptr, 0.0);
+}
+
+extern "C" void zg_adam_soft_step(dtype id, StreamWrapper w, void* params, void* grads, void* m, void* v, const zg_segment* seg, len_t n_seg,
+                                  len_t t_first, double lr, double beta1, double beta2, double eps, int clip, double max_norm, double delta,
+                                  void* norms, void* step_counter, void* target, double tau) {
+  if (id != SINGLE) { set_error(kUnsupported, "zg_adam_soft_step: only SINGLE is implemented"); return; }
+  if (!target) { set_error(kBadArgument, "zg_adam_soft_step: NULL target"); return; }
+  adam_step(as_stream(w), (float*)params, (float*)grads, (float*)m, (float*)v, seg, n_seg, t_first, lr, beta1, beta2, eps, clip, max_norm, delta,
+            (float*)norms, nullptr, (unsigned long long*)step_counter, 1, (float*)target, tau);
 }
 
 extern "C" void zg_adam_step(dtype id, StreamWrapper w, void* params, void* grads, void* m, void* v, const zg_segment* seg, len_t n_seg,

@@ -567,7 +567,23 @@ class CudaDevice:
                            p.lr, int(p.clip), p.max_norm, p.delta, p.norms.ptr if p.norms is not None else None,
                            int(bool(getattr(p, 'zero_grads', False))))
 
+    def q_head_supported(self, dtype: int, batch: int, actions: int) -> bool:
+        return bool(self.L.zg_q_head_supported(dtype, batch, actions))
+
+    def q_head(self, p):
+        self.L.zg_q_head(p.q.dtype, self.stream, p.batch, p.n_actions, p.qn.ptr, p.q.ptr, p.actions.ptr, p.rewards.ptr, p.dones.ptr, p.gamma,
+                         p.q_clip, p.beta, p.maxq.ptr, p.targets.ptr, p.chosen.ptr, p.offsets.ptr, p.loss.ptr, p.dchosen.ptr, p.dq.ptr, p.dbias.ptr)
+
     def adam(self, p):
+        if p.soft_target is not None:
+            if p.bf16_copy is not None or not p.advance_counter:
+                raise ValueError("adam: a soft target update goes with a whole fp32 step")
+            self.L.zg_adam_soft_step(p.params.dtype, self.stream, p.params.ptr, p.grads.ptr, p.m.ptr, p.v.ptr,
+                                     self._segments(p.segments), len(p.segments), p.t_first, p.lr, p.beta1, p.beta2, p.eps,
+                                     2 if p.clip == "given" else int(bool(p.clip)), p.max_norm, p.delta,
+                                     p.norms.ptr if p.norms is not None else None,
+                                     p.step_counter.ptr if p.step_counter is not None else None, p.soft_target.ptr, p.tau)
+            return
         self.L.zg_adam_step_part(p.params.dtype, self.stream, p.params.ptr, p.grads.ptr, p.m.ptr, p.v.ptr,
                                  self._segments(p.segments), len(p.segments), p.t_first, p.lr, p.beta1, p.beta2, p.eps,
                                  2 if p.clip == "given" else int(bool(p.clip)), p.max_norm, p.delta,

@@ -61,35 +61,45 @@ class DqnTrainer:
         self.target._set_host_state(state[half:])
 
     def _step(self, states: DeviceSlice, actions: DeviceSlice, next_states: DeviceSlice, rewards: DeviceSlice, dones: DeviceSlice):
-        d, B, C, qc = self.dev, self.B, self.C, self.q_clip
+        d, B, C = self.dev, self.B, self.C
         pol, tgt = self.policy, self.target
-        # ---- targets (gradients disabled in the reference): a chain of small kernels that does not depend
-        # on the policy net, so it runs on a side stream beside the policy forward
+        # ---- both forward passes (gradients disabled in the reference for the target net): independent chains of
+        # small kernels; zero_grad of the policy net rides on the side stream
         with d.branch(1):
             qn = tgt.forward(next_states)
-            d.dispatch(opspec.clamp_fwd(qn, qn, -qc, qc))
-            d.dispatch(opspec.max_along(qn, [B, C], self.maxq, [B, 1], 1))
-            d.dispatch(opspec.mul(self.maxq, self.gamma_s, self.tmp))          # gamma * max
-            d.dispatch(opspec.sub(self.one_s, dones, self.targets))            # 1 - done
-            d.dispatch(opspec.mul(self.tmp, self.targets, self.tmp))           # masked
-            d.dispatch(opspec.add(rewards, self.tmp, self.targets))            # r + ...
-            d.dispatch(opspec.clamp_fwd(self.targets, self.targets, -qc, qc))
-            # the two zero fills the loss and the gather backward accumulate into (ensure_grad(0))
-            d.mem_fill(self.dq, 0.0)
-            d.mem_fill(pol.dact[-1], 0.0)
-        # ---- policy forward, clamp outside the graph, gather by action
+            d.mem_fill(pol._grads, 0.0)
         q_all = pol.forward(states)
+        pol._zero_due = False
+        d.join()
+        # ---- targets, gather by action, loss and its gradient w.r.t. all Q values, last bias gradient
+        fused = d.q_head_supported(SINGLE, B, C)
+        if fused:
+            d.dispatch(opspec.q_head(qn, q_all, actions, rewards, dones, B, C, self.gamma, self.q_clip, 1.0, self.maxq, self.targets, self.q,
+                                     self.offsets, self.loss, self.dq, pol.dact[-1], pol._db[-1]))
+        else:
+            self._head(qn, q_all, actions, rewards, dones)
+        pol.backward(states, last_bias_done=fused)
+        # ---- Adam, and the soft update of the target parameters behind it
+        pol.update(soft_target=tgt.params, tau=self.tau)
+
+    def _head(self, qn, q_all, actions, rewards, dones):
+        """opspec.q_head as separate ops (more actions than it is built for)."""
+        d, B, C, qc = self.dev, self.B, self.C, self.q_clip
+        d.dispatch(opspec.clamp_fwd(qn, qn, -qc, qc))
+        d.dispatch(opspec.max_along(qn, [B, C], self.maxq, [B, 1], 1))
+        d.dispatch(opspec.mul(self.maxq, self.gamma_s, self.tmp))          # gamma * max
+        d.dispatch(opspec.sub(self.one_s, dones, self.targets))            # 1 - done
+        d.dispatch(opspec.mul(self.tmp, self.targets, self.tmp))           # masked
+        d.dispatch(opspec.add(rewards, self.tmp, self.targets))            # r + ...
+        d.dispatch(opspec.clamp_fwd(self.targets, self.targets, -qc, qc))
+        # the two zero fills the loss and the gather backward accumulate into (ensure_grad(0))
+        d.mem_fill(self.dq, 0.0)
+        d.mem_fill(self.policy.dact[-1], 0.0)
         d.dispatch(opspec.clamp_fwd(q_all, q_all, -qc, qc))
         d.gather_rows(q_all, actions, B, C, self.q, self.offsets)
-        d.join()  # the targets and the cleared gradients are ready
-        # ---- loss and its gradient w.r.t. the gathered values
         d.dispatch(opspec.smooth_l1(self.q, self.targets, 1.0, self.loss, self.dq))
-        # ---- gather backward: scatter into a zero gradient of all Q values
-        d.dispatch(opspec.scatter_add(self.dq, self.offsets, pol.dact[-1]))
-        pol.backward(states, last_bias_done=False)
-        pol.update()
-        # ---- soft update of the target parameters (one kernel over the flat buffer)
-        d.soft_update(pol.params, tgt.params, self.tau)
+        # gather backward: scatter into a zero gradient of all Q values
+        d.dispatch(opspec.scatter_add(self.dq, self.offsets, self.policy.dact[-1]))
 
     def read_loss(self) -> float:
         return float(self.dev.to_numpy(self.loss)[0])

@@ -295,7 +295,8 @@ class MlpTrainer:
         if last:
             self.t += len(self.segments)  # host mirror (eager steps only; read_t() is the truth)
 
-    def update(self):
+    def update(self, soft_target: Optional[DeviceSlice] = None, tau: float = 0.0):
+        """`soft_target` (Adam): a target network's flat parameters, moved towards the updated ones by tau."""
         d = self.dev
         self._settle()
         if self.opt == "sgd":
@@ -305,7 +306,7 @@ class MlpTrainer:
         elif self.opt == "adam":
             d.dispatch(opspec.adam(self.params, self._grads, self.m, self.v, self.segments, self.t + 1, self.lr, self.beta1,
                                    self.beta2, self.eps, self.clip, self.max_norm, self.delta, self.norms,
-                                   self.params_bf16 if self.bf16 else None, self.t_dev))
+                                   self.params_bf16 if self.bf16 else None, self.t_dev, soft_target=soft_target, tau=tau))
             self.t += len(self.segments)  # host mirror (eager steps only; read_t() is the truth)
         elif self.opt != "none":
             raise ValueError(self.opt)

@@ -537,6 +537,34 @@ class adam:
     bf16_copy: Optional[Any] = None
     step_counter: Optional[Any] = None  # device u64: tensor updates so far (graph-replay safe step count)
     advance_counter: bool = True  # False: read step_counter without advancing it (one optimizer step as several calls, see zg_adam_step_part)
+    soft_target: Optional[Any] = None   # target network's parameters, laid out like params: tau * params + (1 - tau) * target after the update
+    tau: float = 0.0
+
+
+@_op("q_head")
+class q_head:
+    """Everything between the forward passes of a Q-learning update and its backward
+    pass as one device op (zg_q_head): targets from the next states' values, the chosen
+    actions' values, smooth L1 loss, its gradient scattered into the Q values and the
+    column sums of that gradient."""
+    qn: Any          # [batch, actions], clamped in place
+    q: Any           # [batch, actions], clamped in place
+    actions: Any     # u64 [batch]
+    rewards: Any
+    dones: Any
+    batch: int
+    n_actions: int
+    gamma: float
+    q_clip: float
+    beta: float
+    maxq: Any
+    targets: Any
+    chosen: Any
+    offsets: Any     # u64 [batch]
+    loss: Any
+    dchosen: Any
+    dq: Any          # [batch, actions]
+    dbias: Any       # [actions]
 
 
 @_op("csr_gcn_propagate")
