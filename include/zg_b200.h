@@ -303,7 +303,7 @@ EXTERN_C void zg_adam_step_part(dtype id, StreamWrapper stream, void* params, vo
                                 int clip, double max_norm, double delta, void* norms, void* bf16_copy, void* step_counter,
                                 int advance_counter);
 /* zg_adam_step followed by the soft update of a target network's parameters (laid out like `params`):
- * target = tau * params + (1 - tau) * target, in the same launch for small models. */
+ * target = tau * params + (1 - tau) * target, in the same launch. */
 EXTERN_C void zg_adam_soft_step(dtype id, StreamWrapper stream, void* params, void* grads, void* m, void* v, const zg_segment* seg, len_t n_seg,
                                 len_t t_first, double lr, double beta1, double beta2, double eps, int clip, double max_norm, double delta,
                                 void* norms, void* step_counter, void* target, double tau);
