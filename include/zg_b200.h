@@ -311,6 +311,12 @@ EXTERN_C void zg_adam_soft_step(dtype id, StreamWrapper stream, void* params, vo
  * shard-local part of the per-tensor gradient norm of host_device.zig:339-346 */
 EXTERN_C void zg_segment_sumsq(dtype id, StreamWrapper stream, const void* x, const zg_segment* seg, len_t n_seg, void* out);
 /* target[i] = tau*src[i] + (1-tau)*target[i] (examples/dqn/src/dqn_agent.zig:111-123) */
+/* Softmax cross-entropy of selected rows (mem_take, softmax_ce and scatter_add as one launch): row r of the loss reads
+ * logits + offsets[r * ld] (a row's offsets are consecutive) and ADDS its gradient into dlogits there; loss and dbias (the
+ * gradient's column sums, may be NULL) are overwritten. */
+EXTERN_C int zg_masked_softmax_ce_supported(dtype id, len_t rows, len_t C);
+EXTERN_C void zg_masked_softmax_ce(dtype id, StreamWrapper stream, const void* logits, const len_t* offsets, const void* labels, int label_kind,
+                                   len_t rows, len_t C, len_t ld, double divisor, void* loss, void* dlogits, void* dbias);
 /* The ops between the forward passes of a Q-learning update and its backward pass as one launch (a dozen ops of the device
  * interface; examples/dqn/src/dqn_agent.zig:111-228).  qn = the target network's values of the next states, q = the
  * policy's of the states, both [batch, actions] and clamped in place; dq, dbias, loss, .. are overwritten. */

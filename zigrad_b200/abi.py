@@ -209,6 +209,8 @@ SIGNATURES = {
     "zg_adam_step": (None, [dtype_t, S, vp, vp, vp, vp, C.POINTER(Segment), len_t, len_t, dbl, dbl, dbl, dbl, i32, dbl, dbl, vp, vp, vp]),
     "zg_adam_step_part": (None, [dtype_t, S, vp, vp, vp, vp, C.POINTER(Segment), len_t, len_t, dbl, dbl, dbl, dbl, i32, dbl, dbl, vp, vp, vp, i32]),
     "zg_adam_soft_step": (None, [dtype_t, S, vp, vp, vp, vp, C.POINTER(Segment), len_t, len_t, dbl, dbl, dbl, dbl, i32, dbl, dbl, vp, vp, vp, dbl]),
+    "zg_masked_softmax_ce_supported": (i32, [dtype_t, len_t, len_t]),
+    "zg_masked_softmax_ce": (None, [dtype_t, S, vp, vp, vp, i32, len_t, len_t, len_t, dbl, vp, vp, vp]),
     "zg_q_head_supported": (i32, [dtype_t, len_t, len_t]),
     "zg_q_head": (None, [dtype_t, S, len_t, len_t, vp, vp, vp, vp, vp, dbl, dbl, dbl, vp, vp, vp, vp, vp, vp, vp, vp]),
     "zg_segment_sumsq": (None, [dtype_t, S, vp, C.POINTER(Segment), len_t, vp]),

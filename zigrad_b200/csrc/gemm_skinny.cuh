@@ -127,10 +127,8 @@ __global__ void __launch_bounds__(kThreads) skinny_k_kernel(const Params p) {
   __syncthreads();
   const float4* b4 = reinterpret_cast<const float4*>(bs);
   float4 cs = make_float4(0.f, 0.f, 0.f, 0.f);
-  uint32_t g_last = 0;
   for (uint64_t idx = (uint64_t)blockIdx.x * kThreads + threadIdx.x; idx < total; idx += stride) {
     const uint32_t row = (uint32_t)(idx / cg), g = (uint32_t)(idx - (uint64_t)row * cg);
-    g_last = g;  // constant per thread: the launcher makes the stride a multiple of cg when column sums are asked for
     float a[KMAX];
 #pragma unroll
     for (int kk = 0; kk < KMAX; ++kk) a[kk] = an[kk];
@@ -165,11 +163,20 @@ __global__ void __launch_bounds__(kThreads) skinny_k_kernel(const Params p) {
     cs.x += v.x; cs.y += v.y; cs.z += v.z; cs.w += v.w;
   }
   if (p.colsum) {
-    // per-CTA column sums in shared memory, then one global atomic per column and CTA
-    atomicAdd(&scol[4 * g_last + 0], cs.x);
-    atomicAdd(&scol[4 * g_last + 1], cs.y);
-    atomicAdd(&scol[4 * g_last + 2], cs.z);
-    atomicAdd(&scol[4 * g_last + 3], cs.w);
+    // The lanes of a warp that hold the same columns fold their sums first (cg, a power of two, divides the stride): per-CTA sums in
+    // shared memory, whose fp32 atomics serialise (2708 x 16 outputs: 9.2 us with 64 threads on each column, 4.7 like this), then
+    // one global atomic per column and CTA.
+    for (uint32_t off = cg; off < 32; off <<= 1) {
+      cs.x += __shfl_xor_sync(0xffffffffu, cs.x, off); cs.y += __shfl_xor_sync(0xffffffffu, cs.y, off);
+      cs.z += __shfl_xor_sync(0xffffffffu, cs.z, off); cs.w += __shfl_xor_sync(0xffffffffu, cs.w, off);
+    }
+    if ((threadIdx.x & 31) < cg) {
+      const uint32_t g = threadIdx.x % cg;  // the columns of every output of this thread
+      atomicAdd(&scol[4 * g + 0], cs.x);
+      atomicAdd(&scol[4 * g + 1], cs.y);
+      atomicAdd(&scol[4 * g + 2], cs.z);
+      atomicAdd(&scol[4 * g + 3], cs.w);
+    }
     __syncthreads();
     for (uint32_t e = threadIdx.x; e < n; e += kThreads) atomicAdd(p.colsum + e, scol[e]);
   }

@@ -1172,6 +1172,93 @@ extern "C" void zg_softmax_ce_fwd_bwd(dtype id, StreamWrapper w, const void* log
   else set_error(kBadArgument, "zg_softmax_ce_fwd_bwd: unknown label kind %d", label_kind);
 }
 
+// Softmax cross-entropy of selected rows (a MaskLayer, its loss and both backward passes: mem_take, softmax_ce and
+// scatter_add in one launch): row r reads logits + offsets[r * ld] and adds its gradient into dlogits there.  A warp per
+// row, lanes along the classes; loss and column sums per CTA, folded by the CTA that draws the last ticket.
+struct MaskedCe {
+  const float* logits;
+  const len_t* offsets;   // [rows, ld] element offsets; a row's are consecutive
+  const void* labels;
+  float *dlogits, *loss, *dbias;
+  float* partial;         // [grid][C + 1]
+  unsigned* ticket;
+  unsigned rows, C, ld;
+  float divisor;
+  int index_labels;
+};
+__global__ void __launch_bounds__(kLThreads) masked_ce_kernel(const MaskedCe a) {
+  extern __shared__ float cols[];  // [warps][C]
+  __shared__ float lsum[kLThreads / 32];
+  __shared__ bool last;
+  pdl_sync();
+  constexpr int W = kLThreads / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, C = (int)a.C;
+  for (int c = lane; c < C; c += 32) cols[warp * C + c] = 0.f;
+  __syncwarp();
+  float loss = 0.f;
+  for (unsigned r = blockIdx.x * W + warp; r < a.rows; r += gridDim.x * W) {
+    const len_t off = __ldg(a.offsets + (size_t)r * a.ld);
+    const float* x = a.logits + off;
+    const float* t = static_cast<const float*>(a.labels) + (size_t)r * C;
+    const len_t lab = a.index_labels ? __ldg(static_cast<const len_t*>(a.labels) + r) : 0;
+    float mx = -INFINITY, se = 0.f;
+    for (int c = lane; c < C; c += 32) mx = fmaxf(mx, x[c]);
+    mx = warp_max(mx);
+    for (int c = lane; c < C; c += 32) se += fast_exp(x[c] - mx);
+    se = warp_sum(se);
+    const float inv = 1.f / se, lse = logf(se);
+    for (int c = lane; c < C; c += 32) {
+      const float d = x[c] - mx, tc = a.index_labels ? ((len_t)c == lab ? 1.f : 0.f) : t[c];
+      if (tc != 0.f) loss -= tc * clamp_logp(d - lse);
+      const float g = (fast_exp(d) * inv - tc) / a.divisor;
+      atomicAdd(a.dlogits + off + c, g);
+      cols[warp * C + c] += g;
+    }
+  }
+  loss = warp_sum(loss);
+  if (lane == 0) lsum[warp] = loss;
+  __syncthreads();
+  float* mine = a.partial + (size_t)blockIdx.x * (C + 1);
+  for (int c = threadIdx.x; c <= C; c += kLThreads) {
+    float s = 0.f;
+    for (int w = 0; w < W; ++w) s += c < C ? cols[w * C + c] : lsum[w];
+    mine[c] = s;
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+    if (last) *a.ticket = 0;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int c = warp; c <= C; c += W) {
+    float s = 0.f;
+    for (unsigned k = lane; k < gridDim.x; k += 32) s += __ldcg(a.partial + (size_t)k * (C + 1) + c);
+    s = warp_sum(s);
+    if (lane == 0) {
+      if (c == C) *a.loss = s / a.divisor;
+      else if (a.dbias) a.dbias[c] = s;
+    }
+  }
+}
+
+extern "C" int zg_masked_softmax_ce_supported(dtype id, len_t rows, len_t C) { return id == SINGLE && rows > 0 && rows <= 0x7fffffffu && C > 0 && C <= 1024 ? 1 : 0; }
+extern "C" void zg_masked_softmax_ce(dtype id, StreamWrapper w, const void* logits, const len_t* offsets, const void* labels, int label_kind, len_t rows,
+                                     len_t C, len_t ld, double divisor, void* loss, void* dlogits, void* dbias) {
+  if (!zg_masked_softmax_ce_supported(id, rows, C) || ld < C || ld > 0xffffffffu) { set_error(kUnsupported, "zg_masked_softmax_ce: %lu rows of %lu (stride %lu)", rows, C, ld); return; }
+  if (label_kind != ZG_LABEL_ONEHOT && label_kind != ZG_LABEL_INDEX) { set_error(kBadArgument, "zg_masked_softmax_ce: unknown label kind %d", label_kind); return; }
+  cudaStream_t s = as_stream(w);
+  const unsigned g = grid_for(rows, kLThreads / 32, 2);
+  unsigned* counters = nullptr;
+  float* partial = static_cast<float*>(workspace(s, sizeof(float) * g * (C + 1), &counters));
+  if (!partial) return;
+  const MaskedCe a{(const float*)logits, offsets, labels, (float*)dlogits, (float*)loss, (float*)dbias, partial, counters,
+                   (unsigned)rows, (unsigned)C, (unsigned)ld, (float)divisor, label_kind == ZG_LABEL_INDEX ? 1 : 0};
+  launch_pdl(masked_ce_kernel, dim3(g), dim3(kLThreads), sizeof(float) * C * (kLThreads / 32), s, a);
+}
+
 // ---------------------------------------------------------------- Q learning
 // Everything between the two forward passes of a Q-learning update and its backward pass, as one launch
 // (examples/dqn/src/dqn_agent.zig:111-228): as the device interface spells it these are a dozen ops over a few kilobytes,
@@ -1253,12 +1340,16 @@ __global__ void __launch_bounds__(kLThreads) q_head_kernel(const QHead a) {
   }
   const float bs = block_sum<float>(loss, sm32);
   float* mine = a.partial + (size_t)blockIdx.x * (A + 1);
-  if (threadIdx.x == 0) mine[A] = bs;
-  __syncthreads();
+  if (threadIdx.x == 0 && gridDim.x > 1) mine[A] = bs;
   for (int c = threadIdx.x; c < A; c += kLThreads) {
     float s = 0.f;
     for (int w = 0; w < kLThreads / 32; ++w) s += cols[w * A + c];
-    mine[c] = s;
+    if (gridDim.x == 1) a.dbias[c] = s;
+    else mine[c] = s;
+  }
+  if (gridDim.x == 1) {
+    if (threadIdx.x == 0) *a.loss = bs / fn;
+    return;
   }
   __threadfence();
   __syncthreads();

@@ -567,6 +567,14 @@ class CudaDevice:
                            p.lr, int(p.clip), p.max_norm, p.delta, p.norms.ptr if p.norms is not None else None,
                            int(bool(getattr(p, 'zero_grads', False))))
 
+    def masked_softmax_ce_supported(self, dtype: int, rows: int, classes: int) -> bool:
+        return bool(self.L.zg_masked_softmax_ce_supported(dtype, rows, classes))
+
+    def masked_softmax_ce(self, p):
+        kind = abi.LABEL_INDEX if p.labels.dtype == USIZE else abi.LABEL_ONEHOT
+        self.L.zg_masked_softmax_ce(p.logits.dtype, self.stream, p.logits.ptr, p.offsets.ptr, p.labels.ptr, kind, p.rows, p.classes, p.ld,
+                                    float(p.loss_div), p.loss.ptr, p.grad.ptr, p.bias_grad.ptr if p.bias_grad is not None else None)
+
     def q_head_supported(self, dtype: int, batch: int, actions: int) -> bool:
         return bool(self.L.zg_q_head_supported(dtype, batch, actions))
 

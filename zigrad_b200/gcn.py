@@ -128,11 +128,14 @@ class GcnTrainer:
         self._mm(self.a1, self.W2, self.h2, N, C, H, False, True, H, H, Cp)                       # h2 = a1 . W2^T
         self._prop(self.h2, self.logits, C, Cp, "bias", self.b2)                                   # A.h2 + b2
         # ---- mask rows, loss, gradient of the masked logits (+ db2 = its column sums)
-        d.mem_take(self.logits, self.offsets, self.mlog)
         d.join()  # the cleared gradient buffers
-        d.dispatch(opspec.softmax_ce(self.mlog, T_masked, M, C, self.loss, self.dm, float(M), accumulate=False, ld=Cp,
-                                     bias_grad=self.db2))
-        d.dispatch(opspec.scatter_add(self.dm, self.offsets, self.dlog))                            # MaskLayer backward
+        if d.masked_softmax_ce_supported(SINGLE, M, C):
+            d.dispatch(opspec.masked_softmax_ce(self.logits, self.offsets, T_masked, M, C, Cp, self.loss, self.dlog, float(M), self.db2))
+        else:
+            d.mem_take(self.logits, self.offsets, self.mlog)
+            d.dispatch(opspec.softmax_ce(self.mlog, T_masked, M, C, self.loss, self.dm, float(M), accumulate=False, ld=Cp,
+                                         bias_grad=self.db2))
+            d.dispatch(opspec.scatter_add(self.dm, self.offsets, self.dlog))                        # MaskLayer backward
         # ---- backward
         self._prop(self.dlog, self.dh2, C, Cp, transpose=True)                                    # dh2 = A^T . dlogits
         with d.branch(0):  # nothing below reads dW2: beside the rest of the backward pass

@@ -541,6 +541,22 @@ class adam:
     tau: float = 0.0
 
 
+@_op("masked_softmax_ce")
+class masked_softmax_ce:
+    """mem_take, softmax_ce and scatter_add of a MaskLayer in front of the loss as one
+    device op: row r reads logits[offsets[r * ld] ..] and adds its gradient into grad there."""
+    logits: Any
+    offsets: Any     # u64 [rows, ld]
+    labels: Any      # one-hot fp32 [rows, classes] or u64 [rows]
+    rows: int
+    classes: int
+    ld: int
+    loss: Any
+    grad: Any        # like logits, accumulated
+    loss_div: float
+    bias_grad: Optional[Any] = None
+
+
 @_op("q_head")
 class q_head:
     """Everything between the forward passes of a Q-learning update and its backward
