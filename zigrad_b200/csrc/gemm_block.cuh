@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(kThreads, MI == 0 ? 2 : 1) gemm_block_kernel(c
   constexpr bool kAsync = sizeof(TI) >= 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   AT* ring = reinterpret_cast<AT*>(smem_raw);
-  __shared__ float col_part[TN];
+  __shared__ float col_part[kThreads / TN][TN];
 
   const uint32_t split = blockIdx.x % p.splits;
   uint32_t tile = blockIdx.x / p.splits;
@@ -304,7 +304,6 @@ __global__ void __launch_bounds__(kThreads, MI == 0 ? 2 : 1) gemm_block_kernel(c
       for (int j = 0; j < MI; ++j)
         red[(group * TM + ty * 4 + (i / 4) * (TM / 2) + i % 4) * TN + tx * 4 + (j / 4) * (TN / 2) + j % 4] = acc[i][j];
   }
-  if (threadIdx.x < TN) col_part[threadIdx.x] = 0.f;
   __syncthreads();
   AT sum[kOut];
 #pragma unroll
@@ -356,9 +355,14 @@ __global__ void __launch_bounds__(kThreads, MI == 0 ? 2 : 1) gemm_block_kernel(c
   }
   if (p.colsum) {
     // a thread's outputs all lie in column threadIdx.x % TN: kThreads and the shares are multiples of TN
-    atomicAdd(&col_part[threadIdx.x % TN], csum);
+    col_part[threadIdx.x / TN][threadIdx.x % TN] = csum;
     __syncthreads();
-    if (threadIdx.x < TN && n0 + threadIdx.x < p.n) atomicAdd(p.colsum + n0 + threadIdx.x, col_part[threadIdx.x]);
+    if (threadIdx.x < TN && n0 + threadIdx.x < p.n) {
+      float s = 0.f;
+#pragma unroll
+      for (int w = 0; w < kThreads / TN; ++w) s += col_part[w][threadIdx.x];
+      atomicAdd(p.colsum + n0 + threadIdx.x, s);
+    }
   }
 }
 

@@ -553,7 +553,8 @@ struct SmemLayout {
   // FP32X3: two sets of four A warps take the slabs in turn
   static constexpr int kThreads = X3 ? 384 : kThreadsTc;  // + kLoadWarps * 32 with direct operands
   static constexpr int kOutPitch = BN + 4;  // floats per row of the staged output tile
-  static_assert(kBM * kOutPitch * 4 <= kStages * kStageBytes, "the output tile is staged in the ring");
+  static constexpr int kColRows = (kThreads + kLoadWarps * 32) / (BN / 4);  // partial column sums behind the tile
+  static_assert((kBM * kOutPitch + kColRows * BN) * 4 <= kStages * kStageBytes, "the output tile and its column sums are staged in the ring");
 };
 
 // One lane's four columns of a row of the staged tile.  VEC: four consecutive columns with 16-byte (fp32) or 8-byte (bf16)
@@ -693,9 +694,10 @@ __device__ __forceinline__ void staged_out_swapped(const Params& p, const float*
 
 // The staged tile (128 x BN floats, pitch BN + 4, all CTAs of a cluster hold partial sums) to C: NT threads, lanes along
 // the rows of C, U rows in flight (a row of a lone CTA is a round trip to memory for C and the mask; one of a cluster
-// already has a load to every rank in flight, two measured slower).  col_part: BN zeroed floats.
+// already has a load to every rank in flight, two measured slower).  The column sums of a CTA are
+// added up in a fixed order behind the tile.
 template <int BN, int NT, bool VEC, int U>
-__device__ __forceinline__ void staged_out(const Params& p, const float* tile, float* col_part, uint32_t split, uint32_t m0, uint32_t n0, uint64_t batch_off) {
+__device__ __forceinline__ void staged_out(const Params& p, float* tile, uint32_t split, uint32_t m0, uint32_t n0, uint64_t batch_off) {
   constexpr int CG = BN / 4, PITCH = BN + 4;
   const uint32_t cg = threadIdx.x % CG, ranks = p.cluster ? p.splits : 1, rank = p.cluster ? split : 0;
   const uint32_t local = VEC ? 4 * cg : cg, stride = VEC ? 1 : CG, col = n0 + local;
@@ -764,12 +766,16 @@ __device__ __forceinline__ void staged_out(const Params& p, const float* tile, f
     }
     if (p.colsum) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) atomicAdd(col_part + local + j * stride, cs[j]);
+      for (int j = 0; j < 4; ++j) tile[kBM * PITCH + threadIdx.x / CG * BN + local + j * stride] = cs[j];
     }
   }
   if (p.colsum) {
     __syncthreads();
-    if (threadIdx.x < BN && n0 + threadIdx.x < p.n) atomicAdd(p.colsum + n0 + threadIdx.x, col_part[threadIdx.x]);
+    if (threadIdx.x < BN && n0 + threadIdx.x < p.n) {
+      float s = 0.f;
+      for (int w = 0; w < NT / CG; ++w) s += tile[kBM * PITCH + w * BN + threadIdx.x];
+      atomicAdd(p.colsum + n0 + threadIdx.x, s);
+    }
   }
 }
 
@@ -797,7 +803,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   uint64_t* accum = bars + 3 * S;   // accumulator complete
   __shared__ uint32_t tmem_base_slot;
   __shared__ volatile int failed;
-  __shared__ float col_part[BN];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // the splits of a tile are neighbours where they form a cluster; else the tiles are, which share their slabs of A in L2
@@ -808,7 +813,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   if (k_end > p.k) k_end = p.k;
   const int KT = (k_end > k_begin) ? (int)((k_end - k_begin + MT::kBK - 1) / MT::kBK) : 0;
 
-  if (threadIdx.x < BN) col_part[threadIdx.x] = 0.f;
   if (threadIdx.x == 0) {
     failed = 0;
     for (int s = 0; s < S; ++s) {
@@ -1135,17 +1139,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   }
   __syncwarp();
   if (!p.tma_epilogue) {
-    const float* tile = reinterpret_cast<const float*>(stage_base);
+    float* tile = reinterpret_cast<float*>(stage_base);
     if (p.cluster) cluster_sync(); else __syncthreads();
     constexpr int NT = SL::kThreads + (DIRECT ? kLoadWarps * 32 : 0);
     const uint64_t batch_off = (uint64_t)batch * p.c_batch_stride;
     if (p.swap) staged_out_swapped<BN, NT>(p, tile, split, tile_m * kBM, tile_n * BN, batch_off);
     else if (p.vec_ok && (p.n & 3u) == 0) {
-      if (p.cluster) staged_out<BN, NT, true, 1>(p, tile, col_part, split, tile_m * kBM, tile_n * BN, batch_off);
-      else staged_out<BN, NT, true, 2>(p, tile, col_part, split, tile_m * kBM, tile_n * BN, batch_off);
+      if (p.cluster) staged_out<BN, NT, true, 1>(p, tile, split, tile_m * kBM, tile_n * BN, batch_off);
+      else staged_out<BN, NT, true, 2>(p, tile, split, tile_m * kBM, tile_n * BN, batch_off);
     } else {
-      if (p.cluster) staged_out<BN, NT, false, 1>(p, tile, col_part, split, tile_m * kBM, tile_n * BN, batch_off);
-      else staged_out<BN, NT, false, 2>(p, tile, col_part, split, tile_m * kBM, tile_n * BN, batch_off);
+      if (p.cluster) staged_out<BN, NT, false, 1>(p, tile, split, tile_m * kBM, tile_n * BN, batch_off);
+      else staged_out<BN, NT, false, 2>(p, tile, split, tile_m * kBM, tile_n * BN, batch_off);
     }
     if (p.cluster) cluster_sync();  // nobody leaves while its partial tile may still be read
   }
