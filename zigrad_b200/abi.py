@@ -9,6 +9,8 @@ fallback implementation.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -275,8 +277,36 @@ def lib() -> C.CDLL:
         fn = getattr(L, name)  # AttributeError here = a declared symbol is not exported
         fn.restype = res
         fn.argtypes = args
+    _bind_fast(L)
     _lib = L
     return L
+
+
+def _bind_fast(L: C.CDLL) -> None:
+    """Replace the ctypes functions by direct calls (host/fastcall.c) wherever every argument is an integer, a pointer, a
+    one-pointer struct or a double; ctypes stays behind them for arguments of other Python types."""
+    path = os.path.join(HERE, "lib", "_fastcall.so")
+    if not os.path.exists(path):
+        raise LibraryMissing("%s not found: build it with `python -m zigrad_b200.build`" % path)
+    loader = importlib.machinery.ExtensionFileLoader("_fastcall", path)
+    fast = importlib.util.module_from_spec(importlib.util.spec_from_loader("_fastcall", loader))
+    loader.exec_module(fast)
+    ret = {None: "v", i32: "i", len_t: "u", vp: "p"}
+
+    def kind(t):
+        if t is dbl:
+            return "d"
+        if t is vp or (isinstance(t, type) and issubclass(t, C._Pointer)):
+            return "p"
+        if isinstance(t, type) and issubclass(t, _Handle):
+            return "s"
+        return "i" if isinstance(t, type) and issubclass(t, C._SimpleCData) and t._type_ in "?bBhHiIlLqQ" else None
+
+    for name, (res, args) in SIGNATURES.items():
+        sig = [kind(t) for t in args]
+        if res in ret and None not in sig and sig.count("d") <= 8 and len(sig) - sig.count("d") <= 26:
+            fn = getattr(L, name)
+            setattr(L, name, fast.function(C.cast(fn, vp).value, "".join(sig), ret[res], fn))
 
 
 class DeviceError(RuntimeError):

@@ -85,6 +85,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError("link failed:\n%s\n%s" % (r.stdout, r.stderr))
+    build_fastcall(force)
     return LIB
 
 
@@ -105,6 +106,23 @@ def build_host_example(force: bool = False) -> str:
     if r.returncode != 0:
         raise RuntimeError("g++ failed for the C++ host example:\n%s\n%s" % (r.stdout, r.stderr))
     return HOST_EXAMPLE
+
+
+FASTCALL = os.path.join(HERE, "lib", "_fastcall.so")
+
+
+def build_fastcall(force: bool = False) -> str:
+    """The CPython binding of the C ABI's calls (zigrad_b200/host/fastcall.c).  gcc and Python's headers only."""
+    import sysconfig
+    src = os.path.join(HERE, "host", "fastcall.c")
+    if not force and os.path.exists(FASTCALL) and os.path.getmtime(FASTCALL) >= os.path.getmtime(src):
+        return FASTCALL
+    os.makedirs(os.path.dirname(FASTCALL), exist_ok=True)
+    cmd = [shutil.which("gcc") or "gcc", "-O2", "-Wall", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], src, "-o", FASTCALL]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("gcc failed for the call binding:\n%s\n%s" % (r.stdout, r.stderr))
+    return FASTCALL
 
 
 if __name__ == "__main__":

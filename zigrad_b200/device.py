@@ -10,7 +10,9 @@ other implementation behind it: without the library or without a GPU it raises.
 from __future__ import annotations
 
 import contextlib
+import functools
 import os
+import struct
 
 import ctypes as C
 from dataclasses import dataclass
@@ -53,8 +55,21 @@ class DeviceOOM(MemoryError):
     """error.DeviceOOM of src/allocators/device_data.zig:44."""
 
 
-def _shape(s: Sequence[int]):
+@functools.lru_cache(maxsize=1024)
+def _shape_of(s: tuple):
     return (abi.len_t * len(s))(*[int(v) for v in s])
+
+
+def _shape(s: Sequence[int]):
+    return _shape_of(tuple(s))  # the library only reads it
+
+
+@functools.lru_cache(maxsize=256)
+def _segments_of(segs: tuple):
+    arr = (abi.Segment * len(segs))()
+    for i, (off, ln) in enumerate(segs):
+        arr[i].offset, arr[i].len = int(off), int(ln)
+    return arr
 
 
 def _f32(v: float):
@@ -267,8 +282,7 @@ class CudaDevice:
         return DeviceSlice(p, n, dtype)
 
     def mem_fill(self, s: DeviceSlice, value: float):
-        v = C.c_float(value) if s.dtype == SINGLE else C.c_double(value)
-        self.L.mem_fill(s.dtype, s.ptr, s.len, C.byref(v), self.stream)
+        self.L.mem_fill(s.dtype, s.ptr, s.len, struct.pack("f" if s.dtype == SINGLE else "d", value), self.stream)
 
     def mem_sequence(self, s: DeviceSlice, initial: float, step: float):
         T = C.c_float if s.dtype == SINGLE else C.c_double
@@ -557,10 +571,7 @@ class CudaDevice:
 
     @staticmethod
     def _segments(segs):
-        arr = (abi.Segment * len(segs))()
-        for i, (off, ln) in enumerate(segs):
-            arr[i].offset, arr[i].len = int(off), int(ln)
-        return arr
+        return _segments_of(tuple(map(tuple, segs)))
 
     def sgd(self, p):
         self.L.zg_sgd_step(p.params.dtype, self.stream, p.params.ptr, p.grads.ptr, self._segments(p.segments), len(p.segments),
