@@ -198,7 +198,8 @@ static size_t max_clusters(unsigned size) {
 }
 
 template <bool AK, bool BK_, int MODE>
-static bool launch_persistent_inst(cudaStream_t s, const CUtensorMap& ta, const CUtensorMap& tb, const tc::Params& p, uint32_t tiles_m,
+static bool launch_persistent_inst(cudaStream_t s, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tcm, const CUtensorMap& tmm,
+                                   const tc::Params& p, uint32_t tiles_m,
                                    uint32_t tiles_n, uint32_t n_tiles) {
   using SL = tc::PersistentSmem<MODE>;
   auto kern = tc::gemm_tc_persistent_kernel<AK, BK_, MODE>;
@@ -207,21 +208,21 @@ static bool launch_persistent_inst(cudaStream_t s, const CUtensorMap& ta, const 
     if (!ZG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SL::kTotal))) return false;
     attr_set = true;
   }
-  const unsigned grid = n_tiles < (uint32_t)sm_count() ? n_tiles : (unsigned)sm_count();
+  const unsigned pairs = std::min<unsigned>(n_tiles, (unsigned)sm_count() / 2);
   // work-item counter: zero between launches (slot 2 of the stream's workspace)
   unsigned* unused = nullptr;
   unsigned* counter = static_cast<unsigned*>(workspace(s, 256, &unused, 2));
   if (!counter) return false;
-  return launch_pdl(kern, dim3(grid), dim3(tc::kThreadsPersistent), (size_t)SL::kTotal, s, ta, tb, p, tiles_m, tiles_n, n_tiles, counter);
+  return launch_pdl_cluster(kern, dim3(2 * pairs), dim3(tc::kThreadsPersistent), (size_t)SL::kTotal, s, 2u, ta, tb, tcm, tmm, p, tiles_m, tiles_n, n_tiles, counter);
 }
 
 template <int MODE>
 static bool launch_persistent(cudaStream_t s, bool a_kmajor, bool b_kmajor, const CUtensorMap& ta, const CUtensorMap& tb,
-                              const tc::Params& p, uint32_t tiles_m, uint32_t tiles_n, uint32_t n_tiles) {
-  if (a_kmajor && b_kmajor) return launch_persistent_inst<true, true, MODE>(s, ta, tb, p, tiles_m, tiles_n, n_tiles);
-  if (a_kmajor && !b_kmajor) return launch_persistent_inst<true, false, MODE>(s, ta, tb, p, tiles_m, tiles_n, n_tiles);
-  if (!a_kmajor && b_kmajor) return launch_persistent_inst<false, true, MODE>(s, ta, tb, p, tiles_m, tiles_n, n_tiles);
-  return launch_persistent_inst<false, false, MODE>(s, ta, tb, p, tiles_m, tiles_n, n_tiles);
+                              const CUtensorMap& tcm, const CUtensorMap& tmm, const tc::Params& p, uint32_t tiles_m, uint32_t tiles_n, uint32_t n_tiles) {
+  if (a_kmajor && b_kmajor) return launch_persistent_inst<true, true, MODE>(s, ta, tb, tcm, tmm, p, tiles_m, tiles_n, n_tiles);
+  if (a_kmajor && !b_kmajor) return launch_persistent_inst<true, false, MODE>(s, ta, tb, tcm, tmm, p, tiles_m, tiles_n, n_tiles);
+  if (!a_kmajor && b_kmajor) return launch_persistent_inst<false, true, MODE>(s, ta, tb, tcm, tmm, p, tiles_m, tiles_n, n_tiles);
+  return launch_persistent_inst<false, false, MODE>(s, ta, tb, tcm, tmm, p, tiles_m, tiles_n, n_tiles);
 }
 
 // fp32 problems with n <= 16 or k <= 16 (see gemm_skinny.cuh).  Returns true when taken.
@@ -320,11 +321,11 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   const len_t M = swap ? n : m, N = swap ? m : n;
   const bool a_kmajor = swap ? tb : !ta;  // the dimension that is contiguous in memory: K, or M / N
   const bool b_kmajor = swap ? !ta : tb;
-  // Large single-pass problems: persistent kernel over 128 x 256 tiles
-  // (at least one tile per SM, k deep enough to amortise the tile hand-over).
+  // Large single-pass problems: persistent kernel over 256 x 256 tiles of CTA pairs
+  // (a tile for half of them at least, k deep enough to amortise the tile hand-over).
   static const bool no_persist = [] { const char* e = getenv("ZG_GEMM_NO_PERSISTENT"); return e && e[0] == '1'; }();
-  const size_t ptiles = ((m + 127) / 128) * ((n + 255) / 256) * nC;
-  const bool persistent = mode != tc::kFP32X3 && !swap && n > 128 && k >= 8 * (size_t)bk && ptiles * 2 >= (size_t)sm_count() &&
+  const size_t ptiles = ((m + tc::kPBM - 1) / tc::kPBM) * ((n + tc::kPBN - 1) / tc::kPBN) * nC, pairs = (size_t)sm_count() / 2;
+  const bool persistent = mode != tc::kFP32X3 && !swap && n > 128 && k >= 8 * (size_t)bk && ptiles * 2 >= pairs &&
                           ptiles <= 0x3fffffffu && !no_persist;
   int bn = persistent ? 256 : (N <= 32 && !direct ? 32 : (N <= 64 ? 64 : 128));
   if (bn < atom) bn = atom;               // MN-major B needs whole column blocks; bf16 has no BN=32 instance
@@ -349,16 +350,17 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   }
 
   unsigned splits = 1;
+  size_t whole = ptiles;
   if (persistent && epilogue == ZG_EPI_NONE && !colsum && c_id == SINGLE) {
-    // K ranges as work items when that fills the last wave better (>= 16 k-slabs per range)
-    const double sms = (double)sm_count();
-    double best = 0.0;
-    for (unsigned sp = 1; sp <= 4; sp *= 2) {
-      if (sp > 1 && k / sp < 16 * (size_t)bk) break;
-      const double items = (double)ptiles * sp;
-      const double eff = items / (std::ceil(items / sms) * sms);
-      if (eff > best + 0.03) { best = eff; splits = sp; }
+    // The tiles of the last wave as K ranges, when those fill it better: its length in k-slabs, with two slabs' time for
+    // what every item costs, over the numbers of ranges (at least 16 slabs each).
+    const size_t rest = ptiles % pairs, slabs = (k + bk - 1) / bk;
+    size_t best = slabs + 2;
+    for (unsigned sp = 2; rest && sp <= 16 && slabs / sp >= 16; ++sp) {
+      const size_t len = (rest * sp + pairs - 1) / pairs * ((slabs + sp - 1) / sp + 2);
+      if (len + slabs / 32 < best) { best = len; splits = sp; }
     }
+    if (splits > 1) whole = ptiles - rest;
   }
   bool cluster = false;
   if (can_split) {
@@ -388,7 +390,7 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   else ok = make_tmap(&tmA, bf16, pa, M, k, na, la, atom, bk, !bf16);
   if (!ok) return true;  // error recorded
   if (b_direct) {}
-  else if (b_kmajor) ok = make_tmap(&tmB, bf16, pb, k, N, nb, lb, bk, bn, false);
+  else if (b_kmajor) ok = make_tmap(&tmB, bf16, pb, k, N, nb, lb, bk, persistent ? tc::kPBN / 2 : bn, false);
   else ok = make_tmap(&tmB, bf16, pb, N, k, nb, lb, atom, bk, !bf16);
   if (!ok) return true;
 
@@ -413,24 +415,35 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   p.alpha = (float)alpha; p.beta = (float)beta; p.epilogue = epilogue;
   p.vec_ok = c_aligned ? 1 : 0;
   p.error_flag = tc_error_flag();
+  // Output through the C tensor map where the epilogue needs nothing from global memory but the bias, in the persistent kernel
+  // also the mask (ZG_GEMM_TMA_EPILOGUE=0 keeps the register path)
+  CUtensorMap tmC;
+  memset(&tmC, 0, sizeof(tmC));
+  static const bool tma_epi_on = [] { const char* e = getenv("ZG_GEMM_TMA_EPILOGUE"); return !(e && e[0] == '0'); }();
+  const bool tma_epi = tma_epi_on && p.vec_ok && !swap && nC <= 0x7fffffffu;
   if (persistent) {
-    const uint32_t tiles_m = (uint32_t)((m + 127) / 128), tiles_n = (uint32_t)((n + 255) / 256);
-    const uint32_t items = (uint32_t)(ptiles * splits);
+    const bool add = splits > 1 || (beta == 1.0 && epilogue == ZG_EPI_NONE && !colsum && c_id == SINGLE);
+    CUtensorMap tmM;
+    memset(&tmM, 0, sizeof(tmM));
+    if (tma_epi && (add || beta == 0.0)) {
+      const bool c16 = c_id == BF16;
+      if (!make_tmap(&tmC, c16, C, n, m, nC, ldc, c16 ? 64 : 32, 32, false)) return true;
+      if (epilogue == ZG_EPI_RELU_MASK && !make_tmap(&tmM, c16, mask, n, m, nC, ldc, c16 ? 64 : 32, 32, false)) return true;
+      p.tma_epilogue = add ? 2 : 1;
+    }
+    p.whole_tiles = (uint32_t)whole;
+    const uint32_t tiles_m = (uint32_t)((m + tc::kPBM - 1) / tc::kPBM), tiles_n = (uint32_t)((n + tc::kPBN - 1) / tc::kPBN);
+    const uint32_t items = (uint32_t)(whole + (ptiles - whole) * splits);
     if (splits > 1) prescale_c<float>(s, static_cast<float*>(C), nC, m, n, ldc, m * ldc, beta);
-    if (mode == tc::kBF16) launch_persistent<tc::kBF16>(s, a_kmajor, b_kmajor, tmA, tmB, p, tiles_m, tiles_n, items);
-    else launch_persistent<tc::kTF32>(s, a_kmajor, b_kmajor, tmA, tmB, p, tiles_m, tiles_n, items);
+    if (mode == tc::kBF16) launch_persistent<tc::kBF16>(s, a_kmajor, b_kmajor, tmA, tmB, tmC, tmM, p, tiles_m, tiles_n, items);
+    else launch_persistent<tc::kTF32>(s, a_kmajor, b_kmajor, tmA, tmB, tmC, tmM, p, tiles_m, tiles_n, items);
     return true;
   }
   p.cluster = cluster ? 1 : 0;
   if (splits > 1 && !cluster) prescale_c<float>(s, static_cast<float*>(C), nC, m, n, ldc, m * ldc, beta);
   dim3 grid((unsigned)((N + bn - 1) / bn * splits), (unsigned)((M + 127) / 128), (unsigned)nC);
   if (grid.y > 65535 || grid.z > 65535) return false;
-  // Output through the C tensor map where the epilogue needs nothing from global memory but the bias
-  // (ZG_GEMM_TMA_EPILOGUE=0 keeps the register path)
-  CUtensorMap tmC;
-  memset(&tmC, 0, sizeof(tmC));
-  static const bool tma_epi_on = [] { const char* e = getenv("ZG_GEMM_TMA_EPILOGUE"); return !(e && e[0] == '0'); }();
-  if (tma_epi_on && c_id == SINGLE && p.vec_ok && !cluster && !swap && !p.colsum && nC <= 0x7fffffffu &&
+  if (tma_epi && c_id == SINGLE && !cluster && !p.colsum &&
       (splits > 1 ? epilogue == ZG_EPI_NONE : (beta == 0.0 && epilogue != ZG_EPI_RELU_MASK))) {
     if (!make_tmap(&tmC, false, C, n, m, nC, ldc, 32, 32, false)) return true;
     p.tma_epilogue = splits > 1 ? 2 : 1;

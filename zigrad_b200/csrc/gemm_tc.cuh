@@ -84,6 +84,7 @@ struct Params {
   uint32_t nA, nB;      // operand batch counts (index wraps)
   uint32_t tiles_n;     // column tiles
   uint32_t splits;      // K splits (gridDim.x = column tiles * splits)
+  uint32_t whole_tiles; // persistent kernel: the first tiles of the list, which are not split
   uint32_t k_per_split; // multiple of BK
   float alpha, beta;
   int epilogue;
@@ -307,6 +308,22 @@ struct ModeTraits {
   static constexpr int kAtomMN = kSlabBytes / kElem;   // M/N elements per 128-byte column block
 };
 
+// Column sums of this warp's 32 x 32 block without shared memory: five exchange rounds, each halving the columns a lane
+// still carries (a lane keeps the half selected by its own bit); lane j ends with column j.
+__device__ __forceinline__ void colsum_chunk(const Params& p, float (&v)[32], uint32_t col0, int lane) {
+#pragma unroll
+  for (int off = 16; off >= 1; off >>= 1) {
+    const bool upper = (lane & off) != 0;
+#pragma unroll
+    for (int j = 0; j < off; ++j) {
+      const float send = upper ? v[j] : v[j + off];
+      const float keep = upper ? v[j + off] : v[j];
+      v[j] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+  }
+  if (col0 + lane < p.n) atomicAdd(p.colsum + col0 + lane, v[0]);
+}
+
 // Epilogue of one 32-column chunk of one accumulator row (registers r, raw
 // fp32 bits): alpha/beta/bias/ReLU/mask, the store (or the split-K reduction
 // into C), and the optional column sums.  `o` = element offset of (row, col0)
@@ -424,22 +441,7 @@ __device__ __forceinline__ void epilogue_chunk(const Params& p, const uint32_t (
       }
     }
   }
-  if (p.colsum) {
-    // Column sums of this warp's 32 x 32 block without shared memory: five
-    // exchange rounds, each halving the columns a lane still carries (a lane
-    // keeps the half selected by its own bit); lane j ends with column j.
-#pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) {
-      const bool upper = (lane & off) != 0;
-#pragma unroll
-      for (int j = 0; j < off; ++j) {
-        const float send = upper ? v[j] : v[j + off];
-        const float keep = upper ? v[j + off] : v[j];
-        v[j] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-      }
-    }
-    if (col0 + lane < p.n) atomicAdd(p.colsum + col0 + lane, v[0]);
-  }
+  if (p.colsum) colsum_chunk(p, v, col0, lane);
 }
 
 // One row of an fp32 A slab (32 k values of row `row` of the 128-row tile) from its shared-memory stage.
