@@ -59,9 +59,23 @@ struct SmceArgs {
 // CTA partials in a fixed warp order -> workspace -> folded by the last CTA
 // (the caller guarantees that this runs in the last CTA only after all
 // partials are visible).
-template <int ITEMS>
-__device__ __forceinline__ void cta_column_partials(const float (&acc)[ITEMS], float* colsum /*smem [32*ITEMS]*/, float* out, int C) {
+template <int ITEMS, int THREADS>
+constexpr int kColumnRows = THREADS > 256 ? THREADS / 32 : 1;  // rows of shared memory below: a warp each, or one in turn
+template <int ITEMS, int THREADS = 256>
+__device__ __forceinline__ void cta_column_partials(const float (&acc)[ITEMS], float* colsum /*smem [rows][32*ITEMS]*/, float* out, int C) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if constexpr (kColumnRows<ITEMS, THREADS> > 1) {
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) colsum[(warp * ITEMS + i) * 32 + lane] = acc[i];
+    __syncthreads();
+    for (int j = threadIdx.x; j < C; j += THREADS) {
+      float s = 0.f;
+#pragma unroll
+      for (int w = 0; w < THREADS / 32; ++w) s += colsum[w * 32 * ITEMS + j];
+      out[j] = s;
+    }
+    return;
+  }
   for (int w = 0; w < kLThreads / 32; ++w) {
     if (warp == w) {
 #pragma unroll
@@ -101,7 +115,8 @@ __device__ __forceinline__ void smce_finish(const SmceArgs& a, float loss_acc, f
   if (threadIdx.x == 0 && a.loss_out) *a.loss_out = s / a.divisor;
   if (a.dbias && a.fold_bias_inline) {
     // `parts` threads per column, each over every parts-th CTA partial, then a shuffle tree
-    const unsigned parts = (C * 8 <= (int)blockDim.x) ? 8u : ((C * 4 <= (int)blockDim.x) ? 4u : ((C * 2 <= (int)blockDim.x) ? 2u : 1u));
+    unsigned parts = 1;
+    while (parts < 32 && C * parts * 2 <= blockDim.x) parts *= 2;
     const unsigned part = threadIdx.x % parts;
     const int per_trip = blockDim.x / parts;
     for (int base = 0; base < C; base += per_trip) {
@@ -145,10 +160,10 @@ __device__ __forceinline__ float grad_scale(const SmceArgs& a, float d) {
 // dlogits written once.  All loads of a trip are issued before the first
 // shuffle, the ROWS independent reductions overlap, and the element loops are
 // branch-free (index labels) so that the compiler can interleave them.
-template <int ITEMS, int ROWS, bool INDEX_LABELS, bool FAST>
-__global__ void __launch_bounds__(kLThreads) softmax_ce_kernel(const SmceArgs a) {
+template <int ITEMS, int ROWS, bool INDEX_LABELS, bool FAST, int THREADS = kLThreads>
+__global__ void __launch_bounds__(THREADS) softmax_ce_kernel(const SmceArgs a) {
   __shared__ float sm32[32];
-  __shared__ float colsum[32 * ITEMS];
+  __shared__ float colsum[kColumnRows<ITEMS, THREADS> * 32 * ITEMS];
   const int lane = threadIdx.x & 31;
   const int C = a.C;
   const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
@@ -248,7 +263,7 @@ __global__ void __launch_bounds__(kLThreads) softmax_ce_kernel(const SmceArgs a)
     }
   }
   float* bias_partial = a.partial + gridDim.x;
-  if (a.dbias) cta_column_partials<ITEMS>(bias_acc, colsum, bias_partial + (size_t)blockIdx.x * C, C);
+  if (a.dbias) cta_column_partials<ITEMS, THREADS>(bias_acc, colsum, bias_partial + (size_t)blockIdx.x * C, C);
   smce_finish(a, loss_acc, sm32);
 }
 
@@ -1004,11 +1019,11 @@ static void launch_smce_rows(cudaStream_t s, SmceArgs a) {
   launch_pdl(softmax_ce_row_kernel<CP, IDX, FAST>, dim3(gr), dim3(kRowThreads), 0, s, a);
 }
 
-template <int ITEMS, int ROWS, bool IDX, bool FAST>
+template <int ITEMS, int ROWS, bool IDX, bool FAST, int THREADS = kLThreads>
 static void launch_smce_warps(cudaStream_t s, SmceArgs a) {
-  static const unsigned resident = resident_ctas(softmax_ce_kernel<ITEMS, ROWS, IDX, FAST>, kLThreads);
+  static const unsigned resident = resident_ctas(softmax_ce_kernel<ITEMS, ROWS, IDX, FAST, THREADS>, THREADS);
   const int C = a.C;
-  const size_t rows_per_cta = (size_t)(kLThreads / 32) * ROWS;
+  const size_t rows_per_cta = (size_t)(THREADS / 32) * ROWS;
   unsigned g = (unsigned)std::min<size_t>((a.rows + rows_per_cta - 1) / rows_per_cta, resident);
   // The bias gradient leaves the kernel as one partial row per CTA.  Few of
   // them are folded by the last CTA to finish; many (wide rows on a large grid)
@@ -1020,7 +1035,7 @@ static void launch_smce_warps(cudaStream_t s, SmceArgs a) {
   a.partial = partial;
   a.counter = counters;
   a.fold_bias_inline = separate_fold ? 0 : 1;
-  if (!launch_pdl(softmax_ce_kernel<ITEMS, ROWS, IDX, FAST>, dim3(g), dim3(kLThreads), 0, s, a)) return;
+  if (!launch_pdl(softmax_ce_kernel<ITEMS, ROWS, IDX, FAST, THREADS>, dim3(g), dim3(THREADS), 0, s, a)) return;
   if (separate_fold) fold_rows_f32(s, partial + g, a.dbias, g, (size_t)C);
 }
 
@@ -1125,6 +1140,17 @@ static void launch_softmax_ce(cudaStream_t s, SmceArgs a) {
       if (C <= 24) return launch_smce_rows_staged<24>(s, a);
       return launch_smce_rows_staged<32>(s, a);
     }
+  }
+  // Few rows: a row per warp, spread over the chip.  Several rows per warp leave most SMs idle and are a longer chain (1000 x
+  // 37 with bias gradient 9.9 us against 6.7, 512 x 300 22 against 8.6, 1000 x 500 42 against 13); so is a thread per row
+  // (100 x 10 5.0 against 3.5, 1000 x 10 5.5 against 4.6) unless the bias gradient, cheap there, is wanted (equal).
+  // Large CTAs, because the last one folds a partial bias gradient per CTA.
+  if (a.rows <= (size_t)sm_count() * 8 && C <= 512 && (C > 32 || !a.dbias)) {
+    if (C <= 32) return launch_smce_warps<1, 1, IDX, false, 1024>(s, a);
+    if (C <= 64) return launch_smce_warps<2, 1, IDX, false, 1024>(s, a);
+    if (C <= 128) return launch_smce_warps<4, 1, IDX, false, 1024>(s, a);
+    if (C <= 256) return launch_smce_warps<8, 1, IDX, false, 512>(s, a);
+    return launch_smce_warps<16, 1, IDX, false, 512>(s, a);
   }
   if (C <= 4) ZG_ROWS(4);
   if (C <= 8) ZG_ROWS(8);
