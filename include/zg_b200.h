@@ -317,6 +317,11 @@ EXTERN_C void zg_segment_sumsq(dtype id, StreamWrapper stream, const void* x, co
 EXTERN_C int zg_masked_softmax_ce_supported(dtype id, len_t rows, len_t C);
 EXTERN_C void zg_masked_softmax_ce(dtype id, StreamWrapper stream, const void* logits, const len_t* offsets, const void* labels, int label_kind,
                                    len_t rows, len_t C, len_t ld, double divisor, void* loss, void* dlogits, void* dbias);
+/* out[n, c] = sum over u < count of A[rows[u], n] * x[rows[u], c] (A^T . x for an x whose only nonzero rows are the listed
+ * ones, each once); C <= 16. */
+EXTERN_C int zg_rows_tn_supported(dtype id, len_t C);
+EXTERN_C void zg_rows_tn(dtype id, StreamWrapper stream, void* out, len_t ldo, const void* A, len_t lda, const void* x, len_t ldx, const len_t* rows,
+                         len_t count, len_t N, len_t C);
 /* The ops between the forward passes of a Q-learning update and its backward pass as one launch (a dozen ops of the device
  * interface; examples/dqn/src/dqn_agent.zig:111-228).  qn = the target network's values of the next states, q = the
  * policy's of the states, both [batch, actions] and clamped in place; dq, dbias, loss, .. are overwritten. */

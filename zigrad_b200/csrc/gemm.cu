@@ -649,6 +649,18 @@ extern "C" void zg_set_math_mode(int mode) {
 }
 extern "C" int zg_get_math_mode(void) { return g_math_mode; }
 
+extern "C" int zg_rows_tn_supported(dtype id, len_t C) { return id == SINGLE && C >= 1 && C <= 16; }
+
+extern "C" void zg_rows_tn(dtype id, StreamWrapper w, void* out, len_t ldo, const void* A, len_t lda, const void* x, len_t ldx, const len_t* rows,
+                           len_t count, len_t N, len_t C) {
+  if (!zg_rows_tn_supported(id, C)) { set_error(kUnsupported, "zg_rows_tn: dtype %d, %lu columns", (int)id, C); return; }
+  if (N == 0) return;
+  if (N > 0xffffffffu) { set_error(kBadArgument, "zg_rows_tn: %lu columns of A", N); return; }
+  auto kern = C <= 4 ? skinny::rows_tn_kernel<4> : (C <= 8 ? skinny::rows_tn_kernel<8> : (C <= 12 ? skinny::rows_tn_kernel<12> : skinny::rows_tn_kernel<16>));
+  launch_pdl(kern, dim3((unsigned)((N + 31) / 32)), dim3(skinny::kRowsThreads), 0, as_stream(w), (float*)out, (size_t)ldo, (const float*)A, (size_t)lda,
+             (const float*)x, (size_t)ldx, rows, (size_t)count, (size_t)N, (int)C);
+}
+
 extern "C" void zg_bmm(dtype id, dtype c_id, StreamWrapper stream, const void* A, const void* B, void* C, len_t nA, len_t nB, len_t nC,
                        len_t m, len_t n, len_t k, bool trans_a, bool trans_b, len_t lda, len_t ldb, len_t ldc, double alpha, double beta,
                        int epilogue, const void* bias, const void* mask_src, void* colsum) {

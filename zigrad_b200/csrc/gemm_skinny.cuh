@@ -228,5 +228,56 @@ __global__ void __launch_bounds__(kThreads) skinny_m_kernel(const Params p, cons
   }
 }
 
+// out[n, c] = sum over u of A[rows[u], n] * x[rows[u], c]: the transposed product with an x of which only `count` rows, all
+// of them listed, are not zero -- a node classifier's gradient behind a mask of labelled nodes.  What it reads is those
+// rows of A instead of all of it: 140 of 2708 rows, 7 columns, 3.8 us against 10.3 for the whole product on the tensor cores.
+// A CTA owns 32 columns of A, its 16 warps every 16th row each (two dependent round trips: index, then row), and the
+// warps' sums meet in shared memory in a fixed order.
+constexpr int kRowsThreads = 512;
+template <int CM>
+__global__ void __launch_bounds__(kRowsThreads) rows_tn_kernel(float* __restrict__ out, size_t ldo, const float* __restrict__ A, size_t lda,
+                                                               const float* __restrict__ x, size_t ldx, const len_t* __restrict__ rows, size_t count,
+                                                               size_t N, int C) {
+  constexpr int kWarps = kRowsThreads / 32, U = 8;
+  __shared__ float part[kWarps][32][CM + 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const size_t n = (size_t)blockIdx.x * 32 + lane;
+  pdl_sync();
+  float acc[CM];
+#pragma unroll
+  for (int c = 0; c < CM; ++c) acc[c] = 0.f;
+  size_t r[U];
+#pragma unroll
+  for (int i = 0; i < U; ++i) r[i] = warp + i * kWarps < count ? (size_t)__ldg(rows + warp + i * kWarps) : 0;
+  for (size_t u0 = warp; u0 < count; u0 += kWarps * U) {
+    float a[U], xv[U];
+#pragma unroll
+    for (int i = 0; i < U; ++i) {
+      const bool ok = u0 + i * kWarps < count;
+      a[i] = ok && n < N ? __ldg(A + r[i] * lda + n) : 0.f;
+      xv[i] = ok && lane < C ? __ldg(x + r[i] * ldx + lane) : 0.f;
+    }
+    const size_t next = u0 + kWarps * U;
+#pragma unroll
+    for (int i = 0; i < U; ++i) r[i] = next + i * kWarps < count ? (size_t)__ldg(rows + next + i * kWarps) : 0;
+#pragma unroll
+    for (int i = 0; i < U; ++i)
+#pragma unroll
+      for (int c = 0; c < CM; ++c) acc[c] = fmaf(a[i], __shfl_sync(0xffffffffu, xv[i], c), acc[c]);
+  }
+#pragma unroll
+  for (int c = 0; c < CM; ++c) part[warp][lane][c] = acc[c];
+  __syncthreads();
+  for (int e = threadIdx.x; e < 32 * C; e += kRowsThreads) {
+    const int row = e / C, c = e % C;
+    const size_t o = (size_t)blockIdx.x * 32 + row;
+    if (o >= N) continue;
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) s += part[w][row][c];
+    out[o * ldo + c] = s;
+  }
+}
+
 }  // namespace skinny
 }  // namespace zg

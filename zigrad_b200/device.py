@@ -578,6 +578,12 @@ class CudaDevice:
                            p.lr, int(p.clip), p.max_norm, p.delta, p.norms.ptr if p.norms is not None else None,
                            int(bool(getattr(p, 'zero_grads', False))))
 
+    def rows_tn_supported(self, dtype: int, classes: int) -> bool:
+        return bool(self.L.zg_rows_tn_supported(dtype, classes))
+
+    def rows_tn(self, p):
+        self.L.zg_rows_tn(p.A.dtype, self.stream, p.out.ptr, p.ldo, p.A.ptr, p.lda, p.x.ptr, p.ldx, p.rows.ptr, p.rows.len, p.n, p.classes)
+
     def masked_softmax_ce_supported(self, dtype: int, rows: int, classes: int) -> bool:
         return bool(self.L.zg_masked_softmax_ce_supported(dtype, rows, classes))
 

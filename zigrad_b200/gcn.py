@@ -57,11 +57,15 @@ class GcnTrainer:
             src, tgt, deg = edges
             rp, ci = edges_to_csr(tgt, src, N)      # forward: grouped by target, neighbours = sources
             rpt, cit = edges_to_csr(src, tgt, N)    # gradient w.r.t. h: grouped by source, neighbours = targets
-            self.csr = tuple(d.from_numpy(a) for a in (rp, ci, rpt, cit))
+            # ... of which the gradient of the logits needs the edges into masked nodes only: it is zero elsewhere
+            into = np.isin(tgt, mask_idx)
+            rpm, cim = edges_to_csr(np.asarray(src)[into], np.asarray(tgt)[into], N)
+            self.csr = tuple(d.from_numpy(a) for a in (rp, ci, rpt, cit, rpm, cim))
             self.deg = d.from_numpy(np.ascontiguousarray(deg, np.float32))
             self.A = None
         else:
             self.A = d.from_numpy(np.ascontiguousarray(A_hat, np.float32))
+        self.mask_rows = d.from_numpy(np.unique(np.asarray(mask_idx, np.uint64)))
         # flat parameters in attach order: W1 [H, Fp], b1 [H], W2 [C, H], b2 [C]
         W1p = np.zeros((H, Fp), np.float32)
         W1p[:, :F] = W1
@@ -101,11 +105,21 @@ class GcnTrainer:
         """out = A.x (+ bias, ReLU) -- dense GEMM with the adjacency, or the CSR walk over the edges."""
         N = self.N
         if self.sparse:
-            rp, ci, rpt, cit = self.csr
+            rp, ci, rpt, cit = self.csr[:4]
             self.dev.dispatch(opspec.csr_gcn_propagate(out, x, self.deg, rpt if transpose else rp, cit if transpose else ci, N, F, ld, ld,
                                                        transpose, epilogue, bias))
         else:
             self._mm(self.A, x, out, N, F, N, transpose, False, N, ld, ld, 0.0, epilogue, bias)
+
+    def _prop_dlogits(self):
+        """dh2 = A^T . dlogits, of which only the masked nodes' rows are not zero (up to a sixth of them it pays to say so)."""
+        d, N, C, Cp = self.dev, self.N, self.C, self.Cp
+        if self.sparse:
+            d.dispatch(opspec.csr_gcn_propagate(self.dh2, self.dlog, self.deg, self.csr[4], self.csr[5], N, C, Cp, Cp, True, "none", None))
+        elif 6 * self.mask_rows.len <= N and d.rows_tn_supported(SINGLE, C):
+            d.dispatch(opspec.rows_tn(self.dh2, Cp, self.A, N, self.dlog, Cp, self.mask_rows, N, C))
+        else:
+            self._prop(self.dlog, self.dh2, C, Cp, transpose=True)
 
     def step(self, T_masked: DeviceSlice):
         """T_masked: one-hot targets of the masked rows, fp32 [M, C] contiguous."""
@@ -137,7 +151,7 @@ class GcnTrainer:
                                          bias_grad=self.db2))
             d.dispatch(opspec.scatter_add(self.dm, self.offsets, self.dlog))                        # MaskLayer backward
         # ---- backward
-        self._prop(self.dlog, self.dh2, C, Cp, transpose=True)                                    # dh2 = A^T . dlogits
+        self._prop_dlogits()                                                                       # dh2 = A^T . dlogits
         with d.branch(0):  # nothing below reads dW2: beside the rest of the backward pass
             self._mm(self.dh2, self.a1, self.dW2, C, H, N, True, False, Cp, H, H, 1.0)            # dW2 += dh2^T . a1
         self._mm(self.dh2, self.W2, self.da1, N, H, C, False, False, Cp, H, H, 0.0, "relu_mask", None, self.a1,
@@ -168,6 +182,6 @@ class GcnTrainer:
         d.sync()
         self._graphs.clear()
         extra = list(self.csr) + [self.deg] if self.sparse else [self.A]
-        for s in extra + [self.X, self.params, self.grads, self.m, self.v, self.norms, self.h1, self.a1, self.h2, self.logits,
+        for s in extra + [self.mask_rows, self.X, self.params, self.grads, self.m, self.v, self.norms, self.h1, self.a1, self.h2, self.logits,
                   self.dlog, self.dh2, self.da1, self.dh1, self.mlog, self.dm, self.offsets, self.loss, self.t_dev]:
             d.mem_cache_free(s)

@@ -541,6 +541,20 @@ class adam:
     tau: float = 0.0
 
 
+@_op("rows_tn")
+class rows_tn:
+    """out[n, c] = sum over the listed rows r of A[r, n] * x[r, c]: A^T . x where all other rows of x are zero."""
+    out: Any
+    ldo: int
+    A: Any
+    lda: int
+    x: Any
+    ldx: int
+    rows: Any        # u64, each once
+    n: int
+    classes: int
+
+
 @_op("masked_softmax_ce")
 class masked_softmax_ce:
     """mem_take, softmax_ce and scatter_add of a MaskLayer in front of the loss as one
