@@ -317,6 +317,11 @@ EXTERN_C void zg_segment_sumsq(dtype id, StreamWrapper stream, const void* x, co
 EXTERN_C int zg_masked_softmax_ce_supported(dtype id, len_t rows, len_t C);
 EXTERN_C void zg_masked_softmax_ce(dtype id, StreamWrapper stream, const void* logits, const len_t* offsets, const void* labels, int label_kind,
                                    len_t rows, len_t C, len_t ld, double divisor, void* loss, void* dlogits, void* dbias);
+/* Forward pass of an MLP on one row as one launch: out[l] = relu(W[l] out[l-1] + b[l]), no ReLU on the last; W[l] is
+ * [dims[l+1], dims[l]].  The arrays are read during the call. */
+EXTERN_C int zg_mlp_forward_supported(dtype id, len_t layers, const len_t* dims);
+EXTERN_C void zg_mlp_forward(dtype id, StreamWrapper stream, const void* X, len_t layers, const len_t* dims, void* const* W, void* const* b,
+                             void* const* out);
 /* out[n, c] = sum over u < count of A[rows[u], n] * x[rows[u], c] (A^T . x for an x whose only nonzero rows are the listed
  * ones, each once); C <= 16. */
 EXTERN_C int zg_rows_tn_supported(dtype id, len_t C);

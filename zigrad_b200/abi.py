@@ -211,6 +211,8 @@ SIGNATURES = {
     "zg_adam_step": (None, [dtype_t, S, vp, vp, vp, vp, C.POINTER(Segment), len_t, len_t, dbl, dbl, dbl, dbl, i32, dbl, dbl, vp, vp, vp]),
     "zg_adam_step_part": (None, [dtype_t, S, vp, vp, vp, vp, C.POINTER(Segment), len_t, len_t, dbl, dbl, dbl, dbl, i32, dbl, dbl, vp, vp, vp, i32]),
     "zg_adam_soft_step": (None, [dtype_t, S, vp, vp, vp, vp, C.POINTER(Segment), len_t, len_t, dbl, dbl, dbl, dbl, i32, dbl, dbl, vp, vp, vp, dbl]),
+    "zg_mlp_forward_supported": (i32, [dtype_t, len_t, vp]),
+    "zg_mlp_forward": (None, [dtype_t, S, vp, len_t, vp, vp, vp, vp]),
     "zg_rows_tn_supported": (i32, [dtype_t, len_t]),
     "zg_rows_tn": (None, [dtype_t, S, vp, len_t, vp, len_t, vp, len_t, vp, len_t, len_t, len_t]),
     "zg_masked_softmax_ce_supported": (i32, [dtype_t, len_t, len_t]),

@@ -11,6 +11,7 @@
 #include "driver_api.h"
 #include "gemm_tc.cuh"
 #include "gemm_tc_persistent.cuh"
+#include "mlp_forward.cuh"
 #include "gemm_skinny.cuh"
 #include "gemm_block.cuh"
 #include "mlp_tail.cuh"
@@ -648,6 +649,36 @@ extern "C" void zg_set_math_mode(int mode) {
   g_math_mode = mode;
 }
 extern "C" int zg_get_math_mode(void) { return g_math_mode; }
+
+// One row of a network whose weights eight SMs read about as fast as a chain of launches starts (see mlp_forward.cuh)
+constexpr size_t kFwdWeights = 200 * 1000;
+extern "C" int zg_mlp_forward_supported(dtype id, len_t layers, const len_t* dims) {
+  if (id != SINGLE || layers == 0 || layers > mlp_fwd::kMaxLayers) return 0;
+  size_t weights = 0, inputs = 0;
+  for (len_t l = 0; l < layers; ++l) {
+    if (dims[l] == 0 || dims[l + 1] == 0 || dims[l] > kFwdWeights || dims[l + 1] > kFwdWeights) return 0;
+    weights += dims[l] * dims[l + 1];
+    inputs += (dims[l] + 3) / 4 * 4;
+  }
+  return weights <= kFwdWeights && inputs * sizeof(float) <= 48 * 1024;
+}
+
+extern "C" void zg_mlp_forward(dtype id, StreamWrapper w, const void* X, len_t layers, const len_t* dims, void* const* W, void* const* b,
+                               void* const* out) {
+  if (!zg_mlp_forward_supported(id, layers, dims)) { set_error(kUnsupported, "zg_mlp_forward: dtype %d, %lu layers", (int)id, layers); return; }
+  mlp_fwd::Params p;
+  memset(&p, 0, sizeof(p));
+  p.X = static_cast<const float*>(X);
+  p.layers = (int)layers;
+  uint32_t at = 0;
+  for (len_t l = 0; l < layers; ++l) {
+    const uint32_t K = (uint32_t)dims[l];
+    p.l[l] = {static_cast<const float*>(W[l]), static_cast<const float*>(b[l]), static_cast<float*>(out[l]), K, (uint32_t)dims[l + 1], at,
+              host_aligned16(W[l]) && K % 4 == 0};
+    at += (K + 3) / 4 * 4;
+  }
+  launch_pdl_cluster(mlp_fwd::mlp_forward_kernel, dim3(mlp_fwd::kCluster), dim3(mlp_fwd::kThreads), at * sizeof(float), as_stream(w), mlp_fwd::kCluster, p);
+}
 
 extern "C" int zg_rows_tn_supported(dtype id, len_t C) { return id == SINGLE && C >= 1 && C <= 16; }
 

@@ -578,6 +578,14 @@ class CudaDevice:
                            p.lr, int(p.clip), p.max_norm, p.delta, p.norms.ptr if p.norms is not None else None,
                            int(bool(getattr(p, 'zero_grads', False))))
 
+    def mlp_forward_supported(self, dtype: int, dims) -> bool:
+        return bool(self.L.zg_mlp_forward_supported(dtype, len(dims) - 1, _shape(dims)))
+
+    def mlp_forward(self, p):
+        n = len(p.dims) - 1
+        ptrs = lambda slices: (abi.vp * n)(*[s.ptr for s in slices])
+        self.L.zg_mlp_forward(p.X.dtype, self.stream, p.X.ptr, n, _shape(p.dims), ptrs(p.W), ptrs(p.b), ptrs(p.out))
+
     def rows_tn_supported(self, dtype: int, classes: int) -> bool:
         return bool(self.L.zg_rows_tn_supported(dtype, classes))
 

@@ -196,6 +196,9 @@ class MlpTrainer:
             # cleared the gradients already.
             self._zero_due = self._zero_due or not self._grads_clear
             self._grads_clear = False
+        if self.fused and not self.bf16 and B == 1 and d.mlp_forward_supported(SINGLE, self.dims):
+            d.dispatch(opspec.mlp_forward(X, self.dims, self.W, self.b, self.act))
+            return self.act[-1]
         for l in range(self.L):
             K, N = self.dims[l], self.dims[l + 1]
             last = l + 1 == self.L

@@ -541,6 +541,17 @@ class adam:
     tau: float = 0.0
 
 
+@_op("mlp_forward")
+class mlp_forward:
+    """The `linear` ops of an MLP's forward pass on one row as one device op: out[l] = relu(W[l] out[l-1] + b[l]), no ReLU on
+    the last layer."""
+    X: Any
+    dims: Any        # widths, input first
+    W: Any           # per layer [dims[l + 1], dims[l]]
+    b: Any
+    out: Any
+
+
 @_op("rows_tn")
 class rows_tn:
     """out[n, c] = sum over the listed rows r of A[r, n] * x[r, c]: A^T . x where all other rows of x are zero."""
