@@ -422,11 +422,13 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   memset(&tmC, 0, sizeof(tmC));
   static const bool tma_epi_on = [] { const char* e = getenv("ZG_GEMM_TMA_EPILOGUE"); return !(e && e[0] == '0'); }();
   const bool tma_epi = tma_epi_on && p.vec_ok && !swap && nC <= 0x7fffffffu;
+  // A store is clipped at a whole 16-byte word: one past n would clear padding columns (a reduction adds zeros to them)
+  const bool tma_store = tma_epi && n * (c_id == SINGLE ? 4 : 2) % 16 == 0;
   if (persistent) {
     const bool add = splits > 1 || (beta == 1.0 && epilogue == ZG_EPI_NONE && !colsum && c_id == SINGLE);
     CUtensorMap tmM;
     memset(&tmM, 0, sizeof(tmM));
-    if (tma_epi && (add || beta == 0.0)) {
+    if (add ? tma_epi : tma_store && beta == 0.0) {
       const bool c16 = c_id == BF16;
       if (!make_tmap(&tmC, c16, C, n, m, nC, ldc, c16 ? 64 : 32, 32, false)) return true;
       if (epilogue == ZG_EPI_RELU_MASK && !make_tmap(&tmM, c16, mask, n, m, nC, ldc, c16 ? 64 : 32, 32, false)) return true;
@@ -445,7 +447,7 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   dim3 grid((unsigned)((N + bn - 1) / bn * splits), (unsigned)((M + 127) / 128), (unsigned)nC);
   if (grid.y > 65535 || grid.z > 65535) return false;
   if (tma_epi && c_id == SINGLE && !cluster && !p.colsum &&
-      (splits > 1 ? epilogue == ZG_EPI_NONE : (beta == 0.0 && epilogue != ZG_EPI_RELU_MASK))) {
+      (splits > 1 ? epilogue == ZG_EPI_NONE : (tma_store && beta == 0.0 && epilogue != ZG_EPI_RELU_MASK))) {
     if (!make_tmap(&tmC, false, C, n, m, nC, ldc, 32, 32, false)) return true;
     p.tma_epilogue = splits > 1 ? 2 : 1;
   }
