@@ -177,7 +177,8 @@ class MlpTrainer:
     def forward(self, X: DeviceSlice):
         if not self.fused:
             return self._forward(X)
-        self._graphs.run(("forward", X.ptr, X.dtype), lambda: self._forward(X), self._host_state, self._set_host_state)
+        key = ("forward", X.ptr, X.dtype, self._grads_clear, self._zero_due)  # what the flags are afterwards depends on both
+        self._graphs.run(key, lambda: self._forward(X), self._host_state, self._set_host_state)
         return self.act[-1]
 
     def _host_state(self):
