@@ -45,6 +45,44 @@ def pair(gpu, request):
     p.free()
 
 
+def test_graph_of_the_caller_then_evaluation_then_update(gpu, pair):
+    (X, T), other = pair.data[0], pair.data[1][0]
+    pair.a.forward(other)
+    gpu.capture.open()
+    pair.a.forward(X)
+    pair.backward(pair.a)
+    gpu.capture.save()
+    pair.a.forward(other)  # evaluation
+    gpu.capture.run()
+    pair.b.forward(X)
+    pair.backward(pair.b)
+    assert pair.check("grads").any()
+    for tr in (pair.a, pair.b):
+        tr.update()
+    gpu.capture.free()
+    pair.check()
+
+
+def test_captured_forward_and_ops_behind_it(gpu):
+    # (not with zero_grads_in_update: a graph captured while the update clears relies on the update)
+    pair = Pair(gpu, opt="sgd")
+    X = pair.data[0][0]
+    gpu.capture.open()
+    pair.a.forward(X)
+    gpu.capture.save()
+    for _ in range(3):
+        gpu.capture.run()
+        pair.backward(pair.a)
+        pair.b.forward(X)
+        pair.backward(pair.b)
+        pair.check("grads")
+        for tr in (pair.a, pair.b):
+            tr.update()
+    gpu.capture.free()
+    pair.check()
+    pair.free()
+
+
 def test_repeated_forward_without_an_update_in_between(gpu, pair):
     X = pair.data[0][0]
     for i in range(8):
@@ -55,3 +93,32 @@ def test_repeated_forward_without_an_update_in_between(gpu, pair):
                 tr.update()
     pair.check("grads")
     pair.check()
+
+
+def test_a_slice_taken_before_shows_zeros_behind_a_forward_pass(gpu):
+    pair = Pair(gpu, opt="adam")
+    held, layer, X = pair.a.grads, pair.a.layer_grads(1), pair.data[0][0]
+    for i in range(5):
+        pair.a.forward(X)
+        assert not gpu.to_numpy(held).any() and not gpu.to_numpy(layer).any(), i
+        pair.backward(pair.a)
+        assert gpu.to_numpy(held).any() and gpu.to_numpy(layer).any(), i
+    gpu.mem_fill(held, 3.0)  # somebody else's writes are cleared as well
+    pair.a.forward(X)
+    assert not gpu.to_numpy(held).any()
+    pair.free()
+
+
+def test_graph_of_the_caller_over_a_trainer_that_never_had_gradients(gpu):
+    pair = Pair(gpu, opt="none")
+    X = pair.data[0][0]
+    gpu.capture.open()
+    pair.a.forward(X)
+    gpu.capture.save()
+    for _ in range(4):
+        pair.a.forward(X)  # nothing to clear
+    pair.backward(pair.a)
+    gpu.capture.run()
+    assert not gpu.to_numpy(pair.a.grads).any()
+    gpu.capture.free()
+    pair.free()

@@ -184,6 +184,10 @@ class CudaDevice:
         self.L.stream_synchronize(self.stream)
         abi.check()
 
+    def capturing(self) -> bool:
+        """What is issued now goes into a graph and is run later."""
+        return bool(self.L.zg_stream_capturing(self.stream))
+
     def make_current(self):
         self.L.zg_set_device(self.device_number)
 

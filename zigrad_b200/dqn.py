@@ -49,7 +49,7 @@ class DqnTrainer:
              dones: DeviceSlice):
         p = self.policy
         key = (states.ptr, actions.ptr, next_states.ptr, rewards.ptr, dones.ptr, self.gamma, self.tau, self.q_clip, p.lr, p.opt, p.beta1,
-               p.beta2, p.eps, p.clip, p.max_norm, p.delta, self.target._grads_clear, p._grads_clear)
+               p.beta2, p.eps, p.clip, p.max_norm, p.delta, self.target._touched)
         self._graphs.run(key, lambda: self._step(states, actions, next_states, rewards, dones), self._host_state, self._set_host_state)
 
     def _host_state(self):
@@ -66,10 +66,11 @@ class DqnTrainer:
         # ---- both forward passes (gradients disabled in the reference for the target net): independent chains of
         # small kernels; zero_grad of the policy net rides on the side stream
         with d.branch(1):
-            qn = tgt.forward(next_states)
-            d.mem_fill(pol._grads, 0.0)
-        q_all = pol.forward(states)
-        pol._zero_due = False
+            if tgt._touched:  # (it has no backward pass: only if somebody holds its gradients)
+                tgt.zero_grad()
+            qn = tgt._layers(next_states)
+            pol.zero_grad()
+        q_all = pol._layers(states)
         d.join()
         # ---- targets, gather by action, loss and its gradient w.r.t. all Q values, last bias gradient
         fused = d.q_head_supported(SINGLE, B, C)

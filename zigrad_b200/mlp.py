@@ -116,7 +116,7 @@ class MlpTrainer:
                                for w, b in zip(weights, biases)])
         d.mem_transfer_htod(flat, self.params)
         d.mem_fill(self._grads, 0.0)
-        self._zero_due = False  # zero_grad was asked for by a forward pass and has not been issued yet
+        self._touched = False  # a gradient has been written, or the buffer handed out
         self._graphs = GraphCache(d)  # repeated steps (replay.py)
         if opt == "adam":
             self.m, self.v = d.mem_cache_alloc(SINGLE, off), d.mem_cache_alloc(SINGLE, off)
@@ -152,51 +152,58 @@ class MlpTrainer:
         d.sync()
 
     # -------------------------------------------------------------- gradients
-    def _settle(self):
-        """Issue the zero_grad that is due (model.zig:57-62) as ONE fill of the flat gradient buffer."""
-        if self._zero_due:
-            self._zero_due = False
-            self.dev.mem_fill(self._grads, 0.0)
+    def _zero_grad_due(self) -> bool:
+        """Whether a forward pass that starts now has to clear the gradients (model.zig:57-62).  Not behind an update that
+        did (zero_grads_in_update), and not while they are the zeros of construction: no backward pass has written them
+        and nobody holds the buffer.  A graph of the caller's clears them all the same, since it may be run later."""
+        due = not self._grads_clear and (self._touched or self.dev.capturing())
+        self._grads_clear = False
+        return due
+
+    def zero_grad(self):
+        """ONE fill of the flat gradient buffer."""
+        self.dev.mem_fill(self._grads, 0.0)
+        self._grads_clear = False
 
     @property
     def grads(self) -> DeviceSlice:
-        self._settle()
+        self._touched = True
         return self._grads
 
     @property
     def dW(self) -> List[DeviceSlice]:
-        self._settle()
+        self._touched = True
         return self._dW
 
     @property
     def db(self) -> List[DeviceSlice]:
-        self._settle()
+        self._touched = True
         return self._db
 
     # ------------------------------------------------------------------ pieces
     def forward(self, X: DeviceSlice):
         if not self.fused:
-            return self._forward(X)
-        key = ("forward", X.ptr, X.dtype, self._grads_clear, self._zero_due)  # what the flags are afterwards depends on both
-        self._graphs.run(key, lambda: self._forward(X), self._host_state, self._set_host_state)
+            return self._layers(X)
+        zero = self._zero_grad_due()
+        self._graphs.run(("forward", X.ptr, X.dtype, zero), lambda: self._forward(X, zero), self._host_state, self._set_host_state)
         return self.act[-1]
 
     def _host_state(self):
-        return self.t, self._grads_clear, self._zero_due
+        return self.t, self._grads_clear, self._touched
 
     def _set_host_state(self, state):
-        self.t, self._grads_clear, self._zero_due = state
+        self.t, self._grads_clear, self._touched = state
 
-    def _forward(self, X: DeviceSlice):
+    def _forward(self, X: DeviceSlice, zero: bool):
+        # The gradients are cleared here, in front of the products: the weight-gradient GEMMs accumulate with beta = 1 as
+        # the reference does.
+        if zero:
+            self.zero_grad()
+        return self._layers(X)
+
+    def _layers(self, X: DeviceSlice):
         d, B = self.dev, self.B
         inp = X
-        if self.fused:
-            # zero_grad is due from here on (the weight-gradient GEMMs accumulate with beta = 1 as the reference
-            # does) and issued when the first gradient is about to be written or somebody looks: a forward pass
-            # alone does not pay for it.  With zero_grads_in_update the previous step's SGD kernel has
-            # cleared the gradients already.
-            self._zero_due = self._zero_due or not self._grads_clear
-            self._grads_clear = False
         if self.fused and not self.bf16 and B == 1 and d.mlp_forward_supported(SINGLE, self.dims):
             d.dispatch(opspec.mlp_forward(X, self.dims, self.W, self.b, self.act))
             return self.act[-1]
@@ -217,7 +224,7 @@ class MlpTrainer:
 
     def loss_and_grad(self, T: DeviceSlice):
         d, B, C = self.dev, self.B, self.dims[-1]
-        self._settle()
+        self._touched = True
         if self.fused:  # the bias gradient of the last layer comes out of the same pass
             d.dispatch(opspec.softmax_ce(self.act[-1], T, B, C, self.loss, self.dact[-1], self.loss_div, accumulate=False,
                                          ld=self.ld_out, bias_grad=self._db[-1]))
@@ -243,7 +250,7 @@ class MlpTrainer:
         wide MLP the update then competes with the persistent GEMMs for memory bandwidth
         and the step got slower (2.39 ms against 2.27 ms with one update after the join)."""
         d, B = self.dev, self.B
-        self._settle()
+        self._touched = True
         if self.fused and not last_bias_done:
             if self.ld_out != self.dims[-1]:
                 raise ValueError("an external output gradient needs unpadded logits (pad_logits=False)")
@@ -306,7 +313,6 @@ class MlpTrainer:
     def update(self, soft_target: Optional[DeviceSlice] = None, tau: float = 0.0):
         """`soft_target` (Adam): a target network's flat parameters, moved towards the updated ones by tau."""
         d = self.dev
-        self._settle()
         if self.opt == "sgd":
             d.dispatch(opspec.sgd(self.params, self._grads, self.segments, self.lr, self.clip, self.max_norm, self.delta, self.norms,
                                   self.zero_grads_in_update))
@@ -323,6 +329,7 @@ class MlpTrainer:
     def layer_grads(self, l: int) -> DeviceSlice:
         """The contiguous slice [dW_l ; db_l] of the flat gradient buffer."""
         off = self.segments[2 * l][0]
+        self._touched = True
         return self._grads.view(off, self.segments[2 * l][1] + self.segments[2 * l + 1][1])
 
     def _forward_backward_tail(self, X: DeviceSlice, T: DeviceSlice, fuse_update: bool = False):
@@ -341,9 +348,9 @@ class MlpTrainer:
         layer's product; no update waits for the join of all streams.  The weights of the
         layers in between are still read by the dX products and are updated after the join."""
         d, B, L = self.dev, self.B, self.L
-        if self._zero_due or not self._grads_clear:
-            d.mem_fill(self._grads, 0.0)
-        self._grads_clear = self._zero_due = False
+        if self._zero_grad_due():
+            self.zero_grad()
+        self._touched = True
 
         in_gemm = fuse_update and self.zero_grads_in_update
         nlr = -float(np.float32(self.lr))  # lr cast f64 -> f32, then negated (optim.zig:103)
@@ -417,8 +424,7 @@ class MlpTrainer:
         if allreduce is not None:
             return self._step(X, T, allreduce)
         key = (X.ptr, X.dtype, T.ptr, T.dtype, self.lr, self.opt, self.beta1, self.beta2, self.eps, self.clip, self.max_norm, self.delta,
-               self.loss_div, self.fused, self.tail, self.fuse_update, self.update_by_layer, self.zero_grads_in_update, self._grads_clear,
-               self._zero_due)
+               self.loss_div, self.fused, self.tail, self.fuse_update, self.update_by_layer, self.zero_grads_in_update, self._grads_clear)
         self._graphs.run(key, lambda: self._step(X, T, None), self._host_state, self._set_host_state)
 
     def _step(self, X: DeviceSlice, T: DeviceSlice, allreduce):
@@ -429,7 +435,7 @@ class MlpTrainer:
                 return
         else:
             by_layer = self.update_by_layer and self.fused and self.opt == "adam" and allreduce is None
-            self._forward(X)
+            self._forward(X, self.fused and self._zero_grad_due())
             self.loss_and_grad(T)
             self.backward(X, update_by_layer=by_layer)
             if by_layer:
