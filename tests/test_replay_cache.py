@@ -1,0 +1,133 @@
+"""The rules by which a trainer's steps become graphs, on a stand-in for the library that records what is asked of it (no
+GPU): what is issued when a capture fails or a step raises, where captures happen, and what a graph is found by."""
+import ctypes as C
+import threading
+
+import numpy as np
+import pytest
+
+from zigrad_b200 import abi, device
+from zigrad_b200.mlp import MlpTrainer, kaiming_uniform
+from zigrad_b200.replay import GraphCache
+
+
+class Library:
+    """Calls by name, with the stream they went to; handles are numbers that are given out once."""
+
+    def __init__(self):
+        self.calls, self.error, self.fail, self.given = [], 0, set(), 0
+        self.open = {}  # graph -> stream
+
+    def _new(self):
+        self.given += 64
+        return self.given
+
+    def init_stream(self):
+        return abi.StreamWrapper(self._new())
+
+    def init_cublas_handle(self, s):
+        return abi.CublasWrapper(self._new())
+
+    def init_cudnn_handle(self, s):
+        return abi.CudnnWrapper(self._new())
+
+    def init_cutensor_handle(self, s):
+        return abi.CutensorWrapper(self._new())
+
+    def init_device(self, n):
+        return None
+
+    def zg_device_available(self):
+        return 1
+
+    def zg_cache_alloc(self, cache, size, stream):
+        return abi.Block(self._new() << 20, self._new())
+
+    def zg_last_error(self):
+        return self.error
+
+    def zg_clear_error(self):
+        self.error = 0
+
+    def zg_stream_capturing(self, s):
+        return int(s.ptr in self.open.values())
+
+    def open_capture(self, s):
+        self.calls.append(("open_capture", s.ptr))
+        if "open" in self.fail:
+            self.error = 1
+            return abi.GraphWrapper(0)
+        g = self._new()
+        self.open[g] = s.ptr
+        return abi.GraphWrapper(g)
+
+    def save_capture(self, g, s):
+        if not g.ptr:
+            return
+        self.calls.append(("save_capture", s.ptr))
+        del self.open[g.ptr]
+        if "save" in self.fail:
+            self.error = 1
+
+    def __getattr__(self, name):
+        def call(*args):
+            streams = [a.ptr for a in args if isinstance(a, abi.StreamWrapper)]
+            self.calls.append((name, streams[0] if streams else None))
+            return 0
+        return call
+
+    def names(self):
+        return [n for n, _ in self.calls]
+
+
+@pytest.fixture()
+def dev(monkeypatch):
+    lib = Library()
+    monkeypatch.setattr(abi, "lib", lambda: lib)
+    monkeypatch.setattr(abi, "check", lambda: None)
+    return device.CudaDevice(0)
+
+
+class Steps:
+    """A step of one launch that counts, in the host's state too."""
+
+    def __init__(self, dev):
+        self.dev, self.t, self.ran = dev, 0, []
+        self.cache = GraphCache(dev)
+        self.hook = lambda: None
+
+    def body(self):
+        d = self.dev
+        self.t += 1
+        with d.branch(0):
+            d.L.kernel(d.stream)
+        self.hook()
+        d.join()
+        self.ran.append(d.capturing())
+
+    def step(self, key=0):
+        self.cache.run(key, self.body, lambda: (self.t,), self._set)
+
+    def _set(self, s):
+        (self.t,) = s
+
+
+def test_third_call_is_captured_and_replayed(dev):
+    s = Steps(dev)
+    for i in range(6):
+        s.step()
+    assert s.ran == [False, False, True] and s.t == 6
+    assert dev.L.names().count("open_capture") == 1 and dev.L.names().count("run_capture") == 4
+    s.cache.clear()
+    assert dev.L.names().count("free_capture") == 1
+
+
+def test_capture_that_does_not_open_issues_the_step_once(dev):
+    s = Steps(dev)
+    s.step()
+    s.step()
+    dev.L.fail.add("open")
+    for i in range(3, 6):
+        s.step()
+        assert s.ran == [False] * i and s.t == i and dev.L.error == 0
+    assert "run_capture" not in dev.L.names() and "save_capture" not in dev.L.names()

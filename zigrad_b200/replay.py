@@ -48,6 +48,10 @@ class GraphCache:
                 return body()
             before = save()
             graph = d.L.open_capture(d.stream)
+            if not graph.ptr:  # what is issued now runs now: once
+                d.L.zg_clear_error()
+                self.evicted = GIVE_UP
+                return body()
             try:
                 body()
             finally:
