@@ -131,3 +131,39 @@ def test_capture_that_does_not_open_issues_the_step_once(dev):
         s.step()
         assert s.ran == [False] * i and s.t == i and dev.L.error == 0
     assert "run_capture" not in dev.L.names() and "save_capture" not in dev.L.names()
+
+
+def test_capture_that_cannot_be_saved_issues_the_step_instead(dev):
+    s = Steps(dev)
+    s.step()
+    s.step()
+    dev.L.fail.add("save")
+    s.step()
+    assert s.ran == [False, False, True, False] and s.t == 3 and dev.L.error == 0
+    assert dev.L.names().count("free_capture") == 1 and "run_capture" not in dev.L.names()
+    s.step()
+    assert s.t == 4 and "run_capture" not in dev.L.names()
+
+
+@pytest.mark.parametrize("call", [1, 2, 3])
+def test_step_that_raises(dev, call):
+    s = Steps(dev)
+
+    def hook():
+        if len(s.ran) + 1 == call:
+            s.hook = lambda: None
+            raise KeyError("from the step")
+
+    s.hook = hook
+    for _ in range(call - 1):
+        s.step()
+    with pytest.raises(KeyError):
+        s.step()
+    assert s.t == (call if call < 3 else 2)  # nothing of a captured step has run
+    names = dev.L.names()
+    assert names.count("open_capture") == names.count("save_capture") == names.count("free_capture") == (1 if call == 3 else 0)
+    dev.join()
+    for _ in range(6):
+        s.step()
+    assert "run_capture" in dev.L.names() and not dev.L.open
+    assert s.t == (call if call < 3 else 2) + 6

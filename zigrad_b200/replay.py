@@ -54,8 +54,14 @@ class GraphCache:
                 return body()
             try:
                 body()
-            finally:
+            except BaseException:  # none of it has run: as before the call, side streams included
                 d.L.save_capture(graph, d.stream)
+                d.L.free_capture(graph, d.stream)
+                d.L.zg_clear_error()
+                d._forked = []
+                restore(before)
+                raise
+            d.L.save_capture(graph, d.stream)
             if d.L.zg_last_error():  # something in it cannot be captured: nothing ran, so issue it after all
                 d.L.zg_clear_error()
                 d.L.free_capture(graph, d.stream)
