@@ -1,5 +1,7 @@
 """Steps that a trainer replays as a graph of its own: same results as op-by-op steps, and never used for a call it was not
 captured from (other buffers, other hyper-parameters, inside a caller's capture or branch)."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -83,4 +85,40 @@ def test_forward_alone_leaves_zeroed_gradients_behind(gpu):
     np.testing.assert_allclose(gW[0].ravel(), 2 * once[:n], rtol=1e-4, atol=1e-7)
     tr.free()
     for s in (X, T):
+        gpu.mem_cache_free(s)
+
+
+def test_work_of_another_thread_stays_out_of_the_graph(gpu):
+    """Fills, copies and synchronisation on the device's stream by a second thread while a step is captured happen there and
+    then, and are not repeated by the steps that replay it."""
+    dims, B = [64, 32, 16], 40
+    Ws, bs = kaiming_uniform(dims, 4)
+    X, T = (gpu.from_numpy(a) for a in synthetic.mlp_batch(B, 64, 16, 1)[:2])
+    a, b = (MlpTrainer(gpu, dims, B, Ws, bs, "sgd") for _ in range(2))
+    b._graphs.evicted = replay.GIVE_UP
+    mine = gpu.from_numpy(np.zeros(1000, np.float32))
+    seen, inner = [], a.loss_and_grad
+
+    def other():
+        gpu.mem_fill(mine, 7.0)
+        seen.append(gpu.to_numpy(mine)[0])
+        gpu.sync()
+
+    def loss_and_grad(T):  # in the middle of the step
+        th = threading.Thread(target=other)
+        th.start()
+        th.join()
+        inner(T)
+
+    a.loss_and_grad = loss_and_grad
+    for i in range(6):
+        gpu.mem_fill(mine, float(i))
+        a.step(X, T)
+        b.step(X, T)
+    assert graphs(a) == 1 and seen == [7.0] * len(seen) and len(seen) == 3
+    assert gpu.to_numpy(mine)[0] == 5.0  # what this thread put there last
+    np.testing.assert_allclose(gpu.to_numpy(a.params), gpu.to_numpy(b.params), rtol=1e-4, atol=1e-6)
+    for tr in (a, b):
+        tr.free()
+    for s in (X, T, mine):
         gpu.mem_cache_free(s)

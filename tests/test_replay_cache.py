@@ -167,3 +167,59 @@ def test_step_that_raises(dev, call):
         s.step()
     assert "run_capture" in dev.L.names() and not dev.L.open
     assert s.t == (call if call < 3 else 2) + 6
+
+
+def test_captures_happen_beside_the_streams_that_others_use(dev):
+    s, main = Steps(dev), dev.stream.ptr
+    seen, mine = [], []
+
+    def hook():  # in the middle of the step
+        th = threading.Thread(target=lambda: (seen.append(dev.stream.ptr), dev.capturing() and seen.append("capturing"), dev.L.copy(dev.stream)))
+        th.start()
+        th.join()
+        mine.append(dev.stream.ptr)
+
+    s.hook = hook
+    for _ in range(5):
+        s.step()
+    assert seen == [main] * 3 and [x for n, x in dev.L.calls if n == "copy"] == [main] * 3
+    assert mine[0] == main and main not in mine[1:]
+    assert [x for n, x in dev.L.calls if n == "open_capture"] == [mine[2]] and mine[1] == mine[2]
+    assert [x for n, x in dev.L.calls if n == "run_capture"] == [main] * 3
+    kernels = [x for n, x in dev.L.calls if n == "kernel"]
+    assert kernels[1] == kernels[2] != kernels[0]  # side streams of their own, too
+    with dev.branch(0):
+        assert dev.stream.ptr == kernels[0]
+    dev.join()
+    assert dev.stream.ptr == main
+
+
+def test_one_thread_captures_at_a_time(dev):
+    first, second = Steps(dev), Steps(dev)
+    for s in (first, second):
+        s.step()
+        s.step()
+
+    def hook():
+        th = threading.Thread(target=second.step)
+        th.start()
+        th.join()
+
+    first.hook = hook
+    first.step()
+    assert first.ran == [False, False, True] and second.ran == [False, False, False] and second.t == 3
+    second.step()
+    assert second.ran[-1] is True and dev.L.names().count("run_capture") == 2
+
+
+def test_stream_chosen_by_the_user_is_everybodys(dev):
+    s, other = Steps(dev), dev.L.init_stream()
+    main, dev.stream = dev.stream, other
+    seen = []
+    th = threading.Thread(target=lambda: seen.append(dev.stream.ptr))
+    th.start()
+    th.join()
+    for _ in range(4):
+        s.step()
+    assert seen == [other.ptr] and "open_capture" not in dev.L.names()
+    dev.stream = main

@@ -13,6 +13,7 @@ import contextlib
 import functools
 import os
 import struct
+import threading
 
 import ctypes as C
 from dataclasses import dataclass
@@ -128,6 +129,32 @@ class ExecutionGraph:
         return g
 
 
+class _Lane:
+    """A stream, the side streams that its branches use and the op contexts bound to it."""
+
+    def __init__(self, L, stream):
+        self.stream = stream
+        self.sides = {}   # by index (branch(k)), created on first use
+        self.forked = []  # side streams used since the last join()
+        self.cublas = L.init_cublas_handle(stream)
+        self.cudnn = L.init_cudnn_handle(stream)
+        self.cutensor = L.init_cutensor_handle(stream)
+
+    def close(self, L):
+        L.deinit_cudnn_handle(self.cudnn)
+        L.deinit_cublas_handle(self.cublas)
+        L.deinit_cutensor_handle(self.cutensor)
+        for st in self.sides.values():
+            L.deinit_stream(st)
+        self.sides = {}
+
+
+class _Issue(threading.local):
+    """Where a thread's ops go: the main lane's stream unless it is inside branch() or apart()."""
+    lane = stream = None      # None: the main lane, `CudaDevice._stream`
+    replaying = False  # a GraphCache (replay.py) is issuing a step
+
+
 class CudaDevice:
     def __init__(self, device_number: int = 0, cache_max_bytes: int = 0, stream: Optional[int] = None):
         self.L = abi.lib()
@@ -136,23 +163,57 @@ class CudaDevice:
         self.device_number = int(device_number)
         self.properties = self.L.init_device(self.device_number)
         abi.check()
-        if stream is None:
-            self.stream = self.L.init_stream()
-            self._own_stream = True
-        else:  # adopt a stream created elsewhere (e.g. by the process's communication library)
-            self.stream = abi.StreamWrapper(stream)
-            self._own_stream = False
-        self.cublas = self.L.init_cublas_handle(self.stream)
-        self.cudnn = self.L.init_cudnn_handle(self.stream)
-        self.cutensor = self.L.init_cutensor_handle(self.stream)
+        self._own_stream = stream is None  # else adopt one created elsewhere (e.g. by the process's communication library)
+        self._main = _Lane(self.L, self.L.init_stream() if stream is None else abi.StreamWrapper(stream))
+        self._apart, self._apart_lock = None, threading.Lock()
+        self._here = _Issue()
+        self.main_stream = self._stream = self._main.stream  # what `stream` is outside a branch() block
         self.cache = self.L.zg_cache_create(self.device_number, cache_max_bytes)
         self.capture = ExecutionGraph(self)
-        self._side = None  # second stream for branches of independent work, created on first use
-        self._sides = {}   # further side streams by index (branch(k), k >= 1)
-        self._forked = []  # side streams used since the last join()
-        self.main_stream = self.stream  # what `stream` is outside a branch() block
-        self.replaying = False  # a GraphCache (replay.py) is issuing a step
         abi.check()
+
+    # Where ops go is each thread's own: a branch, or a step that is being captured, in one thread leaves the others'
+    # ops on the main stream.
+    @property
+    def stream(self) -> abi.StreamWrapper:
+        return self._here.stream or self._stream
+
+    @stream.setter
+    def stream(self, s: abi.StreamWrapper):
+        self._stream = s
+
+    @property
+    def lane(self) -> _Lane:
+        return self._here.lane or self._main
+
+    @property
+    def cublas(self):
+        return self.lane.cublas
+
+    @property
+    def cudnn(self):
+        return self.lane.cudnn
+
+    @property
+    def cutensor(self):
+        return self.lane.cutensor
+
+    @contextlib.contextmanager
+    def apart(self):
+        """This thread's ops go to streams that nobody else uses (one thread at a time: None is yielded, and nothing changes,
+        while another one is in here).  The caller orders them against the main stream."""
+        if not self._apart_lock.acquire(blocking=False):
+            yield None
+            return
+        here, was = self._here, (self._here.lane, self._here.stream)
+        try:
+            if self._apart is None:
+                self._apart = _Lane(self.L, self.L.init_stream())
+            here.lane, here.stream = self._apart, self._apart.stream
+            yield self._apart
+        finally:
+            here.lane, here.stream = was
+            self._apart_lock.release()
 
     # ------------------------------------------------------------ lifecycle
     def deinit(self):
@@ -161,17 +222,12 @@ class CudaDevice:
         self.sync()
         self.capture.free()
         self.L.zg_cache_destroy(self.cache)
-        self.L.deinit_cudnn_handle(self.cudnn)
-        self.L.deinit_cublas_handle(self.cublas)
-        self.L.deinit_cutensor_handle(self.cutensor)
-        if self._side is not None:
-            self.L.deinit_stream(self._side)
-            self._side = None
-        for st in self._sides.values():
-            self.L.deinit_stream(st)
-        self._sides = {}
+        if self._apart is not None:
+            self._apart.close(self.L)
+            self.L.deinit_stream(self._apart.stream)
+        self._main.close(self.L)
         if self._own_stream:
-            self.L.deinit_stream(self.stream)
+            self.L.deinit_stream(self.main_stream)
         self.L = None
 
     def reference(self):
@@ -202,35 +258,31 @@ class CudaDevice:
         if os.environ.get("ZG_NO_BRANCH") == "1":  # everything in issue order on the main stream
             yield
             return
-        if k == 0:
-            if self._side is None:
-                self._side = self.L.init_stream()
-            side = self._side
-        else:
-            if k not in self._sides:
-                self._sides[k] = self.L.init_stream()
-            side = self._sides[k]
-        main = self.stream
+        here, lane, main = self._here, self.lane, self.stream
+        side = lane.sides.get(k)
+        if side is None:
+            side = lane.sides[k] = self.L.init_stream()
         self.L.zg_stream_wait(side, main)
         for j in after:
-            other = self._side if j == 0 else self._sides.get(j)
+            other = lane.sides.get(j)
             if other is not None and other.ptr != side.ptr:
                 self.L.zg_stream_wait(side, other)
-        if all(side.ptr != f.ptr for f in self._forked):
-            self._forked.append(side)
-        self.stream = side
+        if all(side.ptr != f.ptr for f in lane.forked):
+            lane.forked.append(side)
+        was, here.stream = here.stream, side
         try:
             yield
         finally:
-            self.stream = main
+            here.stream = was
 
     def join(self):
         """The main stream waits for every side stream used since the last join
         (only those: a wait on a stream that is not part of a running capture
         would break the capture)."""
-        for st in self._forked:
+        lane = self.lane
+        for st in lane.forked:
             self.L.zg_stream_wait(self.stream, st)
-        self._forked = []
+        lane.forked = []
 
     # --------------------------------------------------------------- memory
     def mem_cache_alloc(self, dtype: int, n: int) -> DeviceSlice:
