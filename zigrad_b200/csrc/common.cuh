@@ -51,6 +51,8 @@ int sm_count();  // SMs of the current device (cached)
 // Slots 0 and 1 are scratch; slot 2 is zero when handed out and every kernel
 // that uses it leaves it zero (arrival counters of multi-CTA reductions).
 void* workspace(cudaStream_t s, size_t bytes, unsigned** counters, int slot = 0);
+// Whether workspace() would give that much now: what is being captured can use only what is there already.
+bool workspace_ready(cudaStream_t s, size_t bytes, int slot);
 
 // y[col] = column sums of x[row, col] (fp32, two-stage, deterministic; uses workspace slot 0)
 void fold_rows_f32(cudaStream_t s, const float* x, float* y, size_t row, size_t col);

@@ -314,6 +314,11 @@ __global__ void __launch_bounds__(kSmallThreads) small_step_kernel(float* params
   cluster.sync();  // nobody leaves while its partial sum may still be read
 }
 
+__global__ void counter_add_kernel(unsigned long long* c, unsigned long long inc) {
+  pdl_sync();
+  *c += inc;
+}
+
 // CTAs of a tensor for small_step_kernel (an element per thread, as far as that goes: divisions and roots bound it), or 0:
 // tensors too long, or more of them than run side by side
 static unsigned small_cluster(const zg_segment* seg, size_t n_seg) {
@@ -406,23 +411,25 @@ static void adam_step(cudaStream_t s, float* P, float* G, float* M, float* V, co
     }
     return tab;
   };
-  if (const unsigned c = clip == 1 && !cp ? small_cluster(seg, n_seg) : 0) {
-    unsigned* ticket = nullptr;
-    if (!workspace(s, 256, &ticket, 2)) return;
+  // The update's last CTA moves the device counter on, by a ticket from slot 2.  On a stream whose first step is being captured
+  // that slot cannot be had any more: the separate kernels then, the counter's behind them.
+  const bool advances = t_dev && advance, own = advances && workspace_ready(s, 256, 2);
+  unsigned* ticket = nullptr;
+  if (own && !workspace(s, 256, &ticket, 2)) return;
+  if (const unsigned c = clip == 1 && !cp && own == advances ? small_cluster(seg, n_seg) : 0) {
     launch_pdl_cluster(small_step_kernel<true>, dim3(c, (unsigned)n_seg), dim3(kSmallThreads), 0, s, c, P, G, M, V, table(0), a, norms, (float)max_norm,
-                       (float)delta, t_dev, lr, ticket, t_dev && advance ? (unsigned long long)n_seg : 0ull, target, (float)tau, 0);
+                       (float)delta, t_dev, lr, ticket, own ? (unsigned long long)n_seg : 0ull, target, (float)tau, 0);
     return;
   }
   if (clip == 1 && !compute_norms(s, G, seg, n_seg, norms)) return;
   for (size_t first = 0; first < n_seg; first += kMaxSeg) {
     const SegTable tab = table(first);
-    unsigned* ticket = nullptr;
-    if (!workspace(s, 256, &ticket, 2)) return;
     const dim3 grid(chunks_for(seg + first, tab.n), tab.n), blk(kOThreads);
-    const unsigned long long inc = (t_dev && advance && first + kMaxSeg >= n_seg) ? (unsigned long long)n_seg : 0ull;
+    const unsigned long long inc = (own && first + kMaxSeg >= n_seg) ? (unsigned long long)n_seg : 0ull;
     auto kern = clip ? (cp ? adam_kernel<true, true> : adam_kernel<true, false>) : (cp ? adam_kernel<false, true> : adam_kernel<false, false>);
     if (!launch_pdl(kern, grid, blk, 0, s, P, G, M, V, tab, a, (const float*)norms, (float)max_norm, (float)delta, cp, t_dev, lr, ticket, inc, target, (float)tau)) return;
   }
+  if (advances && !own) launch_pdl(counter_add_kernel, dim3(1), dim3(1), 0, s, t_dev, (unsigned long long)n_seg);
 }
 
 extern "C" void zg_adam_step_part(dtype id, StreamWrapper w, void* params, void* grads, void* m, void* v, const zg_segment* seg, len_t n_seg,

@@ -213,6 +213,16 @@ void* workspace(cudaStream_t s, size_t bytes, unsigned** counters, int slot) {
   return static_cast<char*>(w.base) + 256;
 }
 
+bool workspace_ready(cudaStream_t s, size_t bytes, int slot) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess || st == cudaStreamCaptureStatusNone) return true;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(g_ws_mu);
+  const auto w = g_ws.find({{dev, slot}, s});
+  return w != g_ws.end() && w->second.bytes >= bytes + 256;
+}
+
 struct GraphBackend {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
