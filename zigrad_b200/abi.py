@@ -286,13 +286,16 @@ def lib() -> C.CDLL:
     return L
 
 
+FASTCALL = os.path.join(HERE, "lib", "_fastcall" + importlib.machinery.EXTENSION_SUFFIXES[0])
+
+
 def _bind_fast(L: C.CDLL) -> None:
     """Replace the ctypes functions by direct calls (host/fastcall.c) wherever every argument is an integer, a pointer, a
-    one-pointer struct or a double; ctypes stays behind them for arguments of other Python types."""
-    path = os.path.join(HERE, "lib", "_fastcall.so")
-    if not os.path.exists(path):
-        raise LibraryMissing("%s not found: build it with `python -m zigrad_b200.build`" % path)
-    loader = importlib.machinery.ExtensionFileLoader("_fastcall", path)
+    one-pointer struct or a double; ctypes stays behind them for arguments of other Python types, and serves every call
+    where there is no such binding (it is written for x86-64; one built for another interpreter has another name)."""
+    if not os.path.exists(FASTCALL):
+        return
+    loader = importlib.machinery.ExtensionFileLoader("_fastcall", FASTCALL)
     fast = importlib.util.module_from_spec(importlib.util.spec_from_loader("_fastcall", loader))
     loader.exec_module(fast)
     ret = {None: "v", i32: "i", len_t: "u", vp: "p"}

@@ -108,12 +108,14 @@ def build_host_example(force: bool = False) -> str:
     return HOST_EXAMPLE
 
 
-FASTCALL = os.path.join(HERE, "lib", "_fastcall.so")
-
-
 def build_fastcall(force: bool = False) -> str:
-    """The CPython binding of the C ABI's calls (zigrad_b200/host/fastcall.c).  gcc and Python's headers only."""
+    """The CPython binding of the C ABI's calls (zigrad_b200/host/fastcall.c).  gcc and Python's headers only.  It speaks the
+    calling convention of x86-64 Linux; elsewhere ctypes serves the calls."""
+    import platform
     import sysconfig
+    from .abi import FASTCALL
+    if platform.machine() != "x86_64" or platform.system() != "Linux":
+        return ""
     src = os.path.join(HERE, "host", "fastcall.c")
     if not force and os.path.exists(FASTCALL) and os.path.getmtime(FASTCALL) >= os.path.getmtime(src):
         return FASTCALL
