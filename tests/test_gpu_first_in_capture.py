@@ -45,3 +45,17 @@ def test_adam(fresh, lens, clip):
     assert fresh.to_numpy(count)[0] == 11 + len(segs)
     fresh.capture.run()
     assert fresh.to_numpy(count)[0] == 11 + 2 * len(segs)
+
+
+
+@pytest.mark.parametrize("rows,cols", [(5000, 33), (4099, 1003), (3000, 512), (70, 64)])
+def test_column_sums_behind_an_op_that_left_work_space(fresh, rows, cols):
+    x = rng(rows).standard_normal((rows, cols)).astype(np.float32)
+    X, Y, S = fresh.from_numpy(x), fresh.from_numpy(np.zeros(cols, np.float32)), fresh.from_numpy(np.zeros(1, np.float32))
+    fresh.dispatch(opspec.sum(X, S))
+    fresh.capture.open()
+    fresh.dispatch(opspec.unbroadcast(X, [rows, cols], Y, [cols], None, 1.0, 0.0))
+    fresh.capture.save()
+    for _ in range(2):
+        fresh.capture.run()
+        assert rel_err(fresh.to_numpy(Y), x.astype(np.float64).sum(0)) <= 1e-5

@@ -143,13 +143,16 @@ void fold_rows_launch(cudaStream_t s, const T* x, T* y, size_t batch, size_t row
   if (col_tiles > 65535 || batch > 65535) { set_error(kBadArgument, "fold_rows: shape too large (%zu col tiles, batch %zu)", col_tiles, batch); return; }
   T* partial = nullptr;
   unsigned* tickets = nullptr;
+  // a ticket per column tile, unless the first such op of a stream is being captured and their slot cannot be had any more
+  const size_t ticket_bytes = sizeof(unsigned) * batch * col_tiles;
+  const int per_tile = chunks > 1 && workspace_ready(s, ticket_bytes, 2);
   if (chunks > 1) {
-    partial = static_cast<T*>(workspace(s, sizeof(T) * batch * col_tiles * chunks * tile, nullptr));
-    tickets = static_cast<unsigned*>(workspace(s, sizeof(unsigned) * batch * col_tiles, nullptr, 2));
+    partial = static_cast<T*>(workspace(s, sizeof(T) * batch * col_tiles * chunks * tile, &tickets));
+    if (per_tile) tickets = static_cast<unsigned*>(workspace(s, ticket_bytes, nullptr, 2));
     if (!partial || !tickets) return;
   }
   auto kern = vec ? fold_rows_kernel<T, true> : fold_rows_kernel<T, false>;
-  launch_pdl(kern, dim3((unsigned)chunks, (unsigned)col_tiles, (unsigned)batch), dim3(kRThreads), 0, s, x, y, partial, tickets, row, col, alpha, beta, 1);
+  launch_pdl(kern, dim3((unsigned)chunks, (unsigned)col_tiles, (unsigned)batch), dim3(kRThreads), 0, s, x, y, partial, tickets, row, col, alpha, beta, per_tile);
 }
 
 void fold_rows_f32(cudaStream_t s, const float* x, float* y, size_t row, size_t col) { fold_rows_launch<float>(s, x, y, 1, row, col, 1.f, 0.f); }
