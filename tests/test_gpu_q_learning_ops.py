@@ -64,3 +64,26 @@ def test_adam_step_with_counter_and_soft_target(gpu, lens, clip):
     assert rel_err(be.down(T), 0.25 * want[0] + 0.75 * t) <= 1e-6
     assert gpu.to_numpy(count)[0] == 11 + len(segs)
     gpu.mem_cache_free(count)
+
+
+@pytest.mark.parametrize("lens,clip", [((200001, 3), False), ((200001, 3), True), ((700, 64, 5), True)])
+def test_adam_counter_over_many_steps(gpu, lens, clip):
+    """Every launch reads the counter that the launch before has moved on, in all of its CTAs."""
+    n, g, steps = sum(lens), rng(sum(lens)), 60
+    segs, off = [], 0
+    for k in lens:
+        segs.append((off, k))
+        off += k
+    p, gr = (g.standard_normal(n).astype(np.float32) for _ in range(2))
+    gr *= 1e-3  # not clipped: the gradients stay
+    be = GpuBackend(gpu)
+    P, G, M, V, N = (be.up(x) for x in (p, gr, np.zeros(n), np.zeros(n), np.zeros(len(segs))))
+    count = gpu.from_numpy(np.zeros(1, np.uint64))
+    want = (p, gr, np.zeros(n, np.float32), np.zeros(n, np.float32))
+    for i in range(steps):
+        gpu.dispatch(opspec.adam(P, G, M, V, segs, 1, 1e-3, clip=clip, max_norm=10.0, norms=N, step_counter=count))
+        want = OracleBackend().adam(*want, segs, 1 + i * len(segs), 1e-3, clip=clip, max_norm=10.0)
+    assert gpu.to_numpy(count)[0] == steps * len(segs)
+    for got, w in zip((P, G, M, V), want):
+        assert rel_err(gpu.to_numpy(got), w) <= 1e-5
+    gpu.mem_cache_free(count)

@@ -152,6 +152,13 @@ struct AdamScalars {
   __device__ __forceinline__ float step_size(float lr, float t) const { return lr * sqrtf(1.f - powf(b2, t)) / (1.f - powf(b1, t)); }
 };
 
+// The device step counter, read before whatever this thread does next: the ticket it draws says that it has been read.
+__device__ __forceinline__ unsigned long long read_counter(const unsigned long long* c) {
+  unsigned long long t;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(t) : "l"(c) : "memory");
+  return t;
+}
+
 // `target` (or nullptr): the soft update of a target network laid out like the parameters, target = tau * p + (1 - tau) *
 // target, in the same pass.
 template <bool CLIP, bool BF16COPY>
@@ -169,13 +176,14 @@ __global__ void __launch_bounds__(kOThreads) adam_kernel(float* params, float* g
   const size_t n = tab.len[seg];
   float lr_t = tab.lr_t[seg];
   if (t_dev) {  // step counter kept on the device (graph replay): t = counter + position of this tensor
-    lr_t = a.step_size(lr, (float)(*t_dev + (unsigned long long)(tab.first + seg + 1)));
-    if (advance) {  // the CTA that draws the last ticket moves the counter on: by then every CTA has read it
-      __syncthreads();
-      if (threadIdx.x == 0 && atomicAdd(ticket, 1u) == gridDim.x * gridDim.y - 1) {
-        *ticket = 0;
-        *t_dev += advance;
-      }
+    __shared__ unsigned long long now;
+    if (threadIdx.x == 0) now = read_counter(t_dev);
+    __syncthreads();
+    lr_t = a.step_size(lr, (float)(now + (unsigned long long)(tab.first + seg + 1)));
+    // the CTA that draws the last ticket moves the counter on: by then every CTA has read it (its one reading thread draws)
+    if (advance && threadIdx.x == 0 && atomicAdd(ticket, 1u) == gridDim.x * gridDim.y - 1) {
+      *ticket = 0;
+      *t_dev = now + advance;
     }
   }
   bool on = false;
@@ -273,13 +281,12 @@ __global__ void __launch_bounds__(kSmallThreads) small_step_kernel(float* params
   if (ADAM && threadIdx.x == kSmallThreads - 1) {
     step = tab.lr_t[seg];
     if (t_dev) {
-      unsigned long long t;
-      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(t) : "l"(t_dev) : "memory");
+      const unsigned long long t = read_counter(t_dev);
       const unsigned drawn = advance ? atomicAdd(ticket, 1u) : 0u;  // on its way while the powers are formed
       step = a.step_size(lr, (float)(t + (unsigned long long)(tab.first + seg + 1)));
       if (advance && drawn == gridDim.x * gridDim.y - 1) {
         *ticket = 0;
-        *t_dev += advance;
+        *t_dev = t + advance;
       }
     }
   }
