@@ -1,6 +1,7 @@
 """The call binding of the C ABI: every argument kind arrives as ctypes would pass it, and what it does not take goes to ctypes."""
 import ctypes as C
 import platform
+import subprocess
 
 import pytest
 
@@ -37,3 +38,32 @@ def test_without_the_binding_ctypes_serves_the_calls(monkeypatch, tmp_path):
 def test_binding_belongs_to_one_interpreter(monkeypatch):
     import sysconfig
     assert abi.FASTCALL.endswith(sysconfig.get_config_var("EXT_SUFFIX")) and sysconfig.get_config_var("py_version_nodot") in abi.FASTCALL
+
+
+def test_what_ctypes_refuses_is_refused():
+    """Handles of another kind, arrays of another type and numbers where a typed pointer is due."""
+    L = abi.lib()
+    S, segs = abi.StreamWrapper(0), (abi.Segment * 1)()
+    clear = lambda seg: L.zg_segment_sumsq(9, S, None, seg, 1, None)
+    for seg in (segs, None):
+        L.zg_clear_error()
+        clear(seg)
+        assert L.zg_last_error() == 5  # called: an unsupported dtype
+    L.zg_clear_error()
+    for bad in (64, b"12345678", (abi.len_t * 2)(), (abi.Block * 1)(), "x"):
+        with pytest.raises((TypeError, C.ArgumentError)):
+            clear(bad)
+    for bad in (abi.CublasWrapper(0), abi.GraphWrapper(0), abi.Block(0, 0), 64, None):
+        with pytest.raises((TypeError, C.ArgumentError)):
+            L.stream_synchronize(bad)
+    assert L.zg_last_error() == 0
+
+
+def test_bool_arguments_are_one_or_zero(tmp_path):
+    src = tmp_path / "f.c"
+    src.write_text("unsigned long f(unsigned long a, unsigned long b) { return a * 1000 + b; }")
+    subprocess.run(["gcc", "-shared", "-fPIC", str(src), "-o", str(tmp_path / "f.so")], check=True)
+    fn = C.CDLL(str(tmp_path / "f.so")).f
+    abi.lib()
+    g = abi._fast.function(C.cast(fn, C.c_void_p).value, "bi", "u", fn, (None, None))
+    assert [g(x, 7) for x in (True, False, 1, 0, 2, -4, 1 << 40)] == [1007, 7, 1007, 7, 1007, 1007, 1007]

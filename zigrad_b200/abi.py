@@ -286,6 +286,7 @@ def lib() -> C.CDLL:
     return L
 
 
+_fast = None  # the binding's module, once loaded
 FASTCALL = os.path.join(HERE, "lib", "_fastcall" + importlib.machinery.EXTENSION_SUFFIXES[0])
 
 
@@ -298,22 +299,29 @@ def _bind_fast(L: C.CDLL) -> None:
     loader = importlib.machinery.ExtensionFileLoader("_fastcall", FASTCALL)
     fast = importlib.util.module_from_spec(importlib.util.spec_from_loader("_fastcall", loader))
     loader.exec_module(fast)
+    global _fast
+    _fast = fast
     ret = {None: "v", i32: "i", len_t: "u", vp: "p"}
 
     def kind(t):
         if t is dbl:
             return "d"
-        if t is vp or (isinstance(t, type) and issubclass(t, C._Pointer)):
+        if t is vp:
             return "p"
+        if isinstance(t, type) and issubclass(t, C._Pointer):
+            return "a"
         if isinstance(t, type) and issubclass(t, _Handle):
             return "s"
-        return "i" if isinstance(t, type) and issubclass(t, C._SimpleCData) and t._type_ in "?bBhHiIlLqQ" else None
+        if t is C.c_bool:
+            return "b"
+        return "i" if isinstance(t, type) and issubclass(t, C._SimpleCData) and t._type_ in "bBhHiIlLqQ" else None
 
     for name, (res, args) in SIGNATURES.items():
         sig = [kind(t) for t in args]
         if res in ret and None not in sig and sig.count("d") <= 8 and len(sig) - sig.count("d") <= 26:
             fn = getattr(L, name)
-            setattr(L, name, fast.function(C.cast(fn, vp).value, "".join(sig), ret[res], fn))
+            types = tuple(t._type_ if k == "a" else t if k == "s" else None for k, t in zip(sig, args))
+            setattr(L, name, fast.function(C.cast(fn, vp).value, "".join(sig), ret[res], fn, types))
 
 
 class DeviceError(RuntimeError):

@@ -4,8 +4,9 @@
  * launch itself costs, and more than a short kernel.  Here a function of the ABI is an object that converts its
  * arguments by a signature string and calls the address directly (zg_bmm: 3.2 -> 0.6 us).
  *
- * Signature characters: i integer (any width; bool), p pointer (int, None, bytes or a ctypes array), s a struct
- * holding one pointer (a ctypes structure), d double; return v nothing, i int, u unsigned long, p pointer.
+ * Signature characters: i integer (any width), b bool, p untyped pointer (int, None, bytes or a ctypes array), a pointer to
+ * a given ctypes type (None or an array of it), s a given struct of one pointer (a ctypes structure), d double; return v
+ * nothing, i int, u unsigned long, p pointer.
  * Under the x86-64 System V convention integers and one-pointer structs take rdi .. r9 and then the stack in order, doubles
  * xmm0 .. xmm7, independently of how they are interleaved, so one call through a prototype with six integers, eight
  * doubles and the rest of the integers serves every signature with at most eight doubles.
@@ -31,6 +32,7 @@ typedef struct {
   int n;
   char ret;
   char sig[MAX_ARGS];
+  PyObject* types[MAX_ARGS]; /* the struct of an s, the element type of an a */
 } Function;
 
 typedef uint64_t (*Generic)(uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, double, double, double, double, double, double, double, double,
@@ -38,7 +40,24 @@ typedef uint64_t (*Generic)(uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, ui
                             uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t);
 
 /* Only what stands for its own memory: a c_void_p or a POINTER object has a buffer too, but holds the address to pass. */
-static PyTypeObject *array_type, *struct_type;  /* ctypes.Array, ctypes.Structure */
+static PyTypeObject* array_type;  /* ctypes.Array */
+static PyObject* type_name;       /* "_type_" */
+
+/* Whether `o` has the memory that argument `a` takes: what is nothing of the kind is for ctypes to convert or to refuse. */
+static int stands(const Function* f, Py_ssize_t a, PyObject* o) {
+  switch (f->sig[a]) {
+    case 's': return PyObject_TypeCheck(o, (PyTypeObject*)f->types[a]);
+    case 'p': return PyBytes_Check(o) || PyObject_TypeCheck(o, array_type);
+    case 'a': {
+      if (!PyObject_TypeCheck(o, array_type)) return 0;
+      PyObject* t = PyObject_GetAttr((PyObject*)Py_TYPE(o), type_name);
+      if (!t) PyErr_Clear();
+      Py_XDECREF(t);
+      return t == f->types[a];
+    }
+  }
+  return 0;
+}
 
 static PyObject* call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* kwnames) {
   Function* f = (Function*)self;
@@ -55,15 +74,17 @@ static PyObject* call(PyObject* self, PyObject* const* args, size_t nargsf, PyOb
       d[nd] = PyFloat_CheckExact(o) ? PyFloat_AS_DOUBLE(o) : PyFloat_AsDouble(o);
       if (d[nd] == -1.0 && PyErr_Occurred()) { PyErr_Clear(); fits = 0; }
       ++nd;
-    } else if (c != 's' && PyLong_Check(o)) {
+    } else if ((c == 'i' || c == 'p') && PyLong_Check(o)) {
       x[ni++] = PyLong_AsUnsignedLongLongMask(o);
       if (PyErr_Occurred()) { PyErr_Clear(); fits = 0; }
-    } else if (c == 'p' && o == Py_None) {
+    } else if (c == 'b' && PyLong_Check(o)) {
+      x[ni++] = (uint64_t)PyObject_IsTrue(o);
+    } else if ((c == 'p' || c == 'a') && o == Py_None) {
       x[ni++] = 0;
-    } else if (nh < 8 && (c == 'p' ? PyBytes_Check(o) || PyType_IsSubtype(Py_TYPE(o), array_type) : c == 's' && PyType_IsSubtype(Py_TYPE(o), struct_type))) {
+    } else if (nh < 8 && stands(f, a, o)) {
       if (PyObject_GetBuffer(o, &held[nh], PyBUF_SIMPLE) != 0) { PyErr_Clear(); fits = 0; break; }
       const Py_buffer* b = &held[nh++];
-      if (c == 'p') x[ni++] = (uint64_t)(uintptr_t)b->buf;
+      if (c != 's') x[ni++] = (uint64_t)(uintptr_t)b->buf;
       else if (b->len == (Py_ssize_t)sizeof(void*)) x[ni++] = *(const uint64_t*)b->buf;
       else fits = 0;
     } else {
@@ -91,6 +112,7 @@ static PyObject* call(PyObject* self, PyObject* const* args, size_t nargsf, PyOb
 
 static void dealloc(PyObject* self) {
   Py_XDECREF(((Function*)self)->fallback);
+  for (int a = 0; a < ((Function*)self)->n; ++a) Py_XDECREF(((Function*)self)->types[a]);
   Py_TYPE(self)->tp_free(self);
 }
 
@@ -108,17 +130,19 @@ static PyTypeObject FunctionType = {
     .tp_flags = Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_VECTORCALL,
 };
 
-/* function(address, signature, return, fallback) */
+/* function(address, signature, return, fallback, types): a type or None per argument */
 static PyObject* make(PyObject* module, PyObject* args) {
   (void)module;
   unsigned long long address;
   const char *sig, *ret;
-  PyObject* fallback;
-  if (!PyArg_ParseTuple(args, "KssO", &address, &sig, &ret, &fallback)) return NULL;
+  PyObject *fallback, *types;
+  if (!PyArg_ParseTuple(args, "KssOO!", &address, &sig, &ret, &fallback, &PyTuple_Type, &types)) return NULL;
   size_t n = strlen(sig), doubles = 0;
   for (size_t i = 0; i < n; ++i) {
-    if (!strchr("ipsd", sig[i])) return PyErr_Format(PyExc_ValueError, "signature %s", sig);
+    if (!strchr("ibpasd", sig[i])) return PyErr_Format(PyExc_ValueError, "signature %s", sig);
     doubles += sig[i] == 'd';
+    if (i >= (size_t)PyTuple_GET_SIZE(types) || (strchr("as", sig[i]) && !PyType_Check(PyTuple_GET_ITEM(types, (Py_ssize_t)i))))
+      return PyErr_Format(PyExc_ValueError, "signature %s: no type for argument %zu", sig, i);
   }
   if (n > MAX_ARGS || doubles > 8 || n - doubles > MAX_INTS || strlen(ret) != 1 || !strchr("viup", ret[0]))
     return PyErr_Format(PyExc_ValueError, "signature %s -> %s", sig, ret);
@@ -130,6 +154,7 @@ static PyObject* make(PyObject* module, PyObject* args) {
   f->n = (int)n;
   f->ret = ret[0];
   memcpy(f->sig, sig, n);
+  for (size_t i = 0; i < n; ++i) f->types[i] = Py_NewRef(PyTuple_GET_ITEM(types, (Py_ssize_t)i));
   return (PyObject*)f;
 }
 
@@ -141,8 +166,8 @@ PyMODINIT_FUNC PyInit__fastcall(void) {
   PyObject* ctypes = PyImport_ImportModule("ctypes");
   if (!ctypes) return NULL;
   array_type = (PyTypeObject*)PyObject_GetAttrString(ctypes, "Array");
-  struct_type = (PyTypeObject*)PyObject_GetAttrString(ctypes, "Structure");
+  type_name = PyUnicode_InternFromString("_type_");
   Py_DECREF(ctypes);
-  if (!array_type || !struct_type) return NULL;
+  if (!array_type || !type_name) return NULL;
   return PyModule_Create(&module_def);
 }
