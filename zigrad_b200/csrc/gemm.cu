@@ -423,18 +423,15 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   static const bool tma_epi_on = [] { const char* e = getenv("ZG_GEMM_TMA_EPILOGUE"); return !(e && e[0] == '0'); }();
   // The unit clips a box at a whole 16-byte word: one past n would write padding columns -- a store clears them, a
   // reduction adds what the accumulator holds there (products with the repeated rows of an element-wise copied operand;
-  // NaN for an infinity times a box's zero fill).  The map of a reduction therefore ends with the last whole word of n,
-  // and the columns behind it are added one by one (as a cluster that sums its tiles and bounds the column instead, a
-  // 16x1433x2708 product took 3 us more).
-  const bool tma_epi = tma_epi_on && p.vec_ok && !swap && nC <= 0x7fffffffu;
-  const bool tma_store = tma_epi && n * (c_id == SINGLE ? 4 : 2) % 16 == 0;
+  // NaN for an infinity times a box's zero fill).  K ranges are then added element by element, which bounds the column.
+  const bool tma_epi = tma_epi_on && p.vec_ok && !swap && nC <= 0x7fffffffu && n * (c_id == SINGLE ? 4 : 2) % 16 == 0;
   if (persistent) {
     const bool add = splits > 1 || (beta == 1.0 && epilogue == ZG_EPI_NONE && !colsum && c_id == SINGLE);
     CUtensorMap tmM;
     memset(&tmM, 0, sizeof(tmM));
-    if (add ? tma_epi : tma_store && beta == 0.0) {
+    if (tma_epi && (add || beta == 0.0)) {
       const bool c16 = c_id == BF16;
-      if (!make_tmap(&tmC, c16, C, add ? n / 4 * 4 : n, m, nC, ldc, c16 ? 64 : 32, 32, false)) return true;
+      if (!make_tmap(&tmC, c16, C, n, m, nC, ldc, c16 ? 64 : 32, 32, false)) return true;
       if (epilogue == ZG_EPI_RELU_MASK && !make_tmap(&tmM, c16, mask, n, m, nC, ldc, c16 ? 64 : 32, 32, false)) return true;
       p.tma_epilogue = add ? 2 : 1;
     }
@@ -451,8 +448,8 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   dim3 grid((unsigned)((N + bn - 1) / bn * splits), (unsigned)((M + 127) / 128), (unsigned)nC);
   if (grid.y > 65535 || grid.z > 65535) return false;
   if (tma_epi && c_id == SINGLE && !cluster && !p.colsum &&
-      (splits > 1 ? epilogue == ZG_EPI_NONE : (tma_store && beta == 0.0 && epilogue != ZG_EPI_RELU_MASK))) {
-    if (!make_tmap(&tmC, false, C, splits > 1 ? n / 4 * 4 : n, m, nC, ldc, 32, 32, false)) return true;
+      (splits > 1 ? epilogue == ZG_EPI_NONE : (beta == 0.0 && epilogue != ZG_EPI_RELU_MASK))) {
+    if (!make_tmap(&tmC, false, C, n, m, nC, ldc, 32, 32, false)) return true;
     p.tma_epilogue = splits > 1 ? 2 : 1;
   }
   if (direct) launch_tc_direct(s, bn, a_kmajor, b_kmajor, tmA, tmB, tmC, p, grid);

@@ -444,16 +444,6 @@ __device__ __forceinline__ void epilogue_chunk(const Params& p, const uint32_t (
   if (p.colsum) colsum_chunk(p, v, col0, lane);
 }
 
-// A reduction's boxes end with the last whole 16-byte word of a row of C: the up to three columns behind it, of this
-// thread's row, one by one.
-__device__ __forceinline__ void add_past_word(const Params& p, const float (&v)[32], bool row_ok, uint64_t o, uint32_t col0) {
-  const uint32_t whole = p.n & ~3u;
-  if (whole == p.n || col0 + 32 <= whole || !row_ok) return;
-#pragma unroll
-  for (uint32_t j = 0; j < 32; ++j)
-    if (col0 + j >= whole && col0 + j < p.n) atomicAdd(p.C + o + j, v[j]);
-}
-
 // One row of an fp32 A slab (32 k values of row `row` of the 128-row tile) from its shared-memory stage.
 // K-major: the row is 128 contiguous bytes whose 16-byte chunks sit at position c ^ (row % 8).
 // MN-major: the stage holds four column blocks of 32 rows; a block is 32 k-rows of 128 bytes (32
@@ -1116,11 +1106,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
         for (int j = 0; j < 8; ++j)
           *reinterpret_cast<float4*>(rowp + ((j ^ (lane & 7)) << 4)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-        if (p.tma_epilogue == 2) {
-          const uint32_t row = tile_m * kBM + q * 32 + lane;
-          add_past_word(p, v, row < p.m, (uint64_t)batch * p.c_batch_stride + (uint64_t)row * p.ldc + col0, col0);
-        }
-        if (col0 < (p.n & ~3u)) ++chunks;
+        ++chunks;
       }
       fence_async_smem();  // generic-proxy writes -> visible to the TMA unit
       __syncwarp();

@@ -438,7 +438,6 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
               *at = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
             }
           }
-          if (p.tma_epilogue == 2) add_past_word(p, v, row_ok, c_off + col0, col0);
           if (p.colsum) {
             if (!row_ok) {
 #pragma unroll
@@ -452,9 +451,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
         __syncwarp();
         if (lane == 0) {
           const int x = (int)(tc.n * BN) + c * width;
-          if (p.tma_epilogue == 2) {
-            if ((uint32_t)x < (p.n & ~3u)) tma_reduce_add_box(&tmC, stg + (box & 1) * 4096, x, (int)row0, (int)tc.batch);
-          } else tma_store_box(&tmC, stg + (box & 1) * 4096, x, (int)row0, (int)tc.batch);
+          if (p.tma_epilogue == 2) tma_reduce_add_box(&tmC, stg + (box & 1) * 4096, x, (int)row0, (int)tc.batch);
+          else tma_store_box(&tmC, stg + (box & 1) * 4096, x, (int)row0, (int)tc.batch);
           bulk_commit_group();
         }
         ++box;
