@@ -157,7 +157,8 @@ class GcnTrainer:
         self._mm(self.dh2, self.W2, self.da1, N, H, C, False, False, Cp, H, H, 0.0, "relu_mask", None, self.a1,
                  colsum=self.db1)                                                                   # da1, db1
         self._prop(self.da1, self.dh1, H, H, transpose=True)                                      # dh1 = A^T . da1
-        self._mm(self.dh1, self.X, self.dW1, H, F, N, True, False, H, Fp, Fp, 1.0)                # dW1 += dh1^T . X
+        # (with the padding columns, which X holds as zeros: rows of whole 16-byte words leave through the tensor map)
+        self._mm(self.dh1, self.X, self.dW1, H, Fp, N, True, False, H, Fp, Fp, 1.0)               # dW1 += dh1^T . X
         d.join()
         # ---- update
         if self.opt == "adam":
