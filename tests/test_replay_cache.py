@@ -2,9 +2,11 @@
 GPU): what is issued when a capture fails or a step raises, where captures happen, and what a graph is found by."""
 import ctypes as C
 import threading
+from fractions import Fraction
 
 import numpy as np
 import pytest
+import torch
 
 from zigrad_b200 import abi, device
 from zigrad_b200.mlp import MlpTrainer, kaiming_uniform
@@ -223,3 +225,34 @@ def test_stream_chosen_by_the_user_is_everybodys(dev):
         s.step()
     assert seen == [other.ptr] and "open_capture" not in dev.L.names()
     dev.stream = main
+
+
+def trainer(dev, **kw):
+    dims = [12, 8, 5]
+    Ws, bs = kaiming_uniform(dims, 1)
+    tr = MlpTrainer(dev, dims, 4, Ws, bs, "sgd", **kw)
+    X, T = dev.mem_cache_alloc(abi.SINGLE, 48), dev.mem_cache_alloc(abi.SINGLE, 20)
+    return tr, lambda: tr.step(X, T)
+
+
+@pytest.mark.parametrize("number", [float, np.float32, np.array, torch.tensor, Fraction], ids=lambda f: f.__name__)
+def test_hyper_parameters_are_found_by_value(dev, number):
+    """Whatever holds the number: it is compared as a number, also if the holder is changed in place or cannot be hashed."""
+    tr, step = trainer(dev)
+    runs = lambda: dev.L.names().count("run_capture")
+    tr.lr = number(0.25)
+    for _ in range(3):
+        step()
+    assert runs() == 1
+    tr.lr = number(0.25)
+    step()
+    assert runs() == 2
+    if hasattr(tr.lr, "fill_") or hasattr(tr.lr, "fill") and tr.lr.__class__ is np.ndarray:
+        (tr.lr.fill_ if hasattr(tr.lr, "fill_") else tr.lr.fill)(0.5)
+    else:
+        tr.lr = number(0.5)
+    step()
+    assert runs() == 2
+    step()
+    step()
+    assert runs() == 3

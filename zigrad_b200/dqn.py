@@ -22,7 +22,7 @@ from . import opspec
 from .abi import SINGLE
 from .device import USIZE, CudaDevice, DeviceSlice
 from .mlp import MlpTrainer
-from .replay import GraphCache
+from .replay import GraphCache, numbers
 
 
 class DqnTrainer:
@@ -48,8 +48,9 @@ class DqnTrainer:
     def step(self, states: DeviceSlice, actions: DeviceSlice, next_states: DeviceSlice, rewards: DeviceSlice,
              dones: DeviceSlice):
         p = self.policy
-        key = (states.ptr, actions.ptr, next_states.ptr, rewards.ptr, dones.ptr, self.gamma, self.tau, self.q_clip, p.lr, p.opt, p.beta1,
-               p.beta2, p.eps, p.clip, p.max_norm, p.delta, self.target._touched)
+        key = (states.ptr, actions.ptr, next_states.ptr, rewards.ptr, dones.ptr,
+               numbers(self.gamma, self.tau, self.q_clip, p.lr, p.beta1, p.beta2, p.eps, p.max_norm, p.delta), p.opt, str(p.clip),
+               self.target._touched)
         self._graphs.run(key, lambda: self._step(states, actions, next_states, rewards, dones), self._host_state, self._set_host_state)
 
     def _host_state(self):

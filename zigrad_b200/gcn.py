@@ -24,7 +24,7 @@ import numpy as np
 from . import opspec
 from .abi import SINGLE
 from .device import USIZE, CudaDevice, DeviceSlice
-from .replay import GraphCache
+from .replay import GraphCache, numbers
 
 
 def _pad4(n: int) -> int:
@@ -123,7 +123,7 @@ class GcnTrainer:
 
     def step(self, T_masked: DeviceSlice):
         """T_masked: one-hot targets of the masked rows, fp32 [M, C] contiguous."""
-        key = (T_masked.ptr, T_masked.dtype, self.opt, self.lr, self.beta1, self.beta2, self.eps, self.clip, self.max_norm, self.delta)
+        key = (T_masked.ptr, T_masked.dtype, numbers(self.lr, self.beta1, self.beta2, self.eps, self.max_norm, self.delta), self.opt, str(self.clip))
         self._graphs.run(key, lambda: self._step(T_masked), lambda: (self.t,), self._set_t)
 
     def _set_t(self, state):

@@ -41,7 +41,7 @@ import numpy as np
 from . import opspec
 from .abi import BF16, SINGLE
 from .device import CudaDevice, DeviceSlice
-from .replay import GraphCache
+from .replay import GraphCache, numbers
 
 
 def kaiming_uniform(dims: Sequence[int], seed: int):
@@ -423,8 +423,8 @@ class MlpTrainer:
         asynchronous on the device stream.  The loss stays in ``self.loss``."""
         if allreduce is not None:
             return self._step(X, T, allreduce)
-        key = (X.ptr, X.dtype, T.ptr, T.dtype, self.lr, self.opt, self.beta1, self.beta2, self.eps, self.clip, self.max_norm, self.delta,
-               self.loss_div, self.fused, self.tail, self.fuse_update, self.update_by_layer, self.zero_grads_in_update, self._grads_clear)
+        key = (X.ptr, X.dtype, T.ptr, T.dtype, numbers(self.lr, self.beta1, self.beta2, self.eps, self.max_norm, self.delta, self.loss_div),
+               self.opt, str(self.clip), self.fused, self.tail, self.fuse_update, self.update_by_layer, self.zero_grads_in_update, self._grads_clear)
         self._graphs.run(key, lambda: self._step(X, T, None), self._host_state, self._set_host_state)
 
     def _step(self, X: DeviceSlice, T: DeviceSlice, allreduce):

@@ -22,6 +22,11 @@ CAPACITY = 8    # graphs (or candidates) per trainer; the one used longest ago g
 GIVE_UP = 32    # evicted graphs after which a trainer stops capturing: its buffers change too often
 
 
+def numbers(*values) -> tuple:
+    """Hyper-parameters as a part of a key: by value, whatever holds them (an array or tensor may be changed in place)."""
+    return tuple(map(float, values))
+
+
 class GraphCache:
     def __init__(self, dev):
         self.dev = dev
