@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
@@ -83,6 +84,21 @@ static inline unsigned grid_for(size_t work_items, size_t per_cta, int ctas_per_
 bool pdl_enabled();  // runtime.cu; off with ZG_PDL=0 in the environment
 
 #ifdef __CUDACC__
+// Dynamic shared memory above 48 KB is allowed per kernel and DEVICE: one of these beside each such launch.
+struct SharedMemoryLimit {
+  std::atomic<uint64_t> devices{0};  // on which the kernel has been told
+  template <typename K>
+  bool raise(K kernel, size_t bytes) {
+    int dev = 0;
+    if (!check_cuda(cudaGetDevice(&dev), "cudaGetDevice", __FILE__, __LINE__)) return false;
+    const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+    if (devices.load(std::memory_order_relaxed) & bit) return true;
+    if (!check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "shared memory limit", __FILE__, __LINE__)) return false;
+    devices.fetch_or(bit, std::memory_order_relaxed);
+    return true;
+  }
+};
+
 // `cluster` > 1: the grid's x dimension is made of thread-block clusters of that many CTAs.
 template <typename... KArgs, typename... Args>
 static inline bool launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, unsigned cluster,

@@ -51,11 +51,8 @@ template <typename TI, typename TC, int TM, int TN, int MI>
 static void launch_block_inst(cudaStream_t s, const void* A, const void* B, void* C, block::Params& p, len_t nC, unsigned splits) {
   using L = block::Layout<TI, TM, TN, MI>;
   auto kern = block::gemm_block_kernel<TI, TC, TM, TN, MI>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (!ZG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kSmem))) return;
-    attr_set = true;
-  }
+  static SharedMemoryLimit limit;
+  if (!limit.raise(kern, L::kSmem)) return;
   p.tiles_m = (uint32_t)((p.m + TM - 1) / TM);
   p.tiles_n = (uint32_t)((p.n + TN - 1) / TN);
   p.splits = splits;
@@ -133,11 +130,8 @@ template <int BN, bool AK, bool BK_, int MODE, bool DIRECT = false>
 static bool launch_tc_inst(cudaStream_t s, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tcm, const tc::Params& p, dim3 grid) {
   using SL = tc::SmemLayout<BN, MODE>;
   auto kern = tc::gemm_tc_kernel<BN, AK, BK_, MODE, DIRECT>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (!ZG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SL::kTotal))) return false;
-    attr_set = true;
-  }
+  static SharedMemoryLimit limit;
+  if (!limit.raise(kern, SL::kTotal)) return false;
   return launch_pdl_cluster(kern, grid, dim3(SL::kThreads + (DIRECT ? tc::kLoadWarps * 32 : 0)), (size_t)SL::kTotal, s, p.cluster ? p.splits : 1, ta, tb, tcm, p);
 }
 
@@ -204,11 +198,8 @@ static bool launch_persistent_inst(cudaStream_t s, const CUtensorMap& ta, const 
                                    uint32_t tiles_n, uint32_t n_tiles) {
   using SL = tc::PersistentSmem<MODE>;
   auto kern = tc::gemm_tc_persistent_kernel<AK, BK_, MODE>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (!ZG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SL::kTotal))) return false;
-    attr_set = true;
-  }
+  static SharedMemoryLimit limit;
+  if (!limit.raise(kern, SL::kTotal)) return false;
   const unsigned pairs = std::min<unsigned>(n_tiles, (unsigned)sm_count() / 2);
   // work-item counter: zero between launches (slot 2 of the stream's workspace)
   unsigned* unused = nullptr;
@@ -484,11 +475,8 @@ template <int CP>
 static bool launch_tail_inst(cudaStream_t s, const CUtensorMap& ta, const CUtensorMap& tk, const CUtensorMap& tn, const CUtensorMap& t1,
                              const CUtensorMap& td1, const CUtensorMap& td0, const tail::Params& p, unsigned grid) {
   auto kern = tail::mlp_tail_kernel<CP>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (!ZG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, tail::kSmemBytes))) return false;
-    attr_set = true;
-  }
+  static SharedMemoryLimit limit;
+  if (!limit.raise(kern, tail::kSmemBytes)) return false;
   return launch_pdl(kern, dim3(grid), dim3(tail::kThreads), (size_t)tail::kSmemBytes, s, ta, tk, tn, t1, td1, td0, p);
 }
 
@@ -496,11 +484,8 @@ template <int CP, int R, int T>
 static bool launch_tail_rows(cudaStream_t s, const tail_rows::Params& p) {
   using L = tail_rows::Layout<CP, R, T>;
   auto kern = tail_rows::mlp_tail_rows_kernel<CP, R, T>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (!ZG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kSmem))) return false;
-    attr_set = true;
-  }
+  static SharedMemoryLimit limit;
+  if (!limit.raise(kern, L::kSmem)) return false;
   return launch_pdl(kern, dim3((p.rows + R - 1) / R), dim3(T), L::kSmem, s, p);
 }
 

@@ -1062,11 +1062,8 @@ static void launch_smce_staged(cudaStream_t s, SmceArgs a) {
   if (n_stages < 2) { set_error(kUnsupported, "zg_softmax_ce_fwd_bwd: rows too wide for the staged kernel"); return; }
   const size_t smem = (size_t)n_stages * stage_bytes;
   auto kern = softmax_ce_staged_kernel<ITEMS, ROWS, SUBL>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (!ZG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024))) return;
-    attr_set = true;
-  }
+  static SharedMemoryLimit limit;
+  if (!limit.raise(kern, 216 * 1024)) return;
   const size_t n_groups = (a.rows + group_rows - 1) / group_rows;
   const unsigned g = (unsigned)std::min<size_t>(n_groups, (size_t)sm_count());
   const bool separate_fold = a.dbias && (size_t)g * C > 32768;
@@ -1087,12 +1084,9 @@ static void launch_smce_rows_staged(cudaStream_t s, SmceArgs a) {
   const int C = a.C;
   const size_t smem = (size_t)kNrStages * ((size_t)kNrRows * C * sizeof(float) + (size_t)kNrRows * sizeof(len_t));
   auto kern = softmax_ce_rows_staged_kernel<CP>;
-  static bool attr_set = false;
+  static SharedMemoryLimit limit;
   static unsigned per_sm = 1;
-  if (!attr_set) {
-    if (!ZG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024))) return;
-    attr_set = true;
-  }
+  if (!limit.raise(kern, 216 * 1024)) return;
   int occ = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kRowThreads, smem) != cudaSuccess || occ < 1) { (void)cudaGetLastError(); occ = 1; }
   per_sm = (unsigned)occ;
