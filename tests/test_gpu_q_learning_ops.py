@@ -87,3 +87,21 @@ def test_adam_counter_over_many_steps(gpu, lens, clip):
     for got, w in zip((P, G, M, V), want):
         assert rel_err(gpu.to_numpy(got), w) <= 1e-5
     gpu.mem_cache_free(count)
+
+
+@pytest.mark.parametrize("opt", ["sgd", "none", "adam"])
+def test_target_net_follows_whatever_updates_the_policy(gpu, opt):
+    B, dims, g = 32, [4, 16, 16, 2], rng(3)
+    tr = DqnTrainer(gpu, dims, B, *kaiming_uniform(dims, 1), tau=0.25)
+    tr.policy.opt = opt
+    batch = [gpu.from_numpy(x) for x in (g.standard_normal(B * 4).astype(np.float32), g.integers(0, 2, B).astype(np.uint64),
+                                         g.standard_normal(B * 4).astype(np.float32), np.ones(B, np.float32), np.zeros(B, np.float32))]
+    gpu.mem_fill(tr.target.params, 0.5)
+    for _ in range(5):
+        before = gpu.to_numpy(tr.target.params).astype(np.float64)
+        tr.step(*batch)
+        want = 0.25 * gpu.to_numpy(tr.policy.params) + 0.75 * before
+        assert rel_err(gpu.to_numpy(tr.target.params), want) <= 1e-6
+    tr.free()
+    for s in batch:
+        gpu.mem_cache_free(s)

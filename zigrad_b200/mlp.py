@@ -311,7 +311,7 @@ class MlpTrainer:
             self.t += len(self.segments)  # host mirror (eager steps only; read_t() is the truth)
 
     def update(self, soft_target: Optional[DeviceSlice] = None, tau: float = 0.0):
-        """`soft_target` (Adam): a target network's flat parameters, moved towards the updated ones by tau."""
+        """`soft_target`: a target network's flat parameters, moved towards the updated ones by tau (Adam: in the same pass)."""
         d = self.dev
         if self.opt == "sgd":
             d.dispatch(opspec.sgd(self.params, self._grads, self.segments, self.lr, self.clip, self.max_norm, self.delta, self.norms,
@@ -324,6 +324,8 @@ class MlpTrainer:
             self.t += len(self.segments)  # host mirror (eager steps only; read_t() is the truth)
         elif self.opt != "none":
             raise ValueError(self.opt)
+        if soft_target is not None and self.opt != "adam":
+            d.soft_update(self.params, soft_target, tau)
 
     # -------------------------------------------------------------------- step
     def layer_grads(self, l: int) -> DeviceSlice:
