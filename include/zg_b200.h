@@ -310,7 +310,6 @@ EXTERN_C void zg_adam_soft_step(dtype id, StreamWrapper stream, void* params, vo
 /* out[j] = sum of squares of segment j (fp64 accumulation, deterministic two-stage): the
  * shard-local part of the per-tensor gradient norm of host_device.zig:339-346 */
 EXTERN_C void zg_segment_sumsq(dtype id, StreamWrapper stream, const void* x, const zg_segment* seg, len_t n_seg, void* out);
-/* target[i] = tau*src[i] + (1-tau)*target[i] (examples/dqn/src/dqn_agent.zig:111-123) */
 /* Softmax cross-entropy of selected rows (mem_take, softmax_ce and scatter_add as one launch): row r of the loss reads
  * logits + offsets[r * ld] (a row's offsets are consecutive) and ADDS its gradient into dlogits there; loss and dbias (the
  * gradient's column sums, may be NULL) are overwritten. */
@@ -334,6 +333,7 @@ EXTERN_C int zg_q_head_supported(dtype id, len_t batch, len_t actions);
 EXTERN_C void zg_q_head(dtype id, StreamWrapper stream, len_t batch, len_t actions, void* qn, void* q, const len_t* action, const void* rewards,
                         const void* dones, double gamma, double q_clip, double beta, void* maxq, void* targets, void* chosen, len_t* offsets,
                         void* loss, void* dchosen, void* dq, void* dbias);
+/* target[i] = tau*src[i] + (1-tau)*target[i] (examples/dqn/src/dqn_agent.zig:111-123) */
 EXTERN_C void zg_soft_update(dtype id, StreamWrapper stream, const void* src, void* target, len_t n, double tau);
 /* fp32 -> bf16 (round to nearest even) and back */
 EXTERN_C void zg_cast(dtype src_id, dtype dst_id, StreamWrapper stream, const void* src, void* dst, len_t n);

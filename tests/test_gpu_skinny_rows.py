@@ -24,3 +24,16 @@ def test_rows_tn(gpu, N, U, C, ld):
     got = be.down(out).reshape(N, ld)
     assert rel_err(got[:, :C], A.T.astype(np.float64) @ x[:, :C]) <= 1e-5
     assert (got[:, C:] == 5.0).all()
+
+
+@pytest.mark.parametrize("k", [12, 16, 124, 128, 132, 512])
+@pytest.mark.parametrize("m,n", [(256, 10), (1001, 16), (255, 7)])
+def test_few_columns_on_both_sides_of_the_longest_row(gpu, m, n, k):
+    """Rows of 16 to 128 floats are walked by a quad of threads; shorter and longer ones take the other kernels."""
+    g = rng(m + n + k)
+    be = GpuBackend(gpu)
+    A, B, bias = (g.standard_normal(s).astype(np.float32) for s in ((m, k), (n, k), (n,)))
+    c = be.up(np.zeros((m, n), np.float32))
+    gpu.dispatch(opspec.linear(be.up(A), be.up(B), c, m, n, k, False, True, k, k, n, 1.0, 0.0, "bias", be.up(bias)))
+    # fp32 sums of k products in any order, or three truncated tf32 products each
+    assert rel_err(be.down(c).reshape(m, n), A.astype(np.float64) @ B.T + bias) <= 1e-5

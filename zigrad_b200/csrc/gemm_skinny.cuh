@@ -5,7 +5,7 @@
 // issues all of its global loads at once, so a launch costs about one memory
 // round trip plus the arithmetic.  Plain FFMA in fp32, sequential accumulation.
 //
-//   skinny_n_kernel: C[m,n] = epi(alpha A[m,k] op(B) + beta C), n <= 16, k <= 512
+//   skinny_n_kernel: C[m,n] = epi(alpha A[m,k] op(B) + beta C), n <= 16, 16 <= k <= 128
 //       four threads per row of A, each a quarter of the row's 16-byte words;
 //       B (n x k) in shared memory; quad reduction by shuffles
 //   skinny_k_kernel: C[m,n] = epi(alpha A[m,k] B[k,n]), k <= 16, n <= 256
