@@ -389,8 +389,8 @@ def test_persistent_gemm_bf16_epilogues(gpu):
 
 @pytest.mark.parametrize("beta", [1.0, 0.0, 0.5])
 def test_persistent_gemm_split_k_weight_gradient(gpu, beta):
-    """160 tiles of 128 x 256 on 148 SMs: the K ranges become work items
-    (vector reductions into C, pre-scaled by beta)."""
+    """80 tiles of 256 x 256 on 74 pairs of SMs: the K ranges of the last wave's tiles become
+    work items (reductions into C, pre-scaled by beta)."""
     m, n, k = 2560, 2048, 4096
     g = rng(5)
     A, B = g.standard_normal((k, m)).astype(np.float32), g.standard_normal((k, n)).astype(np.float32)

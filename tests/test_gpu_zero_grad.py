@@ -122,3 +122,15 @@ def test_graph_of_the_caller_over_a_trainer_that_never_had_gradients(gpu):
     assert not gpu.to_numpy(pair.a.grads).any()
     gpu.capture.free()
     pair.free()
+
+
+def test_without_fused_ops_backward_overwrites(gpu):
+    """Op by op every gradient is written once per backward pass; a second one gives the same, not the sum."""
+    pair = Pair(gpu, opt="sgd", fused=False)
+    pair.a.forward(pair.data[0][0])
+    pair.backward(pair.a)
+    once = gpu.to_numpy(pair.a.grads).copy()
+    pair.a.loss_and_grad(pair.data[0][1])
+    pair.a.backward(pair.data[0][0])
+    np.testing.assert_allclose(gpu.to_numpy(pair.a.grads), once, rtol=1e-5, atol=1e-8)
+    pair.free()

@@ -1057,9 +1057,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   }
 
   // ---------------------------------------------------------------- epilogue
-  // Each epilogue thread owns one accumulator row: 32 consecutive columns per
-  // tcgen05.ld, i.e. one full 128-byte line of C, read (beta / mask) and
-  // written with 128-bit accesses straight from registers.
+  // Each of these threads owns one accumulator row and takes 32 consecutive columns of it per tcgen05.ld: into swizzled
+  // boxes for the TMA unit, or into the staged tile that all warps then finish.
   if (warp >= 4 && warp < 8) {
     const int q = warp - 4;  // TMEM lane quadrant
     const bool have_acc = (KT > 0) && mbar_wait(accum, 0, &failed);

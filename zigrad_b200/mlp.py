@@ -17,7 +17,9 @@ Two op sequences produce the same tensors:
   once per step, so where the reference fills it with zeros and accumulates
   (beta = 1) the op writes it (beta = 0), and what the dX chain does not need runs on
   the side stream: at batch 100 the fills were 8 of 27 launches of about 2.5 us each.
-* ``fused=True``  -- one zero fill of the flat gradient buffer, ``linear`` ops
+  A second ``backward()`` therefore gives the same gradients, as it did with the fills.
+* ``fused=True``  -- one zero fill of the flat gradient buffer per forward pass (a second
+  ``backward()`` behind it accumulates), ``linear`` ops
   with bias / ReLU / ReLU-mask epilogues, bias gradients taken from the loss
   kernel (last layer) and from the dX GEMM epilogues (hidden layers): 10 kernel
   launches + 1 memset for the three-layer model.  When the last two layers have
