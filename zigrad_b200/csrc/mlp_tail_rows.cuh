@@ -5,8 +5,9 @@
 // rows are 2 us of the chip's FFMA rate), so the rows are spread thin: 28 per CTA (two CTAs on each of 148 SMs hold 8288
 // rows), 16 while those leave SMs idle, instead of the 128 of a tensor-core tile with its operand splits and TMEM
 // round trips.  The products are packed pairs (fma.rn.f32x2), which leaves every other issue slot to the shared-memory
-// reads -- whose wavefronts bound the larger batches (68 % of the pipe at 8192 rows).  Measured against the tensor-core
-// kernel: 64 rows 6.5 us (14.9), 1000 rows 7.1 (17.6), 4000 9.8 (17.9), 8192 13.7 (16.2); 16384 rows in two waves 28 (18.8).
+// reads -- whose wavefronts bound the larger batches (68 % of the pipe at 8192 rows).  Measured (the op alone, replayed): 64
+// rows 5.9 us, 1000 6.7, 4000 9.3, 8192 13.6, 8288 13.8; the tensor-core kernel 14.9 to 17.9 below that, 16.2 at 8289 and 16.5 at
+// 16384, where this one in two waves took 28.
 //
 //   product 1  thread = 4 rows x 4 columns, k in pairs along 16-byte words of act0 and W1 rows (both natural layout, rows
 //              132 floats apart: conflict-free); KG groups of threads share k = 128 and meet in shared memory
