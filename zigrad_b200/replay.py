@@ -24,7 +24,10 @@ GIVE_UP = 32    # evicted graphs after which a trainer stops capturing: its buff
 
 def numbers(*values) -> tuple:
     """Hyper-parameters as a part of a key: by value, whatever holds them (an array or tensor may be changed in place)."""
-    return tuple(map(float, values))
+    for v in values:
+        if v.__class__ is not float:
+            return tuple(map(float, values))
+    return values
 
 
 class GraphCache:
@@ -38,7 +41,8 @@ class GraphCache:
         is given the state to set after a replay, in which every int has advanced as it did when captured."""
         d = self.dev
         here = d._here
-        if here.replaying or d._main.forked or d.stream.ptr != d.main_stream.ptr or self.evicted >= GIVE_UP or d.capturing():
+        if (here.replaying or here.stream is not None or d._stream is not d.main_stream or d._main.forked or self.evicted >= GIVE_UP
+                or d.L.zg_stream_capturing(d.main_stream)):
             return body()
         key = (key, d.L.zg_get_math_mode())
         hit = self.entries.get(key)
