@@ -130,6 +130,12 @@ template <typename... KArgs, typename... Args>
 static inline bool launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
   return launch_pdl_cluster(kernel, grid, block, smem, s, 1, static_cast<KArgs>(args)...);
 }
+// A CTA whose bounded wait ran out may have copies and tensor-core work of its own under way.  They end within
+// microseconds; it stays a millisecond, so that nothing lands in shared or tensor memory it has given back.
+__device__ __noinline__ inline void outstay_own_work() {
+  const long long start = clock64();
+  while (clock64() - start < 2000000) __nanosleep(1000);
+}
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_sync() { pdl_wait(); pdl_trigger(); }

@@ -1158,6 +1158,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   // ---------------------------------------------------------------- teardown
   tc_fence_before();
   __syncthreads();
+  if (failed) outstay_own_work();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_d, kTmemCols);

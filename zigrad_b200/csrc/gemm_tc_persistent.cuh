@@ -470,6 +470,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
   if (failed) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_rank((const void*)&failed, rank ^ 1)), "r"(1) : "memory");
   tc_fence_before();
   __syncthreads();
+  if (failed) outstay_own_work();
   cluster_sync();  // nobody's MMAs, loads or arrivals are under way any more
   if (warp == 1) {
     tc_fence_after();

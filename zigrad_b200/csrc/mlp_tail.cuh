@@ -605,6 +605,7 @@ mlp_tail_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   // ---------------------------------------------------------------- teardown
   tc_fence_before();
   __syncthreads();
+  if (failed) outstay_own_work();
   if (warp == kIssuer) {
     tc_fence_after();
     tmem_dealloc(tmem, kTmCols);
