@@ -54,6 +54,8 @@ int sm_count();  // SMs of the current device (cached)
 void* workspace(cudaStream_t s, size_t bytes, unsigned** counters, int slot = 0);
 // Whether workspace() would give that much now: what is being captured can use only what is there already.
 bool workspace_ready(cudaStream_t s, size_t bytes, int slot);
+// Tickets back to zero on the current device, which must be idle: after a kernel that gave up and left some drawn.
+void clear_workspace_tickets();
 
 // y[col] = column sums of x[row, col] (fp32, two-stage, deterministic; uses workspace slot 0)
 void fold_rows_f32(cudaStream_t s, const float* x, float* y, size_t row, size_t col);

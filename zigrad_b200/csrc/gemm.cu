@@ -574,7 +574,9 @@ void check_tc_errors() {
   if (!f) return;
   int v = 0;
   if (cudaMemcpy(&v, f, sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess && v) {
+    cudaDeviceSynchronize();
     cudaMemset(f, 0, sizeof(int));
+    clear_workspace_tickets();  // the next launches count from zero again
     cudaDeviceSynchronize();
     set_error(kKernelTimeout, "a kernel gave up waiting on a pipeline barrier");
   }

@@ -171,8 +171,9 @@ struct Workspace {
   size_t bytes = 0;
 };
 static std::mutex g_ws_mu;
-static std::map<std::pair<std::pair<int, int>, cudaStream_t>, Workspace> g_ws;
-static std::vector<void*> g_ws_retired;
+using WorkspaceKey = std::pair<std::pair<int, int>, cudaStream_t>;  // (device, slot), stream
+static std::map<WorkspaceKey, Workspace> g_ws;
+static std::vector<std::pair<WorkspaceKey, Workspace>> g_ws_retired;
 
 bool pdl_enabled() {
   static const bool on = [] {
@@ -205,7 +206,7 @@ void* workspace(cudaStream_t s, size_t bytes, unsigned** counters, int slot) {
     // The outgrown buffer is retired, not freed: graphs captured earlier on this stream hold its
     // address in their kernel nodes and may be replayed after this call.  Capacities double, so all
     // retired buffers together are smaller than the live one; they go back with the process.
-    if (w.base) g_ws_retired.push_back(w.base);
+    if (w.base) g_ws_retired.push_back({{{dev, slot}, s}, w});
     w.base = p;
     w.bytes = cap;
   }
@@ -221,6 +222,17 @@ bool workspace_ready(cudaStream_t s, size_t bytes, int slot) {
   std::lock_guard<std::mutex> lk(g_ws_mu);
   const auto w = g_ws.find({{dev, slot}, s});
   return w != g_ws.end() && w->second.bytes >= bytes + 256;
+}
+
+void clear_workspace_tickets() {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(g_ws_mu);
+  auto clear = [dev](const WorkspaceKey& key, const Workspace& w) {
+    if (key.first.first == dev && w.base) ZG_CUDA(cudaMemset(w.base, 0, key.first.second == 2 ? w.bytes : 256));
+  };
+  for (const auto& w : g_ws) clear(w.first, w.second);
+  for (const auto& w : g_ws_retired) clear(w.first, w.second);  // graphs captured with them may run again
 }
 
 struct GraphBackend {
