@@ -6,6 +6,7 @@
 // per thread) with a scalar tail, falling back to a scalar loop when a
 // pointer is not 16-byte aligned.  Grids are sized in multiples of the SM
 // count (grid_for).
+#include <algorithm>
 #include <cstring>
 
 #include "common.cuh"
@@ -54,33 +55,29 @@ __global__ void __launch_bounds__(kThreads) map_kernel(T* out, const T* a, const
   if constexpr (VEC) {
     const size_t nvec = n / N;
     size_t v = tid;
-    // unrolled body: kUnroll vectors per thread per trip, all loads first
-    for (; v + (kUnroll - 1) * nthreads < nvec; v += kUnroll * nthreads) {
+    // kUnroll vectors per thread and trip, all loads before the first store.  The last trip is the same code with bounds: as a
+    // loop over single vectors behind it, a few hundred threads took three round trips to memory after everybody else was
+    // done (4.1 M elements in L2, three inputs: 5.9 us, so 5.4; 8.4 M, three inputs: 17.2 and 14.5).
+    for (; v < nvec; v += kUnroll * nthreads) {
       Pack<T, N> ra[kUnroll], rb[kUnroll], rc[kUnroll];
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u) {
         const size_t e = (v + u * nthreads) * N;
-        ra[u] = ldv(a + e);
-        if constexpr (NIN >= 2) rb[u] = ldv(b + e);
-        if constexpr (NIN >= 3) rc[u] = ldv(c + e);
+        if (v + u * nthreads < nvec) {
+          ra[u] = ldv(a + e);
+          if constexpr (NIN >= 2) rb[u] = ldv(b + e);
+          if constexpr (NIN >= 3) rc[u] = ldv(c + e);
+        }
       }
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u) {
+        if (v + u * nthreads >= nvec) continue;
         Pack<T, N> r;
 #pragma unroll
         for (int j = 0; j < N; ++j)
           r.v[j] = f(ra[u].v[j], NIN >= 2 ? rb[u].v[j] : T(0), NIN >= 3 ? rc[u].v[j] : T(0));
         stv(out + (v + u * nthreads) * N, r);
       }
-    }
-    for (; v < nvec; v += nthreads) {
-      const size_t e = v * N;
-      Pack<T, N> ra = ldv(a + e), rb, rc, r;
-      if constexpr (NIN >= 2) rb = ldv(b + e);
-      if constexpr (NIN >= 3) rc = ldv(c + e);
-#pragma unroll
-      for (int j = 0; j < N; ++j) r.v[j] = f(ra.v[j], NIN >= 2 ? rb.v[j] : T(0), NIN >= 3 ? rc.v[j] : T(0));
-      stv(out + e, r);
     }
     for (size_t i = nvec * N + tid; i < n; i += nthreads)
       out[i] = f(a[i], NIN >= 2 ? b[i] : T(0), NIN >= 3 ? c[i] : T(0));
@@ -93,7 +90,8 @@ template <typename T, int NIN, typename F>
 void launch_map(cudaStream_t s, T* out, const T* a, const T* b, const T* c, size_t n, F f) {
   if (n == 0) return;
   bool vec = host_aligned16(out) && host_aligned16(a) && (NIN < 2 || host_aligned16(b)) && (NIN < 3 || host_aligned16(c));
-  const unsigned g = grid_for(n, (size_t)kThreads * VecOf<T>::N * kUnroll);
+  // a vector per thread while that leaves SMs idle (100x128: 1.5 -> 1.3 us), then as many as a thread has in flight
+  const unsigned g = std::max(grid_for(n, (size_t)kThreads * VecOf<T>::N * kUnroll), grid_for(n, (size_t)kThreads * VecOf<T>::N, 1));
   if (vec) launch_pdl(map_kernel<T, NIN, true, F>, dim3(g), dim3(kThreads), 0, s, out, a, b, c, n, f);
   else launch_pdl(map_kernel<T, NIN, false, F>, dim3(g), dim3(kThreads), 0, s, out, a, b, c, n, f);
   ZG_LAUNCH_CHECK();
@@ -152,6 +150,44 @@ __global__ void __launch_bounds__(kThreads) bcast_kernel(T* out, const T* lng, c
   }
 }
 
+// The same with rows of at least 32 elements: a thread keeps its column (16 bytes of columns where rows allow), reads its
+// element of the short operand once and goes down the rows, kRows of them in flight.  Over the flat index every vector of a
+// ragged row fetched four single elements of the short operand through L1, twice what the long one and the result take
+// there (4099 x 1003 6.6 -> 6.3 us, 8192 x 1024 9.8 -> 6.8, 100 x 128 2.0 -> 1.35).
+template <typename T, bool SHORT_IS_X, bool VEC, typename F>
+__global__ void __launch_bounds__(kThreads) bcast_rows_kernel(T* out, const T* lng, const T* sht, size_t R, size_t L, F f) {
+  constexpr int N = VEC ? VecOf<T>::N : 1, kRows = VEC ? 4 : 8;
+  struct alignas(N * sizeof(T)) Word { T v[N]; };
+  pdl_sync();
+  const size_t c = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * N;
+  if (c >= L) return;
+  const Word s = *reinterpret_cast<const Word*>(sht + c);
+  const size_t step = (size_t)gridDim.y * blockDim.y;
+  for (size_t r = (size_t)blockIdx.y * blockDim.y + threadIdx.y; r < R; r += kRows * step) {
+    Word x[kRows];
+#pragma unroll
+    for (int u = 0; u < kRows; ++u)
+      if (r + u * step < R) x[u] = *reinterpret_cast<const Word*>(lng + (r + u * step) * L + c);
+#pragma unroll
+    for (int u = 0; u < kRows; ++u) {
+      if (r + u * step >= R) continue;
+#pragma unroll
+      for (int j = 0; j < N; ++j) x[u].v[j] = SHORT_IS_X ? f(s.v[j], x[u].v[j]) : f(x[u].v[j], s.v[j]);
+      *reinterpret_cast<Word*>(out + (r + u * step) * L + c) = x[u];
+    }
+  }
+}
+
+template <typename T, bool SHORT_IS_X, bool VEC, typename F>
+void launch_bcast_rows(cudaStream_t s, T* out, const T* lng, const T* sht, size_t R, size_t L, F f) {
+  constexpr size_t N = VEC ? VecOf<T>::N : 1, rows = VEC ? 4 : 8;
+  unsigned bx = 32;
+  while (bx < (unsigned)kThreads && bx * N < L) bx *= 2;
+  const unsigned by = kThreads / bx;
+  const size_t gx = (L + bx * N - 1) / (bx * N), want = (R + by * rows - 1) / (by * rows), cap = std::max<size_t>(1, (size_t)sm_count() * 8 / gx);
+  launch_pdl(bcast_rows_kernel<T, SHORT_IS_X, VEC, F>, dim3((unsigned)gx, (unsigned)std::min<size_t>({want, cap, 65535})), dim3(bx, by), 0, s, out, lng, sht, R, L, f);
+}
+
 struct AddOp { template <typename T> __device__ T operator()(T a, T b) const { return a + b; } };
 struct SubOp { template <typename T> __device__ T operator()(T a, T b) const { return a - b; } };
 struct MulOp { template <typename T> __device__ T operator()(T a, T b) const { return a * b; } };
@@ -179,6 +215,13 @@ void binary_dispatch(cudaStream_t s, const T* x, const T* y, T* z, size_t xl, si
   const T* sht = short_is_x ? x : y;
   const size_t L = short_is_x ? xl : yl;
   const bool vec = host_aligned16(z) && host_aligned16(lng);
+  if (L >= 32 && L <= 0x7fffffffu) {
+    const bool rows16 = vec && host_aligned16(sht) && L % VecOf<T>::N == 0;
+    if (short_is_x) rows16 ? launch_bcast_rows<T, true, true>(s, z, lng, sht, zl / L, L, f) : launch_bcast_rows<T, true, false>(s, z, lng, sht, zl / L, L, f);
+    else rows16 ? launch_bcast_rows<T, false, true>(s, z, lng, sht, zl / L, L, f) : launch_bcast_rows<T, false, false>(s, z, lng, sht, zl / L, L, f);
+    ZG_LAUNCH_CHECK();
+    return;
+  }
   const unsigned g = grid_for(zl, (size_t)kThreads * VecOf<T>::N * 2);
   if (short_is_x) {
     if (vec) launch_pdl(bcast_kernel<T, true, true, F>, dim3(g), dim3(kThreads), 0, s, z, lng, sht, zl, L, f);
@@ -253,37 +296,32 @@ __device__ __forceinline__ double dev_tanh(double x) { return tanh(x); }
 __device__ __forceinline__ float dev_pow(float x, float e) { return powf(x, e); }
 __device__ __forceinline__ double dev_pow(double x, double e) { return pow(x, e); }
 
-template <typename T>
+// (a kernel per function: a choice between them for every element keeps the compiler from interleaving the elements)
+template <typename T, int OP>
 struct UnaryF {
-  int op;
   T p;
   __device__ T operator()(T x, T, T) const {
-    switch (op) {
-      case ZG_UN_POW: return dev_pow(x, p);  // p = exponent
-      case ZG_UN_EXP: return dev_exp(x);
-      case ZG_UN_SQRT: return dev_sqrt(x);
-      case ZG_UN_RSQRT: return T(1) / dev_sqrt(x > p ? x : p);  // 1/sqrt(max(x, eps))
-      case ZG_UN_TANH: return dev_tanh(x);
-      default: return T(1) / (T(1) + dev_exp(-x));
-    }
+    if constexpr (OP == ZG_UN_POW) return dev_pow(x, p);  // p = exponent
+    else if constexpr (OP == ZG_UN_EXP) return dev_exp(x);
+    else if constexpr (OP == ZG_UN_SQRT) return dev_sqrt(x);
+    else if constexpr (OP == ZG_UN_RSQRT) return T(1) / dev_sqrt(x > p ? x : p);  // 1/sqrt(max(x, eps))
+    else if constexpr (OP == ZG_UN_TANH) return dev_tanh(x);
+    else return T(1) / (T(1) + dev_exp(-x));
   }
 };
-template <typename T>
+template <typename T, int OP>
 struct UnaryBwdF {  // inputs (v, y_g, x_g)
-  int op;
   T p;
   __device__ T operator()(T v, T yg, T xg) const {
-    switch (op) {
-      case ZG_UN_EXP: return xg + v * yg;
-      case ZG_UN_SQRT: return (v < p) ? xg : xg + T(0.5) / dev_sqrt(v) * yg;
-      case ZG_UN_RSQRT: {
-        if (v < p) return xg;
-        const T inv = T(1) / (v * dev_sqrt(v));
-        return xg + (T(-0.5) * inv) * yg;
-      }
-      case ZG_UN_TANH: return xg + (T(1) - v * v) * yg;
-      default: return xg + v * (T(1) - v) * yg;
+    if constexpr (OP == ZG_UN_EXP) return xg + v * yg;
+    else if constexpr (OP == ZG_UN_SQRT) return (v < p) ? xg : xg + T(0.5) / dev_sqrt(v) * yg;
+    else if constexpr (OP == ZG_UN_RSQRT) {
+      if (v < p) return xg;
+      const T inv = T(1) / (v * dev_sqrt(v));
+      return xg + (T(-0.5) * inv) * yg;
     }
+    else if constexpr (OP == ZG_UN_TANH) return xg + (T(1) - v * v) * yg;
+    else return xg + v * (T(1) - v) * yg;
   }
 };
 
@@ -534,11 +572,26 @@ extern "C" void pow_exp(dtype id, StreamWrapper w, const void* x, void* y, len_t
 }
 extern "C" void zg_unary_fwd(dtype id, StreamWrapper w, int op, const void* x, void* y, len_t n, double p) {
   if (op < ZG_UN_EXP || op > ZG_UN_POW) { set_error(kBadArgument, "zg_unary_fwd: unknown op %d", op); return; }
-  ZG_FLOAT_SWITCH("zg_unary_fwd", id, (launch_map<T, 1>(as_stream(w), (T*)y, (const T*)x, (const T*)nullptr, (const T*)nullptr, n, UnaryF<T>{op, (T)p})));
+#define ZG_UNARY_FWD(OP) \
+  if (op == OP) ZG_FLOAT_SWITCH("zg_unary_fwd", id, (launch_map<T, 1>(as_stream(w), (T*)y, (const T*)x, (const T*)nullptr, (const T*)nullptr, n, UnaryF<T, OP>{(T)p})))
+  ZG_UNARY_FWD(ZG_UN_EXP);
+  ZG_UNARY_FWD(ZG_UN_SQRT);
+  ZG_UNARY_FWD(ZG_UN_RSQRT);
+  ZG_UNARY_FWD(ZG_UN_TANH);
+  ZG_UNARY_FWD(ZG_UN_SIGM);
+  ZG_UNARY_FWD(ZG_UN_POW);
+#undef ZG_UNARY_FWD
 }
 extern "C" void zg_unary_bwd(dtype id, StreamWrapper w, int op, const void* v, const void* y_g, void* x_g, len_t n, double p) {
   if (op < ZG_UN_EXP || op > ZG_UN_SIGM) { set_error(kBadArgument, "zg_unary_bwd: unknown op %d", op); return; }
-  ZG_FLOAT_SWITCH("zg_unary_bwd", id, (launch_map<T, 3>(as_stream(w), (T*)x_g, (const T*)v, (const T*)y_g, (const T*)x_g, n, UnaryBwdF<T>{op, (T)p})));
+#define ZG_UNARY_BWD(OP) \
+  if (op == OP) ZG_FLOAT_SWITCH("zg_unary_bwd", id, (launch_map<T, 3>(as_stream(w), (T*)x_g, (const T*)v, (const T*)y_g, (const T*)x_g, n, UnaryBwdF<T, OP>{(T)p})))
+  ZG_UNARY_BWD(ZG_UN_EXP);
+  ZG_UNARY_BWD(ZG_UN_SQRT);
+  ZG_UNARY_BWD(ZG_UN_RSQRT);
+  ZG_UNARY_BWD(ZG_UN_TANH);
+  ZG_UNARY_BWD(ZG_UN_SIGM);
+#undef ZG_UNARY_BWD
 }
 
 extern "C" void zg_pow_bwd(dtype id, StreamWrapper w, const void* x, const void* y_g, void* x_g, len_t n, double exponent, double eps) {
