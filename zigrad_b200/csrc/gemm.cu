@@ -14,6 +14,7 @@
 #include "mlp_forward.cuh"
 #include "gemm_skinny.cuh"
 #include "gemm_block.cuh"
+#include "gemm_f64.cuh"
 #include "mlp_tail.cuh"
 #include "mlp_tail_rows.cuh"
 #include "../../include/blas_conflux.h"
@@ -63,6 +64,53 @@ static void launch_block_inst(cudaStream_t s, const void* A, const void* B, void
                      static_cast<const TI*>(B), static_cast<TC*>(C), p);
 }
 
+template <int TN, bool A_K, bool B_K>
+static void launch_f64_inst(cudaStream_t s, const void* A, const void* B, void* C, const f64::Params& p) {
+  using L = f64::Layout<TN, A_K, B_K>;
+  auto kern = f64::gemm_f64_kernel<TN, A_K, B_K>;
+  static SharedMemoryLimit limit;
+  if (!limit.raise(kern, L::kSmem)) return;
+  launch_pdl(kern, dim3(std::min<unsigned>(p.tiles, (unsigned)sm_count())), dim3(f64::kThreads), L::kSmem, s, static_cast<const double*>(A),
+             static_cast<const double*>(B), static_cast<double*>(C), p);
+}
+
+static int* tc_error_flag();
+
+// The tile width whose busiest SM has the least to do: the tensor instruction takes TN cycles per k of a 64 x TN tile, and a
+// tile about 300 cycles beside.
+static void launch_f64(cudaStream_t s, const void* A, const void* B, void* C, const block::Params& q, len_t nC) {
+  f64::Params p;
+  memset(&p, 0, sizeof(p));
+  p.nA = q.nA; p.nB = q.nB; p.m = q.m; p.n = q.n; p.k = q.k; p.lda = q.lda; p.ldb = q.ldb; p.ldc = q.ldc;
+  p.a_stride = q.a_stride; p.b_stride = q.b_stride; p.c_stride = q.c_stride;
+  p.alpha = q.alpha; p.beta = q.beta; p.bias = q.bias; p.mask = static_cast<const double*>(q.mask); p.epilogue = q.epilogue;
+  p.error_flag = tc_error_flag();
+  const size_t sms = (size_t)sm_count(), tiles_m = (p.m + f64::TM - 1) / f64::TM;
+  size_t tn = 0;
+  double best = 0;
+  for (const size_t w : {64, 48, 32}) {
+    const double tiles = (double)tiles_m * (double)((p.n + w - 1) / w) * (double)nC;
+    const double cost = std::ceil(tiles / (double)sms) * ((double)w * (double)p.k + 300.0);
+    if (!tn || cost < best) { tn = w; best = cost; }
+  }
+  const size_t tiles = tiles_m * ((p.n + tn - 1) / tn) * nC;
+  if (tiles > 0x7fffffffu) { set_error(kBadArgument, "gemm: grid too large (m=%lu, batches=%lu)", (len_t)p.m, nC); return; }
+  p.tiles_m = (uint32_t)tiles_m;
+  p.tiles_n = (uint32_t)((p.n + tn - 1) / tn);
+  p.tiles = (uint32_t)tiles;
+#define ZG_F64_CASE(TNV)                                                             \
+  if (tn == TNV) {                                                                   \
+    if (!q.ta && q.tb) return launch_f64_inst<TNV, true, true>(s, A, B, C, p);       \
+    if (!q.ta) return launch_f64_inst<TNV, true, false>(s, A, B, C, p);              \
+    if (q.tb) return launch_f64_inst<TNV, false, true>(s, A, B, C, p);               \
+    return launch_f64_inst<TNV, false, false>(s, A, B, C, p);                        \
+  }
+  ZG_F64_CASE(64)
+  ZG_F64_CASE(48)
+  ZG_F64_CASE(32)
+#undef ZG_F64_CASE
+}
+
 template <typename TI, typename TC>
 static void launch_block(cudaStream_t s, const void* A, const void* B, void* C, len_t nA, len_t nB, len_t nC, len_t m, len_t n, len_t k,
                          bool ta, bool tb, len_t lda, len_t ldb, len_t ldc, double alpha, double beta, int epilogue, const void* bias,
@@ -75,13 +123,9 @@ static void launch_block(cudaStream_t s, const void* A, const void* B, void* C, 
   p.bias = static_cast<const float*>(bias); p.mask = mask; p.colsum = static_cast<float*>(colsum);
   const size_t t64 = ((m + 63) / 64) * ((n + 63) / 64) * nC, t32 = ((m + 31) / 32) * ((n + 31) / 32) * nC;
   if constexpr (sizeof(TI) == 8) {
-    // The tile whose busiest SM has the least to do (an SM holds two CTAs of any of them; a 64 x 64 tile costs about 5 %
-    // less per multiply-add than a 64 x 32 one), split over clusters while SMs are left over.
-    const size_t t6432 = ((m + 63) / 64) * ((n + 31) / 32) * nC, sms = (size_t)sm_count();
-    const double w64 = (double)((t64 + sms - 1) / sms) * 4.0, w6432 = (double)((t6432 + sms - 1) / sms) * 2.1;
-    if (t64 * 2 <= sms) launch_block_inst<TI, TC, 32, 32, 0>(s, A, B, C, p, nC, block_splits(t32, k));
-    else if (w64 <= w6432) launch_block_inst<TI, TC, 64, 64, 0>(s, A, B, C, p, nC, 1);
-    else launch_block_inst<TI, TC, 64, 32, 0>(s, A, B, C, p, nC, 1);
+    // Half a 64 x 64 tile per SM or less: 32 x 32 tiles split over clusters.  (An fp64 caller has no column sums.)
+    if (t64 * 2 <= (size_t)sm_count()) launch_block_inst<TI, TC, 32, 32, 0>(s, A, B, C, p, nC, block_splits(t32, k));
+    else launch_f64(s, A, B, C, p, nC);
   } else {
     // 64 x 64 tiles (half the copies per multiply-add) once there is one for every SM; below that, parallelism counts
     // for more: 1000x301x501 takes 21 us with 32 x 32, 30 with 64 x 64; 4096x1023x1023 379 and 280
