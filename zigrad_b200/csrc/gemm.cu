@@ -371,12 +371,6 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   // adds them into C with TMA reductions instead (128x784x1024: 7.2 us against 8.8), which also allows more
   // than eight.  What cannot split, or only in two, halves BN when there are too few tiles to occupy the SMs
   // (8192x128x784: 12.6 us in 64-wide tiles, 14.4 as two splits of 128-wide ones).
-  const size_t min_slabs = mode == tc::kFP32X3 ? 4 : 12;  // per split: a three-pass slab costs 450 to 750 cycles, a single-pass one 130
-  const bool can_split = !persistent && k >= 2 * min_slabs * (size_t)bk && tiles * (bn == 128 ? 3 : 2) <= sm_share();
-  if (!persistent && !can_split && bn == 128 && tiles * 2 <= sm_share() && N > 64) {
-    bn = 64;
-    tiles = ((M + 127) / 128) * ((N + bn - 1) / bn) * nC;
-  }
   bool c_aligned;
   {
     const size_t ce = (c_id == SINGLE) ? 4 : 2;
@@ -384,7 +378,30 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
     if (mask) c_aligned = c_aligned && host_aligned16(mask);
     if (bias) c_aligned = c_aligned && host_aligned16(bias);
   }
-
+  const size_t min_slabs = mode == tc::kFP32X3 ? 4 : 12;  // per split: a three-pass slab costs 450 to 750 cycles, a single-pass one 130
+  const bool can_split = !persistent && k >= 2 * min_slabs * (size_t)bk && tiles * (bn == 128 ? 3 : 2) <= sm_share();
+  // (in a cluster; a plain product of 128-wide tiles reduces through the tensor map)
+  auto cluster_splits = [&](size_t t) {
+    unsigned sp = (unsigned)std::max<size_t>(1, std::min({sm_share() / t, (size_t)k / (min_slabs * bk), (size_t)8}));
+    while (sp > 1 && t > max_clusters(sp)) --sp;
+    return sp;
+  };
+  const bool reduces = epilogue == ZG_EPI_NONE && !colsum && c_id == SINGLE && c_aligned && !swap && bn == 128;
+  const size_t tiles64 = ((M + 127) / 128) * ((N + 63) / 64) * nC;
+  if (!persistent && !can_split && bn == 128 && tiles * 2 <= sm_share() && N > 64) {
+    bn = 64;
+    tiles = tiles64;
+  } else if (can_split && mode == tc::kFP32X3 && bn == 128 && !reduces && tiles64 <= sm_share()) {
+    // Three-pass tiles in clusters: a 128-wide one takes about 0.6 us per slab, 6.8 us beside it and 1.4 more in a cluster of
+    // eight, a 64-wide one 0.37 and 5.8 (launch, first loads, staging, the cluster's sum).  1000x301x501 11.8 us in 128-wide
+    // tiles, 9.8 in 64-wide ones; 4096x128x256 9.2 and 7.2; 1000x501x1000 12.3 and 12.5.
+    auto slabs = [&](unsigned sp) { return (double)((k + (size_t)bk * sp - 1) / ((size_t)bk * sp)); };
+    const unsigned s128 = cluster_splits(tiles), s64 = cluster_splits(tiles64);
+    if (5.8 + 0.37 * slabs(s64) < 6.8 + 0.6 * slabs(s128) + (s128 == 8 ? 1.4 : 0.0)) {
+      bn = 64;
+      tiles = tiles64;
+    }
+  }
   unsigned splits = 1;
   size_t whole = ptiles;
   if (persistent && epilogue == ZG_EPI_NONE && !colsum && c_id == SINGLE) {
@@ -400,11 +417,10 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   }
   bool cluster = false;
   if (can_split) {
-    const bool reduces = epilogue == ZG_EPI_NONE && !colsum && c_id == SINGLE && c_aligned && !swap && bn == 128;
-    splits = (unsigned)std::max<size_t>(1, std::min(sm_share() / tiles, k / (min_slabs * bk)));
-    if (!reduces) {
-      splits = std::min(splits, 8u);
-      while (splits > 1 && tiles > max_clusters(splits)) --splits;
+    if (reduces) {
+      splits = (unsigned)std::max<size_t>(1, std::min(sm_share() / tiles, k / (min_slabs * bk)));
+    } else {
+      splits = cluster_splits(tiles);
       cluster = splits > 1;
     }
   }

@@ -139,7 +139,11 @@ class MlpTrainer:
         # tensor cores; the reference op sequence keeps them contiguous.
         C = self.dims[-1]
         self.ld_out = (C + 3) // 4 * 4 if (fused and pad_logits) else C
-        self.ld = [self.dims[l + 1] if l + 1 < self.L else self.ld_out for l in range(self.L)]
+        # Rows of the hidden activations and their gradients: whole 16-byte words for the same reason, of the products that read
+        # them only the weights' own rows are then left to be copied element by element (1000-501-301-37 with narrower tiles,
+        # gemm.cu: 100 -> 92 us a step).
+        word = (8 if bf16 else 4) if (fused and pad_logits) else 1
+        self.ld = [-(-self.dims[l + 1] // word) * word if l + 1 < self.L else self.ld_out for l in range(self.L)]
         self.act = [d.mem_cache_alloc(act_t if l + 1 < self.L else SINGLE, self.B * self.ld[l]) for l in range(self.L)]
         self.dact = [d.mem_cache_alloc(act_t if l + 1 < self.L else SINGLE, self.B * self.ld[l]) for l in range(self.L)]
         if self.ld_out != C:
@@ -203,6 +207,10 @@ class MlpTrainer:
             self.zero_grad()
         return self._layers(X)
 
+    def _ld_in(self, l: int) -> int:
+        """Row stride of layer l's input: the caller's dense rows, or an activation's."""
+        return self.dims[0] if l == 0 else self.ld[l - 1]
+
     def _layers(self, X: DeviceSlice):
         d, B = self.dev, self.B
         inp = X
@@ -210,11 +218,11 @@ class MlpTrainer:
             d.dispatch(opspec.mlp_forward(X, self.dims, self.W, self.b, self.act))
             return self.act[-1]
         for l in range(self.L):
-            K, N = self.dims[l], self.dims[l + 1]
+            K, N, ldx = self.dims[l], self.dims[l + 1], self._ld_in(l)
             last = l + 1 == self.L
             if self.fused:
                 W = self.Wb[l] if self.bf16 else self.W[l]
-                d.dispatch(opspec.linear(inp, W, self.act[l], B, N, K, False, True, K, K, self.ld[l], 1.0, 0.0,
+                d.dispatch(opspec.linear(inp, W, self.act[l], B, N, K, False, True, ldx, K, self.ld[l], 1.0, 0.0,
                                          "bias" if last else "bias_relu", self.b[l]))
             else:
                 d.dispatch(opspec.bmm_acc(inp, self.W[l], self.act[l], (1, B, K), (1, K, N), (1, B, N), False, True, K, K, N, 1.0, 0.0))
@@ -274,12 +282,12 @@ class MlpTrainer:
                 # stream (a parallel branch of a captured step), forked here where dY
                 # is ready, and runs next to this layer's dX GEMM.
                 with d.branch():
-                    d.dispatch(opspec.linear(dy, a_in, self._dW[l], N, K, B, True, False, ldy, K, K, 1.0, 1.0))
+                    d.dispatch(opspec.linear(dy, a_in, self._dW[l], N, K, B, True, False, ldy, self._ld_in(l), K, 1.0, 1.0))
                     if on_layer_grads is not None:
                         on_layer_grads(l)
                 if l > 0:  # dX = dY . W, zeroed where the previous activation is <= 0
                     W = self.Wb[l] if self.bf16 else self.W[l]
-                    d.dispatch(opspec.linear(dy, W, self.dact[l - 1], B, K, N, False, False, ldy, K, K, 1.0, 0.0,
+                    d.dispatch(opspec.linear(dy, W, self.dact[l - 1], B, K, N, False, False, ldy, K, self.ld[l - 1], 1.0, 0.0,
                                              "relu_mask", None, self.act[l - 1], colsum=self._db[l - 1]))
                 if update_by_layer:
                     with d.branch(1, after=(0,)):
@@ -373,7 +381,7 @@ class MlpTrainer:
         inp = X
         for l in range(L - 2):  # the layers in front of the tail
             K, N = self.dims[l], self.dims[l + 1]
-            d.dispatch(opspec.linear(inp, self.W[l], self.act[l], B, N, K, False, True, K, K, self.ld[l], 1.0, 0.0, "bias_relu", self.b[l]))
+            d.dispatch(opspec.linear(inp, self.W[l], self.act[l], B, N, K, False, True, self._ld_in(l), K, self.ld[l], 1.0, 0.0, "bias_relu", self.b[l]))
             inp = self.act[l]
         h1, h2, C = self.dims[L - 2], self.dims[L - 1], self.dims[L]
         d.dispatch(opspec.mlp_tail(self.act[L - 3], self.W[L - 2], self.b[L - 2], self.W[L - 1], self.b[L - 1], T, B, h1, h2, C,
@@ -400,12 +408,12 @@ class MlpTrainer:
             a_in = X if l == 0 else self.act[l - 1]
             if l == 0:  # nothing else is left on the main stream: the largest weight gradient runs there
                 Cw, a = target(0)
-                d.dispatch(opspec.linear(self.dact[l], a_in, Cw, N, K, B, True, False, N, K, K, a, 1.0, sm_budget=share.get(0, 0)))
+                d.dispatch(opspec.linear(self.dact[l], a_in, Cw, N, K, B, True, False, self.ld[l], K, K, a, 1.0, sm_budget=share.get(0, 0)))
                 update([weight(0)])
             else:
                 with d.branch(0):
-                    d.dispatch(opspec.linear(self.dact[l], a_in, self._dW[l], N, K, B, True, False, N, K, K, 1.0, 1.0))
-                d.dispatch(opspec.linear(self.dact[l], self.W[l], self.dact[l - 1], B, K, N, False, False, N, K, K, 1.0, 0.0,
+                    d.dispatch(opspec.linear(self.dact[l], a_in, self._dW[l], N, K, B, True, False, self.ld[l], self._ld_in(l), K, 1.0, 1.0))
+                d.dispatch(opspec.linear(self.dact[l], self.W[l], self.dact[l - 1], B, K, N, False, False, self.ld[l], K, self.ld[l - 1], 1.0, 0.0,
                                          "relu_mask", None, self.act[l - 1], colsum=self._db[l - 1]))
         d.join()
         if fuse_update:
