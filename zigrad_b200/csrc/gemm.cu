@@ -15,6 +15,7 @@
 #include "gemm_skinny.cuh"
 #include "gemm_block.cuh"
 #include "gemm_f64.cuh"
+#include "gemm_repack.cuh"
 #include "mlp_tail.cuh"
 #include "mlp_tail_rows.cuh"
 #include "../../include/blas_conflux.h"
@@ -324,6 +325,26 @@ static size_t sm_share() {
 }
 extern "C" void zg_bmm_sm_budget(int sms) { g_next_sm_budget = sms > 0 ? sms : 0; }
 
+// Operands without 16-byte rows copied into the stream's work space with them (gemm_repack.cuh); a pointer and leading dimension
+// are replaced where they are copied.  False: no work space for it (more than 256 MB, or it would have to grow inside a capture).
+template <typename T>
+static bool repack_operands(cudaStream_t s, const void*& A, uint64_t rows_a, uint64_t cols_a, len_t& lda, bool copy_a, const void*& B, uint64_t rows_b,
+                            uint64_t cols_b, len_t& ldb, bool copy_b) {
+  constexpr uint64_t E = 16 / sizeof(T);
+  auto words = [](uint64_t cols) { return (cols + E - 1) / E; };
+  const uint64_t wa = copy_a ? rows_a * words(cols_a) : 0, wb = copy_b ? rows_b * words(cols_b) : 0;
+  const uint64_t at_b = (wa * 16 + 255) / 256 * 256, bytes = at_b + wb * 16;
+  if (bytes > ((uint64_t)256 << 20) || !workspace_ready(s, bytes, 1)) return false;
+  char* ws = static_cast<char*>(workspace(s, bytes, nullptr, 1));
+  if (!ws) return false;
+  const repack::Operand a{A, ws, lda, (uint32_t)cols_a, (uint32_t)words(cols_a), wa}, b{B, ws + at_b, ldb, (uint32_t)cols_b, (uint32_t)words(cols_b), wb};
+  const unsigned grid = grid_for(std::max(wa, wb), 512);
+  if (!launch_pdl(repack::repack_kernel<T>, dim3(grid, copy_a && copy_b ? 2 : 1), dim3(256), 0, s, copy_a ? a : b, b)) return false;
+  if (copy_a) { A = a.dst; lda = words(cols_a) * E; }
+  if (copy_b) { B = b.dst; ldb = words(cols_b) * E; }
+  return true;
+}
+
 // Returns true when the tensor-core path took the problem.
 static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A, const void* B, void* C, len_t nA, len_t nB, len_t nC,
                             len_t m, len_t n, len_t k, bool ta, bool tb, len_t lda, len_t ldb, len_t ldc, double alpha, double beta,
@@ -335,8 +356,7 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   const size_t es = bf16 ? 2 : 4;
   // operands whose rows a TMA box cannot address: fp32 ones are copied element by element (direct_slab)
   bool a_direct = !host_aligned16(A) || (lda * es) % 16 != 0, b_direct = !host_aligned16(B) || (ldb * es) % 16 != 0;
-  const bool direct = a_direct || b_direct;
-  if (direct && bf16) return false;
+  bool direct = a_direct || b_direct;
   if (m == 0 || n == 0 || nC == 0) return false;
   if (m > 0x7fffffffu || n > 0x7fffffffu || k > 0x7fffffffu || ldc > 0xffffffffu) return false;
   // Small problems are a latency chain on the tensor cores (descriptor fetch, TMA round trip, operand split, MMA,
@@ -348,6 +368,15 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   static const bool force = [] { const char* e = getenv("ZG_GEMM_FORCE_TC"); return e && e[0] == '1'; }();
   const double macs = (double)((m + 31) / 32 * 32) * (double)((n + 31) / 32 * 32) * (double)k * (double)nC;  // its tiles are 32 x 32
   if (!force && macs < small) return false;
+  // Measured crossovers of the copy: bf16 against the FFMA kernel 10 M multiply-adds (8.0 us either way; 30 M: 17 and 9), fp32
+  // against the element-wise ring 500 M (1000x501x1001 16 us either way; 2001x1001x1001 36 and 29).
+  if (direct && macs >= (bf16 ? 1.5e7 : 1e9)) {
+    const uint64_t ra = nA * (ta ? k : m), ca = ta ? m : k, rb = nB * (tb ? n : k), cb = tb ? k : n;
+    if (bf16 ? repack_operands<__nv_bfloat16>(s, A, ra, ca, lda, a_direct, B, rb, cb, ldb, b_direct)
+             : repack_operands<float>(s, A, ra, ca, lda, a_direct, B, rb, cb, ldb, b_direct))
+      a_direct = b_direct = direct = false;
+  }
+  if (direct && bf16) return false;
 
   const int atom = bf16 ? 64 : 32;        // M/N elements per 128-byte column block
   const int bk = bf16 ? 64 : 32;
