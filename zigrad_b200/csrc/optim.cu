@@ -19,9 +19,25 @@ struct SegTable {
   unsigned long long offset[kMaxSeg];
   unsigned long long len[kMaxSeg];
   float lr_t[kMaxSeg];  // Adam: bias-corrected step size of the segment
+  // CTAs [first_cta[j], first_cta[j + 1]) work on segment j: shares that go with the lengths, so that all end together.  With
+  // the same number for every segment (a second grid dimension) half of a network's CTAs were those of biases.  Norms and
+  // Adam over 4 matrices of 4 to 17 M elements and their biases, behind the products of a training step (with the clock
+  // those leave): 70 + 347 us, so 59 + 305; on their own, with data and clock cold, both forms take 300 to 308.
+  unsigned first_cta[kMaxSeg + 1];
   int n;
   int first;  // index of the first segment of this launch in the caller's list
 };
+
+// This CTA's segment, its place among the segment's CTAs and their number
+struct Share { int seg; unsigned cta, ctas; };
+__device__ __forceinline__ Share share_of(const SegTable& tab) {
+  int lo = 0, hi = tab.n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (tab.first_cta[mid] <= blockIdx.x) lo = mid; else hi = mid - 1;
+  }
+  return {lo, blockIdx.x - tab.first_cta[lo], tab.first_cta[lo + 1] - tab.first_cta[lo]};
+}
 
 // fp32 elements from p up to the next 16-byte boundary
 __device__ __forceinline__ size_t misalign_elems(const void* p) { return ((16u - (unsigned)(reinterpret_cast<uintptr_t>(p) & 15u)) & 15u) >> 2; }
@@ -29,16 +45,16 @@ __device__ __forceinline__ bool same_phase(const void* a, const void* b) {
   return ((reinterpret_cast<uintptr_t>(a) ^ reinterpret_cast<uintptr_t>(b)) & 15u) == 0;
 }
 
-// norms[first + j] = ||g_j||_2 for every segment of the table.  grid = (chunks, n);
-// chunk partials are folded by the last CTA of each segment in index order.
+// norms[first + j] = ||g_j||_2 for every segment of the table; the partial sums of its CTAs are folded by the last CTA of each segment in index order.
 __global__ void __launch_bounds__(kOThreads) seg_nrm2_kernel(const float* __restrict__ g, const __grid_constant__ SegTable tab,
                                                              float* norms, double* partial, unsigned* counters, int squares) {
   __shared__ double sm[32];
+  const Share sh = share_of(tab);
+  const int seg = sh.seg;
   pdl_sync();
-  const int seg = blockIdx.y;
   const float* p = g + tab.offset[seg];
   const size_t n = tab.len[seg];
-  const size_t nth = (size_t)gridDim.x * blockDim.x, tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t nth = (size_t)sh.ctas * blockDim.x, tid = (size_t)sh.cta * blockDim.x + threadIdx.x;
   // scalar head up to the first 16-byte boundary, 128-bit body (4 loads in flight per thread), scalar tail
   size_t head = misalign_elems(p);
   if (head > n) head = n;
@@ -61,20 +77,20 @@ __global__ void __launch_bounds__(kOThreads) seg_nrm2_kernel(const float* __rest
   for (size_t i = head + nv * 4 + tid; i < n; i += nth) acc += p[i] * p[i];
   acc = (acc + a1) + (a2 + a3);
   const double bs = block_sum<double>((double)acc, sm);
-  double* mine = partial + (size_t)seg * gridDim.x;
-  if (threadIdx.x == 0) mine[blockIdx.x] = bs;
+  double* mine = partial + tab.first_cta[seg];
+  if (threadIdx.x == 0) mine[sh.cta] = bs;
   __threadfence();
   __shared__ bool last;
   if (threadIdx.x == 0) {
     const unsigned t = atomicAdd(counters + 1 + seg, 1u);
-    last = (t == gridDim.x - 1);
+    last = (t == sh.ctas - 1);
     if (last) counters[1 + seg] = 0;
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
   double s = 0.0;
-  for (unsigned k = threadIdx.x; k < gridDim.x; k += blockDim.x) s += __ldcg(mine + k);
+  for (unsigned k = threadIdx.x; k < sh.ctas; k += blockDim.x) s += __ldcg(mine + k);
   s = block_sum<double>(s, sm);
   if (threadIdx.x == 0) norms[tab.first + seg] = squares ? (float)s : (float)sqrt(s);  // squares: the caller sums them over shards first
 }
@@ -90,16 +106,17 @@ __device__ __forceinline__ float clip_factor(const float* norms, int idx, float 
 template <bool CLIP>
 __global__ void __launch_bounds__(kOThreads) sgd_kernel(float* params, float* grads, const __grid_constant__ SegTable tab, float nlr,
                                                         const float* __restrict__ norms, float max_norm, float delta, const int zero) {
+  const Share sh = share_of(tab);
+  const int seg = sh.seg;
   pdl_sync();
-  const int seg = blockIdx.y;
   float* p = params + tab.offset[seg];
   float* g = grads + tab.offset[seg];
   const size_t n = tab.len[seg];
   bool on = false;
   float f = 1.f;
   if (CLIP) f = clip_factor(norms, tab.first + seg, max_norm, delta, &on);
-  const size_t nth = (size_t)gridDim.x * blockDim.x;
-  const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t nth = (size_t)sh.ctas * blockDim.x;
+  const size_t tid = (size_t)sh.cta * blockDim.x + threadIdx.x;
   if (same_phase(p, g) && (reinterpret_cast<uintptr_t>(p) & 3u) == 0) {
     size_t head = misalign_elems(p);
     if (head > n) head = n;
@@ -162,12 +179,13 @@ __device__ __forceinline__ unsigned long long read_counter(const unsigned long l
 // `target` (or nullptr): the soft update of a target network laid out like the parameters, target = tau * p + (1 - tau) *
 // target, in the same pass.
 template <bool CLIP, bool BF16COPY>
-__global__ void __launch_bounds__(kOThreads) adam_kernel(float* params, float* grads, float* ms, float* vs, const __grid_constant__ SegTable tab,
+__global__ void __launch_bounds__(kOThreads, 4) adam_kernel(float* params, float* grads, float* ms, float* vs, const __grid_constant__ SegTable tab,
                                                          const AdamScalars a, const float* __restrict__ norms, float max_norm,
                                                          float delta, __nv_bfloat16* copy, unsigned long long* t_dev, float lr,
                                                          unsigned* ticket, unsigned long long advance, float* target, float tau) {
+  const Share sh = share_of(tab);
+  const int seg = sh.seg;
   pdl_sync();
-  const int seg = blockIdx.y;
   const size_t off = tab.offset[seg];
   float* p = params + off;
   float* g = grads + off;
@@ -181,7 +199,7 @@ __global__ void __launch_bounds__(kOThreads) adam_kernel(float* params, float* g
     __syncthreads();
     lr_t = a.step_size(lr, (float)(now + (unsigned long long)(tab.first + seg + 1)));
     // the CTA that draws the last ticket moves the counter on: by then every CTA has read it (its one reading thread draws)
-    if (advance && threadIdx.x == 0 && atomicAdd(ticket, 1u) == gridDim.x * gridDim.y - 1) {
+    if (advance && threadIdx.x == 0 && atomicAdd(ticket, 1u) == gridDim.x - 1) {
       *ticket = 0;
       *t_dev = now + advance;
     }
@@ -189,7 +207,7 @@ __global__ void __launch_bounds__(kOThreads) adam_kernel(float* params, float* g
   bool on = false;
   float f = 1.f;
   if (CLIP) f = clip_factor(norms, tab.first + seg, max_norm, delta, &on);
-  const size_t nth = (size_t)gridDim.x * blockDim.x, tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t nth = (size_t)sh.ctas * blockDim.x, tid = (size_t)sh.cta * blockDim.x + threadIdx.x;
   auto one = [&](float& gi, float& mi, float& vi, float& pi) {
     if (CLIP && on) gi *= f;
     a.apply(gi, mi, vi, pi, lr_t);
@@ -217,8 +235,7 @@ __global__ void __launch_bounds__(kOThreads) adam_kernel(float* params, float* g
   float4* mq = reinterpret_cast<float4*>(m + head);
   float4* vq = reinterpret_cast<float4*>(v + head);
   float4* pq = reinterpret_cast<float4*>(p + head);
-  for (size_t k = tid; k < nv; k += nth) {
-    float4 gv = gq[k], mv = mq[k], vv = vq[k], pv = pq[k];
+  auto four = [&](size_t k, float4 gv, float4 mv, float4 vv, float4 pv) {
     one(gv.x, mv.x, vv.x, pv.x);
     one(gv.y, mv.y, vv.y, pv.y);
     one(gv.z, mv.z, vv.z, pv.z);
@@ -239,7 +256,16 @@ __global__ void __launch_bounds__(kOThreads) adam_kernel(float* params, float* g
       o.y = *reinterpret_cast<const uint32_t*>(&hi);
       *reinterpret_cast<uint2*>(copy + off + head + 4 * k) = o;
     }
+  };
+  // two words of each of the four arrays in flight per thread
+  size_t k = tid;
+  for (; k + nth < nv; k += 2 * nth) {
+    const size_t l = k + nth;
+    const float4 g0 = gq[k], g1 = gq[l], m0 = mq[k], m1 = mq[l], v0 = vq[k], v1 = vq[l], p0 = pq[k], p1 = pq[l];
+    four(k, g0, m0, v0, p0);
+    four(l, g1, m1, v1, p1);
   }
+  if (k < nv) four(k, gq[k], mq[k], vq[k], pq[k]);
   for (size_t i = head + nv * 4 + tid; i < n; i += nth) scalar(i);
 }
 
@@ -336,30 +362,36 @@ static unsigned small_cluster(const zg_segment* seg, size_t n_seg) {
   return mx <= kSmallLen && n_seg <= (size_t)kMaxSeg && n_seg * c <= (size_t)sm_count() * 3 / 4 ? c : 0;
 }
 
-static unsigned chunks_for(const zg_segment* seg, size_t n_seg) {
-  size_t mx = 0;
-  for (size_t j = 0; j < n_seg; ++j) mx = seg[j].len > mx ? seg[j].len : mx;
-  size_t c = (mx + (size_t)kOThreads * 4 - 1) / ((size_t)kOThreads * 4);
-  size_t cap = (size_t)sm_count() * 8 / (n_seg ? n_seg : 1);
-  if (cap < 8) cap = 8;
-  if (c > cap) c = cap;
-  return (unsigned)(c < 1 ? 1 : c);
+// Offsets, lengths and shares of the segments from `first` on: CTAs of at least four elements a thread, `per_sm` of them on an SM
+static SegTable seg_table(const zg_segment* seg, size_t n_seg, size_t first, int per_sm) {
+  SegTable tab;
+  memset(&tab, 0, sizeof(tab));
+  tab.n = (int)((n_seg - first) < (size_t)kMaxSeg ? (n_seg - first) : kMaxSeg);
+  tab.first = (int)first;
+  size_t total = 0;
+  for (int j = 0; j < tab.n; ++j) {
+    tab.offset[j] = seg[first + j].offset;
+    tab.len[j] = seg[first + j].len;
+    total += seg[first + j].len;
+  }
+  size_t per = (total + (size_t)sm_count() * per_sm - 1) / ((size_t)sm_count() * per_sm);
+  if (per < (size_t)kOThreads * 4) per = (size_t)kOThreads * 4;
+  for (int j = 0; j < tab.n; ++j) {
+    const size_t c = (tab.len[j] + per / 2) / per;
+    tab.first_cta[j + 1] = tab.first_cta[j] + (unsigned)(c < 1 ? 1 : c);
+  }
+  return tab;
 }
 
 static bool compute_norms(cudaStream_t s, const float* grads, const zg_segment* seg, size_t n_seg, float* norms, int squares = 0) {
   if (!norms) { set_error(kBadArgument, "optimizer: clip requested but norms scratch is NULL"); return false; }
   for (size_t first = 0; first < n_seg; first += kMaxSeg) {
-    SegTable tab;
-    memset(&tab, 0, sizeof(tab));
-    tab.n = (int)((n_seg - first) < (size_t)kMaxSeg ? (n_seg - first) : kMaxSeg);
-    tab.first = (int)first;
-    for (int j = 0; j < tab.n; ++j) { tab.offset[j] = seg[first + j].offset; tab.len[j] = seg[first + j].len; }
-    unsigned chunks = chunks_for(seg + first, tab.n);
-    if (chunks > 256) chunks = 256;
+    const SegTable tab = seg_table(seg, n_seg, first, 5);
+    const unsigned ctas = tab.first_cta[tab.n];
     unsigned* counters = nullptr;
-    double* partial = static_cast<double*>(workspace(s, sizeof(double) * chunks * tab.n, &counters));
+    double* partial = static_cast<double*>(workspace(s, sizeof(double) * ctas, &counters));
     if (!partial) return false;
-    if (!launch_pdl(seg_nrm2_kernel, dim3(chunks, tab.n), dim3(kOThreads), 0, s, grads, tab, norms, partial, counters, squares)) return false;
+    if (!launch_pdl(seg_nrm2_kernel, dim3(ctas), dim3(kOThreads), 0, s, grads, tab, norms, partial, counters, squares)) return false;
   }
   return true;
 }
@@ -375,10 +407,7 @@ extern "C" void zg_sgd_step(dtype id, StreamWrapper w, void* params, void* grads
   cudaStream_t s = as_stream(w);
   const float nlr = -(float)lr;  // lr cast f64 -> f32, then negated (optim.zig:103)
   if (const unsigned c = clip == 1 && norms ? small_cluster(seg, n_seg) : 0) {
-    SegTable tab;
-    memset(&tab, 0, sizeof(tab));
-    tab.n = (int)n_seg;
-    for (int j = 0; j < tab.n; ++j) { tab.offset[j] = seg[j].offset; tab.len[j] = seg[j].len; }
+    const SegTable tab = seg_table(seg, n_seg, 0, 1);
     launch_pdl_cluster(small_step_kernel<false>, dim3(c, (unsigned)n_seg), dim3(kSmallThreads), 0, s, c, (float*)params, (float*)grads, (float*)nullptr,
                        (float*)nullptr, tab, AdamScalars{}, (float*)norms, (float)max_norm, (float)delta, (unsigned long long*)nullptr, nlr,
                        (unsigned*)nullptr, 0ull, (float*)nullptr, 0.f, zero_grads);
@@ -387,12 +416,8 @@ extern "C" void zg_sgd_step(dtype id, StreamWrapper w, void* params, void* grads
   if (clip == 1 && !compute_norms(s, (const float*)grads, seg, n_seg, (float*)norms)) return;
   if (clip == 2 && !norms) { set_error(kBadArgument, "optimizer: clip with given norms but norms is NULL"); return; }
   for (size_t first = 0; first < n_seg; first += kMaxSeg) {
-    SegTable tab;
-    memset(&tab, 0, sizeof(tab));
-    tab.n = (int)((n_seg - first) < (size_t)kMaxSeg ? (n_seg - first) : kMaxSeg);
-    tab.first = (int)first;
-    for (int j = 0; j < tab.n; ++j) { tab.offset[j] = seg[first + j].offset; tab.len[j] = seg[first + j].len; }
-    const dim3 grid(chunks_for(seg + first, tab.n), tab.n);
+    const SegTable tab = seg_table(seg, n_seg, first, 6);
+    const dim3 grid(tab.first_cta[tab.n]);
     if (clip) launch_pdl(sgd_kernel<true>, grid, dim3(kOThreads), 0, s, (float*)params, (float*)grads, tab, nlr, (const float*)norms, (float)max_norm, (float)delta, zero_grads);
     else launch_pdl(sgd_kernel<false>, grid, dim3(kOThreads), 0, s, (float*)params, (float*)grads, tab, nlr, (const float*)nullptr, 0.f, 0.f, zero_grads);
   }
@@ -406,13 +431,8 @@ static void adam_step(cudaStream_t s, float* P, float* G, float* M, float* V, co
   const AdamScalars a{beta1, beta2, 1.f - beta1, 1.f - beta2, (float)eps_};
   if (clip && !norms) { set_error(kBadArgument, "optimizer: clip %s but norms is NULL", clip == 2 ? "with given norms" : "requested"); return; }
   auto table = [&](size_t first) {
-    SegTable tab;
-    memset(&tab, 0, sizeof(tab));
-    tab.n = (int)((n_seg - first) < (size_t)kMaxSeg ? (n_seg - first) : kMaxSeg);
-    tab.first = (int)first;
+    SegTable tab = seg_table(seg, n_seg, first, 4);
     for (int j = 0; j < tab.n; ++j) {
-      tab.offset[j] = seg[first + j].offset;
-      tab.len[j] = seg[first + j].len;
       const float t_f = (float)(t_first + first + j);  // counter advances once per tensor (optim.zig:189)
       tab.lr_t[j] = lr * std::sqrt(1.f - std::pow(beta2, t_f)) / (1.f - std::pow(beta1, t_f));
     }
@@ -431,7 +451,7 @@ static void adam_step(cudaStream_t s, float* P, float* G, float* M, float* V, co
   if (clip == 1 && !compute_norms(s, G, seg, n_seg, norms)) return;
   for (size_t first = 0; first < n_seg; first += kMaxSeg) {
     const SegTable tab = table(first);
-    const dim3 grid(chunks_for(seg + first, tab.n), tab.n), blk(kOThreads);
+    const dim3 grid(tab.first_cta[tab.n]), blk(kOThreads);
     const unsigned long long inc = (own && first + kMaxSeg >= n_seg) ? (unsigned long long)n_seg : 0ull;
     auto kern = clip ? (cp ? adam_kernel<true, true> : adam_kernel<true, false>) : (cp ? adam_kernel<false, true> : adam_kernel<false, false>);
     if (!launch_pdl(kern, grid, blk, 0, s, P, G, M, V, tab, a, (const float*)norms, (float)max_norm, (float)delta, cp, t_dev, lr, ticket, inc, target, (float)tau)) return;
