@@ -310,6 +310,9 @@ EXTERN_C void zg_adam_soft_step(dtype id, StreamWrapper stream, void* params, vo
 /* out[j] = sum of squares of segment j (fp64 accumulation, deterministic two-stage): the
  * shard-local part of the per-tensor gradient norm of host_device.zig:339-346 */
 EXTERN_C void zg_segment_sumsq(dtype id, StreamWrapper stream, const void* x, const zg_segment* seg, len_t n_seg, void* out);
+/* x[offset .. offset + len) = value for every segment, one launch: the parts of a gradient buffer that a step accumulates
+ * into, where it writes the rest (model.zig:57-62 fills them all) */
+EXTERN_C void zg_fill_segments(dtype id, StreamWrapper stream, void* x, const zg_segment* seg, len_t n_seg, double value);
 /* Softmax cross-entropy of selected rows (mem_take, softmax_ce and scatter_add as one launch): row r of the loss reads
  * logits + offsets[r * ld] (a row's offsets are consecutive) and ADDS its gradient into dlogits there; loss and dbias (the
  * gradient's column sums, may be NULL) are overwritten. */

@@ -1,5 +1,5 @@
 """Broadcasts and column sums at the edges of the kernels that keep a column per thread: rows shorter and longer than a warp,
-ragged and between words, one CTA of rows and more, both types.  Broadcasts are single
+ragged and between words, one CTA of rows and more, both types; and the fill of segments.  Broadcasts are single
 operations (exact); a column sum of at most 4099 values in fp32 1e-5, in fp64 1e-13 of the largest."""
 import numpy as np
 import pytest
@@ -40,3 +40,13 @@ def test_column_sums(gpu, rows, col, ty):
     X, Y = be.up(x, ty), be.up(y, ty)
     gpu.dispatch(opspec.unbroadcast(X, [rows, col], Y, [col], None, 1.0, 0.5))
     assert rel_err(be.down(Y), x.astype(np.float64).sum(0) + 0.5 * y) <= (1e-5 if ty == np.float32 else 1e-13)
+
+
+def test_fill_segments(gpu):
+    be = GpuBackend(gpu)
+    x = np.arange(70000, dtype=np.float32)
+    X, want, segs = be.up(x), x.copy(), [(3, 1), (10, 0), (17, 60000), (69999, 1)] + [(61000 + 100 * i, i) for i in range(60)]
+    gpu.fill_segments(X, segs, -2.5)
+    for off, n in segs:
+        want[off:off + n] = -2.5
+    np.testing.assert_array_equal(be.down(X), want)

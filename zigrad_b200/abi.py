@@ -220,6 +220,7 @@ SIGNATURES = {
     "zg_q_head_supported": (i32, [dtype_t, len_t, len_t]),
     "zg_q_head": (None, [dtype_t, S, len_t, len_t, vp, vp, vp, vp, vp, dbl, dbl, dbl, vp, vp, vp, vp, vp, vp, vp, vp]),
     "zg_segment_sumsq": (None, [dtype_t, S, vp, C.POINTER(Segment), len_t, vp]),
+    "zg_fill_segments": (None, [dtype_t, S, vp, C.POINTER(Segment), len_t, dbl]),
     "zg_soft_update": (None, [dtype_t, S, vp, vp, len_t, dbl]),
     "zg_cast": (None, [dtype_t, dtype_t, S, vp, vp, len_t]),
     # ---- peer-memory all-reduce

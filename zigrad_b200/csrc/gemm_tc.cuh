@@ -95,7 +95,8 @@ struct Params {
   // TMA unit -- 1: plain store (no split-K, beta == 0, epilogue NONE / BIAS / BIAS_RELU, no column
   // sums), 2: reduce-add into C (split-K partial products; C pre-scaled by beta).  Whole 128-byte
   // lines leave the SM instead of 16-byte pieces of 32 different lines per instruction, and boxes that
-  // hang over the edge of C are clipped by the unit.  0: register path below.
+  // hang over the edge of C are clipped by the unit.  3 (persistent kernel): whole tiles are stored, K ranges added into
+  // tiles that were cleared.  0: register path below.
   int tma_epilogue;
   // Split K over the CTAs of a cluster: every CTA stages its partial tile in shared memory, rank r sums rows r,
   // r + splits, ... of all of them through distributed shared memory in rank order and applies the epilogue.

@@ -451,7 +451,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
         __syncwarp();
         if (lane == 0) {
           const int x = (int)(tc.n * BN) + c * width;
-          if (p.tma_epilogue == 2) tma_reduce_add_box(&tmC, stg + (box & 1) * 4096, x, (int)row0, (int)tc.batch);
+          if (p.tma_epilogue == 2 || (p.tma_epilogue == 3 && tc.split != kNoSplit)) tma_reduce_add_box(&tmC, stg + (box & 1) * 4096, x, (int)row0, (int)tc.batch);
           else tma_store_box(&tmC, stg + (box & 1) * 4096, x, (int)row0, (int)tc.batch);
           bulk_commit_group();
         }

@@ -347,6 +347,14 @@ __global__ void __launch_bounds__(kSmallThreads) small_step_kernel(float* params
   cluster.sync();  // nobody leaves while its partial sum may still be read
 }
 
+// Segments of a flat buffer set to a value: what a step clears of its gradients when the rest is about to be written.
+__global__ void __launch_bounds__(kOThreads) fill_segments_kernel(float* x, const __grid_constant__ SegTable tab, float value) {
+  const Share sh = share_of(tab);
+  pdl_sync();
+  float* p = x + tab.offset[sh.seg];
+  for (size_t i = (size_t)sh.cta * blockDim.x + threadIdx.x; i < tab.len[sh.seg]; i += (size_t)sh.ctas * blockDim.x) p[i] = value;
+}
+
 __global__ void counter_add_kernel(unsigned long long* c, unsigned long long inc) {
   pdl_sync();
   *c += inc;
@@ -420,6 +428,14 @@ extern "C" void zg_sgd_step(dtype id, StreamWrapper w, void* params, void* grads
     const dim3 grid(tab.first_cta[tab.n]);
     if (clip) launch_pdl(sgd_kernel<true>, grid, dim3(kOThreads), 0, s, (float*)params, (float*)grads, tab, nlr, (const float*)norms, (float)max_norm, (float)delta, zero_grads);
     else launch_pdl(sgd_kernel<false>, grid, dim3(kOThreads), 0, s, (float*)params, (float*)grads, tab, nlr, (const float*)nullptr, 0.f, 0.f, zero_grads);
+  }
+}
+
+extern "C" void zg_fill_segments(dtype id, StreamWrapper w, void* x, const zg_segment* seg, len_t n_seg, double value) {
+  if (id != SINGLE) { set_error(kUnsupported, "zg_fill_segments: only SINGLE is implemented"); return; }
+  for (size_t first = 0; first < n_seg; first += kMaxSeg) {
+    const SegTable tab = seg_table(seg, n_seg, first, 6);
+    launch_pdl(fill_segments_kernel, dim3(tab.first_cta[tab.n]), dim3(kOThreads), 0, as_stream(w), (float*)x, tab, (float)value);
   }
 }
 

@@ -683,6 +683,9 @@ class CudaDevice:
     def segment_sumsq(self, x: DeviceSlice, segments, out: DeviceSlice):
         self.L.zg_segment_sumsq(x.dtype, self.stream, x.ptr, self._segments(segments), len(segments), out.ptr)
 
+    def fill_segments(self, x: DeviceSlice, segments, value: float):
+        self.L.zg_fill_segments(x.dtype, self.stream, x.ptr, self._segments(segments), len(segments), value)
+
     def soft_update(self, src: DeviceSlice, target: DeviceSlice, tau: float):
         self.L.zg_soft_update(src.dtype, self.stream, src.ptr, target.ptr, src.len, tau)
 

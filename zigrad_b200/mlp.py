@@ -171,6 +171,28 @@ class MlpTrainer:
         self.dev.mem_fill(self._grads, 0.0)
         self._grads_clear = False
 
+    def _large(self, l: int) -> bool:
+        """Whether layer l's weight gradient has enough output tiles (64 of 128 x 128) to fill the chip without K ranges that
+        are added into a cleared C.  Smaller ones are cleared with the biases, in one launch of about 2 us."""
+        return self.segments[2 * l][1] >= 1 << 20
+
+    def clear_for_backward(self):
+        """The gradients that a fused backward pass(fresh=True) accumulates into: all but those of large weights."""
+        large = {2 * l for l in range(self.L) if self._large(l)}
+        if not large:
+            return self.zero_grad()
+        runs, end = [], -1  # neighbours as one segment
+        for j, (off, n) in enumerate(self.segments):
+            if j in large:
+                continue
+            if off == end:
+                runs[-1][1] += n
+            else:
+                runs.append([off, n])
+            end = off + n
+        self.dev.fill_segments(self._grads, runs, 0.0)
+        self._grads_clear = False
+
     @property
     def grads(self) -> DeviceSlice:
         self._touched = True
@@ -242,7 +264,7 @@ class MlpTrainer:
             d.dispatch(opspec.softmax_ce(self.act[-1], T, B, C, self.loss, self.dact[-1], self.loss_div, accumulate=False))
 
     def backward(self, X: DeviceSlice, last_bias_done: bool = True, on_layer_grads: Optional[Callable[[int], None]] = None,
-                 update_by_layer: bool = False):
+                 update_by_layer: bool = False, fresh: bool = False):
         """Backward from dact[L-1].  `last_bias_done`: the bias gradient of the last
         layer was already produced by the loss kernel (fused path); pass False when
         dact[L-1] comes from elsewhere (e.g. the DQN's gather backward).
@@ -258,7 +280,10 @@ class MlpTrainer:
         over all tensors (zg_adam_step_part keeps every tensor's position in the step
         count); the caller must not call update() for this step.  Off by default: on the
         wide MLP the update then competes with the persistent GEMMs for memory bandwidth
-        and the step got slower (2.39 ms against 2.27 ms with one update after the join)."""
+        and the step got slower (2.39 ms against 2.27 ms with one update after the join).
+        `fresh` (fused path): the gradients of large weights are written (beta = 0), whatever the
+        buffer holds, and the others are zero already (clear_for_backward): what zeroing the
+        whole buffer and accumulating gives, without the two passes over it."""
         d, B = self.dev, self.B
         self._touched = True
         if self.fused and not last_bias_done:
@@ -282,7 +307,8 @@ class MlpTrainer:
                 # stream (a parallel branch of a captured step), forked here where dY
                 # is ready, and runs next to this layer's dX GEMM.
                 with d.branch():
-                    d.dispatch(opspec.linear(dy, a_in, self._dW[l], N, K, B, True, False, ldy, self._ld_in(l), K, 1.0, 1.0))
+                    d.dispatch(opspec.linear(dy, a_in, self._dW[l], N, K, B, True, False, ldy, self._ld_in(l), K, 1.0,
+                                             0.0 if fresh and self._large(l) else 1.0))
                     if on_layer_grads is not None:
                         on_layer_grads(l)
                 if l > 0:  # dX = dY . W, zeroed where the previous activation is <= 0
@@ -447,9 +473,13 @@ class MlpTrainer:
                 return
         else:
             by_layer = self.update_by_layer and self.fused and self.opt == "adam" and allreduce is None
-            self._forward(X, self.fused and self._zero_grad_due())
+            # The whole step is issued here: of its gradients only those it accumulates into have to be cleared (a fill of
+            # all of them is 35 us of the wide network's step, and the additions read the 218 MB once more)
+            if self.fused and self._zero_grad_due():
+                self.clear_for_backward()
+            self._layers(X)
             self.loss_and_grad(T)
-            self.backward(X, update_by_layer=by_layer)
+            self.backward(X, update_by_layer=by_layer, fresh=self.fused)
             if by_layer:
                 return
         if allreduce is not None:
