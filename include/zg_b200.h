@@ -310,6 +310,20 @@ EXTERN_C void zg_adam_soft_step(dtype id, StreamWrapper stream, void* params, vo
 /* out[j] = sum of squares of segment j (fp64 accumulation, deterministic two-stage): the
  * shard-local part of the per-tensor gradient norm of host_device.zig:339-346 */
 EXTERN_C void zg_segment_sumsq(dtype id, StreamWrapper stream, const void* x, const zg_segment* seg, len_t n_seg, void* out);
+/* The weight gradients of a fully connected network over `rows` rows, one launch: for each layer dW [out, in] = dy^T x and
+ * db [out] = column sums of dy (ndtensor.zig:1092-1136), both overwritten; then, where W and b are given, the SGD step
+ * W += (-lr) dW, b += (-lr) db (src/nn/optim.zig:100-122 without clipping).  dW, db, W and b are dense and may each be NULL. */
+typedef struct {
+  const void* dy; /* [rows, out], rows ld_dy elements apart */
+  const void* x;  /* [rows, in], rows ld_x elements apart */
+  void* dW;
+  void* db;
+  void* W;
+  void* b;
+  len_t out, in, ld_dy, ld_x;
+} zg_weight_grad;
+EXTERN_C int zg_weight_grads_supported(dtype id, const zg_weight_grad* g, len_t n, len_t rows);
+EXTERN_C void zg_weight_grads(dtype id, StreamWrapper stream, const zg_weight_grad* g, len_t n, len_t rows, double lr);
 /* x[offset .. offset + len) = value for every segment, one launch: the parts of a gradient buffer that a step accumulates
  * into, where it writes the rest (model.zig:57-62 fills them all) */
 EXTERN_C void zg_fill_segments(dtype id, StreamWrapper stream, void* x, const zg_segment* seg, len_t n_seg, double value);

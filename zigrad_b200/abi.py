@@ -79,6 +79,10 @@ class Segment(C.Structure):
     _fields_ = [("offset", len_t), ("len", len_t)]
 
 
+class WeightGrad(C.Structure):
+    _fields_ = [(n, vp) for n in ("dy", "x", "dW", "db", "W", "b")] + [(n, len_t) for n in ("out", "inp", "ld_dy", "ld_x")]
+
+
 ADD, MIN, MAX, MUL = 0, 1, 2, 3
 EPI_NONE, EPI_BIAS, EPI_BIAS_RELU, EPI_RELU_MASK = 0, 1, 2, 3
 MATH_FP32X3, MATH_TF32, MATH_FFMA = 0, 1, 2
@@ -220,6 +224,8 @@ SIGNATURES = {
     "zg_q_head_supported": (i32, [dtype_t, len_t, len_t]),
     "zg_q_head": (None, [dtype_t, S, len_t, len_t, vp, vp, vp, vp, vp, dbl, dbl, dbl, vp, vp, vp, vp, vp, vp, vp, vp]),
     "zg_segment_sumsq": (None, [dtype_t, S, vp, C.POINTER(Segment), len_t, vp]),
+    "zg_weight_grads_supported": (C.c_int, [dtype_t, C.POINTER(WeightGrad), len_t, len_t]),
+    "zg_weight_grads": (None, [dtype_t, S, C.POINTER(WeightGrad), len_t, len_t, dbl]),
     "zg_fill_segments": (None, [dtype_t, S, vp, C.POINTER(Segment), len_t, dbl]),
     "zg_soft_update": (None, [dtype_t, S, vp, vp, len_t, dbl]),
     "zg_cast": (None, [dtype_t, dtype_t, S, vp, vp, len_t]),

@@ -576,6 +576,44 @@ void bmm_dispatch(dtype id, dtype c_id, cudaStream_t s, const void* A, const voi
   else set_error(kUnsupported, "bmm: unsupported dtype combination %d -> %d", (int)id, (int)c_id);
 }
 
+// ---- the weight gradients of a network on few rows as one launch (gemm_block.cuh)
+// Where the products would go to the block kernel one by one (up to 5e7 multiply-adds, see try_tensor_core), all of them
+// together: above that the tensor cores gain more than the launches cost.
+static bool weight_grads_ok(dtype id, const zg_weight_grad* g, len_t n, len_t rows) {
+  if (id != SINGLE || n == 0 || n > (len_t)block::kGroupMax || rows == 0 || rows > 4096) return false;
+  double macs = 0;
+  for (len_t i = 0; i < n; ++i) {
+    if (g[i].out == 0 || g[i].in == 0 || g[i].out > 0x7fffffffu || g[i].in > 0x7fffffffu || g[i].ld_dy > 0x7fffffffu || g[i].ld_x > 0x7fffffffu) return false;
+    macs += (double)((g[i].out + 31) / 32 * 32) * (double)((g[i].in + 31) / 32 * 32) * (double)rows;
+  }
+  return macs <= 5e7;
+}
+extern "C" int zg_weight_grads_supported(dtype id, const zg_weight_grad* g, len_t n, len_t rows) { return weight_grads_ok(id, g, n, rows) ? 1 : 0; }
+
+extern "C" void zg_weight_grads(dtype id, StreamWrapper w, const zg_weight_grad* g, len_t n, len_t rows, double lr) {
+  if (!weight_grads_ok(id, g, n, rows)) { set_error(kUnsupported, "zg_weight_grads: dtype %d, %lu products over %lu rows", (int)id, n, rows); return; }
+  block::Group q;
+  memset(&q, 0, sizeof(q));
+  size_t tiles = 0;
+  for (len_t i = 0; i < n; ++i) {
+    if (!g[i].dy || !g[i].x) { set_error(kBadArgument, "zg_weight_grads: NULL operand"); return; }
+    const uint32_t tn = (uint32_t)((g[i].in + 31) / 32), tm = (uint32_t)((g[i].out + 31) / 32);
+    q.item[i] = {static_cast<const float*>(g[i].dy), static_cast<const float*>(g[i].x), static_cast<float*>(g[i].dW), static_cast<float*>(g[i].W),
+                 static_cast<float*>(g[i].db), static_cast<float*>(g[i].b), (uint32_t)g[i].out, (uint32_t)g[i].in, (uint32_t)g[i].ld_dy,
+                 (uint32_t)g[i].ld_x, tn, (uint32_t)tiles};
+    tiles += (size_t)tn * tm;
+  }
+  q.items = (uint32_t)n;
+  q.k = (uint32_t)rows;
+  q.splits = block_splits(tiles, rows);
+  q.k_per_split = q.splits > 1 ? (uint32_t)(((rows + q.splits - 1) / q.splits + 7) / 8 * 8) : (uint32_t)rows;
+  q.nlr = -(float)lr;  // lr cast f64 -> f32, then negated (optim.zig:103)
+  using L = block::Layout<float, 32, 32, 4>;
+  static SharedMemoryLimit limit;
+  if (!limit.raise(block::weight_grads_kernel, L::kSmem)) return;
+  launch_pdl_cluster(block::weight_grads_kernel, dim3((unsigned)(tiles * q.splits)), dim3(block::kThreads), L::kSmem, as_stream(w), q.splits, q);
+}
+
 // ---- fused middle of the MLP step (mlp_tail.cuh)
 template <int CP>
 static bool launch_tail_inst(cudaStream_t s, const CUtensorMap& ta, const CUtensorMap& tk, const CUtensorMap& tn, const CUtensorMap& t1,
@@ -605,7 +643,9 @@ void mlp_tail_launch(cudaStream_t s, len_t rows, len_t h1, len_t h2, len_t C, co
   }
   if (rows > 0x7fffffffu || ld_out < C || ld_out > 0xffffffffu) { set_error(kBadArgument, "zg_mlp_tail_fwd_bwd: rows %lu, ld_out %lu", rows, ld_out); return; }
   if (label_kind != ZG_LABEL_ONEHOT && label_kind != ZG_LABEL_INDEX) { set_error(kBadArgument, "zg_mlp_tail_fwd_bwd: unknown label kind %d", label_kind); return; }
-  const void* ptrs[] = {act0, W1, b1, W2, b2, labels, act1, logits, loss_out, dlogits, dact1, dact0, db2, db1, db0};
+  // no bias gradients: a grouped launch behind this one forms them with the weights' (row kernel only)
+  const bool sums = db2 || db1 || db0 || rows > (len_t)sm_count() * 2 * 28;
+  const void* ptrs[] = {act0, W1, b1, W2, b2, labels, act1, logits, loss_out, dlogits, dact1, dact0, sums ? db2 : act0, sums ? db1 : act0, sums ? db0 : act0};
   for (const void* q : ptrs)
     if (!q) { set_error(kBadArgument, "zg_mlp_tail_fwd_bwd: NULL argument"); return; }
   if (!host_aligned16(act0) || !host_aligned16(W1) || !host_aligned16(act1) || !host_aligned16(dact1) || !host_aligned16(dact0)) {

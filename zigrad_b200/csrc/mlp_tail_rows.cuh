@@ -45,7 +45,7 @@ struct Params {
   float* dlogits;         // [rows, ld_out]
   float* dact1;           // [rows, 64]
   float* dact0;           // [rows, 128]
-  float* db2;             // [C]   column sums are ADDED (the gradient buffer is zero at the start of a step)
+  float* db2;             // [C]   column sums are ADDED (the gradient buffer is zero at the start of a step); none: all NULL
   float* db1;             // [64]
   float* db0;             // [128]
   float* loss_out;        // one scalar, overwritten
@@ -343,7 +343,8 @@ __global__ void __launch_bounds__(kThreads, 2) mlp_tail_rows_kernel(const Params
     }
   }
   __syncthreads();
-  if (t < kH1) {
+  if (!p.db0) {
+  } else if (t < kH1) {
     float s = 0.f;
 #pragma unroll
     for (int w = 0; w < R / 4; ++w) s += sum0[w * kH1 + t];

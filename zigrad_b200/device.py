@@ -73,6 +73,14 @@ def _segments_of(segs: tuple):
     return arr
 
 
+@functools.lru_cache(maxsize=256)
+def _weight_grads_of(items: tuple):
+    arr = (abi.WeightGrad * len(items))()
+    for i, it in enumerate(items):
+        arr[i] = abi.WeightGrad(*it)
+    return arr
+
+
 def _f32(v: float):
     return C.byref(C.c_float(v))
 
@@ -618,8 +626,19 @@ class CudaDevice:
     def mlp_tail(self, p):
         kind = abi.LABEL_INDEX if p.labels.dtype == USIZE else abi.LABEL_ONEHOT
         self.L.zg_mlp_tail_fwd_bwd(p.act0.dtype, self.stream, p.rows, p.h1, p.h2, p.classes, p.act0.ptr, p.W1.ptr, p.b1.ptr, p.W2.ptr,
-                                   p.b2.ptr, p.labels.ptr, kind, p.ld_out, float(p.loss_div), p.act1.ptr, p.logits.ptr, p.loss.ptr,
-                                   p.dlogits.ptr, p.dact1.ptr, p.dact0.ptr, p.db2.ptr, p.db1.ptr, p.db0.ptr, int(p.weights_ready))
+                                p.b2.ptr, p.labels.ptr, kind, p.ld_out, float(p.loss_div), p.act1.ptr, p.logits.ptr, p.loss.ptr,
+                                p.dlogits.ptr, p.dact1.ptr, p.dact0.ptr, *(b.ptr if b is not None else None for b in (p.db2, p.db1, p.db0)),
+                                int(p.weights_ready))
+
+    @staticmethod
+    def _weight_grads(items):
+        return _weight_grads_of(tuple(tuple(s.ptr if isinstance(s, DeviceSlice) else s for s in it) for it in items))
+
+    def weight_grads_supported(self, dtype: int, items, rows: int) -> bool:
+        return bool(self.L.zg_weight_grads_supported(dtype, self._weight_grads(items), len(items), rows))
+
+    def weight_grads(self, p):
+        self.L.zg_weight_grads(p.items[0][0].dtype, self.stream, self._weight_grads(p.items), len(p.items), p.rows, p.lr)
 
     def smooth_l1(self, p):
         self.L.zg_smooth_l1_fwd_bwd(p.pred.dtype, self.stream, p.pred.ptr, p.target.ptr, p.pred.len, p.beta, p.loss.ptr,

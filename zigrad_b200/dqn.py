@@ -64,13 +64,15 @@ class DqnTrainer:
     def _step(self, states: DeviceSlice, actions: DeviceSlice, next_states: DeviceSlice, rewards: DeviceSlice, dones: DeviceSlice):
         d, B, C = self.dev, self.B, self.C
         pol, tgt = self.policy, self.target
+        grouped = pol.grouped
         # ---- both forward passes (gradients disabled in the reference for the target net): independent chains of
         # small kernels; zero_grad of the policy net rides on the side stream
         with d.branch(1):
             if tgt._touched:  # (it has no backward pass: only if somebody holds its gradients)
                 tgt.zero_grad()
             qn = tgt._layers(next_states)
-            pol.zero_grad()
+            if not grouped:
+                pol.zero_grad()
         q_all = pol._layers(states)
         d.join()
         # ---- targets, gather by action, loss and its gradient w.r.t. all Q values, last bias gradient
@@ -80,7 +82,10 @@ class DqnTrainer:
                                      self.offsets, self.loss, self.dq, pol.dact[-1], pol._db[-1]))
         else:
             self._head(qn, q_all, actions, rewards, dones)
-        pol.backward(states, last_bias_done=fused)
+        if grouped:
+            pol.backward_grouped(states)
+        else:
+            pol.backward(states, last_bias_done=fused)
         # ---- Adam, and the soft update of the target parameters behind it
         pol.update(soft_target=tgt.params, tau=self.tau)
 

@@ -155,6 +155,9 @@ class MlpTrainer:
             d.cast(self.params, self.params_bf16)
             self.Wb = [self.params_bf16.view(self.segments[2 * l][0], self.segments[2 * l][1]) for l in range(self.L)]
             self.dlogits_bf16 = d.mem_cache_alloc(BF16, self.B * self.ld_out)
+        # Whether the weight gradients of a step go out as one op behind the dX chain (opspec.weight_grads): fused fp32 on few
+        # rows, where the products one by one are launches of 2 to 4 us on forked streams.
+        self.grouped = fused and not bf16 and not self.update_by_layer and d.weight_grads_supported(SINGLE, self._group_items(None, False), self.B)
         d.sync()
 
     # -------------------------------------------------------------- gradients
@@ -331,6 +334,38 @@ class MlpTrainer:
                     self._dw_op(l, dy, a_in)
         d.join()  # the gradients are complete before anything that follows on the main stream
 
+    # ------------------------------------------------- few rows: one launch for all weight gradients
+    def _group_items(self, X: Optional[DeviceSlice], update: bool):
+        keep = not (update and self.zero_grads_in_update)  # the gradients are written unless nobody sees them past the step
+        items = []
+        for l in range(self.L):
+            items.append((self.dact[l], X if l == 0 else self.act[l - 1], self._dW[l] if keep else None, self._db[l] if keep else None,
+                          self.W[l] if update else None, self.b[l] if update else None, self.dims[l + 1], self.dims[l], self.ld[l],
+                          self._ld_in(l)))
+        return items
+
+    def _weight_grads(self, X: DeviceSlice, update: bool):
+        """All weight and bias gradients from dact[] (overwritten, so nothing had to be cleared), and the SGD step."""
+        self.dev.dispatch(opspec.weight_grads(self._group_items(X, update), self.B, self.lr))
+        if update:
+            self._grads_clear = self.zero_grads_in_update
+
+    def backward_grouped(self, X: DeviceSlice, update: bool = False):
+        """backward() from dact[L-1] where `grouped`: the dX chain, then everything else in one launch."""
+        d, B = self.dev, self.B
+        self._touched = True
+        for l in range(self.L - 1, 0, -1):
+            K, N = self.dims[l], self.dims[l + 1]
+            d.dispatch(opspec.linear(self.dact[l], self.W[l], self.dact[l - 1], B, K, N, False, False, self.ld[l], K, self.ld[l - 1], 1.0, 0.0,
+                                     "relu_mask", None, self.act[l - 1]))
+        self._weight_grads(X, update)
+
+    def _clear_unwritten(self, update: bool):
+        """The zero_grad of a grouped step: only where its gradients are not written."""
+        if self._zero_grad_due() and update and self.zero_grads_in_update:
+            self.zero_grad()
+        self._touched = True
+
     def _dw_op(self, l: int, dy: DeviceSlice, a_in: DeviceSlice):
         B, K, N = self.B, self.dims[l], self.dims[l + 1]
         self.dev.dispatch(opspec.bmm_acc(dy, a_in, self._dW[l], (1, N, B), (1, B, K), (1, N, K), True, False, N, K, K, 1.0, 0.0))
@@ -386,7 +421,10 @@ class MlpTrainer:
         layer's product; no update waits for the join of all streams.  The weights of the
         layers in between are still read by the dX products and are updated after the join."""
         d, B, L = self.dev, self.B, self.L
-        if self._zero_grad_due():
+        grouped = self.grouped
+        if grouped:
+            self._clear_unwritten(fuse_update)
+        elif self._zero_grad_due():
             self.zero_grad()
         self._touched = True
 
@@ -412,8 +450,14 @@ class MlpTrainer:
         h1, h2, C = self.dims[L - 2], self.dims[L - 1], self.dims[L]
         d.dispatch(opspec.mlp_tail(self.act[L - 3], self.W[L - 2], self.b[L - 2], self.W[L - 1], self.b[L - 1], T, B, h1, h2, C,
                                    self.ld_out, self.loss_div, self.act[L - 2], self.act[L - 1], self.loss, self.dact[L - 1],
-                                   self.dact[L - 2], self.dact[L - 3], self._db[L - 1], self._db[L - 2], self._db[L - 3],
+                                   self.dact[L - 2], self.dact[L - 3], *([None] * 3 if grouped else [self._db[L - 1], self._db[L - 2], self._db[L - 3]]),
                                    weights_ready=L - 2 >= 1))
+        if grouped:
+            for l in range(L - 3, 0, -1):
+                K, N = self.dims[l], self.dims[l + 1]
+                d.dispatch(opspec.linear(self.dact[l], self.W[l], self.dact[l - 1], B, K, N, False, False, self.ld[l], K, self.ld[l - 1], 1.0, 0.0,
+                                         "relu_mask", None, self.act[l - 1]))
+            return self._weight_grads(X, fuse_update)
         # the weight gradients of the two tail layers are independent of each other and of everything that follows:
         # one side stream each.
         # With one layer in front of the tail, its weight gradient (main stream) runs beside the two of the tail:
@@ -473,6 +517,13 @@ class MlpTrainer:
                 return
         else:
             by_layer = self.update_by_layer and self.fused and self.opt == "adam" and allreduce is None
+            if self.grouped:
+                fuse = self.opt == "sgd" and not self.clip and allreduce is None
+                self._clear_unwritten(fuse)
+                self._layers(X)
+                self.loss_and_grad(T)
+                self.backward_grouped(X, fuse)
+                return None if fuse else self._reduce_and_update(allreduce)
             # The whole step is issued here: of its gradients only those it accumulates into have to be cleared (a fill of
             # all of them is 35 us of the wide network's step, and the additions read the 218 MB once more)
             if self.fused and self._zero_grad_due():
@@ -482,6 +533,9 @@ class MlpTrainer:
             self.backward(X, update_by_layer=by_layer, fresh=self.fused)
             if by_layer:
                 return
+        self._reduce_and_update(allreduce)
+
+    def _reduce_and_update(self, allreduce):
         if allreduce is not None:
             fused = getattr(allreduce, "reduce_and_sgd", None)
             if fused is not None and self.opt == "sgd" and not self.clip:

@@ -462,13 +462,23 @@ class softmax_ce:
     bias_grad: Optional[Any] = None  # [classes]: column sums of the gradient written
 
 
+@_op("weight_grads")
+class weight_grads:
+    """Every layer's weight and bias gradient as one device op (zg_weight_grads): dW = dy^T x and
+    db = column sums of dy over `rows` rows, overwritten; where W and b are given, the SGD step behind them.
+    items: (dy, x, dW, db, W, b, out, in, ld_dy, ld_x) per layer, dW .. b each possibly None."""
+    items: Any
+    rows: int
+    lr: float = 0.0
+
+
 @_op("mlp_tail")
 class mlp_tail:
     """The last two Linear layers of an MLP with their loss and the backward pass
     down to the gradient of the layer before them, as one device op
     (zg_mlp_tail_fwd_bwd): act1 = relu(act0 W1^T + b1), logits = act1 W2^T + b2,
     softmax cross-entropy forward/backward, dact1, dact0 and the three bias
-    gradients (added into db2 / db1 / db0)."""
+    gradients (added into db2 / db1 / db0; all None: left to weight_grads)."""
     act0: Any       # [rows, h1]
     W1: Any         # [h2, h1]
     b1: Any
