@@ -255,6 +255,15 @@ EXTERN_C void zg_mlp_tail_fwd_bwd(dtype id, StreamWrapper stream, len_t rows, le
                                   const void* labels, int label_kind, len_t ld_out, double loss_div,
                                   void* act1, void* logits, void* loss_out, void* dlogits, void* dact1, void* dact0,
                                   void* db2, void* db1, void* db0, int weights_ready);
+/* The same with the classifier's weight gradient: dW2 [C, h2] += dlogits^T act1 (fp32 atomics; NULL: not formed).  For as many
+ * rows as zg_mlp_tail_forms_dw2 says.  db2, db1 and db0 may all be NULL there: a zg_weight_grads call behind this one forms
+ * them. */
+EXTERN_C int zg_mlp_tail_forms_dw2(len_t rows);
+EXTERN_C void zg_mlp_tail_step(dtype id, StreamWrapper stream, len_t rows, len_t h1, len_t h2, len_t C,
+                               const void* act0, const void* W1, const void* b1, const void* W2, const void* b2,
+                               const void* labels, int label_kind, len_t ld_out, double loss_div,
+                               void* act1, void* logits, void* loss_out, void* dlogits, void* dact1, void* dact0,
+                               void* db2, void* db1, void* db0, int weights_ready, void* dW2);
 
 /* -------------------------------------------------------------- optimizers
  * One launch over a whole parameter set.  The tensors of a model live back to

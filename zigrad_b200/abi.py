@@ -211,6 +211,9 @@ SIGNATURES = {
     "zg_mlp_tail_supported": (i32, [dtype_t, len_t, len_t, len_t]),
     "zg_mlp_tail_fwd_bwd": (None, [dtype_t, S, len_t, len_t, len_t, len_t, vp, vp, vp, vp, vp, vp, i32, len_t, dbl,
                                    vp, vp, vp, vp, vp, vp, vp, vp, vp, i32]),
+    "zg_mlp_tail_forms_dw2": (i32, [len_t]),
+    "zg_mlp_tail_step": (None, [dtype_t, S, len_t, len_t, len_t, len_t, vp, vp, vp, vp, vp, vp, i32, len_t, dbl,
+                                   vp, vp, vp, vp, vp, vp, vp, vp, vp, i32] + [vp]),
     "zg_sgd_step": (None, [dtype_t, S, vp, vp, C.POINTER(Segment), len_t, dbl, i32, dbl, dbl, vp, i32]),
     "zg_adam_step": (None, [dtype_t, S, vp, vp, vp, vp, C.POINTER(Segment), len_t, len_t, dbl, dbl, dbl, dbl, i32, dbl, dbl, vp, vp, vp]),
     "zg_adam_step_part": (None, [dtype_t, S, vp, vp, vp, vp, C.POINTER(Segment), len_t, len_t, dbl, dbl, dbl, dbl, i32, dbl, dbl, vp, vp, vp, i32]),

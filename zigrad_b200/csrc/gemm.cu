@@ -635,7 +635,7 @@ static bool launch_tail_rows(cudaStream_t s, const tail_rows::Params& p) {
 
 void mlp_tail_launch(cudaStream_t s, len_t rows, len_t h1, len_t h2, len_t C, const void* act0, const void* W1, const void* b1, const void* W2,
                      const void* b2, const void* labels, int label_kind, len_t ld_out, double loss_div, void* act1, void* logits, void* loss_out,
-                     void* dlogits, void* dact1, void* dact0, void* db2, void* db1, void* db0, int weights_ready) {
+                     void* dlogits, void* dact1, void* dact0, void* db2, void* db1, void* db0, int weights_ready, void* dW2) {
   if (rows == 0) return;
   if (h1 != (len_t)tail::kH1 || h2 != (len_t)tail::kH2 || C == 0 || C > (len_t)tail::kCMax) {
     set_error(kUnsupported, "zg_mlp_tail_fwd_bwd: widths %lu -> %lu -> %lu (built for %d -> %d -> at most %d)", h1, h2, C, tail::kH1, tail::kH2, tail::kCMax);
@@ -654,6 +654,7 @@ void mlp_tail_launch(cudaStream_t s, len_t rows, len_t h1, len_t h2, len_t C, co
   }
   if (ld_out > (len_t)tail::kCMax) { set_error(kBadArgument, "zg_mlp_tail_fwd_bwd: ld_out %lu above %d", ld_out, tail::kCMax); return; }
   const unsigned sms = (unsigned)sm_count();
+  if (dW2 && rows > (len_t)sms * 2 * 28) { set_error(kUnsupported, "zg_mlp_tail_step: dW2 of %lu rows", rows); return; }
   if (rows <= (len_t)sms * 2 * 28) {  // one wave of the row kernel; 16 rows per CTA while 28 would leave SMs idle
     unsigned* counters = nullptr;
     float* partial = static_cast<float*>(workspace(s, sizeof(float) * ((rows + 15) / 16), &counters));
@@ -665,7 +666,7 @@ void mlp_tail_launch(cudaStream_t s, len_t rows, len_t h1, len_t h2, len_t C, co
     p.labels = labels; p.label_index = label_kind == ZG_LABEL_INDEX ? 1 : 0;
     p.act1 = static_cast<float*>(act1); p.dact1 = static_cast<float*>(dact1); p.dact0 = static_cast<float*>(dact0);
     p.logits = static_cast<float*>(logits); p.dlogits = static_cast<float*>(dlogits);
-    p.db2 = static_cast<float*>(db2); p.db1 = static_cast<float*>(db1); p.db0 = static_cast<float*>(db0);
+    p.db2 = static_cast<float*>(db2); p.db1 = static_cast<float*>(db1); p.db0 = static_cast<float*>(db0); p.dW2 = static_cast<float*>(dW2);
     p.loss_out = static_cast<float*>(loss_out); p.loss_partial = partial; p.counter = counters;
     p.rows = (uint32_t)rows; p.C = (uint32_t)C; p.ld_out = (uint32_t)ld_out;
     p.divisor = (float)loss_div; p.inv_divisor = 1.f / p.divisor;
@@ -766,18 +767,26 @@ using namespace zg;
 namespace zg {
 void mlp_tail_launch(cudaStream_t s, len_t rows, len_t h1, len_t h2, len_t C, const void* act0, const void* W1, const void* b1, const void* W2,
                      const void* b2, const void* labels, int label_kind, len_t ld_out, double loss_div, void* act1, void* logits, void* loss_out,
-                     void* dlogits, void* dact1, void* dact0, void* db2, void* db1, void* db0, int weights_ready);
+                     void* dlogits, void* dact1, void* dact0, void* db2, void* db1, void* db0, int weights_ready, void* dW2);
 }
 extern "C" int zg_mlp_tail_supported(dtype id, len_t h1, len_t h2, len_t C) {
   return (id == SINGLE && g_math_mode != ZG_MATH_FFMA && h1 == (len_t)tail::kH1 && h2 == (len_t)tail::kH2 && C >= 1 && C <= (len_t)tail::kCMax) ? 1 : 0;
+}
+extern "C" int zg_mlp_tail_forms_dw2(len_t rows) { return rows <= (len_t)sm_count() * 2 * 28 ? 1 : 0; }
+extern "C" void zg_mlp_tail_step(dtype id, StreamWrapper stream, len_t rows, len_t h1, len_t h2, len_t C, const void* act0, const void* W1,
+                                 const void* b1, const void* W2, const void* b2, const void* labels, int label_kind, len_t ld_out,
+                                 double loss_div, void* act1, void* logits, void* loss_out, void* dlogits, void* dact1, void* dact0,
+                                 void* db2, void* db1, void* db0, int weights_ready, void* dW2) {
+  if (id != SINGLE) { set_error(kUnsupported, "zg_mlp_tail_fwd_bwd: only SINGLE is implemented"); return; }
+  mlp_tail_launch(as_stream(stream), rows, h1, h2, C, act0, W1, b1, W2, b2, labels, label_kind, ld_out, loss_div, act1, logits, loss_out,
+                  dlogits, dact1, dact0, db2, db1, db0, weights_ready, dW2);
 }
 extern "C" void zg_mlp_tail_fwd_bwd(dtype id, StreamWrapper stream, len_t rows, len_t h1, len_t h2, len_t C, const void* act0, const void* W1,
                                     const void* b1, const void* W2, const void* b2, const void* labels, int label_kind, len_t ld_out,
                                     double loss_div, void* act1, void* logits, void* loss_out, void* dlogits, void* dact1, void* dact0,
                                     void* db2, void* db1, void* db0, int weights_ready) {
-  if (id != SINGLE) { set_error(kUnsupported, "zg_mlp_tail_fwd_bwd: only SINGLE is implemented"); return; }
-  mlp_tail_launch(as_stream(stream), rows, h1, h2, C, act0, W1, b1, W2, b2, labels, label_kind, ld_out, loss_div, act1, logits, loss_out,
-                  dlogits, dact1, dact0, db2, db1, db0, weights_ready);
+  zg_mlp_tail_step(id, stream, rows, h1, h2, C, act0, W1, b1, W2, b2, labels, label_kind, ld_out, loss_div, act1, logits, loss_out, dlogits, dact1,
+                   dact0, db2, db1, db0, weights_ready, nullptr);
 }
 
 extern "C" void zg_set_math_mode(int mode) {

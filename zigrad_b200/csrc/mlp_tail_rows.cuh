@@ -48,6 +48,7 @@ struct Params {
   float* db2;             // [C]   column sums are ADDED (the gradient buffer is zero at the start of a step); none: all NULL
   float* db1;             // [64]
   float* db0;             // [128]
+  float* dW2;             // [C, 64] or NULL: dlogits^T act1 is ADDED, too
   float* loss_out;        // one scalar, overwritten
   float* loss_partial;    // workspace: one float per CTA
   unsigned* counter;      // workspace: ticket, zero before and after
@@ -263,6 +264,7 @@ __global__ void __launch_bounds__(kThreads, 2) mlp_tail_rows_kernel(const Params
     for (int h = 0; h < NV; ++h) {
       const int col = 4 * q + h * 4 * L::kLanes;
       *reinterpret_cast<float4*>(dact1s + row * kPitch2 + col) = x[h];
+      if (p.dW2) *reinterpret_cast<float4*>(part + row * kPitch2 + col) = a1[h];
       // column sums over the warp's rows
 #pragma unroll
       for (int o = L::kLanes; o < 32; o <<= 1) {
@@ -283,6 +285,26 @@ __global__ void __launch_bounds__(kThreads, 2) mlp_tail_rows_kernel(const Params
     __threadfence();
     is_last = atomicAdd(p.counter, 1u) == gridDim.x - 1;
     if (is_last) *p.counter = 0;
+  }
+
+  // ---- the classifier's weight gradient, whose operands are both here: a thread per class and four columns.  As a launch of
+  // its own beside the other weight gradients it takes the places of the SMs that the next layer's product waits for: a step of 8192
+  // rows 53.0 -> 47.2 us.
+  if (p.dW2) {
+    const bool wide = aligned16(p.dW2);
+    for (int e = t; e < C * (kH2 / 4); e += kThreads) {
+      const int c = e / (kH2 / 4), col = e % (kH2 / 4) * 4;
+      float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+      for (int r = 0; r < R; ++r) {
+        const float g = dls[r * (CP + 1) + c];
+        const float4 a = *reinterpret_cast<const float4*>(part + r * kPitch2 + col);
+        s.x = fmaf(g, a.x, s.x); s.y = fmaf(g, a.y, s.y); s.z = fmaf(g, a.z, s.z); s.w = fmaf(g, a.w, s.w);
+      }
+      float* dst = p.dW2 + c * kH2 + col;
+      if (wide) atomicAdd(reinterpret_cast<float4*>(dst), s);
+      else { atomicAdd(dst, s.x); atomicAdd(dst + 1, s.y); atomicAdd(dst + 2, s.z); atomicAdd(dst + 3, s.w); }
+    }
   }
 
   // ---- product 2: dact1 W1, masked by act0

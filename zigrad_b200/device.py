@@ -625,10 +625,13 @@ class CudaDevice:
 
     def mlp_tail(self, p):
         kind = abi.LABEL_INDEX if p.labels.dtype == USIZE else abi.LABEL_ONEHOT
-        self.L.zg_mlp_tail_fwd_bwd(p.act0.dtype, self.stream, p.rows, p.h1, p.h2, p.classes, p.act0.ptr, p.W1.ptr, p.b1.ptr, p.W2.ptr,
+        self.L.zg_mlp_tail_step(p.act0.dtype, self.stream, p.rows, p.h1, p.h2, p.classes, p.act0.ptr, p.W1.ptr, p.b1.ptr, p.W2.ptr,
                                 p.b2.ptr, p.labels.ptr, kind, p.ld_out, float(p.loss_div), p.act1.ptr, p.logits.ptr, p.loss.ptr,
                                 p.dlogits.ptr, p.dact1.ptr, p.dact0.ptr, *(b.ptr if b is not None else None for b in (p.db2, p.db1, p.db0)),
-                                int(p.weights_ready))
+                                int(p.weights_ready), p.dW2.ptr if p.dW2 is not None else None)
+
+    def mlp_tail_forms_dw2(self, rows: int) -> bool:
+        return bool(self.L.zg_mlp_tail_forms_dw2(rows))
 
     @staticmethod
     def _weight_grads(items):

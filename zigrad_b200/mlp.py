@@ -74,6 +74,22 @@ def split_sm_shares(sms: int, tiles0: int, tiles1: int, k_slabs: int):
     return best
 
 
+def shares_by_finish(sms: int, tiles0: int, tiles1: int, k_slabs: int, late: int = 4):
+    """Shares of `sms` SMs for the same two products where the second starts behind a fork of the stream, about `late` k-slabs'
+    time (3 us) after the first: those with which the later of the two ends soonest.  At batch 8192 split_sm_shares gives the
+    second 15 SMs, and it ended 4 us after everybody else (with the classifier's
+    gradient out of the way as well, mlp_tail, the step went from 53.0 to 47.2 us)."""
+    best = None
+    for s0 in range(1, sms // tiles0 + 1):
+        s1 = (sms - tiles0 * s0) // tiles1
+        if s1 < 1:
+            break
+        end = max(-(-k_slabs // s0), -(-k_slabs // s1) + late)
+        if best is None or end <= best[0]:
+            best = (end, tiles0 * s0, tiles1 * s1)
+    return best and best[1:]
+
+
 class MlpTrainer:
     def __init__(self, dev: CudaDevice, dims: Sequence[int], batch: int, weights, biases, opt: str = "sgd",
                  lr: float = 0.01, beta1: float = 0.9, beta2: float = 0.999, eps: float = 1e-8, clip: bool = False,
@@ -429,14 +445,16 @@ class MlpTrainer:
         self._touched = True
 
         in_gemm = fuse_update and self.zero_grads_in_update
+        in_tail = not grouped and d.mlp_tail_forms_dw2(B)  # the classifier's weight gradient comes out of the tail op as well
+        by_gemm = (0, L - 2) if in_tail else (0, L - 2, L - 1)  # layers whose update rides in their gradient's product
         nlr = -float(np.float32(self.lr))  # lr cast f64 -> f32, then negated (optim.zig:103)
 
         def target(l):  # (C, alpha) of layer l's weight-gradient product
-            return (self.W[l], nlr) if in_gemm and l in (0, L - 2, L - 1) else (self._dW[l], 1.0)
+            return (self.W[l], nlr) if in_gemm and l in by_gemm else (self._dW[l], 1.0)
 
         def update(segs):
             if in_gemm:
-                segs = [sg for sg in segs if sg not in [self.segments[2 * l] for l in (0, L - 2, L - 1)]]
+                segs = [sg for sg in segs if sg not in [self.segments[2 * l] for l in by_gemm]]
             if fuse_update and segs:
                 d.dispatch(opspec.sgd(self.params, self._grads, segs, self.lr, False, self.max_norm, self.delta, self.norms,
                                       self.zero_grads_in_update))
@@ -451,7 +469,7 @@ class MlpTrainer:
         d.dispatch(opspec.mlp_tail(self.act[L - 3], self.W[L - 2], self.b[L - 2], self.W[L - 1], self.b[L - 1], T, B, h1, h2, C,
                                    self.ld_out, self.loss_div, self.act[L - 2], self.act[L - 1], self.loss, self.dact[L - 1],
                                    self.dact[L - 2], self.dact[L - 3], *([None] * 3 if grouped else [self._db[L - 1], self._db[L - 2], self._db[L - 3]]),
-                                   weights_ready=L - 2 >= 1))
+                                   weights_ready=L - 2 >= 1, dW2=self._dW[L - 1] if in_tail else None))
         if grouped:
             for l in range(L - 3, 0, -1):
                 K, N = self.dims[l], self.dims[l + 1]
@@ -468,11 +486,13 @@ class MlpTrainer:
             d.dispatch(opspec.linear(self.dact[L - 2], self.act[L - 3], Cw, h2, h1, B, True, False, h2, h1, h1, a, 1.0,
                                      sm_budget=share.get(L - 2, 0)))
             update([weight(L - 2)])
-        with d.branch(1):
-            Cw, a = target(L - 1)
-            d.dispatch(opspec.linear(self.dact[L - 1], self.act[L - 2], Cw, C, h2, B, True, False, self.ld_out, h2, h2, a, 1.0))
-            # the tail op wrote the bias gradients of its two layers and of the layer in front of it
-            update([weight(L - 1)] + [bias(l) for l in (L - 3, L - 2, L - 1)])
+        if fuse_update or not in_tail:
+            with d.branch(1):
+                if not in_tail:
+                    Cw, a = target(L - 1)
+                    d.dispatch(opspec.linear(self.dact[L - 1], self.act[L - 2], Cw, C, h2, B, True, False, self.ld_out, h2, h2, a, 1.0))
+                # the tail op wrote the bias gradients of its two layers and of the layer in front of it
+                update([weight(L - 1)] + [bias(l) for l in (L - 3, L - 2, L - 1)])
         for l in range(L - 3, -1, -1):
             K, N = self.dims[l], self.dims[l + 1]
             a_in = X if l == 0 else self.act[l - 1]
@@ -496,7 +516,7 @@ class MlpTrainer:
         layer's output is a few rows and goes to a small FFMA kernel that fits beside the others)."""
         if self._dw_shares is None:
             t0, t1 = (-(-self.dims[l + 1] // 128) * -(-self.dims[l] // 128) for l in (0, 1))
-            best = split_sm_shares(self.dev.sm_count(), t0, t1, -(-self.B // 32))
+            best = shares_by_finish(self.dev.sm_count(), t0, t1, -(-self.B // 32))
             self._dw_shares = {0: best[0], 1: best[1]} if best else {}
         return self._dw_shares
 

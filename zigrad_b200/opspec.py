@@ -501,6 +501,7 @@ class mlp_tail:
     db1: Any
     db0: Any
     weights_ready: bool = False
+    dW2: Any = None  # added to where the device forms it (mlp_tail_forms_dw2)
 
 
 @_op("smooth_l1")
