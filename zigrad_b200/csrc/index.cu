@@ -118,36 +118,42 @@ __device__ __forceinline__ float csr_add(float acc, float (&v)[NE * FW / 32], fl
   return acc;
 }
 
+// Rows of up to kShortRow neighbours -- most, of a graph with a handful of edges per node -- are taken FW / 4 lanes each, so
+// that a warp has 4 to 16 of them in flight and a graph of 20011 nodes starts all of its chains (row bounds, neighbours, their
+// features) at once instead of two or three per warp one after the other; a lane adds its four features up in edge order.
+// The longer ones are dealt to the CTA's warps, a row each (a warp's own 8 or 16 rows hold up to half a dozen of them).
+constexpr int kShortRow = 8, kMiddleQueue = 512;
 constexpr int kHubRow = 64, kHubQueue = 64, kGatherWarps = kIThreads / 32 - 1;
 
-template <int FW>
+// VEC: rows of x hold whole 16-byte words at aligned addresses, and F fits into FW
+template <int FW, bool VEC>
 __global__ void __launch_bounds__(kIThreads) csr_gcn_propagate_kernel(float* out, const float* __restrict__ x, const float* __restrict__ deg,
                                                                       const len_t* __restrict__ row_ptr, const len_t* __restrict__ col,
                                                                       size_t n_rows, size_t F, size_t ld_x, size_t ld_out, int mode,
                                                                       int epilogue, const float* __restrict__ bias) {
   constexpr int EW = FW == 32 ? 16 : 32, kBatch = kGatherWarps * EW;  // neighbours per gathering warp, per batch
   __shared__ float batch[2][kBatch][FW];
-  __shared__ uint32_t queue[kHubQueue];
-  __shared__ unsigned queued;
-  if (threadIdx.x == 0) queued = 0;
+  __shared__ uint32_t queue[kHubQueue], middle[VEC ? kMiddleQueue : 1];
+  __shared__ unsigned queued, waiting;
+  if (threadIdx.x == 0) queued = waiting = 0;
   __syncthreads();
   pdl_sync();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane / FW, jl = lane % FW;
-  const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
+  const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5, first = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   auto store = [&](size_t r, size_t j, float acc) {
     if (epilogue == ZG_EPI_BIAS || epilogue == ZG_EPI_BIAS_RELU) acc += bias[j];
     if (epilogue == ZG_EPI_BIAS_RELU) acc = acc > 0.f ? acc : 0.f;
     out[r * ld_out + j] = acc;
   };
-  for (size_t r = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n_rows; r += warps) {
-    const len_t k0 = __ldg(row_ptr + r), k1 = __ldg(row_ptr + r + 1);
+  // a row by the whole warp, or onto the CTA's queue
+  auto whole_row = [&](size_t r, len_t k0, len_t k1) {
     if (k1 - k0 > kHubRow) {
       unsigned at = 0;
       if (lane == 0) at = atomicAdd(&queued, 1u);
       at = __shfl_sync(0xffffffffu, at, 0);
       if (at < kHubQueue) {
         if (lane == 0) queue[at] = (uint32_t)r;
-        continue;
+        return;
       }
     }
     const float dr = __ldg(deg + r);
@@ -165,6 +171,71 @@ __global__ void __launch_bounds__(kIThreads) csr_gcn_propagate_kernel(float* out
       }
       if (jok && g == 0) store(r, j0 + jl, acc);
     }
+  };
+  if constexpr (VEC) {
+    constexpr int LW = FW / 4, RW = 32 / LW;  // lanes per row, rows per warp
+    const int sub = lane % LW;
+    for (size_t r0 = first * RW; r0 < n_rows; r0 += warps * RW) {
+      const size_t r = r0 + lane / LW;
+      const bool in = r < n_rows;
+      const len_t k0 = in ? __ldg(row_ptr + r) : 0, k1 = in ? __ldg(row_ptr + r + 1) : 0;
+      const int n = k1 - k0 <= kShortRow ? (int)(k1 - k0) : 0;
+      const float dr = in ? __ldg(deg + r) : 0.f;
+      const size_t j = 4 * sub < F ? 4 * sub : 0;  // (lanes past the last word read the first one)
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int e = 0; e < kShortRow; e += 4) {
+        if (!__any_sync(0xffffffffu, e < n)) break;
+        uint32_t c[4];
+        float d[4];
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) c[u] = e + u < n ? (uint32_t)__ldg(col + k0 + e + u) : 0u;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          d[u] = __ldg(deg + c[u]);
+          v[u] = __ldg(reinterpret_cast<const float4*>(x + (size_t)c[u] * ld_x + j));
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (e + u >= n) continue;
+          if (mode == 0) {
+            const float s = d[u] * dr;
+            acc.x += s * v[u].x; acc.y += s * v[u].y; acc.z += s * v[u].z; acc.w += s * v[u].w;
+          } else {
+            acc.x += (v[u].x * dr) * d[u]; acc.y += (v[u].y * dr) * d[u]; acc.z += (v[u].z * dr) * d[u]; acc.w += (v[u].w * dr) * d[u];
+          }
+        }
+      }
+      if (in && k1 - k0 <= kShortRow) {
+        if (4 * sub + 0 < F) store(r, 4 * sub + 0, acc.x);
+        if (4 * sub + 1 < F) store(r, 4 * sub + 1, acc.y);
+        if (4 * sub + 2 < F) store(r, 4 * sub + 2, acc.z);
+        if (4 * sub + 3 < F) store(r, 4 * sub + 3, acc.w);
+      }
+      bool longer = in && sub == 0 && k1 - k0 > kShortRow;
+      if (longer) {  // for whichever warp of the CTA is free
+        const unsigned at = atomicAdd(&waiting, 1u);
+        if (at < kMiddleQueue) {
+          middle[at] = (uint32_t)r;
+          longer = false;
+        }
+      }
+      unsigned rest = __ballot_sync(0xffffffffu, longer);
+      while (rest) {
+        const int from = __ffs(rest) - 1;
+        rest &= rest - 1;
+        whole_row(r0 + from / LW, __shfl_sync(0xffffffffu, k0, from), __shfl_sync(0xffffffffu, k1, from));
+      }
+    }
+    __syncthreads();
+    const unsigned n = waiting < kMiddleQueue ? waiting : kMiddleQueue;
+    for (unsigned i = warp; i < n; i += kIThreads / 32) {
+      const size_t r = middle[i];
+      whole_row(r, __ldg(row_ptr + r), __ldg(row_ptr + r + 1));
+    }
+  } else {
+    for (size_t r = first; r < n_rows; r += warps) whole_row(r, __ldg(row_ptr + r), __ldg(row_ptr + r + 1));
   }
   __syncthreads();
   const unsigned hubs = queued < kHubQueue ? queued : kHubQueue;
@@ -177,11 +248,15 @@ __global__ void __launch_bounds__(kIThreads) csr_gcn_propagate_kernel(float* out
       const float* xj = x + j0 + (jok ? jl : 0);
       float acc = 0.f;
       const len_t rounds = (k1 - k0 + kBatch - 1) / kBatch;
+      // (the neighbours of a batch are on their way during the batch before: a gather waits for one round trip, not two)
+      auto neighbour = [&](len_t kc) { return (warp > 0 && lane < EW && kc + lane < k1) ? (uint32_t)__ldg(col + kc + lane) : 0u; };
+      uint32_t next = neighbour(k0 + (warp - 1) * EW);
       for (len_t i = 0; i <= rounds; ++i) {
         if (warp > 0) {
           const len_t kc = k0 + i * kBatch + (warp - 1) * EW;
           if (i < rounds && kc < k1) {
-            const uint32_t c = (lane < EW && kc + lane < k1) ? (uint32_t)__ldg(col + kc + lane) : 0u;
+            const uint32_t c = next;
+            next = neighbour(kc + kBatch);
             const float dc = __ldg(deg + c);
             constexpr int N = EW * FW / 32, G = 32 / FW;
             float v[N];
@@ -345,8 +420,12 @@ extern "C" void zg_csr_gcn_propagate(dtype id, StreamWrapper w, void* out, const
   if (epilogue != ZG_EPI_NONE && !bias) { set_error(kBadArgument, "zg_csr_gcn_propagate: bias epilogue without bias"); return; }
   if (n_rows > 0xffffffffu) { set_error(kBadArgument, "zg_csr_gcn_propagate: %lu rows", n_rows); return; }
   // lane groups as wide as the feature row: 8 features take 4 neighbours per step, 32 one
-  auto kern = n_feat <= 8 ? csr_gcn_propagate_kernel<8> : (n_feat <= 16 ? csr_gcn_propagate_kernel<16> : csr_gcn_propagate_kernel<32>);
-  launch_pdl(kern, dim3(grid_for(n_rows, kIThreads / 32)), dim3(kIThreads), 0, as_stream(w), (float*)out, (const float*)x,
+  const bool vec = n_feat <= 32 && ld_x % 4 == 0 && ld_x >= (n_feat + 3) / 4 * 4 && host_aligned16(x);
+  auto kern = n_feat <= 8 ? (vec ? csr_gcn_propagate_kernel<8, true> : csr_gcn_propagate_kernel<8, false>)
+                          : (n_feat <= 16 ? (vec ? csr_gcn_propagate_kernel<16, true> : csr_gcn_propagate_kernel<16, false>)
+                                          : (vec ? csr_gcn_propagate_kernel<32, true> : csr_gcn_propagate_kernel<32, false>));
+  const size_t per_warp = vec ? (n_feat <= 8 ? 16 : (n_feat <= 16 ? 8 : 4)) : 1;
+  launch_pdl(kern, dim3(grid_for(n_rows, kIThreads / 32 * per_warp)), dim3(kIThreads), 0, as_stream(w), (float*)out, (const float*)x,
              (const float*)deg, row_ptr, col_idx, (size_t)n_rows, (size_t)n_feat, (size_t)ld_x, (size_t)ld_out, transpose_form ? 1 : 0, epilogue,
              (const float*)bias);
 }
