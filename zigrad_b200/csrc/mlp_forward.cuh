@@ -5,7 +5,7 @@
 // in registers (they do not depend on the layer before, so the first ones of the next layer are requested before the
 // cluster meets), and the result goes straight into the shared memory of all eight CTAs.
 // Bound by the chain (two cluster barriers and three reductions) and, as the weights grow, by what eight SMs can read.
-// Measured, one row, against the chain: 784-128-64-10 6.0 us (9.1), 64-64-10 3.7 (5.0), 256-256-256-256-10 10.3 (10.9), 512-512-10 7.2
+// Measured, one row, against the chain: 784-128-64-10 5.5 us (9.1), 64-64-10 3.7 (5.0), 256-256-256-256-10 9.7 (10.9), 512-512-10 7.2
 // (6.9).  More rows cost it a microsecond each and the chain nothing (784-128-64-10, 2 rows: 8.0 and 9.0; 4: 9.4 and 9.2).
 #pragma once
 
@@ -35,7 +35,10 @@ struct Params {
   Layer l[kMaxLayers];
 };
 
-__device__ __forceinline__ void fetch(float4 (&w)[kQuads], const Layer& L, uint32_t n, uint32_t k0, int lane) {
+// The weights of output n from k0 on; with the first of them its bias, which would otherwise be a round trip of its own behind
+// each of the cluster's barriers (784-128-64-10 5.7 -> 5.5 us, 256-256-256-256-10 10.1 -> 9.7)
+__device__ __forceinline__ void fetch(float4 (&w)[kQuads], float& bias, const Layer& L, uint32_t n, uint32_t k0, int lane) {
+  if (k0 == 0) bias = __ldg(L.b + n);
   const float* row = L.W + (size_t)n * L.K;
 #pragma unroll
   for (int j = 0; j < kQuads; ++j) {
@@ -63,7 +66,8 @@ static __global__ void __launch_bounds__(kThreads) mlp_forward_kernel(const __gr
   for (uint32_t i = p.l[0].K + threadIdx.x; i < last.at + (last.K + 3) / 4 * 4; i += kThreads) in[i] = 0.f;  // for the words past a row's end
   pdl_sync();
   float4 w[kQuads];
-  if (first < p.l[0].N) fetch(w, p.l[0], first, 0, lane);
+  float next_bias = 0.f;
+  if (first < p.l[0].N) fetch(w, next_bias, p.l[0], first, 0, lane);
   for (uint32_t i = threadIdx.x; i < p.l[0].K; i += kThreads) in[i] = p.X[i];
   cluster.sync();  // all inputs are in place, and the other CTAs run
   for (int l = 0; l < p.layers; ++l) {
@@ -72,7 +76,7 @@ static __global__ void __launch_bounds__(kThreads) mlp_forward_kernel(const __gr
     const float* x = in + L.at;
     for (uint32_t n = first; n < L.N; n += kStep) {
       float acc = 0.f;
-      const float bias = __ldg(L.b + n);
+      const float bias = next_bias;
       for (uint32_t k0 = 0; k0 < L.K; k0 += kChunk) {
 #pragma unroll
         for (int j = 0; j < kQuads; ++j) {
@@ -86,9 +90,9 @@ static __global__ void __launch_bounds__(kThreads) mlp_forward_kernel(const __gr
           }
         }
         // the next weights: of this row, of this warp's next output, or of its first one in the next layer
-        if (k0 + kChunk < L.K) fetch(w, L, n, k0 + kChunk, lane);
-        else if (n + kStep < L.N) fetch(w, L, n + kStep, 0, lane);
-        else if (!end && first < p.l[l + 1].N) fetch(w, p.l[l + 1], first, 0, lane);
+        if (k0 + kChunk < L.K) fetch(w, next_bias, L, n, k0 + kChunk, lane);
+        else if (n + kStep < L.N) fetch(w, next_bias, L, n + kStep, 0, lane);
+        else if (!end && first < p.l[l + 1].N) fetch(w, next_bias, p.l[l + 1], first, 0, lane);
       }
       float v = warp_sum(acc) + bias;
       if (!end) {
@@ -98,7 +102,7 @@ static __global__ void __launch_bounds__(kThreads) mlp_forward_kernel(const __gr
       if (lane == kCluster) L.out[n] = v;
     }
     if (!end) {
-      if (first >= L.N && first < p.l[l + 1].N) fetch(w, p.l[l + 1], first, 0, lane);
+      if (first >= L.N && first < p.l[l + 1].N) fetch(w, next_bias, p.l[l + 1], first, 0, lane);
       cluster.sync();
     }
   }
