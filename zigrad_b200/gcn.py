@@ -76,20 +76,23 @@ class GcnTrainer:
             self.segments.append((off, n))
             off += n
         self.params = d.from_numpy(flat)
-        self.grads = d.mem_cache_alloc(SINGLE, off)
+        # the gradients and, behind them, the gradient of the logits: what a step clears
+        at = -(-off // 64) * 64
+        self.cleared = d.mem_cache_alloc(SINGLE, at + N * Cp)
+        self.grads, self.dlog = self.cleared.view(0, off), self.cleared.view(at, N * Cp)
         self.m, self.v = d.mem_cache_alloc(SINGLE, off), d.mem_cache_alloc(SINGLE, off)
         self.norms = d.mem_cache_alloc(SINGLE, 4)
         self.t_dev = d.from_numpy(np.zeros(1, np.uint64))  # Adam's counter on the device (graph-replay safe)
-        for s in (self.grads, self.m, self.v):
+        for s in (self.cleared, self.m, self.v):
             d.mem_fill(s, 0.0)
         v = lambda buf, i: buf.view(self.segments[i][0], self.segments[i][1])
         self.W1, self.b1, self.W2, self.b2 = (v(self.params, i) for i in range(4))
         self.dW1, self.db1, self.dW2, self.db2 = (v(self.grads, i) for i in range(4))
         alloc = lambda n: d.mem_cache_alloc(SINGLE, n)
         self.h1, self.a1, self.h2, self.logits = alloc(N * H), alloc(N * H), alloc(N * Cp), alloc(N * Cp)
-        self.dlog, self.dh2, self.da1, self.dh1 = alloc(N * Cp), alloc(N * Cp), alloc(N * H), alloc(N * H)
+        self.dh2, self.da1, self.dh1 = alloc(N * Cp), alloc(N * H), alloc(N * H)
         self.mlog, self.dm = alloc(M * Cp), alloc(M * Cp)
-        for s in (self.h2, self.logits, self.dlog, self.dh2, self.mlog, self.dm):
+        for s in (self.h2, self.logits, self.dh2, self.mlog, self.dm):
             d.mem_fill(s, 0.0)
         # MaskLayer as flat offsets: row r of the mask -> Cp consecutive elements of node mask_idx[r]
         offs = (np.asarray(mask_idx, np.uint64)[:, None] * np.uint64(Cp) + np.arange(Cp, dtype=np.uint64)[None, :]).ravel()
@@ -131,18 +134,24 @@ class GcnTrainer:
 
     def _step(self, T_masked: DeviceSlice):
         d, N, F, H, C, Fp, Cp, M = self.dev, self.N, self.F, self.H, self.C, self.Fp, self.Cp, self.M
-        # zero_grad (model.zig:49-54) and the zero gradient the MaskLayer backward scatters into: nothing in
-        # the forward pass needs them, so the two fills run on a side stream beside it
-        with d.branch(1):
-            d.mem_fill(self.grads, 0.0)
-            d.mem_fill(self.dlog, 0.0)
+        # zero_grad (model.zig:49-54) and the zero gradient the MaskLayer backward scatters into, one fill.  Nothing in the
+        # forward pass needs them, but while the fill is small the fork and the join, which keeps the loss from being launched
+        # while the last propagation still runs, cost more than it does: 0.16 MB 49.5 us a step in front of the forward pass,
+        # 51.3 beside it; 1.5 MB 82.5 and 82.2; 3 MB 98.5 and 96.6.
+        beside = self.cleared.nbytes > 1 << 20
+        if beside:
+            with d.branch(1):
+                d.mem_fill(self.cleared, 0.0)
+        else:
+            d.mem_fill(self.cleared, 0.0)
         # ---- forward
         self._mm(self.X, self.W1, self.h1, N, H, F, False, True, Fp, Fp, H)                       # h1 = X . W1^T
         self._prop(self.h1, self.a1, H, H, "bias_relu", self.b1)                                   # relu(A.h1 + b1)
         self._mm(self.a1, self.W2, self.h2, N, C, H, False, True, H, H, Cp)                       # h2 = a1 . W2^T
         self._prop(self.h2, self.logits, C, Cp, "bias", self.b2)                                   # A.h2 + b2
         # ---- mask rows, loss, gradient of the masked logits (+ db2 = its column sums)
-        d.join()  # the cleared gradient buffers
+        if beside:
+            d.join()
         if d.masked_softmax_ce_supported(SINGLE, M, C):
             d.dispatch(opspec.masked_softmax_ce(self.logits, self.offsets, T_masked, M, C, Cp, self.loss, self.dlog, float(M), self.db2))
         else:
@@ -183,6 +192,6 @@ class GcnTrainer:
         d.sync()
         self._graphs.clear()
         extra = list(self.csr) + [self.deg] if self.sparse else [self.A]
-        for s in extra + [self.mask_rows, self.X, self.params, self.grads, self.m, self.v, self.norms, self.h1, self.a1, self.h2, self.logits,
-                  self.dlog, self.dh2, self.da1, self.dh1, self.mlog, self.dm, self.offsets, self.loss, self.t_dev]:
+        for s in extra + [self.mask_rows, self.X, self.params, self.cleared, self.m, self.v, self.norms, self.h1, self.a1, self.h2, self.logits,
+                  self.dh2, self.da1, self.dh1, self.mlog, self.dm, self.offsets, self.loss, self.t_dev]:
             d.mem_cache_free(s)
