@@ -6,6 +6,7 @@
 #include <cmath>
 #include <cstring>
 
+#include <cooperative_groups.h>
 #include "common.cuh"
 #include "async_copy.cuh"
 #include "../../include/nn_conflux.h"
@@ -1103,12 +1104,149 @@ static void launch_smce_rows_staged(cudaStream_t s, SmceArgs a) {
   launch_pdl(kern, dim3(g), dim3(kRowThreads), smem, s, a);
 }
 
+// Few rows of at most 128 classes: G lanes per row, ITEMS values each, and one cluster for the whole call.  What such a call
+// takes on the kernels for the whole chip is their chain of round trips (4 to 7 us for a few KB).  Here the next row's values and labels are in flight during this
+// one's sums, everything stays in registers, and the partial sums of the loss and the bias gradient meet in shared memory
+// over one cluster barrier instead of through memory, a fence, a ticket and the last CTA's loads.
+// MASKED: row r is the one that starts at logits + offsets[r * ld_offsets], and its gradient is added there (rows may repeat).
+constexpr int kCeThreads = 1024, kCeCluster = 8;
+template <int G, int ITEMS, bool INDEX_LABELS, bool MASKED>
+__global__ void __launch_bounds__(kCeThreads) ce_cluster_kernel(const SmceArgs a, const len_t* __restrict__ offsets, size_t ld_offsets) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  constexpr int W = kCeThreads / 32, CM = G * ITEMS;
+  __shared__ float part[W][CM + 1], sums[CM + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = lane % G, C = a.C;
+  const size_t step = (size_t)gridDim.x * (kCeThreads / G);
+  size_t base = (size_t)blockIdx.x * (kCeThreads / G) + warp * (32 / G);  // the warp's first row: its lanes stay together
+  pdl_sync();
+  float nx[ITEMS], nt[ITEMS], sum[ITEMS], loss = 0.f;
+  size_t n_at = 0;
+  int n_lab = -1;
+  auto fetch = [&](size_t r) {
+    if (r >= a.rows) return;
+    n_at = MASKED ? (size_t)__ldg(offsets + r * ld_offsets) : r * a.ld;
+    if constexpr (INDEX_LABELS) {
+      const len_t l = static_cast<const len_t*>(a.labels)[r];
+      n_lab = l < (len_t)C ? (int)l : -1;
+    }
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      const int c = c0 + G * i;
+      if (c >= C) continue;
+      if (!MASKED) nx[i] = a.logits[n_at + c];
+      if (!INDEX_LABELS) nt[i] = static_cast<const float*>(a.labels)[r * (size_t)C + c];
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) nx[i] = nt[i] = sum[i] = 0.f;
+  fetch(base + lane / G);
+  for (; base < a.rows; base += step) {
+    const size_t r = base + lane / G, at = n_at;
+    const bool row = r < a.rows;
+    const int lab = n_lab;
+    float x[ITEMS], t[ITEMS], mx = -INFINITY, se = 0.f;
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      const int c = c0 + G * i;
+      x[i] = !row || c >= C ? -INFINITY : (MASKED ? a.logits[at + c] : nx[i]);
+      t[i] = INDEX_LABELS ? (c == lab ? 1.f : 0.f) : nt[i];
+    }
+    fetch(r + step);
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) mx = fmaxf(mx, x[i]);
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    float d[ITEMS];
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      d[i] = x[i] - mx;
+      x[i] = row && c0 + G * i < C ? fast_exp(d[i]) : 0.f;
+      se += x[i];
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
+    if (!row) continue;
+    const float inv = 1.f / se, lse = logf(se);
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      const int c = c0 + G * i;
+      if (c >= C) continue;
+      const float p = x[i] * inv;
+      if (t[i] != 0.f) loss -= t[i] * clamp_logp(d[i] - lse);
+      const float g = grad_scale<false>(a, p - t[i]);
+      sum[i] += g;
+      if constexpr (MASKED) atomicAdd(a.dlogits + at + c, g);
+      else {
+        if (a.probs_out) a.probs_out[at + c] = p;
+        if (a.dlogits) a.dlogits[at + c] = a.accumulate ? a.dlogits[at + c] + g : g;
+      }
+    }
+  }
+  loss = warp_sum(loss);
+  if (lane == 0) part[warp][CM] = loss;
+  if (a.dbias) {
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+#pragma unroll
+      for (int o = 16; o >= G; o >>= 1) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], o);
+      if (lane < G) part[warp][c0 + G * i] = sum[i];
+    }
+  }
+  __syncthreads();
+  const int j = CM - (int)threadIdx.x;  // thread 0: the loss
+  const bool mine = j == CM || (j >= 0 && j < C && a.dbias);
+  if (mine) {
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < W; ++w) s += part[w][j];
+    sums[j] = s;
+  }
+  if (gridDim.x > 1) cluster.sync();
+  if (blockIdx.x == 0 && mine) {
+    float v[kCeCluster], s = 0.f;
+#pragma unroll
+    for (unsigned k = 0; k < kCeCluster; ++k) v[k] = k < gridDim.x ? *cluster.map_shared_rank(&sums[j], k) : 0.f;
+#pragma unroll
+    for (unsigned k = 0; k < kCeCluster; ++k) s += v[k];
+    if (j < CM) a.dbias[j] = s;
+    else if (a.loss_out) *a.loss_out = s / a.divisor;
+  }
+  if (gridDim.x > 1) cluster.sync();  // nobody leaves while its sums may still be read
+}
+
+// Up to how many trips of the cluster (1024 rows of 8 classes, 512 of 16, else 256) its serial chain, 2.8 us and 0.8 to 1.5
+// a trip, is shorter than a launch over the whole chip.  With onehot labels and no bias gradient / with it, us, chip -> cluster:
+//   64 x 10    3.5 -> 2.2 / 4.0 -> 2.2    2500 x 7    5.3 -> 4.4 / 6.2 -> 4.5    1500 x 16   6.5 -> 4.4 / 7.2 -> 4.5
+//   600 x 20   4.6 -> 4.6 / 6.7 -> 4.7    300 x 37    4.3 -> 4.2 / 5.8 -> 4.5    1000 x 37   4.8 -> 6.3 / 6.7 -> 6.5
+//   140 x 128  4.7 -> 3.9 / 5.5 -> 3.7    300 x 100   5.0 -> 5.5 / 6.2 -> 5.6    4000 x 7    5.3 -> 5.4 / 6.4 -> 5.5
+// masked (whose kernel for the whole chip is slower):  140 x 7 4.4 -> 2.8   1000 x 7 5.4 -> 3.0   8000 x 7 9.9 -> 9.1
+//   2500 x 16  7.0 -> 6.5, 4000 8.1 -> 9.0   1500 x 20 7.7 -> 7.8   2500 x 37 14.2 -> 12.3, 4000 14.6 -> 17.6   2500 x 128 35 -> 17
+template <bool MASKED>
+static size_t ce_cluster_trips(int C, bool bias) {
+  if (MASKED) return C <= 8 ? 8 : (C <= 32 ? 5 : (C <= 64 ? 10 : 16));
+  return C <= 8 ? 3 : (C <= 16 ? 4 : (bias ? (C <= 64 ? 4 : 2) : (C <= 64 ? 2 : 1)));
+}
+template <bool IDX, bool MASKED>
+static bool launch_ce_cluster(cudaStream_t s, const SmceArgs& a, const len_t* offsets, size_t ld_offsets) {
+  const size_t lanes = a.C <= 8 ? 8 : (a.C <= 16 ? 16 : 32), per_cta = kCeThreads / lanes;
+  if (a.C > 128 || a.rows > ce_cluster_trips<MASKED>(a.C, a.dbias != nullptr) * kCeCluster * per_cta) return false;
+  const unsigned n = (unsigned)std::min<size_t>((a.rows + per_cta - 1) / per_cta, kCeCluster);
+  auto* kernel = a.C <= 8 ? ce_cluster_kernel<8, 1, IDX, MASKED>
+               : a.C <= 16 ? ce_cluster_kernel<16, 1, IDX, MASKED>
+               : a.C <= 32 ? ce_cluster_kernel<32, 1, IDX, MASKED>
+               : a.C <= 64 ? ce_cluster_kernel<32, 2, IDX, MASKED> : ce_cluster_kernel<32, 4, IDX, MASKED>;
+  launch_pdl_cluster(kernel, dim3(n), dim3(kCeThreads), 0, s, n, a, offsets, ld_offsets);
+  return true;
+}
+
 template <bool IDX>
 static void launch_softmax_ce(cudaStream_t s, SmceArgs a) {
   const int C = a.C;
   int e = 0;
   a.inv_divisor = 1.f / a.divisor;
   a.exact_inv = (std::frexp(a.divisor, &e) == 0.5f && std::isnormal(a.inv_divisor)) ? 1 : 0;
+  if (launch_ce_cluster<IDX, false>(s, a, nullptr, 0)) return;
   const bool fast = a.exact_inv && a.dlogits && !a.accumulate && !a.probs_out;
 #define ZG_ROWS(CPV) return fast ? launch_smce_rows<CPV, IDX, true>(s, a) : launch_smce_rows<CPV, IDX, false>(s, a)
 #define ZG_WARPS(I, R) return fast ? launch_smce_warps<I, R, IDX, true>(s, a) : launch_smce_warps<I, R, IDX, false>(s, a)
@@ -1135,9 +1273,9 @@ static void launch_softmax_ce(cudaStream_t s, SmceArgs a) {
       return launch_smce_rows_staged<32>(s, a);
     }
   }
-  // Few rows: a row per warp, spread over the chip.  Several rows per warp leave most SMs idle and are a longer chain (1000 x
-  // 37 with bias gradient 9.9 us against 6.7, 512 x 300 22 against 8.6, 1000 x 500 42 against 13); so is a thread per row
-  // (100 x 10 5.0 against 3.5, 1000 x 10 5.5 against 4.6) unless the bias gradient, cheap there, is wanted (equal).
+  // Still few rows: a row per warp, spread over the chip.  Several rows per warp leave most SMs idle and are a longer chain (1000
+  // x 37 with bias gradient 9.9 us against 6.7, 512 x 300 22 against 8.6, 1000 x 500 42 against 13); so is a thread per row
+  // (1000 x 20 7.5 against 4.6) unless the bias gradient, cheap there, is wanted (equal).
   // Large CTAs, because the last one folds a partial bias gradient per CTA.
   if (a.rows <= (size_t)sm_count() * 8 && C <= 512 && (C > 32 || !a.dbias)) {
     if (C <= 32) return launch_smce_warps<1, 1, IDX, false, 1024>(s, a);
@@ -1270,6 +1408,11 @@ extern "C" void zg_masked_softmax_ce(dtype id, StreamWrapper w, const void* logi
   if (!zg_masked_softmax_ce_supported(id, rows, C) || ld < C || ld > 0xffffffffu) { set_error(kUnsupported, "zg_masked_softmax_ce: %lu rows of %lu (stride %lu)", rows, C, ld); return; }
   if (label_kind != ZG_LABEL_ONEHOT && label_kind != ZG_LABEL_INDEX) { set_error(kBadArgument, "zg_masked_softmax_ce: unknown label kind %d", label_kind); return; }
   cudaStream_t s = as_stream(w);
+  SmceArgs few;
+  memset(&few, 0, sizeof(few));
+  few.logits = (const float*)logits; few.labels = labels; few.rows = rows; few.C = (int)C; few.divisor = (float)divisor;
+  few.loss_out = (float*)loss; few.dlogits = (float*)dlogits; few.dbias = (float*)dbias;
+  if (label_kind == ZG_LABEL_INDEX ? launch_ce_cluster<true, true>(s, few, offsets, ld) : launch_ce_cluster<false, true>(s, few, offsets, ld)) return;
   const unsigned g = grid_for(rows, kLThreads / 32, 2);
   unsigned* counters = nullptr;
   float* partial = static_cast<float*>(workspace(s, sizeof(float) * g * (C + 1), &counters));
