@@ -19,16 +19,19 @@ Two op sequences produce the same tensors:
   the side stream: at batch 100 the fills were 8 of 27 launches of about 2.5 us each.
   A second ``backward()`` therefore gives the same gradients, as it did with the fills.
 * ``fused=True``  -- one zero fill of the flat gradient buffer per forward pass (a second
-  ``backward()`` behind it accumulates), ``linear`` ops
+  ``backward()`` behind it accumulates; ``step()`` clears only what it accumulates into and
+  writes the gradients of large weights), ``linear`` ops
   with bias / ReLU / ReLU-mask epilogues, bias gradients taken from the loss
   kernel (last layer) and from the dX GEMM epilogues (hidden layers): 10 kernel
   launches + 1 memset for the three-layer model.  When the last two layers have
   the widths the ``mlp_tail`` op is built for (128 -> 64 -> at most 16 classes:
   the MNIST model), ``step()`` replaces everything between the first layer's
-  forward GEMM and the weight gradients by that one op; with plain SGD and no
-  reduction between backward and update the weight updates then ride in the
-  gradient GEMMs' epilogues (``fuse_update``): 6 launches per step (forward
-  GEMM, tail, three independent weight-gradient GEMMs, the biases' update).
+  forward GEMM and the weight gradients by that one op, which where it can
+  (``mlp_tail_forms_dw2``) forms the classifier's weight gradient as well; with plain SGD and no
+  reduction between backward and update the updates of the other two weights then ride in their
+  gradient GEMMs' epilogues (``fuse_update``): 5 launches per step (forward
+  GEMM, tail, two weight-gradient GEMMs, the update of the last layer and the biases).
+  On few rows (``grouped``) all weight gradients, the biases' and the SGD step are one launch: 3 per step.
 
 Parameters, gradients and optimizer state live in flat buffers in attach
 order (W0, b0, W1, b1, ...), which is what a data-parallel step all-reduces
@@ -36,6 +39,7 @@ order (W0, b0, W1, b1, ...), which is what a data-parallel step all-reduces
 """
 from __future__ import annotations
 
+import contextlib
 from typing import Callable, List, Optional, Sequence
 
 import numpy as np
@@ -90,6 +94,42 @@ def shares_by_finish(sms: int, tiles0: int, tiles1: int, k_slabs: int, late: int
     return best and best[1:]
 
 
+def late_weight_gradients(sms: int, dims: Sequence[int], batch: int):
+    """{layer: SMs} of the weight gradients that run side by side behind the dX chain instead of each beside a product of it.
+    A product that occupies an SM per CTA and splits its k over whatever SMs there are leaves nothing for another one: the
+    chain's next product waited for the weight gradient's CTAs to leave.  Behind the chain they share the SMs, an output tile's
+    K ranges as even as they come, and pay the fixed part of such a product once.
+
+    Considered are those that go to the tensor cores (from 50 M multiply-adds) while all their 128 x 128 tiles together find an
+    SM each -- larger ones fill the chip whatever the order -- and whose layers' dX products are one wave of tiles: the last of
+    several leaves SMs that a weight gradient beside it fills (16 % slower without).  Not where the rows of X are no whole words: the
+    first gradient then splits in clusters only (1.5 % faster on average, a third of them slower).  They go late
+    where one after the other takes 1.4 times as long as together, at 6 us and 0.6 for a slab of k.
+    650 networks of random widths, 2 to 4 layers, 300 to 15000 rows: 7 % faster on average, 3 % of them 1 % slower or more.
+    Steps, us, beside -> behind: 1000-501-301-37 at 1000 rows 80.6 -> 72.8, 4000 rows 158 -> 146; 784-512-256-10 at 1000 66 -> 59;
+    512-512-512-512 at 2000 106 -> 94; 1024-1024-1024-40 at 1024 125 -> 112."""
+    pad, slabs = lambda n: -(-n // 32) * 32, -(-batch // 32)
+    big = [l for l in range(len(dims) - 1) if dims[l + 1] > 16 and pad(dims[l + 1]) * pad(dims[l]) * batch >= 5e7]
+    tiles = {l: -(-dims[l + 1] // 128) * -(-dims[l] // 128) for l in big}
+    if 0 not in big or dims[0] % 4 or sum(tiles.values()) > sms:
+        return {}
+    time = lambda ranges: 6 + 0.6 * -(-slabs // ranges)
+    alone = {l: time(max(1, min(sms // tiles[l], slabs // 4))) for l in big}
+    late = [0] + sorted((l for l in big if l and -(-batch // 128) * -(-dims[l] // 128) <= sms), key=lambda l: -tiles[l])
+    best, found = 0.0, {}
+    while len(late) > 1:  # (without the smallest, and so on: what finds too few SMs here holds up all of them)
+        ranges, left = {l: 1 for l in late}, sms - sum(tiles[l] for l in late)
+        while fit := [l for l in late if tiles[l] <= left and ranges[l] < slabs // 4]:
+            l = min(fit, key=lambda l: (ranges[l], -tiles[l]))
+            ranges[l] += 1
+            left -= tiles[l]
+        before, after = sum(alone[l] for l in late), time(min(ranges.values()))
+        if before >= 1.4 * after and before - after > best:
+            best, found = before - after, {l: tiles[l] * ranges[l] for l in late}
+        late.pop()
+    return found
+
+
 class MlpTrainer:
     def __init__(self, dev: CudaDevice, dims: Sequence[int], batch: int, weights, biases, opt: str = "sgd",
                  lr: float = 0.01, beta1: float = 0.9, beta2: float = 0.999, eps: float = 1e-8, clip: bool = False,
@@ -116,6 +156,7 @@ class MlpTrainer:
             raise ValueError("no mlp_tail kernel for the widths %s" % self.dims[-3:])
         self.tail = can_tail if tail is None else bool(tail)
         self._dw_shares = None
+        self._late = late_weight_gradients(dev.sm_count(), self.dims, self.B) if fused and not bf16 else {}
         self.update_by_layer = bool(update_by_layer)
         # the tail path applies plain SGD from inside the backward pass (see _forward_backward_tail) unless told not to
         self.fuse_update = bool(fuse_update) and self.tail
@@ -309,6 +350,14 @@ class MlpTrainer:
             if self.ld_out != self.dims[-1]:
                 raise ValueError("an external output gradient needs unpadded logits (pad_logits=False)")
             d.dispatch(opspec.unbroadcast(self.dact[-1], [B, self.dims[-1]], self._db[-1], [self.dims[-1]], None, 1.0, 0.0))
+        # (a caller that starts on each layer's gradients as they come gets them as they come)
+        late = self._late if on_layer_grads is None and not update_by_layer else {}
+
+        def weight_gradient(l, dy, a_in):
+            K, N = self.dims[l], self.dims[l + 1]
+            d.dispatch(opspec.linear(dy, a_in, self._dW[l], N, K, B, True, False, self.ld[l], self._ld_in(l), K, 1.0,
+                                     0.0 if fresh and self._large(l) else 1.0, sm_budget=late.get(l, 0)))
+
         for l in range(self.L - 1, -1, -1):
             K, N = self.dims[l], self.dims[l + 1]
             a_in = X if l == 0 else self.act[l - 1]
@@ -325,11 +374,11 @@ class MlpTrainer:
                 # The weight gradient does not feed the dX chain: it goes to the side
                 # stream (a parallel branch of a captured step), forked here where dY
                 # is ready, and runs next to this layer's dX GEMM.
-                with d.branch():
-                    d.dispatch(opspec.linear(dy, a_in, self._dW[l], N, K, B, True, False, ldy, self._ld_in(l), K, 1.0,
-                                             0.0 if fresh and self._large(l) else 1.0))
-                    if on_layer_grads is not None:
-                        on_layer_grads(l)
+                if l not in late:
+                    with d.branch():
+                        weight_gradient(l, dy, a_in)
+                        if on_layer_grads is not None:
+                            on_layer_grads(l)
                 if l > 0:  # dX = dY . W, zeroed where the previous activation is <= 0
                     W = self.Wb[l] if self.bf16 else self.W[l]
                     d.dispatch(opspec.linear(dy, W, self.dact[l - 1], B, K, N, False, False, ldy, K, self.ld[l - 1], 1.0, 0.0,
@@ -348,6 +397,9 @@ class MlpTrainer:
                     d.dispatch(opspec.bmm_acc(dy, self.W[l], self.dact[l - 1], (1, B, N), (1, N, K), (1, B, K), False, False, N, K, K, 1.0, 0.0))
                 else:
                     self._dw_op(l, dy, a_in)
+        for k, l in enumerate(sorted(late, reverse=True)):
+            with (d.branch(1 + k) if l > 0 else contextlib.nullcontext()):  # (not behind those beside the chain)
+                weight_gradient(l, self.dact[l], X if l == 0 else self.act[l - 1])
         d.join()  # the gradients are complete before anything that follows on the main stream
 
     # ------------------------------------------------- few rows: one launch for all weight gradients
@@ -433,8 +485,8 @@ class MlpTrainer:
           W += (-lr) * dY^T X (alpha = -lr, beta = 1, C = W): no gradient tensor, no update launch;
         * otherwise each weight gradient is followed, on its own stream, by the SGD update
           of that one tensor.
-        The biases, whose gradients the tail op has finished, are updated behind the last
-        layer's product; no update waits for the join of all streams.  The weights of the
+        The biases and the last layer, whose gradients the tail op has finished, are updated by a
+        launch of their own (behind the last layer's product where that op does not form it); no update waits for the join of all streams.  The weights of the
         layers in between are still read by the dX products and are updated after the join."""
         d, B, L = self.dev, self.B, self.L
         grouped = self.grouped
