@@ -118,11 +118,13 @@ __device__ __forceinline__ float csr_add(float acc, float (&v)[NE * FW / 32], fl
   return acc;
 }
 
-// Rows of up to kShortRow neighbours -- most, of a graph with a handful of edges per node -- are taken FW / 4 lanes each, so
+// VEC (many rows): rows of up to kShortRow neighbours -- most, of a graph with a handful of edges per node -- are taken FW / 4 lanes each, so
 // that a warp has 4 to 16 of them in flight and a graph of 20011 nodes starts all of its chains (row bounds, neighbours, their
 // features) at once instead of two or three per warp one after the other; a lane adds its four features up in edge order.
 // The longer ones are dealt to the CTA's warps, a row each (a warp's own 8 or 16 rows hold up to half a dozen of them).
-constexpr int kShortRow = 8, kMiddleQueue = 512;
+template <int FW>
+constexpr int kShortRow = FW == 8 ? 16 : 8;  // (at 8 features 16 of them: 30000 nodes of 7.5 edges 20.5 us, with 8 21.7)
+constexpr int kMiddleQueue = 512;
 constexpr int kHubRow = 64, kHubQueue = 64, kGatherWarps = kIThreads / 32 - 1;
 
 // VEC: rows of x hold whole 16-byte words at aligned addresses, and F fits into FW
@@ -179,12 +181,12 @@ __global__ void __launch_bounds__(kIThreads) csr_gcn_propagate_kernel(float* out
       const size_t r = r0 + lane / LW;
       const bool in = r < n_rows;
       const len_t k0 = in ? __ldg(row_ptr + r) : 0, k1 = in ? __ldg(row_ptr + r + 1) : 0;
-      const int n = k1 - k0 <= kShortRow ? (int)(k1 - k0) : 0;
+      const int n = k1 - k0 <= kShortRow<FW> ? (int)(k1 - k0) : 0;
       const float dr = in ? __ldg(deg + r) : 0.f;
       const size_t j = 4 * sub < F ? 4 * sub : 0;  // (lanes past the last word read the first one)
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int e = 0; e < kShortRow; e += 4) {
+      for (int e = 0; e < kShortRow<FW>; e += 4) {
         if (!__any_sync(0xffffffffu, e < n)) break;
         uint32_t c[4];
         float d[4];
@@ -207,13 +209,13 @@ __global__ void __launch_bounds__(kIThreads) csr_gcn_propagate_kernel(float* out
           }
         }
       }
-      if (in && k1 - k0 <= kShortRow) {
+      if (in && k1 - k0 <= kShortRow<FW>) {
         if (4 * sub + 0 < F) store(r, 4 * sub + 0, acc.x);
         if (4 * sub + 1 < F) store(r, 4 * sub + 1, acc.y);
         if (4 * sub + 2 < F) store(r, 4 * sub + 2, acc.z);
         if (4 * sub + 3 < F) store(r, 4 * sub + 3, acc.w);
       }
-      bool longer = in && sub == 0 && k1 - k0 > kShortRow;
+      bool longer = in && sub == 0 && k1 - k0 > kShortRow<FW>;
       if (longer) {  // for whichever warp of the CTA is free
         const unsigned at = atomicAdd(&waiting, 1u);
         if (at < kMiddleQueue) {
@@ -420,7 +422,11 @@ extern "C" void zg_csr_gcn_propagate(dtype id, StreamWrapper w, void* out, const
   if (epilogue != ZG_EPI_NONE && !bias) { set_error(kBadArgument, "zg_csr_gcn_propagate: bias epilogue without bias"); return; }
   if (n_rows > 0xffffffffu) { set_error(kBadArgument, "zg_csr_gcn_propagate: %lu rows", n_rows); return; }
   // lane groups as wide as the feature row: 8 features take 4 neighbours per step, 32 one
-  const bool vec = n_feat <= 32 && ld_x % 4 == 0 && ld_x >= (n_feat + 3) / 4 * 4 && host_aligned16(x);
+  // A warp per row while two or three waves of warps do: fewer CTAs of several rows per warp leave SMs idle, and the longer
+  // rows queue up in each.  Nodes x edges per node, us, a warp per row against rows by lanes (up to 16 features / 32):
+  //   500 x 7.5 3.9 and 7.5 / 4.3 and 6.7      3749 x 4.5 5.3 and 10.4 / 6.2 and 8.2     9000 x 4.5 9.2 and 8.0 / 9.4 and 9.1
+  //   16000 x 7.5 12.9 and 14.6 / 16.5 and 15.3   20011 x 4.5 13.1 and 11.1 / 15.1 and 12.4   50000 x 4.5 25.8 and 16.9 / 31 and 22
+  const bool vec = n_feat <= 32 && n_rows > (size_t)(n_feat <= 16 ? 128 : 64) * sm_count() && ld_x % 4 == 0 && ld_x >= (n_feat + 3) / 4 * 4 && host_aligned16(x);
   auto kern = n_feat <= 8 ? (vec ? csr_gcn_propagate_kernel<8, true> : csr_gcn_propagate_kernel<8, false>)
                           : (n_feat <= 16 ? (vec ? csr_gcn_propagate_kernel<16, true> : csr_gcn_propagate_kernel<16, false>)
                                           : (vec ? csr_gcn_propagate_kernel<32, true> : csr_gcn_propagate_kernel<32, false>));
