@@ -36,13 +36,15 @@ def test_few_rows(gpu, R, C, index):
     gpu.dispatch(opspec.softmax_ce(x, T, R, C, ls, dl, div, accumulate=True, ld=ld, bias_grad=db, probs=pr))
     # a probability: the exponential (2^-22, and 2^-24 |x - max| of the rounded product), its sum and the reciprocal
     eps = 2.0 ** -22 + 2.0 ** -24 * np.ptp(z64, axis=1).max() + 2.0 ** -22
-    got = be.down(dl).reshape(R, ld)
-    assert np.abs(be.down(pr).reshape(R, ld)[:, :C] - p).max() <= 2 * eps
+    probs, bias, lo = (gpu.to_numpy(v) for v in (pr, db, ls))
+    got = be.down(dl).reshape(R, ld)  # (frees them all)
+    probs = probs.reshape(R, ld)
+    assert np.abs(probs[:, :C] - p).max() <= 2 * eps
     assert np.abs(got[:, :C] - (old[:, :C] + dz)).max() <= 2 * eps / div + 2.0 ** -23 * np.abs(old).max()
-    assert np.array_equal(got[:, C:], old[:, C:]) and not be.down(pr).reshape(R, ld)[:, C:].any()
+    assert np.array_equal(got[:, C:], old[:, C:]) and not probs[:, C:].any()
     n = R + 16
-    assert np.abs(gpu.to_numpy(db) - dz.sum(0)).max() <= (2 * eps * p.sum(0).max() + 2.0 ** -24 * n * (p + t).sum(0).max()) / div + 1e-9
-    assert abs(gpu.to_numpy(ls)[0] - loss) <= (2 * eps + 2.0 ** -24 * (R / 8 + 64)) * max(1.0, abs(loss)) * max(1.0, R / div)
+    assert np.abs(bias - dz.sum(0)).max() <= (2 * eps * p.sum(0).max() + 2.0 ** -24 * n * (p + t).sum(0).max()) / div + 1e-9
+    assert abs(lo[0] - loss) <= (2 * eps + 2.0 ** -24 * (R / 8 + 64)) * max(1.0, abs(loss)) * max(1.0, R / div)
 
 
 @pytest.mark.parametrize("index", [False, True])
@@ -63,9 +65,10 @@ def test_few_masked_rows(gpu, R, C, index):
     T = be.up(lab.astype(np.uint64), np.uint64) if index else be.up(np.eye(C, dtype=np.float32)[lab])
     gpu.dispatch(opspec.masked_softmax_ce(x, o, T, R, C, ld, ls, dl, float(R), db))
     eps = 2.0 ** -21 + 2.0 ** -24 * 10
+    bias, lo = gpu.to_numpy(db), gpu.to_numpy(ls)
     got, times = be.down(dl).reshape(N, ld), np.bincount(mask).max()
     assert np.abs(got - want).max() <= times * (2 * eps / R + 2.0 ** -23 * (np.abs(old).max() + times / R))
     assert np.array_equal(got[:, C:], old[:, C:])
-    assert np.abs(gpu.to_numpy(db) - d.sum(0)).max() <= 2 * eps + 2.0 ** -24 * (R / 8 + 64)
+    assert np.abs(bias - d.sum(0)).max() <= 2 * eps + 2.0 ** -24 * (R / 8 + 64)
     loss = -np.take_along_axis(lp, lab[:, None], 1).sum() / R
-    assert abs(gpu.to_numpy(ls)[0] - loss) <= (2 * eps + 2.0 ** -24 * (R / 8 + 64)) * max(1.0, loss)
+    assert abs(lo[0] - loss) <= (2 * eps + 2.0 ** -24 * (R / 8 + 64)) * max(1.0, loss)
