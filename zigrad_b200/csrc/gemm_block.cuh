@@ -15,7 +15,8 @@
 // way into shared memory: both operands are kept [k][row], so a thread's operands are 16-byte reads.
 // Measured (operands in L2, one launch of a replayed chain): 64x128x784 + bias + ReLU 4.1 us (13.8 as 5 K splits of
 // one 128-row tensor-core tile, 49.7 for one row on the 64x64 tile kernel this one replaced), 128x784x64 4.8 (7.9),
-// 64x10x64 3.1 (6.3), 1000x501x1000 unaligned 49 (66), fp64 4 x 500x389x640 94 (105).
+// 64x10x64 3.1 (6.3), 1000x501x1000 unaligned 49 (66).  fp64 with more than half a
+// 64x64 tile per SM runs in gemm_f64.cuh.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -145,8 +146,7 @@ __device__ __forceinline__ void load4(const T* p, T (&v)[4]) {
 }
 
 // D (8 x 8) += A (8 x 4) * B (4 x 8) in fp64: lane l holds A[l / 4][l % 4], B[l % 4][l / 4] and D[l / 4][2 (l % 4)], [.. + 1].
-// Against DFMA it halves the shared-memory reads per multiply-add, which is what bounded the fp64 tiles:
-// 4 x 500x389x640 89 -> 54 us (105 on the kernel before).
+// Against DFMA it halves the shared-memory reads per multiply-add.
 __device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
 }
