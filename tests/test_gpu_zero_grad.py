@@ -134,3 +134,22 @@ def test_without_fused_ops_backward_overwrites(gpu):
     pair.a.backward(pair.data[0][0])
     np.testing.assert_allclose(gpu.to_numpy(pair.a.grads), once, rtol=1e-5, atol=1e-8)
     pair.free()
+
+
+@pytest.mark.parametrize("dims", [DIMS, [784, 128, 64, 10]], ids=str)
+def test_step_leaves_the_gradients_it_declares_clear(gpu, dims):
+    """zero_grads_in_update: behind a step every gradient is zero, so that the next forward pass need not clear them, an update
+    without a backward pass moves nothing, and a loss of the caller's adds into zeros."""
+    pair = Pair(gpu, dims, opt="sgd", zero_grads_in_update=True)
+    (X, T), other = pair.data[0], pair.data[1][0]
+    for i in range(4):  # op by op, then as a kept graph
+        for tr in (pair.a, pair.b):
+            tr.step(X, T)
+            assert not gpu.to_numpy(tr._grads).any(), i
+            tr.forward(other)
+            assert not gpu.to_numpy(tr._grads).any(), i
+            before = gpu.to_numpy(tr.params).copy()
+            tr.update()
+            np.testing.assert_array_equal(gpu.to_numpy(tr.params), before)
+        pair.check()
+    pair.free()

@@ -149,6 +149,7 @@ class MlpTrainer:
         if zero_grads_in_update and not (fused and opt == "sgd"):
             raise ValueError("zero_grads_in_update needs the fused ops and SGD")
         self.zero_grads_in_update, self._grads_clear = bool(zero_grads_in_update), False
+        self._bias_with_weights = False  # the loss leaves the last bias gradient to the op that forms the weights' (a grouped step)
         # the fused middle of the step (opspec.mlp_tail): on by default wherever the library has a kernel for the widths
         can_tail = (fused and not bf16 and self.L >= 3 and
                     dev.mlp_tail_supported(SINGLE, self.dims[-3], self.dims[-2], self.dims[-1]))
@@ -319,7 +320,7 @@ class MlpTrainer:
         self._touched = True
         if self.fused:  # the bias gradient of the last layer comes out of the same pass
             d.dispatch(opspec.softmax_ce(self.act[-1], T, B, C, self.loss, self.dact[-1], self.loss_div, accumulate=False,
-                                         ld=self.ld_out, bias_grad=self._db[-1]))
+                                         ld=self.ld_out, bias_grad=None if self._bias_with_weights else self._db[-1]))
         else:
             d.dispatch(opspec.softmax_ce(self.act[-1], T, B, C, self.loss, self.dact[-1], self.loss_div, accumulate=False))
 
@@ -593,7 +594,12 @@ class MlpTrainer:
                 fuse = self.opt == "sgd" and not self.clip and allreduce is None
                 self._clear_unwritten(fuse)
                 self._layers(X)
-                self.loss_and_grad(T)
+                # (nothing else clears what the loss would write where the gradients are not kept)
+                self._bias_with_weights = True
+                try:
+                    self.loss_and_grad(T)
+                finally:
+                    self._bias_with_weights = False
                 self.backward_grouped(X, fuse)
                 return None if fuse else self._reduce_and_update(allreduce)
             # The whole step is issued here: of its gradients only those it accumulates into have to be cleared (a fill of
