@@ -104,7 +104,9 @@ def late_weight_gradients(sms: int, dims: Sequence[int], batch: int):
     SM each -- larger ones fill the chip whatever the order -- and whose layers' dX products are one wave of tiles: the last of
     several leaves SMs that a weight gradient beside it fills (16 % slower without).  Not where the rows of X are no whole words: the
     first gradient then splits in clusters only (1.5 % faster on average, a third of them slower).  They go late
-    where one after the other takes 1.4 times as long as together, at 6 us and 0.6 for a slab of k.
+    where one after the other takes 1.4 times as long as together, at 6 us and 0.6 for a slab of k, and only where each keeps a
+    third of the K ranges that it has by itself: the error of a product grows with the length of a range, at a third of the
+    rate that one accumulator for all three passes had (gemm_tc.cuh), against which this was compared.
     650 networks of random widths, 2 to 4 layers, 300 to 15000 rows: 7 % faster on average, 3 % of them 1 % slower or more.
     Steps, us, beside -> behind: 1000-501-301-37 at 1000 rows 80.6 -> 72.8, 4000 rows 158 -> 146; 784-512-256-10 at 1000 66 -> 59;
     512-512-512-512 at 2000 106 -> 94; 1024-1024-1024-40 at 1024 125 -> 112."""
@@ -114,7 +116,13 @@ def late_weight_gradients(sms: int, dims: Sequence[int], batch: int):
     if 0 not in big or dims[0] % 4 or sum(tiles.values()) > sms:
         return {}
     time = lambda ranges: 6 + 0.6 * -(-slabs // ranges)
-    alone = {l: time(max(1, min(sms // tiles[l], slabs // 4))) for l in big}
+    ranges_alone = {l: max(1, min(sms // tiles[l], slabs // 4)) for l in big}
+    alone = {l: time(ranges_alone[l]) for l in big}
+    starts = [sum((dims[j] + 1) * dims[j + 1] for j in range(l)) for l in range(len(dims) - 1)]
+
+    def used(l, ranges):  # what gemm.cu makes of it: narrower tiles of two SMs each, clusters where rows are no whole words
+        return 1 if ranges < 3 else (ranges if dims[l] % 4 == 0 and starts[l] % 4 == 0 else min(ranges, 8))
+
     late = [0] + sorted((l for l in big if l and -(-batch // 128) * -(-dims[l] // 128) <= sms), key=lambda l: -tiles[l])
     best, found = 0.0, {}
     while len(late) > 1:  # (without the smallest, and so on: what finds too few SMs here holds up all of them)
@@ -124,7 +132,8 @@ def late_weight_gradients(sms: int, dims: Sequence[int], batch: int):
             ranges[l] += 1
             left -= tiles[l]
         before, after = sum(alone[l] for l in late), time(min(ranges.values()))
-        if before >= 1.4 * after and before - after > best:
+        exact = all(3 * used(l, ranges[l]) >= used(l, ranges_alone[l]) for l in late)
+        if exact and before >= 1.4 * after and before - after > best:
             best, found = before - after, {l: tiles[l] * ranges[l] for l in late}
         late.pop()
     return found
