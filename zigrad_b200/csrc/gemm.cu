@@ -204,7 +204,7 @@ static bool launch_tc_mode(cudaStream_t s, int bn, bool a_kmajor, bool b_kmajor,
     if (!a_kmajor && b_kmajor) return launch_tc_inst<BNV, false, true, MODE>(s, ta, tb, tcm, p, grid); \
     return launch_tc_inst<BNV, false, false, MODE>(s, ta, tb, tcm, p, grid);                       \
   }
-  if constexpr (MODE != tc::kBF16) { ZG_TC_CASE(32) }
+  if constexpr (!tc::ModeTraits<MODE>::kBf16) { ZG_TC_CASE(32) }
   ZG_TC_CASE(64)
   ZG_TC_CASE(128)
 #undef ZG_TC_CASE
@@ -382,16 +382,21 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   static const bool force = [] { const char* e = getenv("ZG_GEMM_FORCE_TC"); return e && e[0] == '1'; }();
   const double macs = (double)((m + 31) / 32 * 32) * (double)((n + 31) / 32 * 32) * (double)k * (double)nC;  // its tiles are 32 x 32
   if (!force && macs < small) return false;
-  // Measured crossovers of the copy: bf16 against the FFMA kernel 10 M multiply-adds (8.0 us either way; 30 M: 17 and 9), fp32
+  // A bf16 product of such operands with an fp32 C went to the FFMA kernel, whose sums round to nearest; on the tensor cores
+  // it takes the form that adds up as exactly (kBF16Sums).  128-wide tiles without a carry from k = 640 on where the FFMA kernel
+  // has no K ranges: 0.96 to 0.15 of that kernel's error there; 64-wide ones with it 1.0 to 0.15 from k = 96 on (below that
+  // 1.1 to 1.3, and the FFMA kernel stays): 130 random shapes up to k = 8000.  2309x3283x565 382 us and 94 like this, 1208x1518x782
+  // 158 and 16; 331x17x2571 12.6 and 13.6.
+  // Measured crossovers of the copy: bf16 with a bf16 C against the FFMA kernel 10 M multiply-adds (8.0 us either way; 30 M: 17 and 9), fp32
   // against the element-wise ring 500 M (1000x501x1001 16 us either way; 2001x1001x1001 36 and 29).
-  if (direct && macs >= (bf16 ? 1.5e7 : 1e9)) {
+  const bool sums = bf16 && direct && c_id == SINGLE;
+  if (direct && macs >= (sums ? 2e7 : (bf16 ? 1.5e7 : 1e9)) && !(sums && k < 96)) {
     const uint64_t ra = nA * (ta ? k : m), ca = ta ? m : k, rb = nB * (tb ? n : k), cb = tb ? k : n;
     if (bf16 ? repack_operands<__nv_bfloat16>(s, A, ra, ca, lda, a_direct, B, rb, cb, ldb, b_direct)
              : repack_operands<float>(s, A, ra, ca, lda, a_direct, B, rb, cb, ldb, b_direct))
       a_direct = b_direct = direct = false;
   }
   if (direct && bf16) return false;
-
   const int atom = bf16 ? 64 : 32;        // M/N elements per 128-byte column block
   const int bk = bf16 ? 64 : 32;
   // A C of few rows is computed as its transpose, so that the long dimension fills the 128 rows of the tile.
@@ -404,9 +409,10 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   // (a tile for half of them at least, k deep enough to amortise the tile hand-over).
   static const bool no_persist = [] { const char* e = getenv("ZG_GEMM_NO_PERSISTENT"); return e && e[0] == '1'; }();
   const size_t ptiles = ((m + tc::kPBM - 1) / tc::kPBM) * ((n + tc::kPBN - 1) / tc::kPBN) * nC, pairs = (size_t)sm_count() / 2;
-  const bool persistent = mode != tc::kFP32X3 && !swap && n > 128 && k >= 8 * (size_t)bk && ptiles * 2 >= pairs &&
+  const bool persistent = mode != tc::kFP32X3 && !sums && !swap && n > 128 && k >= 8 * (size_t)bk && ptiles * 2 >= pairs &&
                           ptiles <= 0x3fffffffu && !no_persist;
   int bn = persistent ? 256 : (N <= 32 && !direct ? 32 : (N <= 64 ? 64 : 128));
+  if (sums) bn = k >= 640 && N > 64 && block_splits(((m + 31) / 32) * ((n + 31) / 32) * nC, k) == 1 ? 128 : 64;
   if (bn < atom) bn = atom;               // MN-major B needs whole column blocks; bf16 has no BN=32 instance
   size_t tiles = ((M + 127) / 128) * ((N + bn - 1) / bn) * nC;
   // Problems with few tiles get their parallelism from K splits.  Up to eight splits form a cluster, which sums its
@@ -421,7 +427,7 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
     if (mask) c_aligned = c_aligned && host_aligned16(mask);
     if (bias) c_aligned = c_aligned && host_aligned16(bias);
   }
-  const size_t min_slabs = mode == tc::kFP32X3 ? 4 : 12;  // per split: a three-pass slab costs 450 to 750 cycles, a single-pass one 130
+  const size_t min_slabs = mode == tc::kFP32X3 || sums ? 4 : 12;  // per split: a three-pass slab costs 450 to 750 cycles, a single-pass one 130
   const bool can_split = !persistent && k >= 2 * min_slabs * (size_t)bk && tiles * (bn == 128 ? 3 : 2) <= sm_share();
   // (in a cluster; a plain product of 128-wide tiles reduces through the tensor map)
   auto cluster_splits = [&](size_t t) {
@@ -431,7 +437,7 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   };
   const bool reduces = epilogue == ZG_EPI_NONE && !colsum && c_id == SINGLE && c_aligned && !swap && bn == 128;
   const size_t tiles64 = ((M + 127) / 128) * ((N + 63) / 64) * nC;
-  if (!persistent && !can_split && bn == 128 && tiles * 2 <= sm_share() && N > 64) {
+  if (!persistent && !can_split && bn == 128 && !sums && tiles * 2 <= sm_share() && N > 64) {
     bn = 64;
     tiles = tiles64;
   } else if (can_split && mode == tc::kFP32X3 && bn == 128 && !reduces && tiles64 <= sm_share()) {
@@ -550,6 +556,7 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
     p.tma_epilogue = splits > 1 ? 2 : 1;
   }
   if (direct) launch_tc_direct(s, bn, a_kmajor, b_kmajor, tmA, tmB, tmC, p, grid);
+  else if (sums) launch_tc_mode<tc::kBF16Sums>(s, bn, a_kmajor, b_kmajor, tmA, tmB, tmC, p, grid);
   else if (mode == tc::kBF16) launch_tc_mode<tc::kBF16>(s, bn, a_kmajor, b_kmajor, tmA, tmB, tmC, p, grid);
   else if (mode == tc::kTF32) launch_tc_mode<tc::kTF32>(s, bn, a_kmajor, b_kmajor, tmA, tmB, tmC, p, grid);
   else launch_tc_mode<tc::kFP32X3>(s, bn, a_kmajor, b_kmajor, tmA, tmB, tmC, p, grid);

@@ -26,6 +26,9 @@
 //   warps 12-19 DIRECT instances only: element-wise copies of operands whose rows no
 //               TMA box can address (1000x501x1000 with 501-float rows: 16 us
 //               against 66 on the FFMA path, 4096x1023x1023 80 against 385)
+//   kBF16Sums   (bf16 operands, fp32 C): an accumulator takes the products of two or four instructions only, two accumulators in
+//               turn, and warps 4-7 add them up in registers, rounding to nearest; the tensor core's own sums
+//               truncate at every instruction (1895x1340x2310 2.4e-6 off in the 2-norm, 1.3e-7 like this)
 //   warps 4-7   read the accumulator (tcgen05.ld: warp q reads TMEM lanes
 //               32q..32q+31, one row per thread); then either staged boxes go to
 //               the TMA unit, or the whole tile is staged in shared memory and
@@ -69,7 +72,7 @@ constexpr int kSplitThreads = kThreadsTc - 64;  // warps 2-7
 constexpr int kSlabBytes = 128;          // bytes of the contiguous dimension per smem row
 constexpr uint32_t kSpinLimit = 1u << 24;  // polls per wait before giving up
 
-enum Mode { kTF32 = 0, kFP32X3 = 1, kBF16 = 2 };
+enum Mode { kTF32 = 0, kFP32X3 = 1, kBF16 = 2, kBF16Sums = 3 };  // kBF16Sums: bf16 operands, fp32 sums that round (below)
 
 struct Params {
   float* C;             // fp32 output (or nullptr when Cb is used)
@@ -302,7 +305,7 @@ __device__ __forceinline__ void bulk_wait_group_read() { asm volatile("cp.async.
 
 template <int MODE>
 struct ModeTraits {
-  static constexpr bool kBf16 = (MODE == kBF16);
+  static constexpr bool kBf16 = (MODE == kBF16 || MODE == kBF16Sums);
   static constexpr int kElem = kBf16 ? 2 : 4;
   static constexpr int kBK = kSlabBytes / kElem;       // elements of K per stage: 32 (fp32) / 64 (bf16)
   static constexpr int kUmmaK = 32 / kElem;            // K per MMA: 8 (tf32) / 16 (bf16)
@@ -553,8 +556,9 @@ struct SmemLayout {
   static constexpr int kStageBytes = kABytes + (X3 ? 2 : 1) * kBBytes;
   static constexpr int kEpiBytes = 0;
   static constexpr int kBudget = 220 * 1024;
-  // FP32X3: a second accumulator behind the first, see the MMA issuer
-  static constexpr int kAccOne = BN < 32 ? 32 : BN, kAccCols = X3 ? 2 * kAccOne : kAccOne;
+  // FP32X3: a second accumulator behind the first, see the MMA issuer; kBF16Sums: the slabs' products take two in turn
+  static constexpr int kAccOne = BN < 32 ? 32 : BN, kAccCols = X3 || MODE == kBF16Sums ? 2 * kAccOne : kAccOne;
+  static constexpr int kInPart = BN == 64 ? 2 : 4;  // kBF16Sums: instructions whose products share an accumulator
   static constexpr int kATmemCols = 64;              // per stage: 32 columns hi + 32 columns lo
   static constexpr int kStagesSmem = (kBudget - kEpiBytes - 1024) / kStageBytes;
   static constexpr int kStagesTmem = X3 ? (512 - kAccCols) / kATmemCols : 8;
@@ -806,7 +810,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   using MT = ModeTraits<MODE>;
   using SL = SmemLayout<BN, MODE>;
   constexpr int S = SL::kStages;
-  constexpr bool X3 = (MODE == kFP32X3);
+  constexpr bool X3 = (MODE == kFP32X3), SUMS = (MODE == kBF16Sums);
   // an A operand in tensor memory is K-major by construction (row m in lane m, one k element per column)
   constexpr uint32_t kIdesc = make_idesc(MT::kBf16, X3 ? false : !A_KMAJOR, !B_KMAJOR, BN);
   constexpr uint32_t kTmemCols = SL::kTmemCols;
@@ -820,6 +824,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   uint64_t* ready = bars + S;       // [S] (X3) split done
   uint64_t* empty = bars + 2 * S;   // [S] MMAs that read the stage retired
   uint64_t* accum = bars + 3 * S;   // accumulator complete
+  uint64_t* part_full = accum + 1;  // [2] (SUMS) a slab's products complete
+  uint64_t* part_empty = accum + 3; // [2] (SUMS) ... and added up
   __shared__ uint32_t tmem_base_slot;
   __shared__ volatile int failed;
 
@@ -840,6 +846,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       mbar_init(&empty[s], 1);
     }
     mbar_init(accum, 1);
+    if constexpr (SUMS) {
+      for (int i = 0; i < 2; ++i) {
+        mbar_init(&part_full[i], 1);
+        mbar_init(&part_empty[i], 4);
+      }
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     prefetch_tmap(&tmA);
     prefetch_tmap(&tmB);
@@ -962,7 +974,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             umma_tmem_a(tmem_d, ta_hi, db, kIdesc, acc);   // Ahi * Bhi
           } else {
             const uint64_t da = desc_pack(da0 + kk * a_step, a_h32);
-            umma<MT::kBf16>(tmem_d, da, db, kIdesc, acc);
+            if constexpr (SUMS) {
+              const int part = (kt * (MT::kBK / MT::kUmmaK) + kk) / SL::kInPart, at = kk % SL::kInPart;
+              if (at == 0 && part >= 2 && !mbar_wait(&part_empty[part & 1], ((part >> 1) & 1) ^ 1, &failed)) break;
+              umma<MT::kBf16>(tmem_d + (part & 1) * SL::kAccOne, da, db, kIdesc, at > 0 ? 1u : 0u);
+              if (at == SL::kInPart - 1) umma_commit(&part_full[part & 1]);
+            } else umma<MT::kBf16>(tmem_d, da, db, kIdesc, acc);
           }
         }
         umma_commit(&empty[s]);  // stage reusable once these MMAs have read it
@@ -1082,7 +1099,60 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   // boxes for the TMA unit, or into the staged tile that all warps then finish.
   if (warp >= 4 && warp < 8) {
     const int q = warp - 4;  // TMEM lane quadrant
-    const bool have_acc = (KT > 0) && mbar_wait(accum, 0, &failed);
+    bool have_acc = KT > 0;
+    if constexpr (SUMS) {
+      // The parts of the sum are added up here, rounding to nearest, and take the accumulator's place.  64-wide tiles carry what
+      // each addition rounds off to the next one (Kahan's summation).
+      constexpr bool CARRY = BN == 64;
+      const uint32_t at = tmem_d + ((uint32_t)(q * 32) << 16);
+      float sum[BN], off[CARRY ? BN : 1];
+#pragma unroll
+      for (int j = 0; j < BN; ++j) {
+        sum[j] = 0.f;
+        if constexpr (CARRY) off[j] = 0.f;
+      }
+      const int parts = KT * (MT::kBK / MT::kUmmaK) / SL::kInPart;
+      for (int part = 0; part < parts; ++part) {
+        const bool got = mbar_wait(&part_full[part & 1], (part >> 1) & 1, &failed);
+        if (!__all_sync(0xffffffffu, got)) { have_acc = false; break; }
+        tc_fence_after();
+#pragma unroll
+        for (int c = 0; c < BN; c += 64) {
+          uint32_t r[32], t[32];
+          tmem_ld32(at + (part & 1) * SL::kAccOne + c, r);
+          tmem_ld32(at + (part & 1) * SL::kAccOne + c + 32, t);
+          tmem_ld_wait();
+          if (c + 64 == BN) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&part_empty[part & 1]);
+          }
+#pragma unroll
+          for (int j = 0; j < 64; ++j) {
+            const float x = __uint_as_float(j < 32 ? r[j % 32] : t[j % 32]);
+            if constexpr (CARRY) {
+              const float y = x - off[j], z = sum[j] + y, e = (z - sum[j]) - y;
+              off[j] = fabsf(e) < INFINITY ? e : 0.f;  // (behind an infinity, or a sum that became one, there is nothing to carry)
+              sum[j] = z;
+            } else {
+              sum[c + j] += x;
+            }
+          }
+        }
+      }
+      if (have_acc) {
+#pragma unroll
+        for (int c = 0; c < BN; c += 32) {
+          uint32_t r[32];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(sum[c + j]);
+          tmem_st32(at + c, r);
+        }
+        tmem_st_wait();
+      }
+    } else {
+      have_acc = have_acc && mbar_wait(accum, 0, &failed);
+    }
     tc_fence_after();
     if (p.tma_epilogue && (KT == 0 || have_acc)) {
       // The stage ring is idle by now (every fetched slab was consumed by MMAs that have completed):
