@@ -97,6 +97,10 @@ enum { ZG_EPI_NONE = 0, ZG_EPI_BIAS = 1, ZG_EPI_BIAS_RELU = 2, ZG_EPI_RELU_MASK 
  * share: the split-K grid is then sized for that many SMs, so that the concurrent launches
  * fit in one wave together instead of pushing one another's CTAs into a second wave. */
 EXTERN_C void zg_bmm_sm_budget(int sms);
+/* The NEXT zg_bmm call of the calling thread, if its operands are bf16 and C fp32, adds its products up with sums that round to
+ * nearest (about 1e-7 off in the 2-norm), as it does for operands without 16-byte rows; the tensor core's own sums truncate
+ * (1e-7 times the square root of the products per sum and more). */
+EXTERN_C void zg_bmm_rounded_sums(int on);
 EXTERN_C int zg_sm_count(void);
 EXTERN_C void zg_bmm(dtype id, dtype c_id, StreamWrapper stream,
                      const void* A, const void* B, void* C,

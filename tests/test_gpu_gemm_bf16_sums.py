@@ -7,6 +7,9 @@ import pytest
 
 import oracle
 from zigrad_b200 import opspec
+from zigrad_b200.abi import BF16
+from zigrad_b200.device import DeviceSlice
+from zigrad_b200.mlp import MlpTrainer, kaiming_uniform
 
 from .backends import GpuBackend
 from .test_gpu_gemm_repack import between_words
@@ -38,6 +41,30 @@ def test_sums_round(gpu, nb, m, n, k, bound, ta, tb):
     op = lambda x, t: (x.transpose(0, 2, 1) if t else x).astype(np.float64)
     want = op(A, ta) @ op(B, tb)
     assert np.linalg.norm(be.down(c).reshape(nb, m, n) - want) <= bound * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("dims,B", [([320, 253, 129, 24], 700), ([64, 72, 56, 152, 36], 1992)], ids=str)
+def test_weight_gradients_of_padded_activations(gpu, dims, B):
+    """Rows of odd hidden widths are padded to whole words; their weight gradients add up as those of dense rows do."""
+    g = rng(B)
+    bits = lambda a: (oracle.round_bf16(a.ravel()).view(np.uint32) >> 16).astype(np.uint16).reshape(a.shape)
+    wide = lambda u: (u.astype(np.uint32) << 16).view(np.float32)
+    X = bits(g.standard_normal((B, dims[0])).astype(np.float32))
+    tr = MlpTrainer(gpu, dims, B, *kaiming_uniform(dims, 3), opt="none", bf16=True, index_labels=True)
+    Xd, Td = gpu.from_numpy(X.view(np.uint16)), gpu.from_numpy(g.integers(0, dims[-1], B).astype(np.uint64))
+    tr.step(DeviceSlice(Xd.ptr, X.size, BF16, 0), Td)
+    grads = tr.get_grads()[0]
+    for l, (K, N) in enumerate(zip(dims[:-1], dims[1:])):
+        if K % 8 == 0 and (N if l + 2 < len(dims) else tr.ld_out) % 8 == 0:
+            continue  # whole words all along: the tensor core's own sums
+        dy = tr.act_numpy(l, grad=True)
+        dy = wide(bits(dy)) if l + 2 == len(dims) else dy
+        a = wide(X) if l == 0 else tr.act_numpy(l - 1)
+        want = dy.astype(np.float64).T @ a
+        assert np.linalg.norm(grads[l] - want) <= 2e-7 * np.linalg.norm(want), l
+    for s in (Xd, Td):
+        gpu.mem_cache_free(s)
+    tr.free()
 
 
 @pytest.mark.parametrize("k", [200, 1300])

@@ -337,6 +337,9 @@ static size_t sm_share() {
   const size_t all = (size_t)sm_count();
   return (g_sm_budget > 0 && (size_t)g_sm_budget < all) ? (size_t)g_sm_budget : all;
 }
+// bf16 operands with 16-byte rows into an fp32 C whose sums shall round all the same (zg_bmm_rounded_sums)
+static thread_local bool g_next_rounded = false, g_rounded = false;
+extern "C" void zg_bmm_rounded_sums(int on) { g_next_rounded = on != 0; }
 extern "C" void zg_bmm_sm_budget(int sms) { g_next_sm_budget = sms > 0 ? sms : 0; }
 
 // Operands without 16-byte rows copied into the stream's work space with them (gemm_repack.cuh); a pointer and leading dimension
@@ -389,8 +392,9 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   // 158 and 16; 331x17x2571 12.6 and 13.6.
   // Measured crossovers of the copy: bf16 with a bf16 C against the FFMA kernel 10 M multiply-adds (8.0 us either way; 30 M: 17 and 9), fp32
   // against the element-wise ring 500 M (1000x501x1001 16 us either way; 2001x1001x1001 36 and 29).
-  const bool sums = bf16 && direct && c_id == SINGLE;
-  if (direct && macs >= (sums ? 2e7 : (bf16 ? 1.5e7 : 1e9)) && !(sums && k < 96)) {
+  const bool sums = bf16 && (direct || g_rounded) && c_id == SINGLE;
+  if (sums && (macs < 2e7 || k < 96)) return false;
+  if (direct && macs >= (bf16 ? 1.5e7 : 1e9)) {
     const uint64_t ra = nA * (ta ? k : m), ca = ta ? m : k, rb = nB * (tb ? n : k), cb = tb ? k : n;
     if (bf16 ? repack_operands<__nv_bfloat16>(s, A, ra, ca, lda, a_direct, B, rb, cb, ldb, b_direct)
              : repack_operands<float>(s, A, ra, ca, lda, a_direct, B, rb, cb, ldb, b_direct))
@@ -568,6 +572,8 @@ void bmm_dispatch(dtype id, dtype c_id, cudaStream_t s, const void* A, const voi
                   const void* bias, const void* mask, void* colsum) {
   g_sm_budget = g_next_sm_budget;
   g_next_sm_budget = 0;
+  g_rounded = g_next_rounded;
+  g_next_rounded = false;
   if (m == 0 || n == 0 || nC == 0) return;
   if (nA == 0 || nB == 0) { set_error(kBadArgument, "bmm: empty operand batch"); return; }
   if (epilogue < ZG_EPI_NONE || epilogue > ZG_EPI_RELU_MASK) { set_error(kBadArgument, "bmm: unknown epilogue %d", epilogue); return; }

@@ -458,6 +458,8 @@ class CudaDevice:
         nA, nB, nC = p.n_batch
         if p.sm_budget:
             self.L.zg_bmm_sm_budget(p.sm_budget)
+        if p.rounded_sums:
+            self.L.zg_bmm_rounded_sums(1)
         self.L.zg_bmm(p.A.dtype, p.C.dtype, self.stream, p.A.ptr, p.B.ptr, p.C.ptr, nA, nB, nC, p.m, p.n, p.k,
                       p.trans_a, p.trans_b, p.lda, p.ldb, p.ldc, p.alpha, p.beta, epi,
                       p.bias.ptr if p.bias is not None else None, p.mask_src.ptr if p.mask_src is not None else None,

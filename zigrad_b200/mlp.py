@@ -365,8 +365,10 @@ class MlpTrainer:
 
         def weight_gradient(l, dy, a_in):
             K, N = self.dims[l], self.dims[l + 1]
+            # (bf16: the padding of the activations' rows does not make the sums any less exact than those of dense rows)
+            ragged = self.bf16 and (K % 8 != 0 or (N if l + 1 < self.L else self.ld_out) % 8 != 0)
             d.dispatch(opspec.linear(dy, a_in, self._dW[l], N, K, B, True, False, self.ld[l], self._ld_in(l), K, 1.0,
-                                     0.0 if fresh and self._large(l) else 1.0, sm_budget=late.get(l, 0)))
+                                     0.0 if fresh and self._large(l) else 1.0, sm_budget=late.get(l, 0), rounded_sums=ragged))
 
         for l in range(self.L - 1, -1, -1):
             K, N = self.dims[l], self.dims[l + 1]

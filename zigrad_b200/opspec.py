@@ -662,3 +662,4 @@ class linear:
     n_batch: tuple = field(default=(1, 1, 1))
     colsum: Optional[Any] = None  # fp32 [n]: column sums of the stored C are added here (a bias gradient)
     sm_budget: int = 0  # > 0: size the split-K grid for this many SMs (GEMMs that run side by side on parallel streams share them)
+    rounded_sums: bool = False  # bf16 operands, fp32 C: sums that round to nearest rather than truncate (zg_bmm_rounded_sums)
