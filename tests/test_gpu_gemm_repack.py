@@ -38,3 +38,61 @@ def test_operands_without_word_rows(gpu, bf16, nb, m, n, k, off, ta, tb):
     op = lambda x, t: (x.transpose(0, 2, 1) if t else x).astype(np.float64)
     want = 0.5 * (op(A, ta) @ op(B, tb)) + 2.0 * C0 + bias
     assert rel_err(be.down(c).reshape(nb, m, n), want) <= (2e-5 if bf16 else 5e-5)
+
+
+def test_without_memory_for_the_copies(gpu):
+    """The kernels that need no copies take over, and no error is left behind."""
+    import torch
+    g, be = rng(3), GpuBackend(gpu)
+    m, n, k = 3001, 3003, 4001  # 48 MB of copies
+
+    def product(m, n, k):
+        A, B = (oracle.round_bf16(g.standard_normal(s).astype(np.float32).ravel()) for s in (m * k, n * k))
+        return between_words(be, A, 1, True), between_words(be, B, 1, True), be.up(np.zeros((m, n), np.float32)), A.reshape(m, k), B.reshape(n, k)
+
+    run = lambda a, b, c, m, n, k: gpu.dispatch(opspec.linear(a, b, c, m, n, k, False, True, k, k, n))
+    for s in ((301, 301, 601), (3001, 3003, 41)):  # the kernels of both ways are loaded
+        run(*product(*s)[:3], *s)
+    a, b, c, A, B = product(m, n, k)
+    gpu.sync()
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - (24 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        run(a, b, c, m, n, k)
+        gpu.sync()  # raises what was recorded
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    want = A[:64].astype(np.float64) @ B.T
+    assert rel_err(be.down(c).reshape(m, n)[:64], want) <= 2e-5
+    run(a, b, c, m, n, k)  # and the copies come back with the memory
+    assert rel_err(be.down(c).reshape(m, n)[:64], want) <= 2e-5
+
+
+@pytest.mark.parametrize("bf16", [True, False])
+def test_two_threads_on_one_stream(gpu, bf16):
+    """A product's copies are its own until it has been launched, whoever else issues products on the same stream."""
+    import threading
+    g, be, m, n, k = rng(5), GpuBackend(gpu), 1001, 1001, 1001
+    jobs, wrong = [], []
+    for _ in range(2):
+        A, B = (g.standard_normal(s).astype(np.float32) for s in ((m, k), (n, k)))
+        if bf16:
+            A, B = (oracle.round_bf16(x.ravel()).reshape(x.shape) for x in (A, B))
+        outs = [be.up(np.zeros((m, n), np.float32)) for _ in range(40)]
+        jobs.append((between_words(be, A, 1, bf16), between_words(be, B, 1, bf16), outs, A.astype(np.float64) @ B.T.astype(np.float64)))
+    start = threading.Barrier(2)
+
+    def issue(a, b, outs):
+        start.wait()
+        for c in outs:
+            gpu.dispatch(opspec.linear(a, b, c, m, n, k, False, True, k, k, n))
+
+    threads = [threading.Thread(target=issue, args=j[:3]) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    gpu.sync()
+    for _, _, outs, want in jobs:
+        wrong += [e for e in (rel_err(be.down(c).reshape(m, n), want) for c in outs) if e > 5e-5]
+    assert not wrong, len(wrong)

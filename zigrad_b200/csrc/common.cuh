@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 
 #include "../../include/decls.h"
 #include "../../include/zg_b200.h"
@@ -52,6 +53,8 @@ int sm_count();  // SMs of the current device (cached)
 // Slots 0 and 1 are scratch; slot 2 is zero when handed out and every kernel
 // that uses it leaves it zero (arrival counters of multi-CTA reductions).
 void* workspace(cudaStream_t s, size_t bytes, unsigned** counters, int slot = 0);
+// The stream's buffer for copies of operands; nullptr, without an error, where it cannot be had
+void* copy_space(cudaStream_t s, size_t bytes, std::unique_lock<std::mutex>& held);
 // Whether workspace() would give that much now: what is being captured can use only what is there already.
 bool workspace_ready(cudaStream_t s, size_t bytes, int slot);
 // Tickets back to zero on the current device, which must be idle: after a kernel that gave up and left some drawn.

@@ -342,17 +342,16 @@ static thread_local bool g_next_rounded = false, g_rounded = false;
 extern "C" void zg_bmm_rounded_sums(int on) { g_next_rounded = on != 0; }
 extern "C" void zg_bmm_sm_budget(int sms) { g_next_sm_budget = sms > 0 ? sms : 0; }
 
-// Operands without 16-byte rows copied into the stream's work space with them (gemm_repack.cuh); a pointer and leading dimension
-// are replaced where they are copied.  False: no work space for it (more than 256 MB, or it would have to grow inside a capture).
+// Operands without 16-byte rows copied with them (gemm_repack.cuh) into the stream's buffer for that; a pointer and leading
+// dimension are replaced where they are copied.  False: no place for them (more than 256 MB, or copy_space() has none).
 template <typename T>
 static bool repack_operands(cudaStream_t s, const void*& A, uint64_t rows_a, uint64_t cols_a, len_t& lda, bool copy_a, const void*& B, uint64_t rows_b,
-                            uint64_t cols_b, len_t& ldb, bool copy_b) {
+                            uint64_t cols_b, len_t& ldb, bool copy_b, std::unique_lock<std::mutex>& held) {
   constexpr uint64_t E = 16 / sizeof(T);
   auto words = [](uint64_t cols) { return (cols + E - 1) / E; };
   const uint64_t wa = copy_a ? rows_a * words(cols_a) : 0, wb = copy_b ? rows_b * words(cols_b) : 0;
   const uint64_t at_b = (wa * 16 + 255) / 256 * 256, bytes = at_b + wb * 16;
-  if (bytes > ((uint64_t)256 << 20) || !workspace_ready(s, bytes, 1)) return false;
-  char* ws = static_cast<char*>(workspace(s, bytes, nullptr, 1));
+  char* ws = bytes > ((uint64_t)256 << 20) ? nullptr : static_cast<char*>(copy_space(s, bytes, held));
   if (!ws) return false;
   const repack::Operand a{A, ws, lda, (uint32_t)cols_a, (uint32_t)words(cols_a), wa}, b{B, ws + at_b, ldb, (uint32_t)cols_b, (uint32_t)words(cols_b), wb};
   const unsigned grid = grid_for(std::max(wa, wb), 512);
@@ -394,10 +393,11 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   // against the element-wise ring 500 M (1000x501x1001 16 us either way; 2001x1001x1001 36 and 29).
   const bool sums = bf16 && (direct || g_rounded) && c_id == SINGLE;
   if (sums && (macs < 2e7 || k < 96)) return false;
+  std::unique_lock<std::mutex> copies;  // until the product has been launched
   if (direct && macs >= (bf16 ? 1.5e7 : 1e9)) {
     const uint64_t ra = nA * (ta ? k : m), ca = ta ? m : k, rb = nB * (tb ? n : k), cb = tb ? k : n;
-    if (bf16 ? repack_operands<__nv_bfloat16>(s, A, ra, ca, lda, a_direct, B, rb, cb, ldb, b_direct)
-             : repack_operands<float>(s, A, ra, ca, lda, a_direct, B, rb, cb, ldb, b_direct))
+    if (bf16 ? repack_operands<__nv_bfloat16>(s, A, ra, ca, lda, a_direct, B, rb, cb, ldb, b_direct, copies)
+             : repack_operands<float>(s, A, ra, ca, lda, a_direct, B, rb, cb, ldb, b_direct, copies))
       a_direct = b_direct = direct = false;
   }
   if (direct && bf16) return false;

@@ -1,5 +1,5 @@
 // Copies of operands whose rows no TMA box can address (base or row pitch no multiple of 16 bytes) with rows of whole 16-byte
-// words, in the stream's work space: one pass over both operands in one launch in front of a tensor-core product.
+// words, in a buffer of the stream's: one pass over both operands in one launch in front of a tensor-core product.
 //
 // For bf16 there is no other way onto the tensor cores: cp.async has no 2-byte form, and the FFMA kernel that took these
 // products does 26 TFLOP/s (2047^3 670 us, 44 like this; 1000x301x501 37 and 9.7).  For fp32 the element-wise ring (DIRECT) pays for every 4-byte copy as often as a

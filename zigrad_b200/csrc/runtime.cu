@@ -1,5 +1,6 @@
 // Device / stream / memory / graph-capture / virtual-memory entry points
 // (include/cuda_utils.h) and the sticky error status (include/zg_b200.h).
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdlib>
@@ -224,6 +225,62 @@ bool workspace_ready(cudaStream_t s, size_t bytes, int slot) {
   return w != g_ws.end() && w->second.bytes >= bytes + 256;
 }
 
+// Copies of operands in front of a product (gemm_repack.cuh) have a buffer per stream of their own, since they are large and the
+// product can do without: its size follows the need (an eighth above it at most), an outgrown one goes back at once unless a
+// graph was captured with it, and the last one goes back with the stream.  Behind a captured one the next is at least twice as
+// large, so that those that had to stay are together smaller than the live one.  Copy and product are two launches: `held` keeps
+// other threads' copies, which may go to the same stream, from coming between them.  nullptr, without an error: what is being
+// captured can use only what is there already, or the device has no memory left.
+struct CopySpace {
+  std::mutex mu;
+  void* base = nullptr;
+  size_t bytes = 0;
+  bool captured = false;
+};
+static std::map<std::pair<int, cudaStream_t>, CopySpace> g_copies;
+
+void* copy_space(cudaStream_t s, size_t bytes, std::unique_lock<std::mutex>& held) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  CopySpace* c = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(g_ws_mu);
+    c = &g_copies[{dev, s}];
+  }
+  held = std::unique_lock<std::mutex>(c->mu);
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  const bool capturing = cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
+  if (c->bytes < bytes) {
+    if (capturing) return nullptr;
+    size_t unit = (size_t)1 << 20;
+    while (unit * 8 < bytes) unit *= 2;
+    size_t cap = (bytes + unit - 1) / unit * unit;
+    if (c->captured) cap = std::max(cap, 2 * c->bytes);
+    else if (c->base) ZG_CUDA(cudaFree(c->base));  // (waits for what still runs)
+    c->base = nullptr;
+    c->bytes = 0;
+    c->captured = false;
+    if (cudaMalloc(&c->base, cap) != cudaSuccess) {
+      (void)cudaGetLastError();
+      c->base = nullptr;
+      return nullptr;
+    }
+    c->bytes = cap;
+  }
+  c->captured = c->captured || capturing;
+  return c->base;
+}
+
+static void release_copy_space(cudaStream_t s) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(g_ws_mu);
+  const auto c = g_copies.find({dev, s});
+  if (c == g_copies.end()) return;
+  if (c->second.base && !c->second.captured) ZG_CUDA(cudaFree(c->second.base));
+  g_copies.erase(c);
+}
+
 void clear_workspace_tickets() {
   int dev = 0;
   cudaGetDevice(&dev);
@@ -331,7 +388,9 @@ extern "C" StreamWrapper init_stream(void) {
   return StreamWrapper{s};
 }
 extern "C" void deinit_stream(StreamWrapper stream) {
-  if (stream.ptr) ZG_CUDA(cudaStreamDestroy(as_stream(stream)));
+  if (!stream.ptr) return;
+  release_copy_space(as_stream(stream));
+  ZG_CUDA(cudaStreamDestroy(as_stream(stream)));
 }
 extern "C" void* zg_host_alloc_pinned(len_t nbytes) {
   void* p = nullptr;
