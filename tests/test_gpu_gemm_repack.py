@@ -2,6 +2,9 @@
 are copied into the work space first, against a float64 product of the same operands.  bf16 inputs are exact in fp32 and
 the sums of k products are fp32: 2e-5 of the largest element (5e-6 seen); fp32 inputs in three TF32 passes: 5e-5, as for
 aligned ones."""
+import sys
+import threading
+
 import numpy as np
 import pytest
 
@@ -25,7 +28,8 @@ def between_words(be, a, off, bf16):
 
 @pytest.mark.parametrize("ta,tb", [(False, False), (False, True), (True, False), (True, True)])
 @pytest.mark.parametrize("bf16,nb,m,n,k,off", [(True, 1, 300, 301, 501, 0), (True, 3, 129, 257, 263, 1), (True, 2, 2049, 513, 130, 7), (True, 1, 1000, 7, 2049, 3),
-                                              (False, 1, 1023, 1001, 1001, 0), (False, 2, 701, 1024, 1003, 3)])
+                                              (False, 1, 1023, 1001, 1001, 0), (False, 2, 701, 1024, 1003, 3),
+                                              (False, 1, 300, 1025, 1001, 1), (False, 1, 250, 1025, 1001, 1), (False, 1, 163, 1429, 1194, 1)])
 def test_operands_without_word_rows(gpu, bf16, nb, m, n, k, off, ta, tb):
     g, be = rng(m + n + k), GpuBackend(gpu)
     A, B = (g.standard_normal(s).astype(np.float32) for s in ((nb, k, m) if ta else (nb, m, k), (1, n, k) if tb else (1, k, n)))
@@ -70,15 +74,15 @@ def test_without_memory_for_the_copies(gpu):
 
 @pytest.mark.parametrize("bf16", [True, False])
 def test_two_threads_on_one_stream(gpu, bf16):
-    """A product's copies are its own until it has been launched, whoever else issues products on the same stream."""
-    import threading
-    g, be, m, n, k = rng(5), GpuBackend(gpu), 1001, 1001, 1001
+    """A product's copies are its own until it has been launched, whoever else issues products on the same stream.  (Without the
+    lock that sees to it a copy of the other thread's has to fall into the few microseconds between two launches: rarely seen here.)"""
+    g, be, m, n, k = rng(5), GpuBackend(gpu), 333, 1001, 1501
     jobs, wrong = [], []
     for _ in range(2):
         A, B = (g.standard_normal(s).astype(np.float32) for s in ((m, k), (n, k)))
         if bf16:
             A, B = (oracle.round_bf16(x.ravel()).reshape(x.shape) for x in (A, B))
-        outs = [be.up(np.zeros((m, n), np.float32)) for _ in range(40)]
+        outs = [be.up(np.zeros((m, n), np.float32)) for _ in range(60)]
         jobs.append((between_words(be, A, 1, bf16), between_words(be, B, 1, bf16), outs, A.astype(np.float64) @ B.T.astype(np.float64)))
     start = threading.Barrier(2)
 
@@ -87,11 +91,14 @@ def test_two_threads_on_one_stream(gpu, bf16):
         for c in outs:
             gpu.dispatch(opspec.linear(a, b, c, m, n, k, False, True, k, k, n))
 
+    was = sys.getswitchinterval()
+    sys.setswitchinterval(1e-6)
     threads = [threading.Thread(target=issue, args=j[:3]) for j in jobs]
     for t in threads:
         t.start()
     for t in threads:
         t.join()
+    sys.setswitchinterval(was)
     gpu.sync()
     for _, _, outs, want in jobs:
         wrong += [e for e in (rel_err(be.down(c).reshape(m, n), want) for c in outs) if e > 5e-5]

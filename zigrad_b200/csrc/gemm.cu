@@ -389,12 +389,19 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
   // has no K ranges: 0.96 to 0.15 of that kernel's error there; 64-wide ones with it 1.0 to 0.15 from k = 96 on (below that
   // 1.1 to 1.3, and the FFMA kernel stays): 130 random shapes up to k = 8000.  2309x3283x565 382 us and 94 like this, 1208x1518x782
   // 158 and 16; 331x17x2571 12.6 and 13.6.
-  // Measured crossovers of the copy: bf16 with a bf16 C against the FFMA kernel 10 M multiply-adds (8.0 us either way; 30 M: 17 and 9), fp32
-  // against the element-wise ring 500 M (1000x501x1001 16 us either way; 2001x1001x1001 36 and 29).
+  // Measured crossovers of the copy: bf16 with a bf16 C against the FFMA kernel 10 M multiply-adds (8.0 us either way; 30 M: 17 and 9).  fp32
+  // against the element-wise ring, which fetches an operand once for every 128 rows or columns of C: from two and a half
+  // times the words of the copy on, and 5 M in all, 15 M with few slabs per tile (160 random shapes: within 1.1 % of the better
+  // of the two, a rule on the multiply-adds 10 %; 468x230x4071 24 and 18 us, 2248x593x5015 138 and 95, 1613x1194x239 13.7 and
+  // 14.6, 100x4097x4097 33 and 51).
+  const double words_a = a_direct ? (double)nA * (double)m * (double)k : 0.0, words_b = b_direct ? (double)nB * (double)n * (double)k : 0.0;
+  const double fetched = (words_a ? (double)nC * (double)m * (double)k : 0.0) * (double)((n + 127) / 128) +
+                         (words_b ? (double)nC * (double)n * (double)k : 0.0) * (double)((m + 127) / 128);
+  const bool copies_pay = fetched >= 2.5 * (words_a + words_b) && fetched >= (k >= 512 ? 5e6 : 1.5e7);
   const bool sums = bf16 && (direct || g_rounded) && c_id == SINGLE;
   if (sums && (macs < 2e7 || k < 96)) return false;
   std::unique_lock<std::mutex> copies;  // until the product has been launched
-  if (direct && macs >= (bf16 ? 1.5e7 : 1e9)) {
+  if (direct && (bf16 ? macs >= 1.5e7 : copies_pay)) {
     const uint64_t ra = nA * (ta ? k : m), ca = ta ? m : k, rb = nB * (tb ? n : k), cb = tb ? k : n;
     if (bf16 ? repack_operands<__nv_bfloat16>(s, A, ra, ca, lda, a_direct, B, rb, cb, ldb, b_direct, copies)
              : repack_operands<float>(s, A, ra, ca, lda, a_direct, B, rb, cb, ldb, b_direct, copies))
@@ -448,9 +455,11 @@ static bool try_tensor_core(dtype id, dtype c_id, cudaStream_t s, const void* A,
     // Three-pass tiles in clusters: a 128-wide one takes about 0.6 us per slab, 6.8 us beside it and 1.4 more in a cluster of
     // eight, a 64-wide one 0.37 and 5.8 (launch, first loads, staging, the cluster's sum).  1000x301x501 11.8 us in 128-wide
     // tiles, 9.8 in 64-wide ones; 4096x128x256 9.2 and 7.2; 1000x501x1000 12.3 and 12.5.
+    // Where the ring copies element by element a slab takes about a microsecond in either (163x1429x1194 19.2 us in 64-wide
+    // tiles of three ranges, 15.2 in 128-wide ones of six; 887x179x3198 19.3 and 21.7).
     auto slabs = [&](unsigned sp) { return (double)((k + (size_t)bk * sp - 1) / ((size_t)bk * sp)); };
     const unsigned s128 = cluster_splits(tiles), s64 = cluster_splits(tiles64);
-    if (5.8 + 0.37 * slabs(s64) < 6.8 + 0.6 * slabs(s128) + (s128 == 8 ? 1.4 : 0.0)) {
+    if (direct ? 3.2 + 0.95 * slabs(s64) < 8.0 + slabs(s128) : 5.8 + 0.37 * slabs(s64) < 6.8 + 0.6 * slabs(s128) + (s128 == 8 ? 1.4 : 0.0)) {
       bn = 64;
       tiles = tiles64;
     }
