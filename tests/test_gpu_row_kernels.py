@@ -19,7 +19,8 @@ def past(s, n):
 
 @pytest.mark.parametrize("ty", [np.float32, np.float64])
 @pytest.mark.parametrize("off", [0, 1])
-@pytest.mark.parametrize("rows,L", [(1, 32), (9, 31), (300, 33), (5000, 36), (7, 1003), (4099, 1003), (33, 2048), (2, 100001)])
+@pytest.mark.parametrize("rows,L", [(1, 32), (9, 31), (300, 33), (5000, 36), (7, 1003), (4099, 1003), (33, 2048), (2, 100001), (3, 40), (801, 64), (70, 257),
+                                    (15001, 33), (15301, 33), (20800, 96), (20801, 97), (20619, 97), (19999, 300), (20003, 301)])
 def test_broadcast(gpu, rows, L, off, ty):
     g, be = rng(rows + L), GpuBackend(gpu)
     x, s = g.standard_normal(rows * L + off).astype(ty), g.standard_normal(L + off).astype(ty)

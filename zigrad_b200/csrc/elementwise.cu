@@ -151,9 +151,8 @@ __global__ void __launch_bounds__(kThreads) bcast_kernel(T* out, const T* lng, c
 }
 
 // The same with rows of at least 32 elements: a thread keeps its column (16 bytes of columns where rows allow), reads its
-// element of the short operand once and goes down the rows, kRows of them in flight.  Over the flat index every vector of a
-// ragged row fetched four single elements of the short operand through L1, twice what the long one and the result take
-// there (4099 x 1003 6.6 -> 6.3 us, 8192 x 1024 9.8 -> 6.8, 100 x 128 2.0 -> 1.35).
+// element of the short operand once and goes down the rows, kRows of them in flight.  Over the flat index every vector
+// fetches four single elements of the short operand through L1, twice what the long one and the result take there.
 template <typename T, bool SHORT_IS_X, bool VEC, typename F>
 __global__ void __launch_bounds__(kThreads) bcast_rows_kernel(T* out, const T* lng, const T* sht, size_t R, size_t L, F f) {
   constexpr int N = VEC ? VecOf<T>::N : 1, kRows = VEC ? 4 : 8;
@@ -181,10 +180,16 @@ __global__ void __launch_bounds__(kThreads) bcast_rows_kernel(T* out, const T* l
 template <typename T, bool SHORT_IS_X, bool VEC, typename F>
 void launch_bcast_rows(cudaStream_t s, T* out, const T* lng, const T* sht, size_t R, size_t L, F f) {
   constexpr size_t N = VEC ? VecOf<T>::N : 1, rows = VEC ? 4 : 8;
-  unsigned bx = 32;
-  while (bx < (unsigned)kThreads && bx * N < L) bx *= 2;
+  // the widest CTA row that leaves next to no more threads without a column than one of a warp does; narrower ones only where a
+  // row of the operands is no wider
+  const size_t words = (L + N - 1) / N;
+  unsigned bx = VEC && words <= 8 ? 8 : (VEC && words <= 16 ? 16 : 32);
+  for (unsigned b = 64; words > 32 && b <= (unsigned)kThreads; b *= 2)
+    if ((words + b - 1) / b * b * 20 <= (words + 31) / 32 * 32 * 21) bx = b;
   const unsigned by = kThreads / bx;
-  const size_t gx = (L + bx * N - 1) / (bx * N), want = (R + by * rows - 1) / (by * rows), cap = std::max<size_t>(1, (size_t)sm_count() * 8 / gx);
+  // CTAs of `rows` rows a thread, of fewer while that leaves SMs idle
+  const size_t gx = (L + bx * N - 1) / (bx * N), sms = (size_t)sm_count(), cap = std::max<size_t>(1, sms * 8 / gx);
+  const size_t want = std::max((R + by * rows - 1) / (by * rows), std::min((R + by - 1) / by, sms * 2 / gx));
   launch_pdl(bcast_rows_kernel<T, SHORT_IS_X, VEC, F>, dim3((unsigned)gx, (unsigned)std::min<size_t>({want, cap, 65535})), dim3(bx, by), 0, s, out, lng, sht, R, L, f);
 }
 
@@ -215,8 +220,12 @@ void binary_dispatch(cudaStream_t s, const T* x, const T* y, T* z, size_t xl, si
   const T* sht = short_is_x ? x : y;
   const size_t L = short_is_x ? xl : yl;
   const bool vec = host_aligned16(z) && host_aligned16(lng);
-  if (L >= 32 && L <= 0x7fffffffu) {
-    const bool rows16 = vec && host_aligned16(sht) && L % VecOf<T>::N == 0;
+  // Down the rows against the flat index, us, 36 widths of 32 to 5000, fp32 and fp64.  Rows of whole words: 1.5 M elements in rows of
+  // 128 3.8 and 2.4, of 32 3.5 and 2.4, 12 M 14.8 and 11.5; beyond what L2 holds equal (fp32) or up to 10 % slower (fp64).
+  // Others move single elements: 0.3 M 2.0 and 1.8; 1.5 M in rows of 33 3.5 and 5.4, of 129 3.7 and 3.4; 4.2 M in rows of 129 6.1
+  // and 7.8, of 257 6.5 and 6.4, of 1003 6.6 and 6.2; 12 M 15 and 16 to 29.
+  const bool rows16 = vec && host_aligned16(sht) && L % VecOf<T>::N == 0;
+  if (L >= 32 && L <= 0x7fffffffu && (rows16 ? zl * sizeof(T) <= (size_t)128 << 20 : zl <= (L >= 256 ? 6000000u : (L >= 96 ? 2000000u : 500000u)))) {
     if (short_is_x) rows16 ? launch_bcast_rows<T, true, true>(s, z, lng, sht, zl / L, L, f) : launch_bcast_rows<T, true, false>(s, z, lng, sht, zl / L, L, f);
     else rows16 ? launch_bcast_rows<T, false, true>(s, z, lng, sht, zl / L, L, f) : launch_bcast_rows<T, false, false>(s, z, lng, sht, zl / L, L, f);
     ZG_LAUNCH_CHECK();
