@@ -382,10 +382,15 @@ static SegTable seg_table(const zg_segment* seg, size_t n_seg, size_t first, int
     tab.len[j] = seg[first + j].len;
     total += seg[first + j].len;
   }
-  size_t per = (total + (size_t)sm_count() * per_sm - 1) / ((size_t)sm_count() * per_sm);
+  const size_t room = (size_t)sm_count() * per_sm;
+  size_t per = (total + room - 1) / room, up = 0;
   if (per < (size_t)kOThreads * 4) per = (size_t)kOThreads * 4;
+  for (int j = 0; j < tab.n; ++j) up += (tab.len[j] + per - 1) / per;
+  // While there is room for it a segment has a CTA for its last elements as well: as a second trip of a few threads they take
+  // as long again (18791 + 989 elements, Adam: 2.8 us, so 2.2).
+  const bool whole = up <= room;
   for (int j = 0; j < tab.n; ++j) {
-    const size_t c = (tab.len[j] + per / 2) / per;
+    const size_t c = (tab.len[j] + (whole ? per - 1 : per / 2)) / per;
     tab.first_cta[j + 1] = tab.first_cta[j] + (unsigned)(c < 1 ? 1 : c);
   }
   return tab;
