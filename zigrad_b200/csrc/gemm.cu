@@ -93,7 +93,7 @@ static int* tc_error_flag();
 
 // The tile width whose busiest SM has the least to do: the tensor instruction takes TN cycles per k of a 64 x TN tile, and a
 // tile about 300 cycles beside.
-static void launch_f64(cudaStream_t s, const void* A, const void* B, void* C, const block::Params& q, len_t nC) {
+static void launch_f64(cudaStream_t s, const void* A, const void* B, void* C, block::Params& q, len_t nC) {
   f64::Params p;
   memset(&p, 0, sizeof(p));
   p.nA = q.nA; p.nB = q.nB; p.m = q.m; p.n = q.n; p.k = q.k; p.lda = q.lda; p.ldb = q.ldb; p.ldc = q.ldc;
@@ -109,6 +109,13 @@ static void launch_f64(cudaStream_t s, const void* A, const void* B, void* C, co
     if (!tn || cost < best) { tn = w; best = cost; }
   }
   const size_t tiles = tiles_m * ((p.n + tn - 1) / tn) * nC;
+  // A slab or two per tile, and C only written: what counts is how many tiles an SM has in flight, and the block kernel has two
+  // (us, it and the persistent one: 28 x 213x121x17 8.0 and 10.6, 6 x 476x348x44 10.0 and 12.9, 9 x 76x1596x20 13.8 and 16.8;
+  // 2 x 632x551x20 8.2 and 8.5, 5 x 1144x635x8 22.3 and 22.6; with C read as well 950x419x6 19 and 9).  A tile per SM or little
+  // more is a chain of copies, of which a [k][row] operand has more than the four copying warps issue in time (4 x 187x603x9
+  // 5.0 and 6.8, 2 x 302x817x60 7.2 and 8.8, with a tile and a fifth per SM 5 x 215x479x14 6.8 and 8.0; with B in rows of k 4 x 672x174x65 8.8 and 7.8).
+  const size_t t64 = tiles_m * ((p.n + 63) / 64) * nC, short_k = t64 * 5 > sms * 6 ? 48 : (q.tb ? 0 : (t64 > sms ? 24 : 80));
+  if (p.n * 16 >= (p.n + 63) / 64 * (64 * 13) && p.beta == 0.0 && p.epilogue != ZG_EPI_RELU_MASK && p.k <= short_k) return launch_block_inst<double, double, 64, 64, 0>(s, A, B, C, q, nC, 1);
   if (tiles > 0x7fffffffu) { set_error(kBadArgument, "gemm: grid too large (m=%lu, batches=%lu)", (len_t)p.m, nC); return; }
   p.tiles_m = (uint32_t)tiles_m;
   p.tiles_n = (uint32_t)((p.n + tn - 1) / tn);

@@ -16,7 +16,7 @@
 // Measured (operands in L2, one launch of a replayed chain): 64x128x784 + bias + ReLU 4.1 us (13.8 as 5 K splits of
 // one 128-row tensor-core tile, 49.7 for one row on the 64x64 tile kernel this one replaced), 128x784x64 4.8 (7.9),
 // 64x10x64 3.1 (6.3), 1000x501x1000 unaligned 49 (66).  fp64 with more than half a
-// 64x64 tile per SM runs in gemm_f64.cuh.
+// 64x64 tile per SM runs in gemm_f64.cuh, but for the shortest sums.
 #pragma once
 
 #include <cooperative_groups.h>
