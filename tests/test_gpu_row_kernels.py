@@ -51,3 +51,14 @@ def test_fill_segments(gpu):
     for off, n in segs:
         want[off:off + n] = -2.5
     np.testing.assert_array_equal(be.down(X), want)
+
+
+@pytest.mark.parametrize("ty", [np.float32, np.float64])
+@pytest.mark.parametrize("rows,d", [(1, 9), (700, 13), (5, 31), (5000, 32), (300, 33), (4099, 45), (3, 288), (2, 1003)])
+def test_row_maxima(gpu, rows, d, ty):
+    g, be = rng(rows + d), GpuBackend(gpu)
+    x = g.standard_normal((rows, d)).astype(ty)
+    x[0] = -np.inf
+    X, Y = be.up(x, ty), be.up(np.zeros(rows), ty)
+    gpu.dispatch(opspec.max_along(X, [rows, d], Y, [rows, 1], 1))
+    np.testing.assert_array_equal(be.down(Y), x.max(1))

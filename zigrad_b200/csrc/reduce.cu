@@ -222,7 +222,8 @@ __global__ void __launch_bounds__(kRThreads) max_along_kernel(const T* __restric
 
 // inner == 1 (the reduced dimension is the contiguous one), d > 8: a warp per
 // output, lanes stride the row with 128-bit loads where the row allows.
-template <typename T>
+// NARROW: rows of at most 32, a load per lane (the eight of the general form: 4289 rows of 13, fp64, 1.8 -> 2.4 us)
+template <typename T, bool NARROW>
 __global__ void __launch_bounds__(kRThreads) max_along_rows_kernel(const T* __restrict__ x, T* __restrict__ y, size_t rows, size_t d) {
   pdl_sync();
   constexpr int V = 16 / sizeof(T);
@@ -232,7 +233,9 @@ __global__ void __launch_bounds__(kRThreads) max_along_rows_kernel(const T* __re
   for (size_t r = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
     const T* xr = x + r * d;
     T mx = -INFINITY;
-    if (vec) {
+    if constexpr (NARROW) {
+      if (lane < d && xr[lane] > mx) mx = xr[lane];
+    } else if (vec) {
       const uint4* xv = reinterpret_cast<const uint4*>(xr);
       const size_t nv = d / V;
       size_t v = lane;
@@ -503,7 +506,7 @@ void max_along_impl(cudaStream_t s, const T* x, const len_t* xs, size_t nd, size
   if (total == 0) return;
   const size_t ylen = total / xs[dim];
   const size_t inner = prod(xs, dim + 1, nd);
-  if (inner == 1 && xs[dim] > 8) launch_pdl(max_along_rows_kernel<T>, dim3(grid_for(ylen, kRThreads / 32)), dim3(kRThreads), 0, s, x, y, ylen, xs[dim]);
+  if (inner == 1 && xs[dim] > 8) launch_pdl(xs[dim] <= 32 ? max_along_rows_kernel<T, true> : max_along_rows_kernel<T, false>, dim3(grid_for(ylen, kRThreads / 32)), dim3(kRThreads), 0, s, x, y, ylen, xs[dim]);
   else launch_pdl(max_along_kernel<T>, dim3(grid_for(ylen, kRThreads)), dim3(kRThreads), 0, s, x, y, ylen, xs[dim], inner);
   ZG_LAUNCH_CHECK();
 }
