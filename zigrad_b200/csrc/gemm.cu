@@ -814,6 +814,7 @@ extern "C" void zg_mlp_tail_fwd_bwd(dtype id, StreamWrapper stream, len_t rows, 
                                     const void* b1, const void* W2, const void* b2, const void* labels, int label_kind, len_t ld_out,
                                     double loss_div, void* act1, void* logits, void* loss_out, void* dlogits, void* dact1, void* dact0,
                                     void* db2, void* db1, void* db0, int weights_ready) {
+  if (id == SINGLE && rows > 0 && !(db2 && db1 && db0)) { set_error(kBadArgument, "zg_mlp_tail_fwd_bwd: NULL argument"); return; }
   zg_mlp_tail_step(id, stream, rows, h1, h2, C, act0, W1, b1, W2, b2, labels, label_kind, ld_out, loss_div, act1, logits, loss_out, dlogits, dact1,
                    dact0, db2, db1, db0, weights_ready, nullptr);
 }
