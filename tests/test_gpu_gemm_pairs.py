@@ -39,3 +39,22 @@ def test_output_paths_of_the_pair_kernel(gpu, m, n, k, ldc, c16, epi, beta):
     assert np.array_equal(got[:, n:], C0[:, n:])
     if epi != "none":
         assert rel_err(be.down(cs), want.sum(0)) <= 1e-4
+
+
+@pytest.mark.parametrize("beta", [0.0, 1.0])
+@pytest.mark.parametrize("nb,m,n,k,ldc", [(1, 3000, 1700, 4104, 1704), (2, 1500, 1780, 2568, 1780), (1, 2817, 1793, 2600, 1796)])
+def test_tiles_of_the_last_wave_as_k_ranges(gpu, nb, m, n, k, ldc, beta):
+    """84 tiles of 256 x 256 for 74 pairs: ten are split in K.  With beta = 0 they are cleared and added to, the others stored,
+    whatever C holds; padding columns stay (n = 1793: element by element)."""
+    g, be = rng(m + n + k), GpuBackend(gpu)
+    A, B = (oracle.round_bf16(g.standard_normal(s).astype(np.float32).ravel()).reshape(s) for s in ((nb, m, k), (1, n, k)))
+    C0 = g.standard_normal((nb, m, ldc)).astype(np.float32)
+    if beta == 0.0:
+        C0[:, ::3, :n] = np.nan
+    c = be.up(C0)
+    gpu.dispatch(opspec.linear(be.up(to_bf16_bits(A), np.uint16), be.up(to_bf16_bits(B), np.uint16), c, m, n, k, False, True, k, k, ldc, 1.0, beta,
+                               n_batch=(nb, 1, nb)))
+    want = A.astype(np.float64) @ B.transpose(0, 2, 1).astype(np.float64) + (C0[:, :, :n] if beta else 0.0)
+    got = be.down(c).reshape(nb, m, ldc)
+    assert rel_err(got[:, :, :n], want) <= 1e-5
+    assert np.array_equal(got[:, :, n:], C0[:, :, n:])
