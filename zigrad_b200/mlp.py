@@ -63,26 +63,13 @@ def kaiming_uniform(dims: Sequence[int], seed: int):
     return Ws, bs
 
 
-def split_sm_shares(sms: int, tiles0: int, tiles1: int, k_slabs: int):
-    """Shares of `sms` SMs for two split-K GEMMs that run side by side, the first on the critical
-    path.  Both are grids of (output tiles x K ranges) CTAs, one CTA per SM, and a CTA's time goes
-    with the 32-deep k-slabs of its range: the first gets as many K ranges as leave the second a
-    range at most 1.3 times as long.  Returns (SMs of the first, SMs of the second) or None."""
-    best = None
-    for s0 in range(1, sms // tiles0 + 1):
-        s1 = (sms - tiles0 * s0) // tiles1
-        if s1 < 1:
-            break
-        if -(-k_slabs // s1) <= 1.3 * -(-k_slabs // s0):
-            best = (tiles0 * s0, tiles1 * s1)
-    return best
-
-
 def shares_by_finish(sms: int, tiles0: int, tiles1: int, k_slabs: int, late: int = 4):
-    """Shares of `sms` SMs for the same two products where the second starts behind a fork of the stream, about `late` k-slabs'
-    time (3 us) after the first: those with which the later of the two ends soonest.  At batch 8192 split_sm_shares gives the
-    second 15 SMs, and it ended 4 us after everybody else (with the classifier's
-    gradient out of the way as well, mlp_tail, the step went from 53.0 to 47.2 us)."""
+    """Shares of `sms` SMs for two split-K GEMMs that run side by side, the second behind a fork of the stream, about `late`
+    k-slabs' time (3 us) after the first.  Both are grids of (output tiles x K ranges) CTAs, one CTA per SM, and a CTA's time
+    goes with the 32-deep k-slabs of its range: the shares with which the later of the two ends soonest, as (SMs of the first,
+    SMs of the second) or None.  At batch 8192 ranges of about the same length for both gave the second 15 SMs, and it ended
+    4 us after everybody else (with the classifier's gradient out of the way as well, mlp_tail, the step went from 53.0 to
+    47.2 us)."""
     best = None
     for s0 in range(1, sms // tiles0 + 1):
         s1 = (sms - tiles0 * s0) // tiles1
