@@ -132,6 +132,9 @@ class MlpTrainer:
                  max_norm: float = 10.0, delta: float = 1e-6, fused: bool = True, loss_div: Optional[int] = None,
                  index_labels: bool = False, bf16: bool = False, pad_logits: bool = True, zero_grads_in_update: bool = False,
                  tail: Optional[bool] = None, fuse_update: bool = True, update_by_layer: bool = False):
+        """`pad_logits`: in the fused path the rows of `act[l]` and `dact[l]`, logits and hidden layers alike, are `ld[l]`
+        elements apart: dims[l + 1] rounded up to whole 16-byte words (fp32 4 elements, hidden bf16 rows 8).  False: dense rows.
+        `act_numpy(l)` is the dense array either way."""
         self.dev, self.dims, self.B, self.L = dev, [int(d) for d in dims], int(batch), len(dims) - 1
         self.opt, self.lr, self.beta1, self.beta2, self.eps = opt, lr, beta1, beta2, eps
         self.clip, self.max_norm, self.delta = clip, max_norm, delta
@@ -563,8 +566,8 @@ class MlpTrainer:
             self._grads_clear = self.zero_grads_in_update
 
     def _dw_sm_shares(self) -> dict:
-        """SMs for each tensor-core weight-gradient GEMM of a three-layer step (layers 0 and 1; the last
-        layer's output is a few rows and goes to a small FFMA kernel that fits beside the others)."""
+        """SMs for each tensor-core weight-gradient GEMM of a three-layer step (layers 0 and 1; the last layer's comes out of
+        the tail op, or goes to a small FFMA kernel that fits beside the others)."""
         if self._dw_shares is None:
             t0, t1 = (-(-self.dims[l + 1] // 128) * -(-self.dims[l] // 128) for l in (0, 1))
             best = shares_by_finish(self.dev.sm_count(), t0, t1, -(-self.B // 32))
