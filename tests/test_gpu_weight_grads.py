@@ -39,3 +39,21 @@ def test_weight_grads_leaves_large_products_to_the_tensor_cores(gpu):
     be = GpuBackend(gpu)
     s = be.up(np.zeros(4, np.float32))
     assert not gpu.weight_grads_supported(s.dtype, [(s, s, s, s, None, None, 512, 4096, 512, 4096)], 1024)
+
+
+@pytest.mark.parametrize("rows", [400, 1000])
+@pytest.mark.parametrize("dims", [(784, 48, 10), (146, 29, 200, 106), (256, 128, 16)], ids=str)
+def test_error_of_the_sums(gpu, dims, rows):
+    """Sums of 16 products that are added up, in the 2-norm: under two roundings of 2^-24 (9.6e-8 to 1.04e-7 seen; 1.11e-7 to
+    1.56e-7 in one chain)."""
+    g, be = rng(rows), GpuBackend(gpu)
+    f = lambda *s: g.standard_normal(s).astype(np.float32)
+    ops = [(f(rows, n), f(rows, k), n, k) for k, n in zip(dims[:-1], dims[1:])]
+    items = [(be.up(dy), be.up(x), be.up(np.zeros((n, k))), None, None, None, n, k, n, k) for dy, x, n, k in ops]
+    if not gpu.weight_grads_supported(items[0][0].dtype, items, rows):
+        pytest.skip("left to the tensor cores")
+    gpu.dispatch(opspec.weight_grads(items, rows))
+    for it, (dy, x, n, k) in zip(items, ops):
+        want = dy.astype(np.float64).T @ x
+        err = np.linalg.norm(gpu.to_numpy(it[2]).reshape(n, k) - want) / np.linalg.norm(want)
+        assert err <= 1.08e-7
