@@ -240,3 +240,24 @@ def test_sharded_step_equals_full_batch(gpu):
         assert_close("db%d" % l, gb[l], orc.db[l])
     for tr, _ in shards:
         tr.free()
+
+
+@pytest.mark.parametrize("bf16", [False, True], ids=["fp32", "bf16"])
+@pytest.mark.parametrize("pad", [True, False])
+def test_rows_of_activations(gpu, pad, bf16):
+    """`ld` says where a row of act[l] and dact[l] starts, act_numpy gives the rows without their padding."""
+    dims, B = [20, 13, 9, 7], 6
+    tr = MlpTrainer(gpu, dims, B, *kaiming_uniform(dims, 3), opt="none", bf16=bf16, pad_logits=pad, index_labels=True)
+    word = 8 if bf16 else 4
+    assert tr.ld == ([-(-n // word) * word for n in dims[1:-1]] + [8] if pad else dims[1:])
+    g = np.random.default_rng(0)
+    X = g.standard_normal((B, dims[0])).astype(np.float32)
+    Xd = gpu.from_numpy((X.view(np.uint32) >> 16).astype(np.uint16) if bf16 else X)
+    tr.forward(Xd)
+    for l, n in enumerate(dims[1:]):
+        assert tr.act[l].len == tr.dact[l].len == B * tr.ld[l]
+        raw = gpu.to_numpy(tr.act[l])
+        raw = (raw.astype(np.uint32) << 16).view(np.float32) if raw.dtype == np.uint16 else raw
+        np.testing.assert_array_equal(tr.act_numpy(l), raw.reshape(B, tr.ld[l])[:, :n])
+    gpu.mem_cache_free(Xd)
+    tr.free()
