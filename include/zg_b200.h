@@ -99,7 +99,7 @@ enum { ZG_EPI_NONE = 0, ZG_EPI_BIAS = 1, ZG_EPI_BIAS_RELU = 2, ZG_EPI_RELU_MASK 
 EXTERN_C void zg_bmm_sm_budget(int sms);
 /* The NEXT zg_bmm call of the calling thread, if its operands are bf16 and C fp32, adds its products up with sums that round to
  * nearest (about 1e-7 off in the 2-norm), as it does for operands without 16-byte rows; the tensor core's own sums truncate
- * (1e-7 times the square root of the products per sum and more). */
+ * (4e-7 to 4e-6 off for sums of hundreds to thousands of products). */
 EXTERN_C void zg_bmm_rounded_sums(int on);
 EXTERN_C int zg_sm_count(void);
 EXTERN_C void zg_bmm(dtype id, dtype c_id, StreamWrapper stream,

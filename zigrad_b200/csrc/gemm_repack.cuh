@@ -2,7 +2,7 @@
 // words, in a buffer of the stream's: one pass over both operands in one launch in front of a tensor-core product.
 //
 // For bf16 there is no other way onto the tensor cores: cp.async has no 2-byte form, and the FFMA kernel that took these
-// products does 26 TFLOP/s (2047^3 670 us, 44 like this; 1000x301x501 37 and 9.7).  For fp32 the element-wise ring (DIRECT) pays for every 4-byte copy as often as a
+// products does 26 TFLOP/s (1000x301x501 37 us, 9.7 like this; into fp32 with sums that round, gemm_tc.cuh, 1208x1518x782 158 and 16).  For fp32 the element-wise ring (DIRECT) pays for every 4-byte copy as often as a
 // slab is fetched, this once: 2047^3 134 -> 89 us.
 // Bound: L1, by the reads.  A thread makes one 16-byte word of a row out of the aligned 4-byte words that hold it (five of
 // them where a row of bf16 starts on an odd element); words that hold no element of the row are not read.
